@@ -11,8 +11,15 @@
 // The decay, dt, the state, y and the norm are float; x, B, C arrive in the element type T.
 //
 // A request's tokens of one step are neighbours in the batch (rows seq_starts[s] .. seq_starts[s+1]),
-// its slot is state_slots[s].  Every (request, head) is scanned by exactly one block, token after token.
+// its slot is state_slots[s].  Every (request, head, block of columns) is scanned by exactly one block: token after token, or
+// (bfloat16, the sizes of ssm_chunk_kernel) 64 tokens at a time as products of matrices.
+#include <limits.h>
+#include <math.h>
+
 #include "common.cuh"
+#if ERB_ELEM == 1
+#include "mma_split.cuh"
+#endif
 
 using namespace erb;
 
@@ -245,9 +252,10 @@ __global__ void __launch_bounds__(512)
 ssm_scan16_kernel(const T* __restrict__ xbc, int channels, const T* __restrict__ proj, int ld, int off_dt,
                   const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
                   float* __restrict__ state, const int* __restrict__ seq_starts, const int* __restrict__ state_slots,
-                  float* __restrict__ y, int H, int P, int N, int G, int PB) {
+                  float* __restrict__ y, int H, int P, int N, int G, int PB, int most_tokens) {
   chain_wait();
   extern __shared__ __align__(16) float smem[];
+  if (seq_starts[blockIdx.y + 1] - seq_starts[blockIdx.y] > most_tokens) return;      // (longer portions: the chunk kernel's)
   const int L = N / NL;
   float* b_s = smem;                                   // [chunk][N]
   float* c_s = b_s + kScanChunk * N;                   // [chunk][N]
@@ -312,6 +320,270 @@ ssm_scan16_kernel(const T* __restrict__ xbc, int channels, const T* __restrict__
   for (int i = 0; i < NL; ++i) s_glob[(size_t)i * P] = S[i];
 }
 
+#if ERB_ELEM == 1
+// The scan of portions of prompts, 64 tokens at a time.  With c_t the sum of the logarithms of the chunk's decays up to and
+// with token t, and S the state before the chunk,
+//     y_t = exp(c_t) S^T C_t + sum_{s <= t} (C_t . B_s) dt_s exp(c_t - c_s) x_s + D x_t
+//     S  <- exp(c_64) S + sum_s B_s (dt_s exp(c_64 - c_s) x_s)^T
+// which are products of matrices.  C, B and x are bfloat16 as they are; every operand that is not (the weights of the second
+// sum, the state, the weighted x of the third) goes in as three bfloat16 pieces (mma_split.cuh), so nothing is rounded to 16
+// bits.  c is summed in double and kept as two floats, since its differences, not its values, matter.
+//
+// What bounds it: the dependent steps of a chunk (two barriers, the products between them), as the walk was bound by the
+// steps of a token.  Block: one (head, request, 32 columns), 16 warps of products and one that makes the next chunk's steps
+// and decays; the state stays in the accumulators' registers.  Between the barriers the work of a chunk is cut into pieces
+// of about the same length: first 10 of the warps make a tile of the weights (C B^T below the diagonal) each, the others the
+// weighted x, and every warp 16 rows x 8 columns of the part of y that comes from the state; then the same 16 x 8 of the
+// part within the chunk, and 16 rows of the state.  (With 8 warps that made their weights in registers, twice over, a chunk
+// took 5.0 us instead of 3.9.)
+constexpr int kChunk = 64, kChunkCols = 32, kChunkWarps = 16;
+
+template <int N>
+struct ChunkSmem {
+  static constexpr int LdN = N + 8, LdP = kChunkCols + 8, LdM = kChunk + 8;   // rows 16 bytes longer than a power of two: no bank conflicts
+  __nv_bfloat16 c[2][kChunk][LdN];
+  __nv_bfloat16 b[2][kChunk][LdN];
+  __nv_bfloat16 x[2][kChunk][LdP];
+  __nv_bfloat16 s[3][N][LdP];                                  // the state before the chunk, in pieces
+  __nv_bfloat16 w[3][kChunk][LdP];                             // the weighted x, in pieces
+  __nv_bfloat16 m[3][kChunk][LdM];                             // the weights of the sum within the chunk, in pieces (tiles above the diagonal unused)
+  float dt[2][kChunk], hi[2][kChunk], lo[2][kChunk];           // step, c_t / ln 2 in two floats
+  float grown[2][kChunk], weight[2][kChunk];                   // exp(c_t), dt_t exp(c_64 - c_t)
+  float total[2];                                              // exp(c_64)
+};
+
+template <int N>
+__global__ void __launch_bounds__((kChunkWarps + 1) * 32)
+ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const __nv_bfloat16* __restrict__ proj, int ld, int off_dt,
+                 const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
+                 float* __restrict__ state, const int* __restrict__ seq_starts, const int* __restrict__ state_slots,
+                 float* __restrict__ y, int H, int P, int G) {
+  chain_wait();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ChunkSmem<N>& sm = *reinterpret_cast<ChunkSmem<N>*>(smem_raw);
+  const int h = blockIdx.x, seq = blockIdx.y, p0 = blockIdx.z * kChunkCols;
+  const int start = seq_starts[seq], n_tok = seq_starts[seq + 1] - start;
+  if (n_tok <= 1) return;                                      // (a single token: the scan kernel's)
+  const int g = h / (H / G), inner = H * P;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qr = lane >> 2, qc = lane & 3;
+  const int n_chunks = (n_tok + kChunk - 1) / kChunk;
+  const __nv_bfloat16* rows = xbc + (size_t)start * channels;
+
+  auto load_stage = [&](int c) {                               // the threads of the products
+    const int buf = c & 1, c0 = c * kChunk;
+    for (int idx = threadIdx.x; idx < kChunk * (N / 8); idx += kChunkWarps * 32) {
+      const int r = idx / (N / 8), e = 8 * (idx % (N / 8));
+      const bool real = c0 + r < n_tok;
+      const __nv_bfloat16* src = rows + (size_t)(real ? c0 + r : 0) * channels + inner + g * N + e;
+      copy16_or_zero(&sm.b[buf][r][e], src, real);
+      copy16_or_zero(&sm.c[buf][r][e], src + G * N, real);
+    }
+    if (threadIdx.x < kChunk * (kChunkCols / 8)) {
+      const int r = threadIdx.x / (kChunkCols / 8), e = 8 * (threadIdx.x % (kChunkCols / 8));
+      const bool real = c0 + r < n_tok;
+      copy16_or_zero(&sm.x[buf][r][e], rows + (size_t)(real ? c0 + r : 0) * channels + h * P + p0 + e, real);
+    }
+    copy_commit();
+  };
+  const float a = -expf(a_log[h]), bias = dt_bias[h];
+  auto make_steps = [&](int c) {                               // the last warp: tokens 2 lane and 2 lane + 1 of chunk c
+    const int buf = c & 1, t0 = c * kChunk + 2 * lane;
+    float dt[2];
+    double la[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      dt[i] = t0 + i < n_tok ? softplus_f(__bfloat162float(proj[(size_t)(start + t0 + i) * ld + off_dt + h]) + bias) : 0.f;
+      la[i] = (double)a * (double)dt[i];
+    }
+    double sum = la[0] + la[1];                                // inclusive scan over the lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
+    }
+    const double all = __shfl_sync(0xffffffffu, sum, 31);
+    const double cum[2] = {sum - la[1], sum};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = 2 * lane + i;
+      const double l2 = cum[i] * 1.4426950408889634;
+      const float hi = (float)l2;
+      sm.dt[buf][r] = dt[i];
+      sm.hi[buf][r] = hi;
+      sm.lo[buf][r] = (float)(l2 - (double)hi);
+      sm.grown[buf][r] = (float)exp(cum[i]);
+      sm.weight[buf][r] = (float)((double)dt[i] * exp(all - cum[i]));
+    }
+    if (lane == 0) sm.total[buf] = (float)exp(all);
+  };
+
+  // the state: warp w holds rows 16 (w mod N/16) .. + 15, columns 8 NTW (w div N/16) .. + 8 NTW - 1
+  constexpr int kRowTiles = N / 16, kColGroups = kChunkWarps / kRowTiles < 4 ? kChunkWarps / kRowTiles : 4, NTW = 4 / kColGroups;
+  const bool holds_state = warp < kRowTiles * kColGroups;
+  const int s_row = 16 * (warp % kRowTiles), s_col = 8 * NTW * (warp / kRowTiles);
+  float S[NTW][4];
+  float* s_glob = state + ((size_t)state_slots[seq] * H + h) * N * P + p0;
+  auto publish = [&]() {                                       // the state's pieces to shared memory
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        uint32_t piece[3];
+        split_pair(S[nt][2 * j], S[nt][2 * j + 1], piece);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          *reinterpret_cast<uint32_t*>(&sm.s[k][s_row + qr + 8 * j][s_col + 8 * nt + 2 * qc]) = piece[k];
+      }
+  };
+  if (warp < kChunkWarps) load_stage(0);
+  else make_steps(0);
+  if (holds_state) {
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float2 v = *reinterpret_cast<const float2*>(s_glob + (size_t)(s_row + qr + 8 * j) * P + s_col + 8 * nt + 2 * qc);
+        S[nt][2 * j] = v.x;
+        S[nt][2 * j + 1] = v.y;
+      }
+    publish();
+  }
+  const int y_row = 16 * (warp >> 2), y_col = 8 * (warp & 3);
+  // the tile of the weights that a warp makes: warps 0 .. 9 take the tiles (row, column) on and below the diagonal
+  const int m_tr = warp < 1 ? 0 : warp < 3 ? 1 : warp < 6 ? 2 : 3;
+  const int m_row = 16 * m_tr, m_col = 16 * (warp - m_tr * (m_tr + 1) / 2);
+  const float dskip = d_skip[h];
+  for (int c = 0; c < n_chunks; ++c) {
+    const int buf = c & 1;
+    if (warp < kChunkWarps) copy_wait<0>();
+    __syncthreads();                                           // chunk c's rows, steps and state pieces are there; stage c - 1 is free
+    if (warp == kChunkWarps) {
+      if (c + 1 < n_chunks) make_steps(c + 1);
+      __syncthreads();
+      continue;
+    }
+    if (c + 1 < n_chunks) load_stage(c + 1);
+    // the part of y that comes from the state
+    float inter[3][4] = {};
+#pragma unroll
+    for (int k = 0; k < N / 16; k += 2) {
+      uint32_t cf[2][4], b[3][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) ldmatrix4(cf[i], &sm.c[buf][y_row + (lane & 15)][16 * (k + i) + 8 * (lane >> 4)]);
+#pragma unroll
+      for (int piece = 0; piece < 3; ++piece) ldmatrix4t(b[piece], &sm.s[piece][16 * k + lane][y_col]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) mma16816(inter[piece], cf[i], b[piece][2 * i], b[piece][2 * i + 1]);
+    }
+    if (warp < 10) {                                           // a tile of the weights
+      float gram[2][2][4] = {};                                // (two chains: a product does not wait for the one before it)
+#pragma unroll
+      for (int k = 0; k < N / 16; ++k) {
+        uint32_t cf[4], b[4];
+        ldmatrix4(cf, &sm.c[buf][m_row + (lane & 15)][16 * k + 8 * (lane >> 4)]);
+        ldmatrix4(b, &sm.b[buf][m_col + (lane & 7) + 8 * (lane >> 4)][16 * k + 8 * ((lane >> 3) & 1)]);
+        mma16816(gram[k & 1][0], cf, b[0], b[1]);
+        mma16816(gram[k & 1][1], cf, b[2], b[3]);
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        const int s = m_col + 8 * nt + 2 * qc;
+        const float2 hs = *reinterpret_cast<const float2*>(&sm.hi[buf][s]), ls = *reinterpret_cast<const float2*>(&sm.lo[buf][s]);
+        const float2 ds = *reinterpret_cast<const float2*>(&sm.dt[buf][s]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int r = m_row + qr + 8 * j;
+          const float hi = sm.hi[buf][r], lo = sm.lo[buf][r];
+          const float v0 = s <= r ? (gram[0][nt][2 * j] + gram[1][nt][2 * j]) * ds.x * exp2f((hi - hs.x) + (lo - ls.x)) : 0.f;
+          const float v1 = s + 1 <= r ? (gram[0][nt][2 * j + 1] + gram[1][nt][2 * j + 1]) * ds.y * exp2f((hi - hs.y) + (lo - ls.y)) : 0.f;
+          uint32_t piece[3];
+          split_pair(v0, v1, piece);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&sm.m[k][r][s]) = piece[k];
+        }
+      }
+    } else {                                                   // weighted x in pieces: 4 columns of one token at a time
+      for (int idx = threadIdx.x - 320; idx < kChunk * (kChunkCols / 4); idx += 192) {
+        const int r = idx >> 3, e = 4 * (idx & 7);
+        float v[4];
+        Pack4<__nv_bfloat16>::load(&sm.x[buf][r][e], v);
+        const float f = sm.weight[buf][r];
+        uint32_t p01[3], p23[3];
+        split_pair(f * v[0], f * v[1], p01);
+        split_pair(f * v[2], f * v[3], p23);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(&sm.w[k][r][e]) = make_uint2(p01[k], p23[k]);
+      }
+    }
+    __syncthreads();                                           // weights and weighted x are complete; nobody reads the state's pieces any more
+    float add[3][NTW][4] = {};
+    if (holds_state) {
+#pragma unroll
+      for (int k = 0; k < kChunk / 16; ++k) {
+        uint32_t bt[4], b[3][4];                               // B^T: 16 state rows x 16 tokens
+        ldmatrix4t(bt, &sm.b[buf][16 * k + (lane & 7) + 8 * (lane >> 4)][s_row + 8 * ((lane >> 3) & 1)]);
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) {
+          if (NTW == 2) ldmatrix4t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col + 8 * (lane >> 4)]);
+          else ldmatrix2t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col]);
+        }
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece)
+#pragma unroll
+          for (int nt = 0; nt < NTW; ++nt) mma16816(add[piece][nt], bt, b[piece][2 * nt], b[piece][2 * nt + 1]);
+      }
+    }
+    float intra[3][4] = {};                                    // the part of y from the chunk's own tokens
+    for (int k = 0; k <= (warp >> 2); k += 2) {
+      uint32_t xb[4], mf[3][4];
+      ldmatrix4t(xb, &sm.x[buf][16 * k + lane][y_col]);        // (rows 16 k .. + 31: the second half may lie behind the diagonal)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (k + i > (warp >> 2)) break;
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) ldmatrix4(mf[piece], &sm.m[piece][y_row + (lane & 15)][16 * (k + i) + 8 * (lane >> 4)]);
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) mma16816(intra[piece], mf[piece], xb[2 * i], xb[2 * i + 1]);
+      }
+    }
+    if (holds_state) {
+      const float total = sm.total[buf];
+#pragma unroll
+      for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[nt][i] = fmaf(total, S[nt][i], (add[2][nt][i] + add[1][nt][i]) + add[0][nt][i]);
+      publish();
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int r = y_row + qr + 8 * j, col = y_col + 2 * qc;
+      if (c * kChunk + r < n_tok) {
+        const float grown = sm.grown[buf][r];
+        const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&sm.x[buf][r][col]));
+        float v[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int q = 2 * j + i;
+          const float before = (inter[2][q] + inter[1][q]) + inter[0][q], own = (intra[2][q] + intra[1][q]) + intra[0][q];
+          v[i] = fmaf(grown, before, own) + dskip * (i ? xv.y : xv.x);
+        }
+        *reinterpret_cast<float2*>(y + (size_t)(start + c * kChunk + r) * inner + h * P + p0 + col) = make_float2(v[0], v[1]);
+      }
+    }
+  }
+  if (holds_state) {
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        *reinterpret_cast<float2*>(s_glob + (size_t)(s_row + qr + 8 * j) * P + s_col + 8 * nt + 2 * qc) =
+            make_float2(S[nt][2 * j], S[nt][2 * j + 1]);
+  }
+}
+#endif  // ERB_ELEM == 1
+
 // One block per (token, part): out = unit_rms(y * silu(z)) * weight over the part's entries.  `gate` may
 // be null (no gate), `x` is float (X32) or T.
 template <typename T, bool X32>
@@ -337,6 +609,23 @@ gated_group_norm_kernel(const void* __restrict__ x_, int x_ld, const T* __restri
     Elem<T>::store(out + (size_t)t * out_ld + i, value(i) * rs * weight[i]);
 }
 
+#if ERB_ELEM == 1
+// Whether the chunk kernel is the faster one: the two costs in microseconds, fitted to both kernels' times over 1 to 64
+// requests of 2 to 500 tokens (8 to 64 heads of 64 x 64 and 64 x 128; within 20 % of them).  The walk costs 0.28 us a token
+// of the longest portion or, when the GPU is full, its blocks' tokens and states; a chunk costs 3.7 us for the longest
+// portion or, when it is full, a share of an SM for every chunk, be it full or not.  One request: from 17 (64 x 128) to 24
+// tokens on; 32 requests of equal length: from 32 (64 x 128) to 48.
+inline bool chunks_pay(int blocks, int N, int n_tokens, int n_seqs, int longest) {
+  if (longest <= 1) return false;
+  const double size = N / 128.0, extra = (double)n_tokens - n_seqs - (longest - 1);      // tokens beyond one of the other requests
+  const double others = extra < n_seqs - 1 ? extra : n_seqs - 1;
+  const double chunks = (longest + 63) / 64 + (others > 0.0 ? others + extra / 64.0 : 0.0);
+  const double walk = fmax(3.0 + 0.28 * longest, blocks * size * (0.0015 * n_tokens + 0.008 * n_seqs));
+  const double chunked = fmax(3.5 + 3.7 * ((longest + 63) / 64), 0.036 * blocks * chunks);
+  return chunked < walk;
+}
+#endif
+
 }  // namespace
 
 ERB_EXPORT int erb_conv_silu(const void* proj, int n_tokens, int ld, int off, int channels, int taps, const void* weight,
@@ -360,9 +649,26 @@ ERB_EXPORT int erb_conv_state_update(const void* proj, int n_seqs, int ld, int o
 
 ERB_EXPORT int erb_ssm_scan(const void* xbc, int channels, const void* proj, int ld, int off_dt, const float* dt_bias,
                             const float* a_log, const float* d_skip, float* state, const int* seq_starts,
-                            const int* state_slots, float* y, int n_seqs, int n_tokens, int H, int P, int N, int G, void* stream) {
+                            const int* state_slots, float* y, int n_seqs, int n_tokens, int longest, int H, int P, int N, int G, void* stream) {
   if (n_seqs <= 0) return ERB_OK;
   if (H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G || P > 512) return fail(ERB_ERR_ARG, "ssm_scan: bad sizes (columns of at most 512)");
+  int most_tokens = INT_MAX;            // what the scan takes: every portion, or single tokens beside the chunk kernel's portions
+#if ERB_ELEM == 1
+  if ((N == 32 || N == 64 || N == 128) && P % kChunkCols == 0 && chunks_pay(H * (P / kChunkCols), N, n_tokens, n_seqs, longest) && channels % 8 == 0 &&
+      !((uintptr_t)xbc & 15) && !((uintptr_t)state & 7) && !((uintptr_t)y & 7)) {
+    const size_t bytes = N == 32 ? sizeof(ChunkSmem<32>) : N == 64 ? sizeof(ChunkSmem<64>) : sizeof(ChunkSmem<128>);
+    auto kern = N == 32 ? ssm_chunk_kernel<32> : N == 64 ? ssm_chunk_kernel<64> : ssm_chunk_kernel<128>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "ssm_scan: %s", cudaGetErrorString(e));
+    launch_chained(kern, dim3(H, n_seqs, P / kChunkCols), dim3((kChunkWarps + 1) * 32), bytes, (cudaStream_t)stream,
+                   (const elem_t*)xbc, channels, (const elem_t*)proj, ld, off_dt, dt_bias, a_log, d_skip, state, seq_starts,
+                   state_slots, y, H, P, G);
+    const int rc = check_launch("ssm_chunk");
+    if (rc || n_seqs == 1) return rc;
+    most_tokens = 1;
+    n_tokens = n_seqs;                  // (below: the shape for single tokens)
+  }
+#endif
   const int PB = P % 32 == 0 ? 32 : (P % 16 == 0 ? 16 : 0);
   // rows per thread: 16 for a step of single tokens (fewer, busier threads: the step is the state's read and write),
   // 8 where portions are walked and that still gives a block of at most 512 threads (twice the warps to hide a token's
@@ -378,7 +684,7 @@ ERB_EXPORT int erb_ssm_scan(const void* xbc, int channels, const void* proj, int
     }
     launch_chained(kern, dim3(H, n_seqs, P / PB), dim3(L * PB), smem16, (cudaStream_t)stream,
                    (const elem_t*)xbc, channels, (const elem_t*)proj, ld, off_dt, dt_bias, a_log, d_skip, state, seq_starts,
-                   state_slots, y, H, P, N, G, PB);
+                   state_slots, y, H, P, N, G, PB, most_tokens);
     return check_launch("ssm_scan");
   }
   int L = 512 / P;                       // threads that share a column of the state

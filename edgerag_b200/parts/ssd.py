@@ -76,7 +76,8 @@ class StateSpaceDuality(Mixer):
         kernels.conv_state_update(proj, inner, conv_state, ctx.n_seqs, ctx.seq_starts, ctx.state_slots)
         y = ctx.buf("ssd.y", (n, inner), torch.float32)
         kernels.ssm_scan(xbc, proj, inner + self.channels, self.dt_bias, self.a_log, self.d_skip,
-                         ctx.state("ssm", call.cache_layer), ctx.n_seqs, ctx.seq_starts, ctx.state_slots, y, self.groups)
+                         ctx.state("ssm", call.cache_layer), ctx.n_seqs, ctx.seq_starts, ctx.state_slots, y, self.groups,
+                         longest=max(ctx.host_q_len))
         normed = ctx.buf("ssd.normed", (n, inner), self.dtype)
         kernels.gated_group_norm(y, self.norm_w, normed, self.eps, self.norm_groups, gate=proj[:, :inner])
         out = ctx.buf("mixer.out", (n, self.hidden), self.dtype)

@@ -1,0 +1,52 @@
+"""The recurrent mixers' kernels that take a portion 64 tokens at a time, at the sizes where they can go wrong: a token beside
+a chunk's end, the smallest and largest states, single tokens beside portions, decays of almost nothing and almost one."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _ssm_reference(xbc, dt_raw, dt_bias, a_log, skip, state, H, P, N, G):
+    n, inner = xbc.shape[0], H * P
+    x = xbc.double()
+    u = x[:, :inner].view(n, H, P)
+    B = x[:, inner: inner + G * N].view(n, G, N).repeat_interleave(H // G, 1)
+    C = x[:, inner + G * N:].view(n, G, N).repeat_interleave(H // G, 1)
+    dt = torch.nn.functional.softplus(dt_raw.double() + dt_bias.double(), threshold=1e9)
+    decay, S, y = torch.exp(-torch.exp(a_log.double()) * dt), state.double().clone(), torch.empty_like(u)
+    for t in range(n):
+        S = S * decay[t, :, None, None] + (dt[t, :, None] * B[t])[:, :, None] * u[t][:, None, :]
+        y[t] = torch.bmm(C[t][:, None], S)[:, 0]
+    return (y + skip.double()[:, None] * u).reshape(n, inner), S
+
+
+@pytest.mark.parametrize("H,P,N,G", [(4, 32, 32, 2), (2, 64, 64, 1), (4, 64, 128, 2)])
+@pytest.mark.parametrize("lens", [[63], [64], [65], [2], [1, 129, 1], [130, 3, 64, 1, 17]])
+@pytest.mark.parametrize("pace", [-6.0, 0.0, 4.0])
+def test_state_space_chunks(H, P, N, G, lens, pace):
+    """Chunks and the walk against float64.  Both are float throughout (a product's operands go in whole, as three pieces), so
+    each entry is within a few hundred roundings of 2^-24 of the largest of the row of sums it belongs to: 3e-5 of the
+    largest result, the band of the tests of the walk."""
+    from edgerag_b200.ops import kernels
+
+    n, slots = sum(lens), [len(lens) - i for i in range(len(lens))]
+    g = torch.Generator().manual_seed(N + n)
+    inner = H * P
+    xbc = (torch.randn(n, inner + 2 * G * N, generator=g) * 0.5).to(torch.bfloat16).cuda()
+    proj = torch.randn(n, 8, generator=g).to(torch.bfloat16).cuda()
+    dt_bias, a_log, skip = torch.randn(H, generator=g).cuda() - 1.0, torch.randn(H, generator=g).cuda() * 0.3 + pace, torch.randn(H, generator=g).cuda()
+    before = torch.randn(len(lens) + 1, H, N, P, generator=g).cuda()
+    starts = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32).cuda()
+    for longest in (1 << 20, 1):                 # portions in chunks (the largest the rule accepts), every token by the walk
+        state, y = before.clone(), torch.full((n, inner), float("nan"), device="cuda")
+        kernels.ssm_scan(xbc, proj, 1, dt_bias, a_log, skip, state, len(lens), starts, torch.tensor(slots, dtype=torch.int32).cuda(), y, G,
+                         longest=longest)
+        at = 0
+        for s, length in enumerate(lens):
+            rows = slice(at, at + length)
+            want_y, want_s = _ssm_reference(xbc[rows], proj[rows, 1: 1 + H], dt_bias, a_log, skip, before[slots[s]], H, P, N, G)
+            assert (y[rows].double() - want_y).abs().max() < 3e-5 * max(1.0, want_y.abs().max()), (s, longest)
+            assert (state[slots[s]].double() - want_s).abs().max() < 3e-5 * max(1.0, want_s.abs().max()), (s, longest)
+            at += length
+        assert torch.equal(state[0], before[0])     # the slot nobody holds
