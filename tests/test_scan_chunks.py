@@ -50,3 +50,29 @@ def test_state_space_chunks(H, P, N, G, lens, pace):
             assert (state[slots[s]].double() - want_s).abs().max() < 3e-5 * max(1.0, want_s.abs().max()), (s, longest)
             at += length
         assert torch.equal(state[0], before[0])     # the slot nobody holds
+
+
+@pytest.mark.parametrize("lens", [[7], [8], [1] * 9, [255], [3, 1, 2, 250, 1], [9, 300]])
+def test_short_convolution_by_eight_channels(lens):
+    """Rows of four taps, with and without a bias, at counts around the lines between the kernels: float sums of five terms
+    rounded once, so within half a unit of bfloat16 (2^-9) of the exact value, and the sums' own 2^-21."""
+    from edgerag_b200.ops import kernels
+
+    n, channels, ld, off, slots = sum(lens), 72, 96, 16, len(lens) + 1
+    g = torch.Generator().manual_seed(n)
+    proj = torch.randn(n, ld, generator=g).to(torch.bfloat16).cuda()
+    weight, bias = torch.randn(channels, 4, generator=g).to(torch.bfloat16).cuda(), torch.randn(channels, generator=g).to(torch.bfloat16).cuda()
+    record = torch.randn(slots, 3, channels, generator=g).cuda()
+    starts = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32).cuda()
+    seq = torch.tensor([s for s, length in enumerate(lens) for _ in range(length)], dtype=torch.int32).cuda()
+    held = torch.arange(len(lens), 0, -1, dtype=torch.int32).cuda()
+    for b in (bias, None):
+        out = torch.full((n, channels), float("nan"), dtype=torch.bfloat16, device="cuda")
+        kernels.conv_silu(proj, off, weight, b, record, seq, starts, held, out)
+        at = 0
+        for s, length in enumerate(lens):
+            x = torch.cat([record[held[s]].double(), proj[at: at + length, off: off + channels].double()], 0)
+            z = sum(x[j: j + length] * weight[:, j].double() for j in range(4)) + (0.0 if b is None else b.double())
+            want = z * torch.sigmoid(z)
+            assert ((out[at: at + length].double() - want).abs() <= want.abs() * 2.0 ** -8.9 + 2.0 ** -20 * z.abs() + 1e-7).all()
+            at += length
