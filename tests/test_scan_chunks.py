@@ -55,7 +55,8 @@ def test_state_space_chunks(H, P, N, G, lens, pace):
 @pytest.mark.parametrize("lens", [[7], [8], [1] * 9, [255], [3, 1, 2, 250, 1], [9, 300]])
 def test_short_convolution_by_eight_channels(lens):
     """Rows of four taps, with and without a bias, at counts around the lines between the kernels: float sums of five terms
-    rounded once, so within half a unit of bfloat16 (2^-9) of the exact value, and the sums' own 2^-21."""
+    rounded once: neighbouring bfloat16 values (8 bits of significand) lie up to 2^-7 of the value apart, so rounding moves it by
+    up to 2^-8 of itself, and the sums' own error is below 2^-20 of them (silu's slope is at most 1.1)."""
     from edgerag_b200.ops import kernels
 
     n, channels, ld, off, slots = sum(lens), 72, 96, 16, len(lens) + 1
@@ -74,5 +75,5 @@ def test_short_convolution_by_eight_channels(lens):
             x = torch.cat([record[held[s]].double(), proj[at: at + length, off: off + channels].double()], 0)
             z = sum(x[j: j + length] * weight[:, j].double() for j in range(4)) + (0.0 if b is None else b.double())
             want = z * torch.sigmoid(z)
-            assert ((out[at: at + length].double() - want).abs() <= want.abs() * 2.0 ** -8.9 + 2.0 ** -20 * z.abs() + 1e-7).all()
+            assert ((out[at: at + length].double() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -20 * z.abs() + 1e-7).all()
             at += length
