@@ -674,6 +674,48 @@ gated_group_norm_kernel(const void* __restrict__ x_, int x_ld, const T* __restri
     Elem<T>::store(out + (size_t)t * out_ld + i, value(i) * rs * weight[i]);
 }
 
+// The same for parts of 128 V entries (V up to 8) and rows whose parts start aligned: a warp per (token, part), 4 V entries a
+// lane held in registers between the sum and the store, so that nothing is read or gated twice.
+// 2,048 tokens of 8 parts of 512: 42 us by the kernel above, 11.4 us; one token 2.9 us by both.
+template <typename T, bool X32, int V>
+__global__ void __launch_bounds__(128)
+gated_group_norm_vec_kernel(const void* __restrict__ x_, int x_ld, const T* __restrict__ gate, int gate_ld,
+                            const float* __restrict__ weight, T* __restrict__ out, int out_ld, int n_items, int parts, float eps) {
+  chain_wait();
+  const int item = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (item >= n_items) return;
+  constexpr int per = 128 * V;
+  const int t = item / parts, lo = (item % parts) * per + 4 * lane;
+  float v[V][4], ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+    if (X32) load4(static_cast<const float*>(x_) + (size_t)t * x_ld + lo + 128 * j, v[j]);
+    else Pack4<T>::load(static_cast<const T*>(x_) + (size_t)t * x_ld + lo + 128 * j, v[j]);
+  }
+  if (gate) {
+    float z[V][4];
+#pragma unroll
+    for (int j = 0; j < V; ++j) Pack4<T>::load(gate + (size_t)t * gate_ld + lo + 128 * j, z[j]);
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[j][i] *= silu_f(z[j][i]);
+  }
+#pragma unroll
+  for (int j = 0; j < V; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ss = fmaf(v[j][i], v[j][i], ss);
+  const float rs = rsqrtf(warp_sum(ss) / (float)per + eps);
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+    float w[4];
+    load4(weight + lo + 128 * j, w);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = v[j][i] * rs * w[i];
+    Pack4<T>::store(out + (size_t)t * out_ld + lo + 128 * j, w);
+  }
+}
+
 #if ERB_ELEM == 1
 // Whether the chunk kernel is the faster one: the two costs in microseconds, fitted to both kernels' times over 1 to 64
 // requests of 2 to 500 tokens (8 to 64 heads of 64 x 64 and 64 x 128; within 20 % of them).  The walk costs 0.28 us a token
@@ -786,6 +828,20 @@ ERB_EXPORT int erb_gated_group_norm(const void* x, int x_is_float, int x_ld, con
                                     void* out, int out_ld, int n_tokens, int width, int parts, float eps, void* stream) {
   if (n_tokens <= 0) return ERB_OK;
   if (width <= 0 || parts <= 0 || width % parts) return fail(ERB_ERR_ARG, "gated_group_norm: the parts must divide the width");
+  const int per = width / parts, V = per / 128;
+  const uintptr_t elem_bits = 4 * sizeof(elem_t) - 1, x_bits = x_is_float ? 15 : elem_bits;
+  if (per % 128 == 0 && (V == 1 || V == 2 || V == 4 || V == 8) && x_ld % 4 == 0 && out_ld % 4 == 0 && (!gate || gate_ld % 4 == 0) &&
+      !(((uintptr_t)gate | (uintptr_t)out) & elem_bits) && !((uintptr_t)x & x_bits) && !((uintptr_t)weight & 15) &&
+      (long long)n_tokens * parts <= 0x7fffffffLL) {
+    const int n_items = n_tokens * parts;
+#define ERB_GROUP_NORM(X32, VV)                                                                                            \
+  launch_chained(gated_group_norm_vec_kernel<elem_t, X32, VV>, dim3((n_items + 3) / 4), dim3(128), 0, (cudaStream_t)stream, x, x_ld, \
+                 (const elem_t*)gate, gate_ld, weight, (elem_t*)out, out_ld, n_items, parts, eps)
+    if (x_is_float) { if (V == 1) ERB_GROUP_NORM(true, 1); else if (V == 2) ERB_GROUP_NORM(true, 2); else if (V == 4) ERB_GROUP_NORM(true, 4); else ERB_GROUP_NORM(true, 8); }
+    else { if (V == 1) ERB_GROUP_NORM(false, 1); else if (V == 2) ERB_GROUP_NORM(false, 2); else if (V == 4) ERB_GROUP_NORM(false, 4); else ERB_GROUP_NORM(false, 8); }
+#undef ERB_GROUP_NORM
+    return check_launch("gated_group_norm");
+  }
   if (x_is_float)
     launch_chained(gated_group_norm_kernel<elem_t, true>, dim3(n_tokens, parts), dim3(256), 0, (cudaStream_t)stream, x, x_ld,
                    (const elem_t*)gate, gate_ld, weight, (elem_t*)out, out_ld, width, parts, eps);

@@ -77,3 +77,37 @@ def test_short_convolution_by_eight_channels(lens):
             want = z * torch.sigmoid(z)
             assert ((out[at: at + length].double() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -20 * z.abs() + 1e-7).all()
             at += length
+
+
+@pytest.mark.parametrize("n,parts,per", [(1, 1, 128), (5, 3, 256), (33, 2, 512), (3, 1, 1024)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_group_norm_by_warps(n, parts, per, gated):
+    """Against float64: float arithmetic (sums of up to 1,024 squares, 2^-20) rounded once to bfloat16 (2^-8 of the value)."""
+    from edgerag_b200.ops import kernels
+
+    g = torch.Generator().manual_seed(per)
+    width = parts * per
+    x, weight = torch.randn(n, width + 4, generator=g).cuda()[:, :width], torch.randn(width, generator=g).cuda()
+    z = torch.randn(n, width + 4, generator=g).to(torch.bfloat16).cuda()[:, 4:] if gated else None
+    out = torch.empty(n, width, dtype=torch.bfloat16, device="cuda")
+    kernels.gated_group_norm(x, weight, out, 1e-5, parts, gate=z)
+    v = x.double() if z is None else x.double() * z.double() * torch.sigmoid(z.double())
+    v = v.view(n, parts, per)
+    want = (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5)).view(n, width) * weight.double()
+    assert ((out.double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -18) + 1e-30).all()
+
+
+@pytest.mark.parametrize("dv", [4, 124, 128, 132, 256, 512, 6])
+def test_head_norm_by_four_values(dv):
+    """As above, one weight vector for all heads (6: not in runs of four, the general kernel)."""
+    from edgerag_b200.ops import kernels
+
+    g = torch.Generator().manual_seed(dv)
+    n, H = 9, 3
+    o, weight = torch.randn(n, H * dv, generator=g).cuda(), torch.randn(dv, generator=g).cuda()
+    z = torch.randn(n, H * dv + 4, generator=g).to(torch.bfloat16).cuda()[:, : H * dv]
+    out = torch.empty(n, H * dv, dtype=torch.bfloat16, device="cuda")
+    kernels.head_norm_gate(o, z, weight, out, H, 1e-5)
+    v, zz = o.double().view(n, H, dv), z.double().reshape(n, H, dv)
+    want = (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5) * weight.double() * zz * torch.sigmoid(zz)).view(n, H * dv)
+    assert ((out.double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -18) + 1e-30).all()
