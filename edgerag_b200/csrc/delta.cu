@@ -20,7 +20,16 @@
 // A request's tokens of one step are neighbours in the batch (rows seq_starts[s] .. seq_starts[s+1]), its slot is
 // state_slots[s]; every (request, head, column) is walked by exactly one thread group, token after token, so the
 // arithmetic of a token does not depend on how the sequence was cut into steps.
+//
+// Portions of prompts (bfloat16 rows, keys of 64 or 128, values of a multiple of 16) are not walked but taken 64 tokens at a
+// time, as products of matrices: see delta_chunk_kernel.  The two forms differ by rounding.
+#include <limits.h>
+#include <math.h>
+
 #include "common.cuh"
+#if ERB_ELEM == 1
+#include "mma_split.cuh"
+#endif
 
 using namespace erb;
 
@@ -67,11 +76,15 @@ template <typename T>
 __global__ void __launch_bounds__(kPrepWarps * 32)
 delta_prepare_kernel(const T* __restrict__ qkv, int channels, const T* __restrict__ proj, int ld, int off_b, int off_a,
                      const float* __restrict__ dt_bias, const float* __restrict__ a_log, DeltaScratch out, int n_items, int H,
-                     int G, int d, int dv, float q_scale) {
+                     int G, int d, int dv, float q_scale, const int* __restrict__ singles) {
   chain_wait();
   const int item = blockIdx.x * kPrepWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (item >= n_items) return;
-  const int t = item / G, kh = item % G;
+  // `at`: the token's place in the scratch.  With `singles` (the step's seq_starts) an item is a request, and only requests of
+  // one token are prepared, each at its own number.
+  const int at = item / G, kh = item % G;
+  if (singles && singles[at + 1] - singles[at] != 1) return;
+  const int t = singles ? singles[at] : at;
   const int dp = pad4(d), dvp = pad4(dv), rep = H / G;
   const T* row = qkv + (size_t)t * channels;
   const T* qs = row + kh * d;
@@ -86,7 +99,7 @@ delta_prepare_kernel(const T* __restrict__ qkv, int channels, const T* __restric
   //  compound along the recurrence)
   const float rk = (float)(1.0 / sqrt((double)warp_sum(sk) + 1e-6));
   const float rq = (float)((double)q_scale / sqrt((double)warp_sum(sq) + 1e-6));
-  float* qd = out.qk + ((size_t)t * G + kh) * 2 * dp;
+  float* qd = out.qk + ((size_t)at * G + kh) * 2 * dp;
   float* kd = qd + dp;
   float kq = 0.f;
   for (int n = lane; n < dp; n += 32) {
@@ -103,10 +116,10 @@ delta_prepare_kernel(const T* __restrict__ qkv, int channels, const T* __restric
       const float beta = (float)(1.0 / (1.0 + exp(-(double)Elem<T>::load(raw + off_b + h))));
       const double z = (double)(Elem<T>::load(raw + off_a + h) + dt_bias[h]);
       const float g = (float)exp(-exp((double)a_log[h]) * (z > 30.0 ? z : log1p(exp(z))));
-      *reinterpret_cast<float4*>(out.sc + ((size_t)t * H + h) * 4) = make_float4(beta, g, kq, 0.f);
+      *reinterpret_cast<float4*>(out.sc + ((size_t)at * H + h) * 4) = make_float4(beta, g, kq, 0.f);
     }
     const T* vs = row + 2 * G * d + h * dv;
-    float* vd = out.vf + ((size_t)t * H + h) * dvp;
+    float* vd = out.vf + ((size_t)at * H + h) * dvp;
     for (int n = lane; n < dvp; n += 32) vd[n] = n < dv ? Elem<T>::load(vs + n) : 0.f;
   }
 }
@@ -118,8 +131,9 @@ delta_prepare_kernel(const T* __restrict__ qkv, int channels, const T* __restric
 template <int L>
 __global__ void __launch_bounds__(512)
 delta_scan_kernel(DeltaScratch in, float* __restrict__ state, const int* __restrict__ seq_starts,
-                  const int* __restrict__ state_slots, float* __restrict__ out, int H, int G, int d, int dv, int PB) {
+                  const int* __restrict__ state_slots, float* __restrict__ out, int H, int G, int d, int dv, int PB, bool singles) {
   chain_wait();
+  if (singles && seq_starts[blockIdx.y + 1] - seq_starts[blockIdx.y] != 1) return;       // (the chunk kernel's)
   extern __shared__ __align__(16) float smem[];
   const int dp = pad4(d), dvp = pad4(dv);
   constexpr int RS = 16 * L;                                   // floats of a staged query or key
@@ -129,7 +143,7 @@ delta_scan_kernel(DeltaScratch in, float* __restrict__ state, const int* __restr
   const int l = threadIdx.x % L, p = threadIdx.x / L;
   const int col = p0 + p;
   const bool live = col < dv;
-  const int start = seq_starts[seq], n_tok = seq_starts[seq + 1] - start;
+  const int start = seq_starts[seq], n_tok = seq_starts[seq + 1] - start, first = singles ? seq : start;   // `first`: place in the scratch
   float* s_glob = state + (((size_t)state_slots[seq] * H + h) * dv + (live ? col : 0)) * d;
   int row_of[4];                                               // first row of each run
 #pragma unroll
@@ -156,14 +170,14 @@ delta_scan_kernel(DeltaScratch in, float* __restrict__ state, const int* __restr
     for (int idx = threadIdx.x; idx < nc * qk4; idx += blockDim.x) {
       const int c = idx / qk4, j = idx % qk4;                  // piece j of the token's [q | k]: to row 2 c or 2 c + 1
       const int which = 4 * j >= dp, e = 4 * j - which * dp;
-      copy16_async(qk_s + (2 * c + which) * RS + e, in.qk + ((size_t)(start + c0 + c) * G + kh) * 2 * dp + 4 * j);
+      copy16_async(qk_s + (2 * c + which) * RS + e, in.qk + ((size_t)(first + c0 + c) * G + kh) * 2 * dp + 4 * j);
     }
     for (int idx = threadIdx.x; idx < nc * v4; idx += blockDim.x) {
       const int c = idx / v4, j = idx % v4;
-      if (4 * j < pb_live) copy16_async(v_s + c * PB + 4 * j, in.vf + ((size_t)(start + c0 + c) * H + h) * dvp + p0 + 4 * j);
+      if (4 * j < pb_live) copy16_async(v_s + c * PB + 4 * j, in.vf + ((size_t)(first + c0 + c) * H + h) * dvp + p0 + 4 * j);
     }
     for (int c = threadIdx.x; c < nc; c += blockDim.x)
-      copy16_async(sc_s + 4 * c, in.sc + ((size_t)(start + c0 + c) * H + h) * 4);
+      copy16_async(sc_s + 4 * c, in.sc + ((size_t)(first + c0 + c) * H + h) * 4);
     copies_commit();
   };
   if (n_tok > 0) stage(0, 0);
@@ -288,28 +302,555 @@ head_norm_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ gat
   }
 }
 
+#if ERB_ELEM == 1
+// ---------------------------------------------------------------------------------------------
+// 64 tokens at a time.  With c_t the sum of the logarithms of the chunk's decays up to and with token t, S the state before the
+// chunk and u_t the token's write (u = beta (v - S^T k) with the state of its time),
+//     u_t + beta_t sum_{s < t} exp(c_t - c_s) (k_t . k_s) u_s  =  beta_t (v_t - exp(c_t) S^T k_t)
+//     o_t = exp(c_t) S^T q_t + sum_{s <= t} exp(c_t - c_s) (q_t . k_s) u_s
+//     S  <- exp(c_64) S + sum_s exp(c_64 - c_s) k_s u_s^T
+// The first line is a triangular system (I + A) U = R whose matrix does not depend on the state: a first kernel, parallel over
+// (chunk, head), makes T = (I + A)^-1 in float and the weights of the second line; the second kernel, parallel over (request,
+// head, 16 columns of values), walks the chunks with products of matrices alone.  The raw queries and keys are bfloat16 as they
+// are (their lengths are factors of rows and columns); every other operand goes in as three bfloat16 pieces (mma_split.cuh), so
+// that nothing is rounded to 16 bits.  c is summed in double and kept as two floats.
+//
+// What bounds it: the three dependent phases of a chunk, and the 64 KB of operands a block reads of it.  The walk took 0.49 us
+// a token (2,048 tokens of 16 heads of 128 x 128: 1,011 us
+// behind 24 us of preparing); the chunks 3.7 us for 64 tokens (142 us for both kernels).  Error against float64: 1.7e-7, as the walk's.
+constexpr int kChunk = 64, kChunkCols = 16, kChunkWarps = 16, kChunkPrepWarps = 8;
+constexpr int kPieceElems = kChunk * kChunk;
+
+// What the first kernel leaves of one (chunk, head): the weights of the second line and T, each as three pieces [64][64] (tiles
+// of 16 x 16 above the diagonal are not written), per token (beta, exp(c) / |k|, exp(c) / |q|, exp(c_64 - c) / |k|), exp(c_64).
+struct ChunkRecord {
+  __nv_bfloat16 p[3][kPieceElems];
+  __nv_bfloat16 t[3][kPieceElems];
+  float4 sc[kChunk];
+  float4 total;
+};
+static_assert(sizeof(ChunkRecord) == 4 * 12548, "copied 16 bytes at a time; the size that callers give the scratch by");
+
+// Chunks before request `seq` (requests of one token have none).
+__device__ __forceinline__ int chunks_before(const int* seq_starts, int seq) {
+  int n = 0;
+  for (int s = threadIdx.x & 31; s < seq; s += 32) {
+    const int len = seq_starts[s + 1] - seq_starts[s];
+    n += len > 1 ? (len + kChunk - 1) / kChunk : 0;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+  return n;
+}
+
+template <int D>
+struct DeltaPrepSmem {
+  __nv_bfloat16 k[kChunk][D + 8], q[kChunk][D + 8];
+  float a[kChunk][kChunk + 4];                                 // A, then T in its place
+  float x[3][16][17];
+  float beta[kChunk], ik[kChunk], iq[kChunk], hi[kChunk], lo[kChunk], grown[kChunk], left[kChunk];
+};
+
+template <int D>
+__global__ void __launch_bounds__(kChunkPrepWarps * 32)
+delta_chunk_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const __nv_bfloat16* __restrict__ proj, int ld, int off_b,
+                           int off_a, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
+                           const int* __restrict__ seq_starts, int n_seqs, ChunkRecord* __restrict__ records, int H, int G, float q_scale) {
+  chain_wait();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  DeltaPrepSmem<D>& sm = *reinterpret_cast<DeltaPrepSmem<D>*>(smem_raw);
+  auto &ks = sm.k, &qs = sm.q;
+  auto &a_s = sm.a;
+  auto &x_s = sm.x;
+  auto &beta_s = sm.beta, &ik_s = sm.ik, &iq_s = sm.iq, &hi_s = sm.hi, &lo_s = sm.lo, &grown_s = sm.grown, &left_s = sm.left;
+  const int h = blockIdx.x, kh = h / (H / G), warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qr = lane >> 2, qc = lane & 3;
+  int seq = -1, c = (int)blockIdx.y, start = 0, n_tok = 0;     // chunk c of request seq
+  for (int s = 0; s < n_seqs; ++s) {
+    start = seq_starts[s];
+    n_tok = seq_starts[s + 1] - start;
+    const int chunks = n_tok > 1 ? (n_tok + kChunk - 1) / kChunk : 0;
+    if (c < chunks) { seq = s; break; }
+    c -= chunks;
+  }
+  if (seq < 0) return;                                         // (the grid is an upper bound)
+  const int c0 = c * kChunk;
+  ChunkRecord& rec = records[(size_t)blockIdx.y * H + h];
+  for (int idx = threadIdx.x; idx < kChunk * (D / 8); idx += blockDim.x) {
+    const int r = idx / (D / 8), e = 8 * (idx % (D / 8));
+    const bool real = c0 + r < n_tok;
+    const __nv_bfloat16* src = qkv + (size_t)(start + (real ? c0 + r : 0)) * channels + kh * D + e;
+    copy16_or_zero(&qs[r][e], src, real);
+    copy16_or_zero(&ks[r][e], src + G * D, real);
+  }
+  copy_commit();
+  if (warp == 0) {                                             // write strengths and decays: tokens 2 lane and 2 lane + 1
+    double lg[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = 2 * lane + i;
+      double beta = 0.0;
+      lg[i] = 0.0;
+      if (c0 + r < n_tok) {
+        const __nv_bfloat16* raw = proj + (size_t)(start + c0 + r) * ld;
+        beta = 1.0 / (1.0 + exp(-(double)__bfloat162float(raw[off_b + h])));
+        const double z = (double)(__bfloat162float(raw[off_a + h]) + dt_bias[h]);
+        lg[i] = -exp((double)a_log[h]) * (z > 30.0 ? z : log1p(exp(z)));
+      }
+      beta_s[r] = (float)beta;
+    }
+    double sum = lg[0] + lg[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
+    }
+    const double all = __shfl_sync(0xffffffffu, sum, 31);
+    const double cum[2] = {sum - lg[1], sum};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = 2 * lane + i;
+      const double l2 = cum[i] * 1.4426950408889634;
+      hi_s[r] = (float)l2;
+      lo_s[r] = (float)(l2 - (double)(float)l2);
+      grown_s[r] = (float)exp(cum[i]);
+      left_s[r] = (float)exp(all - cum[i]);
+    }
+    if (lane == 0) rec.total = make_float4((float)exp(all), 0.f, 0.f, 0.f);
+  }
+  copy_wait<0>();
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kChunk / kChunkPrepWarps; ++i) {         // lengths, a row at a time (the roots in double, as the walk's)
+    const int r = warp + kChunkPrepWarps * i;
+    float sk = 0.f, sq = 0.f;
+#pragma unroll
+    for (int e = 0; e < D / 64; ++e) {
+      const float2 kv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ks[r][2 * lane + 64 * e]));
+      const float2 qv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qs[r][2 * lane + 64 * e]));
+      sk = fmaf(kv.x, kv.x, sk); sk = fmaf(kv.y, kv.y, sk);
+      sq = fmaf(qv.x, qv.x, sq); sq = fmaf(qv.y, qv.y, sq);
+    }
+    sk = warp_sum(sk);
+    sq = warp_sum(sq);
+    if (lane == 0) {
+      ik_s[r] = (float)(1.0 / sqrt((double)sk + 1e-6));
+      iq_s[r] = (float)((double)q_scale / sqrt((double)sq + 1e-6));
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < kChunk) {
+    const int r = threadIdx.x;
+    rec.sc[r] = make_float4(beta_s[r], grown_s[r] * ik_s[r], grown_s[r] * iq_s[r], left_s[r] * ik_s[r]);
+  }
+  // the tiles on and below the diagonal: 10 of k . k, 10 of q . k
+  for (int item = warp; item < 20; item += kChunkPrepWarps) {
+    const bool is_q = item >= 10;
+    const int tile = is_q ? item - 10 : item, tr = tile < 1 ? 0 : tile < 3 ? 1 : tile < 6 ? 2 : 3;
+    const int row = 16 * tr, col = 16 * (tile - tr * (tr + 1) / 2);
+    float acc[2][2][4] = {};
+#pragma unroll
+    for (int k = 0; k < D / 16; ++k) {
+      uint32_t a[4], b[4];
+      ldmatrix4(a, is_q ? &qs[row + (lane & 15)][16 * k + 8 * (lane >> 4)] : &ks[row + (lane & 15)][16 * k + 8 * (lane >> 4)]);
+      ldmatrix4(b, &ks[col + (lane & 7) + 8 * (lane >> 4)][16 * k + 8 * ((lane >> 3) & 1)]);
+      mma16816(acc[k & 1][0], a, b[0], b[1]);
+      mma16816(acc[k & 1][1], a, b[2], b[3]);
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int r = row + qr + 8 * j, s = col + 8 * nt + 2 * qc;
+        float v[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float decay = exp2f((hi_s[r] - hi_s[s + i]) + (lo_s[r] - lo_s[s + i]));
+          const float dot = (acc[0][nt][2 * j + i] + acc[1][nt][2 * j + i]) * ik_s[s + i];
+          v[i] = is_q ? (s + i <= r ? dot * iq_s[r] * decay : 0.f) : (s + i < r ? dot * ik_s[r] * decay * beta_s[r] : 0.f);
+        }
+        if (is_q) {
+          uint32_t piece[3];
+          split_pair(v[0], v[1], piece);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&rec.p[k][r * kChunk + s]) = piece[k];
+        } else {
+          a_s[r][s] = v[0];
+          a_s[r][s + 1] = v[1];
+        }
+      }
+  }
+  __syncthreads();
+  // T = (I + A)^-1 in place of A, by blocks of 16: the diagonal ones column by column, then the others by rising distance from
+  // the diagonal, T_ij = -T_ii sum_k A_ik T_kj (k from j to i - 1).  A tile of A is read for the last time before its place is
+  // taken: A_ik is needed for the T_ij with j <= k, at distances >= that of (i, k); X holds a distance's sums.
+  float tcol[16];
+  if (warp < 4 && lane < 16) {
+    const int b = 16 * warp;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float v = i == lane ? 1.f : 0.f;
+#pragma unroll
+      for (int k = 0; k < i; ++k) v = fmaf(-a_s[b + i][b + k], tcol[k], v);
+      tcol[i] = v;
+    }
+  }
+  __syncthreads();
+  if (warp < 4 && lane < 16) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) a_s[16 * warp + i][16 * warp + lane] = tcol[i];
+  }
+  __syncthreads();
+  {
+    const int er = threadIdx.x >> 4, ec = threadIdx.x & 15;    // a thread's entry of a tile
+    // Distances 1 to 3; the tiles of A at larger distances than the current one are still A.  T_kj for k > j lies at a smaller
+    // distance and has been made.  A_ik with i - k < distance has been overwritten, so the sums use copies: x = T_ii^-1 parts
+    // are avoided by multiplying with A from registers saved before.
+    float a_keep[3][16];                                       // this thread's rows of A at distance 1 (tiles (1,0), (2,1), (3,2)): row er
+    float a_keep2[2][16];                                      // and at distance 2 (tiles (2,0), (3,1))
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+      for (int k = 0; k < 16; ++k) a_keep[b][k] = a_s[16 * (b + 1) + er][16 * b + k];
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int k = 0; k < 16; ++k) a_keep2[b][k] = a_s[16 * (b + 2) + er][16 * b + k];
+#pragma unroll
+    for (int dist = 1; dist < 4; ++dist) {
+      __syncthreads();
+#pragma unroll
+      for (int b = 0; b < 4 - dist; ++b) {                     // tile (b + dist, b)
+        const int i = b + dist;
+        float x = 0.f;
+#pragma unroll
+        for (int kb = b; kb < i; ++kb) {                       // A tile (i, kb), at distance i - kb
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const float av = i - kb == 1 ? a_keep[kb][k] : i - kb == 2 ? a_keep2[kb < 2 ? kb : 0][k] : a_s[16 * i + er][16 * kb + k];
+            x = fmaf(av, a_s[16 * kb + k][16 * b + ec], x);
+          }
+        }
+        x_s[b][er][ec] = x;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int b = 0; b < 4 - dist; ++b) {
+        const int i = b + dist;
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v = fmaf(a_s[16 * i + er][16 * i + k], x_s[b][k][ec], v);
+        a_s[16 * i + er][16 * b + ec] = -v;
+      }
+    }
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < kPieceElems / 4; idx += blockDim.x) {
+    const int r = idx / (kChunk / 4), e = 4 * (idx % (kChunk / 4));
+    if (e >= 16 * (r / 16 + 1)) continue;
+    const float4 v = *reinterpret_cast<const float4*>(&a_s[r][e]);
+    uint32_t p01[3], p23[3];
+    split_pair(v.x, v.y, p01);
+    split_pair(v.z, v.w, p23);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(&rec.t[k][r * kChunk + e]) = make_uint2(p01[k], p23[k]);
+  }
+}
+
+// grid (H, requests, columns / 16).  Phases of a chunk, a barrier after each:
+//   1  warps 0-7: R = beta (v - exp(c) S^T k), a 16 x 8 tile each;  warps 8-15: S^T q, kept in registers
+//   2  warps 0-7: U = T R, and U as the state will take it;  warps 8-15 wait
+//   3  warps 0-7: the state, in accumulators (D / 16 tiles of 16 keys);  warps 8-15: o
+// The next chunk's operands are copied meanwhile.
+template <int D>
+struct DeltaChunkSmem {
+  static constexpr int LdD = D + 8, LdC = kChunkCols + 8;      // rows 16 bytes longer than a power of two: no bank conflicts
+  struct Stage {
+    __nv_bfloat16 k[kChunk][LdD];
+    __nv_bfloat16 q[kChunk][LdD];
+    __nv_bfloat16 p[3][kPieceElems];                           // rows of 128 bytes, 16-byte pieces exchanged by the row's number
+    __nv_bfloat16 t[3][kPieceElems];
+    __nv_bfloat16 v[kChunk][LdC];
+    float4 sc[kChunk];
+    float4 total;
+  } stage[2];
+  __nv_bfloat16 s[3][D][LdC];                                  // the state before the chunk, in pieces
+  __nv_bfloat16 r[3][kChunk][LdC];
+  __nv_bfloat16 u[3][kChunk][LdC];
+  __nv_bfloat16 w[3][kChunk][LdC];                             // exp(c_64 - c) / |k| u
+};
+
+template <int D>
+__global__ void __launch_bounds__(kChunkWarps * 32)
+delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const ChunkRecord* __restrict__ records, float* __restrict__ state,
+                   const int* __restrict__ seq_starts, const int* __restrict__ state_slots, float* __restrict__ out, int H, int G, int dv) {
+  chain_wait();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typedef DeltaChunkSmem<D> Smem;
+  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+  const int h = blockIdx.x, seq = blockIdx.y, p0 = blockIdx.z * kChunkCols, kh = h / (H / G);
+  const int start = seq_starts[seq], n_tok = seq_starts[seq + 1] - start;
+  if (n_tok <= 1) return;                                      // (a single token is walked)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qr = lane >> 2, qc = lane & 3;
+  const int n_chunks = (n_tok + kChunk - 1) / kChunk;
+  const ChunkRecord* rec0 = records + (size_t)chunks_before(seq_starts, seq) * H + h;
+  const __nv_bfloat16* rows = qkv + (size_t)start * channels;
+
+  auto load_stage = [&](int c) {
+    typename Smem::Stage& st = sm.stage[c & 1];
+    const int c0 = c * kChunk;
+    const ChunkRecord* rec = rec0 + (size_t)c * H;
+    for (int idx = threadIdx.x; idx < kChunk * (D / 8); idx += kChunkWarps * 32) {
+      const int r = idx / (D / 8), e = 8 * (idx % (D / 8));
+      const bool real = c0 + r < n_tok;
+      const __nv_bfloat16* src = rows + (size_t)(real ? c0 + r : 0) * channels + kh * D + e;
+      copy16_or_zero(&st.q[r][e], src, real);
+      copy16_or_zero(&st.k[r][e], src + G * D, real);
+    }
+    for (int idx = threadIdx.x; idx < 3 * kChunk * (kChunk / 8); idx += kChunkWarps * 32) {
+      const int row = idx >> 3, r = row & (kChunk - 1), piece = row / kChunk, e = idx & 7;
+      if (e >= 2 * (r / 16 + 1)) continue;                     // (above the diagonal)
+      const int dst = r * kChunk + 8 * (e ^ (r & 7));
+      copy16_or_zero(&st.p[piece][dst], &rec->p[piece][r * kChunk + 8 * e], true);
+      copy16_or_zero(&st.t[piece][dst], &rec->t[piece][r * kChunk + 8 * e], true);
+    }
+    if (threadIdx.x < 2 * kChunk) {
+      const int r = threadIdx.x >> 1, e = 8 * (threadIdx.x & 1);
+      const bool real = c0 + r < n_tok;
+      copy16_or_zero(&st.v[r][e], rows + (size_t)(real ? c0 + r : 0) * channels + 2 * G * D + h * dv + p0 + e, real);
+    } else if (threadIdx.x < 3 * kChunk) {
+      copy16_or_zero(&st.sc[threadIdx.x - 2 * kChunk], &rec->sc[threadIdx.x - 2 * kChunk], true);
+    } else if (threadIdx.x == 3 * kChunk) {
+      copy16_or_zero(&st.total, &rec->total, true);
+    }
+    copy_commit();
+  };
+
+  // the state (stored [values][keys]): warp w < 8 holds keys 16 (w mod D/16) .. + 15, values 8 NTW (w div D/16) .. + 8 NTW - 1
+  constexpr int kRowTiles = D / 16, NTW = kRowTiles / 4;
+  const int s_row = 16 * (warp % kRowTiles), s_col = 8 * NTW * (warp / kRowTiles);
+  float S[NTW][4];
+  float* s_glob = state + (((size_t)state_slots[seq] * H + h) * dv + p0) * D;
+  auto publish = [&]() {
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        uint32_t piece[3];
+        split_pair(S[nt][2 * j], S[nt][2 * j + 1], piece);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          *reinterpret_cast<uint32_t*>(&sm.s[k][s_row + qr + 8 * j][s_col + 8 * nt + 2 * qc]) = piece[k];
+      }
+  };
+  load_stage(0);
+  if (warp < 8) {
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) S[nt][i] = s_glob[(size_t)(s_col + 8 * nt + 2 * qc + (i & 1)) * D + s_row + qr + 8 * (i >> 1)];
+    publish();
+  }
+  const int row = 16 * ((warp & 7) >> 1), col = 8 * (warp & 1);       // a warp's tile of R, U and o
+  // 16 x 8 of M X for a lower-triangular M in pieces (swizzled rows) and X in pieces, the six products that matter
+  auto triangular = [&](const __nv_bfloat16 (*m)[kPieceElems], const __nv_bfloat16 (*x)[kChunk][Smem::LdC], float* result) {
+    float acc[3][4] = {};
+    for (int k = 0; k <= row; k += 16) {
+      uint32_t a[3][4], b[3][2];
+      const int r = row + (lane & 15), e = (k >> 3) + (lane >> 4);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        ldmatrix4(a[i], &m[i][r * kChunk + 8 * (e ^ (r & 7))]);
+        ldmatrix2t(b[i], &x[i][k + (lane & 15)][col]);
+      }
+      mma16816(acc[0], a[0], b[0][0], b[0][1]);
+      mma16816(acc[1], a[0], b[1][0], b[1][1]);
+      mma16816(acc[2], a[0], b[2][0], b[2][1]);
+      mma16816(acc[1], a[1], b[0][0], b[0][1]);
+      mma16816(acc[2], a[1], b[1][0], b[1][1]);
+      mma16816(acc[2], a[2], b[0][0], b[0][1]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) result[i] = (acc[2][i] + acc[1][i]) + acc[0][i];
+  };
+  for (int c = 0; c < n_chunks; ++c) {
+    typename Smem::Stage& st = sm.stage[c & 1];
+    copy_wait<0>();
+    __syncthreads();                                           // chunk c's operands and the state's pieces are there
+    if (c + 1 < n_chunks) load_stage(c + 1);
+    float from_state[4];                                       // 16 x 8 of k S (warps 0-7) or q S, rows as they came
+    {
+      float acc[3][4] = {};
+      const __nv_bfloat16 (*m)[Smem::LdD] = warp < 8 ? st.k : st.q;
+#pragma unroll
+      for (int k = 0; k < D / 16; k += 2) {
+        uint32_t a[2][4], b[3][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) ldmatrix4(a[i], &m[row + (lane & 15)][16 * (k + i) + 8 * (lane >> 4)]);
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) ldmatrix4t(b[piece], &sm.s[piece][16 * k + lane][col]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int piece = 0; piece < 3; ++piece) mma16816(acc[piece], a[i], b[piece][2 * i], b[piece][2 * i + 1]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) from_state[i] = (acc[2][i] + acc[1][i]) + acc[0][i];
+    }
+    if (warp < 8) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int r = row + qr + 8 * j;
+        const float4 sc = st.sc[r];
+        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.v[r][col + 2 * qc]));
+        uint32_t piece[3];
+        split_pair(sc.x * fmaf(-sc.y, from_state[2 * j], v.x), sc.x * fmaf(-sc.y, from_state[2 * j + 1], v.y), piece);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&sm.r[k][r][col + 2 * qc]) = piece[k];
+      }
+    }
+    __syncthreads();                                           // R is there; the state's pieces have been read
+    if (warp < 8) {
+      float u[4];
+      triangular(st.t, sm.r, u);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int r = row + qr + 8 * j;
+        const float left = st.sc[r].w;
+        uint32_t piece[3], weighted[3];
+        split_pair(u[2 * j], u[2 * j + 1], piece);
+        split_pair(left * u[2 * j], left * u[2 * j + 1], weighted);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          *reinterpret_cast<uint32_t*>(&sm.u[k][r][col + 2 * qc]) = piece[k];
+          *reinterpret_cast<uint32_t*>(&sm.w[k][r][col + 2 * qc]) = weighted[k];
+        }
+      }
+    }
+    __syncthreads();                                           // U is there
+    if (warp < 8) {
+      float add[3][NTW][4] = {};
+#pragma unroll
+      for (int k = 0; k < kChunk / 16; ++k) {
+        uint32_t kt[4], b[3][4];                               // K^T: 16 keys x 16 tokens
+        ldmatrix4t(kt, &st.k[16 * k + (lane & 7) + 8 * (lane >> 4)][s_row + 8 * ((lane >> 3) & 1)]);
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) {
+          if (NTW == 2) ldmatrix4t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col + 8 * (lane >> 4)]);
+          else ldmatrix2t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col]);
+        }
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece)
+#pragma unroll
+          for (int nt = 0; nt < NTW; ++nt) mma16816(add[piece][nt], kt, b[piece][2 * nt], b[piece][2 * nt + 1]);
+      }
+      const float total = st.total.x;
+#pragma unroll
+      for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[nt][i] = fmaf(total, S[nt][i], (add[2][nt][i] + add[1][nt][i]) + add[0][nt][i]);
+      publish();
+    } else {
+      float own[4];
+      triangular(st.p, sm.u, own);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int r = row + qr + 8 * j;
+        if (c * kChunk + r < n_tok) {
+          const float grown = st.sc[r].z;
+          *reinterpret_cast<float2*>(out + ((size_t)(start + c * kChunk + r) * H + h) * dv + p0 + col + 2 * qc) =
+              make_float2(fmaf(grown, from_state[2 * j], own[2 * j]), fmaf(grown, from_state[2 * j + 1], own[2 * j + 1]));
+        }
+      }
+    }
+  }
+  if (warp < 8) {
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s_glob[(size_t)(s_col + 8 * nt + 2 * qc + (i & 1)) * D + s_row + qr + 8 * (i >> 1)] = S[nt][i];
+  }
+}
+
+inline bool chunk_sizes(int d, int dv) { return (d == 64 || d == 128) && dv % kChunkCols == 0; }
+inline long long chunk_records(int n_tokens, int n_seqs, int H) { return (long long)(n_tokens / kChunk + n_seqs) * H; }
+
+// Whether the chunks are the faster form: both costs in microseconds, fitted to the times of 1 to 64 requests of 2 to 500 tokens
+// (4 to 16 heads of 64 x 48 and 128 x 128).  The walk costs 0.49 us a token of the longest portion or, when the GPU is full,
+// its blocks' tokens and states; the chunks cost two more launches, 3.7 us a chunk of the longest portion or, when the GPU is
+// full, a share of an SM for every chunk, be it full or not, and requests of one token are then walked by themselves.  One
+// request: from 32 tokens on; 32 requests of equal length: from about 50.
+inline bool chunks_pay(int blocks, int n_tokens, int n_seqs, int longest) {
+  if (longest <= 1) return false;
+  const double extra = (double)n_tokens - n_seqs - (longest - 1);      // tokens beyond one of the other requests
+  const double others = fmax(0.0, fmin(extra, n_seqs - 1.0)), singles = n_seqs - 1.0 - others;
+  const double own = (longest + 63) / 64, chunks = own + (others > 0.0 ? others + extra / 64.0 : 0.0);
+  const double walk = fmax(6.0 + 0.49 * longest, blocks * (0.00086 * n_tokens + 0.0024 * n_seqs));
+  return 15.0 + fmax(3.7 * own, 0.0384 * blocks * chunks) + 0.003 * blocks * singles < walk;
+}
+
+#define ERB_DELTA_CHUNKS 1
+#else
+inline bool chunk_sizes(int, int) { return false; }
+#define ERB_DELTA_CHUNKS 0
+#endif  // ERB_ELEM == 1
+
 }  // namespace
 
-// Floats of the scratch that erb_delta_scan needs for a step of n_tokens tokens.
-ERB_EXPORT long long erb_delta_scratch_floats(int n_tokens, int H, int G, int d, int dv) {
-  return (long long)delta_scratch_floats(n_tokens, H, G, d, dv);
+// Floats of the scratch that erb_delta_scan needs for a step of n_tokens tokens, and (n_seqs > 0) what it needs to take portions
+// of prompts in chunks: the chunks' records, and the walk's scratch for requests of one token.
+ERB_EXPORT long long erb_delta_scratch_floats(int n_tokens, int n_seqs, int H, int G, int d, int dv) {
+  long long need = (long long)delta_scratch_floats(n_tokens, H, G, d, dv);
+#if ERB_DELTA_CHUNKS
+  if (n_seqs > 0 && n_tokens > n_seqs && chunk_sizes(d, dv)) {
+    const long long chunks = chunk_records(n_tokens, n_seqs, H) * (long long)(sizeof(ChunkRecord) / 4) + (long long)delta_scratch_floats(n_seqs, H, G, d, dv);
+    if (chunks > need) need = chunks;
+  }
+#endif
+  return need;
 }
 
 ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, int ld, int off_b, int off_a,
                               const float* dt_bias, const float* a_log, float* state, const int* seq_starts,
-                              const int* state_slots, float* out, float* scratch, int n_seqs, int n_tokens, int H, int G, int d,
-                              int dv, void* stream) {
+                              const int* state_slots, float* out, float* scratch, long long scratch_floats, int n_seqs, int n_tokens,
+                              int longest, int H, int G, int d, int dv, void* stream) {
   if (n_seqs <= 0 || n_tokens <= 0) return ERB_OK;
   if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 || d > 32 * kDeltaRows)
     return fail(ERB_ERR_ARG, "delta_scan: bad sizes (%d heads over %d, keys of %d up to %d)", H, G, d, 32 * kDeltaRows);
   if (channels < 2 * G * d + H * dv) return fail(ERB_ERR_ARG, "delta_scan: rows too narrow");
   if (!scratch || ((uintptr_t)scratch & 15)) return fail(ERB_ERR_ARG, "delta_scan: the scratch must be 16-byte aligned");
-  const DeltaScratch sc = delta_scratch(scratch, n_tokens, H, G, d, dv);
-  const long long items = (long long)n_tokens * G;
+  bool singles = false;                  // whether the walk is left with the requests of one token
+  int walk_tokens = n_tokens;
+#if ERB_DELTA_CHUNKS
+  if (chunk_sizes(d, dv) && n_tokens > n_seqs && chunks_pay(H * (dv / kChunkCols), n_tokens, n_seqs, longest) && channels % 8 == 0 &&
+      !(((uintptr_t)qkv | (uintptr_t)scratch) & 15) && !((uintptr_t)out & 7) && n_tokens / kChunk + n_seqs <= 65535 &&
+      scratch_floats >= erb_delta_scratch_floats(n_tokens, n_seqs, H, G, d, dv)) {
+    ChunkRecord* records = reinterpret_cast<ChunkRecord*>(scratch);
+    auto prep = d == 64 ? delta_chunk_prepare_kernel<64> : delta_chunk_prepare_kernel<128>;
+    const size_t prep_bytes = d == 64 ? sizeof(DeltaPrepSmem<64>) : sizeof(DeltaPrepSmem<128>);
+    cudaError_t e = cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_bytes);
+    if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "delta_scan: %s", cudaGetErrorString(e));
+    launch_chained(prep, dim3(H, n_tokens / kChunk + n_seqs), dim3(kChunkPrepWarps * 32), prep_bytes, (cudaStream_t)stream, (const elem_t*)qkv,
+                   channels, (const elem_t*)proj, ld, off_b, off_a, dt_bias, a_log, seq_starts, n_seqs, records, H, G, 1.f / sqrtf((float)d));
+    int rc = check_launch("delta_chunk_prepare");
+    if (rc) return rc;
+    const size_t bytes = d == 64 ? sizeof(DeltaChunkSmem<64>) : sizeof(DeltaChunkSmem<128>);
+    auto kern = d == 64 ? delta_chunk_kernel<64> : delta_chunk_kernel<128>;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "delta_scan: %s", cudaGetErrorString(e));
+    launch_chained(kern, dim3(H, n_seqs, dv / kChunkCols), dim3(kChunkWarps * 32), bytes, (cudaStream_t)stream, (const elem_t*)qkv,
+                   channels, records, state, seq_starts, state_slots, out, H, G, dv);
+    if ((rc = check_launch("delta_chunk")) || n_seqs == 1) return rc;
+    singles = true;
+    walk_tokens = n_seqs;
+    scratch += chunk_records(n_tokens, n_seqs, H) * (long long)(sizeof(ChunkRecord) / 4);
+  }
+#endif
+  const DeltaScratch sc = delta_scratch(scratch, walk_tokens, H, G, d, dv);
+  const long long items = (long long)walk_tokens * G;
   if (items > 0x7fffffffLL) return fail(ERB_ERR_UNSUPPORTED, "delta_scan: %d tokens of %d key heads", n_tokens, G);
   launch_chained(delta_prepare_kernel<elem_t>, dim3((unsigned)((items + kPrepWarps - 1) / kPrepWarps)), dim3(kPrepWarps * 32), 0,
                  (cudaStream_t)stream, (const elem_t*)qkv, channels, (const elem_t*)proj, ld, off_b, off_a, dt_bias, a_log, sc,
-                 (int)items, H, G, d, dv, 1.f / sqrtf((float)d));
+                 (int)items, H, G, d, dv, 1.f / sqrtf((float)d), singles ? seq_starts : nullptr);
   int rc = check_launch("delta_prepare");
   if (rc) return rc;
   int L = 1;
@@ -328,7 +869,7 @@ ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, i
       if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "delta_scan: %s", cudaGetErrorString(e));                        \
     }                                                                                                                   \
     launch_chained(kern, dim3(H, n_seqs, cblocks), dim3(LL * PB), smem, (cudaStream_t)stream, sc, state, seq_starts,    \
-                   state_slots, out, H, G, d, dv, PB);                                                                  \
+                   state_slots, out, H, G, d, dv, PB, singles);                                                         \
   } break;
   switch (L) {
     ERB_DELTA_CASE(1)

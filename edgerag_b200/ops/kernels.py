@@ -124,7 +124,7 @@ _SIGNATURES = {
                            c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                            c_void_p, c_void_p, c_int, c_int, c_void_p],
     "erb_delta_scan": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                       c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "erb_head_norm_gate": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
     "erb_moe_route": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p],
@@ -1383,16 +1383,25 @@ def gated_group_norm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, e
 DELTA_MAX_KEY_DIM = 512      # entries of a key the scan kernel holds per column (32 lanes of 16)
 
 
-def delta_scratch_floats(n_tokens: int, n_heads: int, n_key_heads: int, key_dim: int, v_dim: int) -> int:
+DELTA_CHUNK_TOKENS = 64      # tokens the chunk kernel takes at a time ...
+DELTA_CHUNK_FLOATS = 12548   # ... and floats it keeps of them per head
+
+
+def delta_scratch_floats(n_tokens: int, n_heads: int, n_key_heads: int, key_dim: int, v_dim: int, n_seqs: int = 0) -> int:
     """Floats of the scratch ``delta_scan`` fills for a step of ``n_tokens`` tokens: per token the unit queries and keys of
-    every key head, three scalars per head and the values, rows padded to 16 bytes."""
+    every key head, three scalars per head and the values, rows padded to 16 bytes.  With ``n_seqs``, the step's requests, it is
+    enough for portions of prompts to be taken in chunks (bfloat16 rows): two 64 x 64 matrices per chunk and head."""
     pad = lambda v: (v + 3) & ~3   # noqa: E731
-    return n_tokens * (n_key_heads * 2 * pad(key_dim) + n_heads * 4 + n_heads * pad(v_dim))
+    per_token = n_key_heads * 2 * pad(key_dim) + n_heads * 4 + n_heads * pad(v_dim)
+    need = n_tokens * per_token
+    if n_seqs > 0 and n_tokens > n_seqs and key_dim in (64, 128) and v_dim % 16 == 0:
+        need = max(need, (n_tokens // DELTA_CHUNK_TOKENS + n_seqs) * n_heads * DELTA_CHUNK_FLOATS + n_seqs * per_token)
+    return need
 
 
 def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
                state: torch.Tensor, n_seqs: int, seq_starts: torch.Tensor, state_slots: torch.Tensor, out: torch.Tensor,
-               n_key_heads: int, key_dim: int, scratch: torch.Tensor | None = None) -> None:
+               n_key_heads: int, key_dim: int, scratch: torch.Tensor | None = None, longest: int | None = None) -> None:
     """The gated delta rule over every request's rows, from and to its record in ``state`` (float ``[slots, heads,
     vdim, key_dim]``, the matrix of a head stored with the value index first).  ``qkv``: convolved and activated rows
     ``[q (key heads * key_dim) | k (the same) | v (heads * vdim)]``; the raw write strengths and decay inputs are
@@ -1400,7 +1409,9 @@ def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt
     made unit vectors (q also times ``key_dim ** -0.5``), ``beta = sigmoid(b)``, ``g = exp(-exp(a_log) * softplus(a +
     dt_bias))``, ``S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q``.  ``out`` float ``[tokens, heads * vdim]``.
     ``scratch``: float, ``delta_scratch_floats`` entries (None: allocated here), where a first kernel leaves every token's
-    unit vectors, scalars and values for the walk along the tokens."""
+    unit vectors, scalars and values for the walk along the tokens.  Where it has room (``n_seqs`` given to that function) and
+    the sizes allow it, long portions are taken in chunks of 64 tokens; ``longest``: the largest number of tokens of a request,
+    by which that is chosen (None: what the totals allow).  The results do not depend on it beyond rounding."""
     _need(qkv, "qkv"); _need(proj, "proj", qkv.dtype, contiguous=False); _need(state, "state", torch.float32)
     _need(out, "out", torch.float32); _need(dt_bias, "dt_bias", torch.float32); _need(a_log, "a_log", torch.float32)
     _need(seq_starts, "seq_starts", torch.int32); _need(state_slots, "state_slots", torch.int32)
@@ -1412,14 +1423,15 @@ def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt
         raise KernelError("delta_scan: shapes disagree")
     need = delta_scratch_floats(n, heads, n_key_heads, d, vdim)
     if scratch is None:
-        scratch = torch.empty(max(need, 4), dtype=torch.float32, device=qkv.device)
+        room = delta_scratch_floats(n, heads, n_key_heads, d, vdim, int(n_seqs) if qkv.dtype == torch.bfloat16 else 0)
+        scratch = torch.empty(max(room, 4), dtype=torch.float32, device=qkv.device)
     _need(scratch, "scratch", torch.float32)
     if scratch.numel() < need:
         raise KernelError("delta_scan: the scratch is too small")
     _call(_fn("delta", _elem(qkv), "erb_delta_scan"), qkv.data_ptr(), qkv.shape[1], proj.data_ptr(),
           proj.stride(0) if n > 1 else proj.shape[1], int(off_b), int(off_a), dt_bias.data_ptr(), a_log.data_ptr(),
-          state.data_ptr(), seq_starts.data_ptr(), state_slots.data_ptr(), out.data_ptr(), scratch.data_ptr(), int(n_seqs), n, heads,
-          int(n_key_heads), d, vdim, _stream())
+          state.data_ptr(), seq_starts.data_ptr(), state_slots.data_ptr(), out.data_ptr(), scratch.data_ptr(), scratch.numel(), int(n_seqs), n,
+          n - int(n_seqs) + 1 if longest is None else int(longest), heads, int(n_key_heads), d, vdim, _stream())
 
 
 def head_norm_gate(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, n_heads: int, eps: float) -> None:

@@ -52,6 +52,56 @@ def test_state_space_chunks(H, P, N, G, lens, pace):
         assert torch.equal(state[0], before[0])     # the slot nobody holds
 
 
+def _delta_reference(qkv, b, a, dt_bias, a_log, state, H, G, d, dv):
+    n, x = qkv.shape[0], qkv.double()
+    unit = lambda z: z / torch.sqrt((z * z).sum(-1, keepdim=True) + 1e-6)      # noqa: E731
+    q = (unit(x[:, : G * d].reshape(n, G, d)) * d ** -0.5).repeat_interleave(H // G, 1)
+    k = unit(x[:, G * d: 2 * G * d].reshape(n, G, d)).repeat_interleave(H // G, 1)
+    v, beta = x[:, 2 * G * d:].reshape(n, H, dv), torch.sigmoid(b.double())
+    g = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(a.double() + dt_bias.double(), threshold=1e9))
+    S, o = state.double().clone(), torch.empty_like(v)
+    for t in range(n):
+        S = S * g[t, :, None, None]
+        u = beta[t, :, None] * (v[t] - torch.bmm(S, k[t, :, :, None])[..., 0])
+        S = S + u[:, :, None] * k[t, :, None, :]
+        o[t] = torch.bmm(S, q[t, :, :, None])[..., 0]
+    return o.reshape(n, H * dv), S
+
+
+@pytest.mark.parametrize("H,G,d,dv", [(2, 1, 64, 16), (4, 2, 64, 48), (2, 2, 128, 128)])
+@pytest.mark.parametrize("lens", [[63], [64], [65], [2], [1, 129, 1], [130, 3, 64, 1, 17]])
+@pytest.mark.parametrize("pace,alike", [(-6.0, True), (-6.0, False), (0.0, False), (4.0, False)])
+def test_delta_chunks(H, G, d, dv, lens, pace, alike):
+    """The delta rule in chunks and walked, against float64, with keys that resemble one another (the triangular system is
+    then far from the identity) and decays of almost one and almost nothing: within the band of the walk's own test (3e-5)."""
+    from edgerag_b200.ops import kernels
+
+    n, m = sum(lens), len(lens)
+    slots = [m - i for i in range(m)]
+    g = torch.Generator().manual_seed(d + n)
+    qkv = torch.randn(n, 2 * G * d + H * dv, generator=g) * 0.5
+    if alike:
+        qkv[:, G * d: 2 * G * d] = torch.randn(1, G * d, generator=g) + 0.3 * torch.randn(n, G * d, generator=g)
+    qkv = qkv.to(torch.bfloat16).cuda()
+    proj = torch.randn(n, 2 * H + 3, generator=g).to(torch.bfloat16).cuda()
+    dt_bias, a_log = torch.randn(H, generator=g).cuda() - 1.0, torch.randn(H, generator=g).cuda() * 0.3 + pace
+    before = 0.3 * torch.randn(m + 1, H, dv, d, generator=g).cuda()
+    starts = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32).cuda()
+    for longest, room in ((1 << 20, m), (1, m), (1 << 20, 0)):      # chunks; the walk; the walk for want of scratch
+        state, out = before.clone(), torch.full((n, H * dv), float("nan"), device="cuda")
+        scratch = torch.full((kernels.delta_scratch_floats(n, H, G, d, dv, room),), float("nan"), device="cuda")
+        kernels.delta_scan(qkv, proj, 1, 2 + H, dt_bias, a_log, state, m, starts, torch.tensor(slots, dtype=torch.int32).cuda(), out, G, d,
+                           scratch, longest=longest)
+        at = 0
+        for s, length in enumerate(lens):
+            rows = slice(at, at + length)
+            want, want_s = _delta_reference(qkv[rows], proj[rows, 1: 1 + H], proj[rows, 2 + H: 2 + 2 * H], dt_bias, a_log, before[slots[s]], H, G, d, dv)
+            assert (out[rows].double() - want).abs().max() < 3e-5 * max(1.0, want.abs().max()), (s, longest)
+            assert (state[slots[s]].double() - want_s).abs().max() < 3e-5 * max(1.0, want_s.abs().max()), (s, longest)
+            at += length
+        assert torch.equal(state[0], before[0])
+
+
 @pytest.mark.parametrize("lens", [[7], [8], [1] * 9, [255], [3, 1, 2, 250, 1], [9, 300]])
 def test_short_convolution_by_eight_channels(lens):
     """Rows of four taps, with and without a bias, at counts around the lines between the kernels: float sums of five terms
