@@ -93,29 +93,6 @@ constexpr uint32_t kIdescO = mma_idesc(BM, HD, true);
 
 // What is done to a scaled score before the softmax.
 constexpr int kScorePlain = 0, kScorePenalty = 1, kScoreCap = 2;
-// tanh(x) = x (t0 + t1 y + ... + t5 y^5), y = x^2 <= 1: the minimax polynomial of tanh(x) / x in y (relative error 6e-7)
-constexpr float kTanh0 = 0.99999941f, kTanh1 = -0.33329042f, kTanh2 = 0.13281434f, kTanh3 = -0.051605674f, kTanh4 = 0.016743115f,
-                kTanh5 = -0.0030670603f;
-
-// Two floats that one instruction multiplies and adds (both rounded as fmaf rounds one).
-struct Two {
-  unsigned long long v;
-  __device__ __forceinline__ Two() {}
-  __device__ __forceinline__ Two(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
-  __device__ __forceinline__ explicit Two(float a) : Two(a, a) {}
-  __device__ __forceinline__ void get(float& a, float& b) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-};
-__device__ __forceinline__ Two operator*(Two a, Two b) {
-  Two d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-  return d;
-}
-__device__ __forceinline__ Two fma2(Two a, Two b, Two c) {
-  Two d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return d;
-}
-
 // GATED: a launch with a gate (a kernel of its own, so that the others keep their registers).
 template <int SCORE, bool GATED>
 __global__ void __launch_bounds__(kThreads, 1)

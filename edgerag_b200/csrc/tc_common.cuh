@@ -61,6 +61,12 @@ __device__ __forceinline__ void mma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_a
       "r"(tmem_a), "l"(b), "r"(idesc), "r"(acc)
       : "memory");
 }
+// True for one lane of the (whole) warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(one));
+  return one != 0;
+}
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -196,6 +202,13 @@ __device__ __forceinline__ void tma_load_rows(uint32_t dst, const CUtensorMap* m
       ::"r"(dst), "l"(map), "r"(0), "r"(row), "r"(bar) : "memory");
 }
 
+// The same from column `col` on (a multiple of 8: copies start on 16-byte boundaries).
+__device__ __forceinline__ void tma_load_box(uint32_t dst, const CUtensorMap* map, int col, int row, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(map), "r"(col), "r"(row), "r"(bar) : "memory");
+}
+
 __device__ __forceinline__ float fast_log2(float x) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -215,6 +228,34 @@ __device__ __forceinline__ float fast_exp2(float x) {          // 2^x, one instr
 // as c2 (1 - 2 / (1 + 2^x)); its error is a few units in the last place of c2, whatever s is.
 __device__ __forceinline__ float capped_score(float x, float c2) { return fmaf(-2.f * c2, fast_rcp(1.f + fast_exp2(x)), c2); }
 
+// tanh(x) = x (t0 + t1 y + ... + t5 y^5), y = x^2 <= 1: the minimax polynomial of tanh(x) / x in y (relative error 6e-7)
+constexpr float kTanh0 = 0.99999941f, kTanh1 = -0.33329042f, kTanh2 = 0.13281434f, kTanh3 = -0.051605674f, kTanh4 = 0.016743115f,
+                kTanh5 = -0.0030670603f;
+
+// Two floats that one instruction multiplies and adds (both rounded as fmaf rounds one).
+struct Two {
+  unsigned long long v;
+  __device__ __forceinline__ Two() {}
+  __device__ __forceinline__ Two(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+  __device__ __forceinline__ explicit Two(float a) : Two(a, a) {}
+  __device__ __forceinline__ void get(float& a, float& b) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+};
+__device__ __forceinline__ Two operator*(Two a, Two b) {
+  Two d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ Two operator+(Two a, Two b) {
+  Two d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ Two fma2(Two a, Two b, Two c) {
+  Two d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return d;
+}
+
 // Tensor maps over a page pool seen as [rows = pages * kv heads * page_size][64 bfloat16] with boxes
 // of `box_rows` rows and the 128-byte swizzle.  Encoding is a host-side computation; the maps are
 // kept per (pool, rows, box) in the library that includes this header.
@@ -233,6 +274,32 @@ inline int pool_map(CUtensorMap* out, const void* pool, unsigned long long rows,
     const CUresult r = cuTensorMapEncodeTiled(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(pool), dims, strides,
                                               box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(ERB_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed (%d)", who, (int)r);
+    if (maps.size() > 4096) maps.clear();
+    it = maps.emplace(key, m).first;
+  }
+  *out = it->second;
+  return ERB_OK;
+}
+
+// A tensor map over `rows` rows of `cols` bfloat16, `ld` elements apart, with boxes of 64 columns x `box_rows` rows and the
+// 128-byte swizzle (columns behind `cols` read as zeros).  Kept like the maps of page pools.
+inline int rows_map(CUtensorMap* out, const void* base, unsigned long long rows, unsigned cols, unsigned long long ld, unsigned box_rows,
+                    const char* who) {
+  static std::map<std::tuple<const void*, unsigned long long, unsigned, unsigned long long, unsigned>, CUtensorMap> maps;
+  static std::mutex mutex;
+  std::lock_guard<std::mutex> lock(mutex);
+  const auto key = std::make_tuple(base, rows, cols, ld, box_rows);
+  auto it = maps.find(key);
+  if (it == maps.end()) {
+    CUtensorMap m;
+    const cuuint64_t dims[2] = {cols, rows};
+    const cuuint64_t strides[1] = {ld * 2};
+    const cuuint32_t box[2] = {64, box_rows};
+    const cuuint32_t elem[2] = {1, 1};
+    const CUresult r = cuTensorMapEncodeTiled(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+                                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ERB_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed (%d)", who, (int)r);
     if (maps.size() > 4096) maps.clear();
     it = maps.emplace(key, m).first;

@@ -106,6 +106,8 @@ _SIGNATURES = {
     "erb_conv_silu": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                       c_void_p, c_void_p, c_void_p],
     "erb_conv_state_update": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
+    "erb_attention_wide_diff": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_float, c_void_p, c_void_p],
     "erb_ssm_scan": [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                      c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "erb_gated_group_norm": [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
@@ -1270,6 +1272,36 @@ def diff_attention_mma(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Te
           seq_starts.data_ptr(), positions.data_ptr(), out.data_ptr(), _ptr(part), int(first_token), int(n_tokens), int(first_seq),
           int(n_seqs), int(n_tiles), int(tile_rows), int(n_heads), int(n_kv), two_dim // 2, v_dim, page_size, int(window),
           int(split_keys), int(n_splits), float(scale), float(softcap), float(lam), float(eps), float(out_scale), _stream())
+
+
+DIFF_WIDE_ROWS = 128       # tokens of one head that a block of the tcgen05 form takes
+
+
+def diff_wide_supported(dtype: torch.dtype, dim: int, v_dim: int, page_size: int) -> bool:
+    """Whether the tcgen05 form for portions takes these sizes: bfloat16, maps of 64, values of 128, pages of 8 to 128 tokens."""
+    return dtype == torch.bfloat16 and dim == 64 and v_dim == 128 and 8 <= page_size <= 128 and page_size & (page_size - 1) == 0
+
+
+def diff_attention_wide(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, block_tables: torch.Tensor,
+                        seq_starts: torch.Tensor, positions: torch.Tensor, out: torch.Tensor, n_heads: int, scale: float, lam: float,
+                        eps: float, out_scale: float, n_blocks: int, status: torch.Tensor, *, window: int = 0,
+                        softcap: float = 0.0) -> None:
+    """``diff_attention`` for portions of prompts on tcgen05: ``seq_starts`` (``[n_seqs + 1]`` token offsets) and ``block_tables``
+    name the sequences; ``n_blocks`` = sum of ``ceil(tokens / DIFF_WIDE_ROWS)`` over them.  ``status``: the word to which a block
+    that gave up waiting reports."""
+    _need(q, "q", torch.bfloat16); _need(k_pages, "k_pages", torch.bfloat16); _need(v_pages, "v_pages", torch.bfloat16)
+    _need(out, "out", torch.bfloat16); _need(block_tables, "block_tables", torch.int32); _need(seq_starts, "seq_starts", torch.int32)
+    _need(positions, "positions", torch.int32); _need(status, "status", torch.int32)
+    n = q.shape[0]
+    n_pages, n_kv, page_size, two_dim = k_pages.shape
+    if not diff_wide_supported(q.dtype, two_dim // 2, v_pages.shape[3], page_size) or two_dim % 2 or q.shape[1] != n_heads * two_dim or \
+            out.shape != (n, n_heads * v_pages.shape[3]) or n_heads % n_kv or tuple(v_pages.shape[:3]) != (n_pages, n_kv, page_size) or \
+            seq_starts.numel() < 2 or block_tables.shape[0] < seq_starts.numel() - 1 or positions.numel() < n:
+        raise KernelError("diff_attention_wide: q, pages and out disagree, or the sizes are not supported")
+    _call(_fn("attention_wide", None, "erb_attention_wide_diff"), q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), n_pages,
+          block_tables.data_ptr(), block_tables.shape[1], seq_starts.data_ptr(), positions.data_ptr(), out.data_ptr(),
+          seq_starts.numel() - 1, int(n_blocks), int(n_heads), int(n_kv), page_size, int(window), float(scale), float(softcap), float(lam),
+          float(eps), float(out_scale), status.data_ptr(), _stream())
 
 
 # --- state-space mixer -------------------------------------------------------------------------

@@ -40,6 +40,7 @@ LIBRARIES: dict[str, tuple[str, tuple[str, ...], bool]] = {
     "moe_tc": ("moe_tc.cu", ("-lcuda",), False),
     "attention_tc": ("attention_tc.cu", ("-lcuda",), False),
     "attention_prefill": ("attention_prefill.cu", ("-lcuda",), False),
+    "attention_wide": ("attention_wide.cu", ("-lcuda",), False),
     "gemm": ("gemm.cu", ("-lcublasLt",), True),
     "linear_tc": ("linear_tc.cu", ("-lcuda",), False),
     "sampling": ("sampling.cu", (), False),

@@ -21,7 +21,7 @@ The kernels of ``csrc/diff_attention.cu`` do the work between the fused input pr
 ``diff_prepare`` (convolution, rotation, cache write), ``diff_attention`` (both maps in one walk over the keys; the
 difference, the head norm and the constant in its epilogue; single tokens with long reaches in splits of the keys),
 ``diff_attention_mma`` (the same on tensor cores for prompt portions in bfloat16: both maps' weights meet one tile of
-values) and, from ``csrc/ssm.cu``, the update of the convolution's state record.
+values), ``diff_attention_wide`` (on tcgen05, maps of 64 and values of 128; ``csrc/attention_wide.cu``) and, from ``csrc/ssm.cu``, the update of the convolution's state record.
 """
 
 from __future__ import annotations
@@ -39,6 +39,12 @@ class DiffAttention(Mixer):
     graph_safe = True
     #: prompt tokens of a step from which the tensor-core kernel (tiles of 64 tokens) takes the portions
     MMA_FROM_TOKENS = 32
+    #: windows from which on the tcgen05 kernel (tiles of 128 tokens and 64 keys) takes them, and how many of its rows a token may
+    #: cost.  700 tokens with a window of 128, 256, 512: 22.7, 26.5, 33.3 us against 23.7, 33.7, 50.9 us by the tensor-core kernel of
+    #: 64 rows (a window of 64: 16.2 against 14.5 us); 16 portions of 8 tokens behind 1,024: 80 us against 75 us, 8 portions of 32
+    #: behind 512: 25 us against 46 us, 17 tokens behind 2,048: 69 us against 133 us.
+    WIDE_FROM_WINDOW = 128
+    WIDE_ROWS_PER_TOKEN = 8
 
     def __init__(self, hidden: int, n_q_heads: int, n_kv_heads: int, dim: int, v_dim: int, scale: float, diff: float,
                  eps: float, dtype: torch.dtype, device: torch.device, window: int = 0, softcap: float = 0.0, conv: int = 0,
@@ -94,6 +100,15 @@ class DiffAttention(Mixer):
         f64 = lambda n: tensors[n].to(dtype=torch.float64, device="cpu")     # noqa: E731
         self.lam = float(torch.exp((f64("lq1") * f64("lk1")).sum()) - torch.exp((f64("lq2") * f64("lk2")).sum()) + self.diff)
 
+    def _wide_blocks(self, ctx, n: int) -> int:
+        """Blocks per head of the tcgen05 kernel for the step's ``n`` tokens of portions; 0: another kernel takes them."""
+        if n < self.MMA_FROM_TOKENS or not kernels.diff_wide_supported(self.dtype, self.dim, self.v_dim, ctx.page_size):
+            return 0
+        if 0 < self.window < self.WIDE_FROM_WINDOW or not self.scale > 0:
+            return 0
+        blocks = sum(-(-length // kernels.DIFF_WIDE_ROWS) for length in ctx.host_q_len[ctx.n_decode:])
+        return blocks if blocks * kernels.DIFF_WIDE_ROWS <= self.WIDE_ROWS_PER_TOKEN * n else 0
+
     def _decode_plan(self, ctx, n_rows: int) -> tuple[int, int]:
         """(keys per split, splits) for the single-token rows: enough blocks for two per SM, splits of a multiple of 64
         keys; a function of the row count, the window and the step's context bound alone."""
@@ -144,7 +159,12 @@ class DiffAttention(Mixer):
                 kernels.diff_attention(q, k_pages, v_pages, tables, ctx.seq_of_token, ctx.positions, out, self.n_q, self.scale,
                                        self.lam, self.eps, 1.0 - self.diff, 0, nd, split_keys=split, n_splits=n_splits, part=part,
                                        **common)
-        if n - nd >= self.MMA_FROM_TOKENS and mma:
+        wide = self._wide_blocks(ctx, n - nd)
+        if wide:
+            # portions of prompts on tcgen05: blocks of 128 tokens of one head
+            kernels.diff_attention_wide(q, k_pages, v_pages, tables[nd:], ctx.seq_starts[nd: ctx.n_seqs + 1], ctx.positions, out, self.n_q,
+                                        self.scale, self.lam, self.eps, 1.0 - self.diff, wide, ctx.status, **common)
+        elif n - nd >= self.MMA_FROM_TOKENS and mma:
             # portions of prompts on tensor cores: blocks of 64 (token, head) rows of one sequence and one kv head
             kernels.diff_attention_mma(q, k_pages, v_pages, tables, ctx.seq_starts, ctx.positions, out, self.n_q, self.scale,
                                        self.lam, self.eps, 1.0 - self.diff, nd, ctx.n_seqs - nd, nd, n - nd,
