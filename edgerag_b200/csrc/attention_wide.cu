@@ -28,6 +28,8 @@
 // cores wait for them.  Tiles of 64 keys leave room in TMEM for two accumulators of 128 columns beside the scores, and in shared
 // memory for three to four tiles beside the queries.  Differential, 2,048 tokens of 16 heads, capped: 240 us by the mma.sync
 // kernel of diff_attention.cu, 74 us by this; without a cap 185 us and 58 us.
+// Rows, 2,048 tokens of 16 heads of 128 + 64 and 128: about 50 us beside 20 us of gathering and up-projecting, where the kernel over
+// latents of 512 took 705 us.
 #include <limits.h>
 #include <stdarg.h>
 #include <stdio.h>
@@ -74,7 +76,7 @@ struct WideArgs {
 template <bool DIFF, int KB, int VB>
 __host__ __device__ constexpr uint32_t q_bytes() { return 2 * (DIFF ? 1 : KB) * kQBlock; }
 template <bool DIFF, int KB, int VB>
-__host__ __device__ constexpr int stages() { return KB == 3 && VB == 2 ? 3 : 4; }
+__host__ __device__ constexpr int stages() { return KB == 3 ? 3 : 4; }
 template <bool DIFF, int KB, int VB>
 __host__ __device__ constexpr uint32_t smem_bytes() {
   return q_bytes<DIFF, KB, VB>() + stages<DIFF, KB, VB>() * (KB + VB) * kKvBlock + kExchangeBytes + 8 * (4 * stages<DIFF, KB, VB>() + 12) + 16 + 1024;
@@ -544,6 +546,54 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   }
 }
 
+// The cache rows that a portion's tokens see, gathered into plain rows: row r of sequence s is key g + r, g the first key of the
+// tile of 64 that holds the first key its first token sees; zeros before that key and behind the last one.  A warp per row.
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const __nv_bfloat16* __restrict__ pages, const int* __restrict__ block_tables, int max_pages,
+                     const int* __restrict__ seq_starts, const int* __restrict__ positions, int rows, int kv_rows, int width, int page_size,
+                     int window, __nv_bfloat16* __restrict__ out) {
+  chain_wait();
+  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  const int s = r / kv_rows;
+  const int lo = first_visible_key(positions[seq_starts[s]], window), key = (lo & ~(BN - 1)) + r - s * kv_rows;
+  const bool real = key >= lo && key <= positions[seq_starts[s + 1] - 1];
+  const uint4* src = reinterpret_cast<const uint4*>(
+      pages + (real ? ((size_t)block_tables[(size_t)s * max_pages + key / page_size] * page_size + key % page_size) * width : 0));
+  uint4* dst = reinterpret_cast<uint4*>(out + (size_t)r * width);
+  for (int c = lane; c < width / 8; c += 32) dst[c] = real ? src[c] : make_uint4(0, 0, 0, 0);
+}
+
+// The rotated parts of the queries: row t holds, per head, `dim` unrotated then `rot` rotated entries; the latter go, turned, to
+// out[token][head][64], zeros behind them.  Pairs (2i, 2i + 1), angle = position * inv_freq[i] in float, cosines and sines times
+// rot_mult.  A block per token: the angles once for all heads.
+__global__ void __launch_bounds__(128)
+latent_q_rows_kernel(const __nv_bfloat16* __restrict__ q, int ld, int heads, int dim, int rot, const int* __restrict__ positions,
+                     const float* __restrict__ inv_freq, int rot_dims, float rot_mult, __nv_bfloat16* __restrict__ out) {
+  chain_wait();
+  __shared__ float2 turn[32];
+  const int t = blockIdx.x;
+  if (threadIdx.x < 32) {
+    float sn = 0.f, cs = 1.f;
+    if (2 * (int)threadIdx.x < rot_dims) {
+      sincosf((float)positions[t] * inv_freq[threadIdx.x], &sn, &cs);
+      sn *= rot_mult; cs *= rot_mult;
+    }
+    turn[threadIdx.x] = make_float2(cs, sn);
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < heads * 32; idx += blockDim.x) {
+    const int h = idx >> 5, i = idx & 31;
+    __nv_bfloat162 v = __floats2bfloat162_rn(0.f, 0.f);
+    if (2 * i < rot) {
+      const float2 u = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(q + (size_t)t * ld + (size_t)h * (dim + rot) + dim + 2 * i));
+      const float2 c = turn[i];
+      v = __floats2bfloat162_rn(u.x * c.x - u.y * c.y, u.y * c.x + u.x * c.y);
+    }
+    *reinterpret_cast<__nv_bfloat162*>(out + ((size_t)t * heads + h) * 64 + 2 * i) = v;
+  }
+}
+
 template <bool DIFF, int KB, int VB, bool CAP>
 int launch(const CUtensorMap& mk, const CUtensorMap& mv, const WideArgs& a, int n_blocks, void* stream, const char* who) {
   auto kern = attention_wide_kernel<DIFF, KB, VB, CAP>;
@@ -595,4 +645,71 @@ ERB_EXPORT int erb_attention_wide_diff(const void* q, const void* k_pages, const
   a.out = (__nv_bfloat16*)out; a.status = status;
   return softcap > 0.f ? launch<true, 2, 2, true>(mk, mv, a, n_blocks, stream, "attention_wide_diff")
                        : launch<true, 2, 2, false>(mk, mv, a, n_blocks, stream, "attention_wide_diff");
+}
+
+// The cache rows of `n_seqs` portions as plain rows: out [n_seqs * kv_rows][width]; kv_rows a multiple of 64 that covers, from the
+// tile of 64 keys with the first key a portion's first token sees, all of its keys.
+ERB_EXPORT int erb_latent_gather(const void* pages, const int* block_tables, int max_pages, const int* seq_starts, const int* positions,
+                                 int n_seqs, int kv_rows, int width, int page_size, int window, void* out, void* stream) {
+  if (n_seqs <= 0 || kv_rows <= 0) return ERB_OK;
+  if (kv_rows % BN || width <= 0 || width % 8 || page_size <= 0 || max_pages <= 0 || window < 0 || (long long)n_seqs * kv_rows > 0x7fffffffLL ||
+      (((uintptr_t)pages | (uintptr_t)out) & 15))
+    return fail(ERB_ERR_ARG, "latent_gather: bad sizes (rows of %d, %d a sequence) or alignment", width, kv_rows);
+  const int rows = n_seqs * kv_rows;
+  launch_chained(latent_gather_kernel, dim3((rows + 7) / 8), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)pages, block_tables,
+                 max_pages, seq_starts, positions, rows, kv_rows, width, page_size, window, (__nv_bfloat16*)out);
+  return check_launch("latent_gather");
+}
+
+ERB_EXPORT int erb_latent_q_rows(const void* q, int n_tokens, int ld, int heads, int dim, int rot, const int* positions, const float* inv_freq,
+                                 int rot_dims, float rot_mult, void* out, void* stream) {
+  if (n_tokens <= 0) return ERB_OK;
+  if (heads <= 0 || dim % 2 || rot % 2 || rot < 0 || rot > 64 || ld % 2 || rot_dims > rot || rot_dims % 2 || (rot_dims > 0 && !inv_freq) ||
+      (((uintptr_t)q | (uintptr_t)out) & 3))
+    return fail(ERB_ERR_ARG, "latent_q_rows: bad sizes (rotated parts of %d, at most 64)", rot);
+  launch_chained(latent_q_rows_kernel, dim3(n_tokens), dim3(128), 0, (cudaStream_t)stream, (const __nv_bfloat16*)q, ld, heads, dim, rot,
+                 positions, inv_freq, rot_dims, rot_mult, (__nv_bfloat16*)out);
+  return check_launch("latent_q_rows");
+}
+
+// Whether erb_attention_wide_rows takes these sizes.
+ERB_EXPORT int erb_attention_wide_rows_supported(int dim, int rot, int v_dim, int rank) {
+  return (dim == 64 || dim == 128) && (v_dim == 64 || v_dim == 128) && rot > 0 && rot <= 64 && rot % 8 == 0 && rank > 0 && rank % 8 == 0;
+}
+
+// Attention over rows: keys of a head are [dim | shared rot], values v_dim.  q: [token][head][dim + rot] (rows q_ld apart, the first
+// `dim` entries of a head are read), q_rot: [token][head][64] from erb_latent_q_rows; kv: [n_seqs * kv_rows][heads][dim + v_dim];
+// latents: [n_seqs * kv_rows][rank + rot] from erb_latent_gather, whose last `rot` columns are the keys' shared part.  All token rows
+// start at the batch's first token; seq_starts as for erb_attention_wide_diff; n_blocks: sum of ceil(length / 256).  sink: float
+// [heads] or null; gate: [token][head] logits (rows gate_ld apart) or null; out: [token][head][v_dim].
+ERB_EXPORT int erb_attention_wide_rows(const void* q, int q_ld, const void* q_rot, const void* kv, const void* latents, const int* seq_starts,
+                                       const int* positions, void* out, int n_seqs, int kv_rows, int n_blocks, int heads, int dim, int rot,
+                                       int v_dim, int rank, int window, float scale, const float* sink, const void* gate, int gate_ld,
+                                       int* status, void* stream) {
+  if (n_seqs <= 0 || n_blocks <= 0) return ERB_OK;
+  if (!erb_attention_wide_rows_supported(dim, rot, v_dim, rank))
+    return fail(ERB_ERR_UNSUPPORTED, "attention_wide_rows: heads of %d + %d and %d over latents of %d", dim, rot, v_dim, rank);
+  if (heads <= 0 || n_blocks > 65535 || kv_rows <= 0 || kv_rows % BN || !status || window < 0 || !(scale > 0.f) ||
+      (long long)n_seqs * kv_rows > 0x7fffffffLL)
+    return fail(ERB_ERR_ARG, "attention_wide_rows: bad sizes or a missing status word");
+  if (q_ld % 8 || (((uintptr_t)q | (uintptr_t)q_rot | (uintptr_t)out | (uintptr_t)kv | (uintptr_t)latents) & 15))
+    return fail(ERB_ERR_UNSUPPORTED, "attention_wide_rows: rows must be 16-byte aligned");
+  const unsigned long long rows = (unsigned long long)n_seqs * kv_rows;
+  const unsigned kv_ld = (unsigned)heads * (dim + v_dim), lat_ld = (unsigned)(rank + rot);
+  CUtensorMap mk, ml;
+  int rc;
+  if ((rc = rows_map(&mk, kv, rows, kv_ld, kv_ld, BN, "attention_wide_rows")) ||
+      (rc = rows_map(&ml, latents, rows, lat_ld, lat_ld, BN, "attention_wide_rows")))
+    return rc;
+  WideArgs a = {};
+  a.q = (const __nv_bfloat16*)q; a.q_ld = q_ld; a.q_head = dim + rot; a.q_rot = (const __nv_bfloat16*)q_rot;
+  a.seq_starts = seq_starts; a.positions = positions; a.n_seqs = n_seqs; a.heads = heads;
+  a.kv_rows = kv_rows; a.k_col = 0; a.v_col = dim; a.kv_head = dim + v_dim; a.rot_col = rank;
+  a.scale_log2 = scale * 1.4426950408889634f;
+  a.window = window; a.sink = sink; a.gate = (const __nv_bfloat16*)gate; a.gate_ld = gate_ld;
+  a.out = (__nv_bfloat16*)out; a.status = status;
+  if (dim == 64) return v_dim == 64 ? launch<false, 2, 1, false>(mk, ml, a, n_blocks, stream, "attention_wide_rows")
+                                    : launch<false, 2, 2, false>(mk, ml, a, n_blocks, stream, "attention_wide_rows");
+  return v_dim == 64 ? launch<false, 3, 1, false>(mk, ml, a, n_blocks, stream, "attention_wide_rows")
+                     : launch<false, 3, 2, false>(mk, ml, a, n_blocks, stream, "attention_wide_rows");
 }

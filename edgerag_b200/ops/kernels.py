@@ -106,6 +106,10 @@ _SIGNATURES = {
     "erb_conv_silu": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                       c_void_p, c_void_p, c_void_p],
     "erb_conv_state_update": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
+    "erb_latent_gather": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    "erb_latent_q_rows": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p, c_void_p],
+    "erb_attention_wide_rows": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                                c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
     "erb_attention_wide_diff": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                 c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_float, c_void_p, c_void_p],
     "erb_ssm_scan": [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -1138,6 +1142,71 @@ def latent_attention_mma(q_lat: torch.Tensor, pages: torch.Tensor, block_tables:
     if n_splits > 1:
         _call(_fn("latent_attention", "bfloat16", "erb_latent_combine"), part.data_ptr(), _ptr(gate), gate_ld, _ptr(sink),
               out.data_ptr(), int(first_token), int(n_tokens), heads, rank, int(n_splits), _stream())
+
+
+LATENT_WIDE_ROWS = 256     # tokens of one head that a block of the kernel over up-projected rows takes
+LATENT_WIDE_KEYS = 64      # ... and keys of its tiles: a portion's rows are a multiple of it
+
+
+def latent_wide_supported(dtype: torch.dtype, dim: int, rot_dim: int, v_dim: int, rank: int) -> bool:
+    """Whether the tcgen05 form over up-projected keys and values takes these sizes: bfloat16, unrotated parts and values of 64 or
+    128, a rotated part of at most 64 and latents in multiples of 8."""
+    return (dtype == torch.bfloat16 and dim in (64, 128) and v_dim in (64, 128) and 0 < rot_dim <= 64 and rot_dim % 8 == 0
+            and rank > 0 and rank % 8 == 0)
+
+
+def latent_gather(pages: torch.Tensor, block_tables: torch.Tensor, seq_starts: torch.Tensor, positions: torch.Tensor, out: torch.Tensor,
+                  kv_rows: int, window: int = 0) -> None:
+    """The cache rows that the tokens of portions see as plain rows: ``out`` ``[n_seqs * kv_rows, width]``; row ``r`` of sequence
+    ``s`` is key ``g + r``, ``g`` the first key of the tile of ``LATENT_WIDE_KEYS`` that holds the first key the portion sees
+    (zeros before that key and behind the portion's last one).  ``seq_starts`` ``[n_seqs + 1]`` and ``block_tables`` name the sequences."""
+    _need(pages, "pages", torch.bfloat16); _need(out, "out", torch.bfloat16); _need(block_tables, "block_tables", torch.int32)
+    _need(seq_starts, "seq_starts", torch.int32); _need(positions, "positions", torch.int32)
+    n_seqs, width = seq_starts.numel() - 1, pages.shape[3]
+    if pages.shape[1] != 1 or n_seqs < 1 or block_tables.shape[0] < n_seqs or out.shape != (n_seqs * kv_rows, width):
+        raise KernelError("latent_gather: pages, tables and out disagree")
+    _call(_fn("attention_wide", None, "erb_latent_gather"), pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
+          seq_starts.data_ptr(), positions.data_ptr(), n_seqs, int(kv_rows), width, pages.shape[2], int(window), out.data_ptr(), _stream())
+
+
+def latent_q_rows(q: torch.Tensor, positions: torch.Tensor, inv_freq: torch.Tensor | None, n_heads: int, dim: int, rot_dim: int,
+                  rot_dims: int, out: torch.Tensor, rot_mult: float = 1.0) -> None:
+    """The rotated parts of the query rows ``[tokens, heads * (dim + rot_dim)]``, turned, to ``out`` ``[tokens, heads, 64]`` (zeros
+    behind the ``rot_dim`` entries)."""
+    _need(q, "q", torch.bfloat16, contiguous=False); _need(out, "out", torch.bfloat16); _need(positions, "positions", torch.int32)
+    _need(inv_freq, "inv_freq", torch.float32)
+    n = q.shape[0]
+    if q.shape[1] != n_heads * (dim + rot_dim) or q.stride(1) != 1 or out.shape != (n, n_heads, 64) or positions.numel() < n:
+        raise KernelError("latent_q_rows: shapes disagree")
+    _call(_fn("attention_wide", None, "erb_latent_q_rows"), q.data_ptr(), n, q.stride(0) if n > 1 else q.shape[1], int(n_heads), int(dim),
+          int(rot_dim), positions.data_ptr(), _ptr(inv_freq), int(rot_dims), float(rot_mult), out.data_ptr(), _stream())
+
+
+def latent_attention_wide(q: torch.Tensor, q_rot: torch.Tensor, kv: torch.Tensor, latents: torch.Tensor, seq_starts: torch.Tensor,
+                          positions: torch.Tensor, out: torch.Tensor, dim: int, rot_dim: int, scale: float, kv_rows: int, n_blocks: int,
+                          status: torch.Tensor, *, gate: torch.Tensor | None = None, sink: torch.Tensor | None = None,
+                          window: int = 0) -> None:
+    """Latent attention for portions of prompts in its up-projected form, on tcgen05: ``kv`` ``[n_seqs * kv_rows, heads * (dim +
+    v_dim)]`` holds every head's keys and values made of ``latents`` (``latent_gather``'s rows, whose last ``rot_dim`` columns
+    are the keys' shared part); ``q`` the query rows, ``q_rot`` their turned parts (``latent_q_rows``); ``out`` ``[tokens, heads,
+    v_dim]``.  ``q``, ``q_rot``, ``gate``, ``out`` and ``positions`` are indexed by the batch's tokens, ``seq_starts`` names
+    the portions, ``n_blocks`` = sum of ``ceil(tokens / LATENT_WIDE_ROWS)`` over them."""
+    _need(q, "q", torch.bfloat16, contiguous=False); _need(q_rot, "q_rot", torch.bfloat16); _need(kv, "kv", torch.bfloat16)
+    _need(latents, "latents", torch.bfloat16); _need(out, "out", torch.bfloat16); _need(seq_starts, "seq_starts", torch.int32)
+    _need(positions, "positions", torch.int32); _need(status, "status", torch.int32); _need(sink, "sink", torch.float32)
+    _need(gate, "gate", torch.bfloat16, contiguous=False)
+    n, heads, v_dim = out.shape
+    rank, n_seqs = latents.shape[1] - rot_dim, seq_starts.numel() - 1
+    if not latent_wide_supported(q.dtype, dim, rot_dim, v_dim, rank) or q.shape != (n, heads * (dim + rot_dim)) or q.stride(1) != 1 or \
+            q_rot.shape != (n, heads, 64) or kv.shape != (n_seqs * kv_rows, heads * (dim + v_dim)) or latents.shape[0] != kv.shape[0] or \
+            n_seqs < 1 or positions.numel() < n:
+        raise KernelError("latent_attention_wide: q, kv, latents and out disagree, or the sizes are not supported")
+    if (gate is not None and (gate.shape != (n, heads) or gate.stride(1) != 1)) or (sink is not None and sink.numel() != heads):
+        raise KernelError("latent_attention_wide: gate must be [tokens, heads] with unit inner stride, one sink per head")
+    _call(_fn("attention_wide", None, "erb_attention_wide_rows"), q.data_ptr(), q.stride(0) if n > 1 else q.shape[1], q_rot.data_ptr(),
+          kv.data_ptr(), latents.data_ptr(), seq_starts.data_ptr(), positions.data_ptr(), out.data_ptr(), n_seqs, int(kv_rows), int(n_blocks),
+          heads, int(dim), int(rot_dim), v_dim, rank, int(window), float(scale), _ptr(sink), _ptr(gate),
+          0 if gate is None else (gate.stride(0) if n > 1 else heads), status.data_ptr(), _stream())
 
 
 # --- differential attention ----------------------------------------------------------------------

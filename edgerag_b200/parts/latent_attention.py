@@ -18,6 +18,11 @@ them after ``Uv_h``.  A scaled rotation may multiply its cosines and sines by a 
 With ``window`` a query sees its last ``window`` cache rows only (itself among them), the pages behind the
 window go back to the pool, and ``gated=False`` leaves the sigmoid gate out.
 
+Portions of prompts are worth the opposite: with many new tokens per cached one it is cheaper to up-project the context once and to
+attend with heads of ``dim + rot_dim`` and values of ``v_dim`` than over rows of ``kv_rank + rot_dim``.  Where the sizes allow it
+(``kernels.latent_wide_supported``) a portion's cache rows are gathered, one product makes every head's keys and values of them,
+and a tcgen05 kernel attends; single tokens stay in the latent space.
+
 The first product reads the mixer's input once for everything that is made from it: queries (or
 their latent), the down-projection of ``[c | kr]`` and the gate logits.
 """
@@ -39,6 +44,8 @@ def _pad8(n: int) -> int:
 @register_part("mixer", "latent_attention")
 class LatentAttention(Mixer):
     graph_safe = True
+    #: bytes that the up-projected keys and values of a step may take
+    WIDE_MAX_BYTES = 1 << 28
 
     def __init__(self, hidden: int, n_heads: int, dim: int, rot_dim: int, v_dim: int, kv_rank: int, scale: float,
                  rot_base: float, rot_dims: int, eps: float, dtype: torch.dtype, device: torch.device, q_rank: int = 0,
@@ -64,7 +71,8 @@ class LatentAttention(Mixer):
         self.in_width = _pad8(self.off_g + self.gate_width)
         self.inv_freq = rotary_frequencies(rot_base, rot_dims, rot_scaling).to(device=device, dtype=torch.float32).contiguous()
         self.rot_mult = rotary_multiplier(rot_scaling)
-        self.w_in = self.w_uq = self.w_uk_t = self.w_uv = self.w_o = None
+        self.w_in = self.w_uq = self.w_uk_t = self.w_uv = self.w_ukv = self.w_o = None
+        self.wide = kernels.latent_wide_supported(dtype, dim, rot_dim, v_dim, kv_rank) and self.scale > 0
         self.kv_norm = self.q_norm = self.sink = None
 
     def cache_spec(self) -> KVGroupSpec:
@@ -107,6 +115,8 @@ class LatentAttention(Mixer):
         # Uk_h^T per head, [H, kv_rank, dim]: the query's unrotated part times it is the absorbed query
         self.w_uk_t = cast(tensors["uk"]).view(H, self.dim, r).transpose(1, 2).contiguous()
         self.w_uv = cast(tensors["uv"]).view(H, self.v_dim, r).contiguous()
+        if self.wide:       # both up-projections head by head, for portions whose context is up-projected
+            self.w_ukv = torch.cat([cast(tensors["uk"]).view(H, self.dim, r), self.w_uv], 1).reshape(-1, r).contiguous()
         self.sink = f32(tensors["sink"]) if self.sink_on else None
         self.w_o = cast(tensors["o"]).contiguous()
 
@@ -121,6 +131,50 @@ class LatentAttention(Mixer):
         if self.window:     # a window of w keys touches at most (w - 1) // split + 2 splits, wherever it lies
             n_splits = min(n_splits, (self.window - 1) // split + 2)
         return split, n_splits
+
+    def _wide_rows(self, ctx) -> int:
+        """Cache rows per portion that the up-projected form of the step's portions takes (0: they stay in the latent space).  A
+        function of the portions' lengths and the step's context bound alone, so that a captured step's choice holds."""
+        if ctx.batch_invariant:
+            return 0
+        lens = ctx.host_q_len[ctx.n_decode:]
+        tile = kernels.LATENT_WIDE_KEYS
+        rows = ctx.max_keys_bound()
+        if self.window:
+            rows = min(rows, self.window + max(lens) + tile - 1)
+        rows = -(-rows // tile) * tile
+        total = rows * len(lens)
+        if 2 * total * self.n_heads * (self.dim + self.v_dim) > self.WIDE_MAX_BYTES:
+            return 0
+        # The form is the faster one for every portion measured, of 2 tokens to 2,048 behind 0 to 8,000 (2,048 tokens of 16 heads of
+        # 128 + 64 over latents of 512: the sublayer 800 us in the latent space, 129 us; 2 tokens behind 2,048: 190 us, 73 us; 17 behind
+        # none: 40 us, 32 us).  But beside single tokens the bound may be theirs, with rows that no portion needs, at 6 us a thousand.
+        return rows if not ctx.n_decode or total <= 32 * sum(lens) + 2048 else 0
+
+    def _attend_wide(self, ctx, q, pages, tables, heads, gate, rows: int) -> None:
+        """The portions' tokens over up-projected keys and values; ``q``, ``gate`` and ``heads`` hold the whole batch's rows."""
+        nd, n, H = ctx.n_decode, q.shape[0], self.n_heads
+        starts = ctx.seq_starts[nd: ctx.n_seqs + 1]
+        seqs = ctx.n_seqs - nd
+        latents = ctx.buf("latent.rows", (seqs * rows, self.kv_rank + self.rot_dim), self.dtype)
+        kernels.latent_gather(pages, tables[nd:], starts, ctx.positions, latents, rows, self.window)
+        kv = ctx.buf("latent.kv", (seqs * rows, H * (self.dim + self.v_dim)), self.dtype)
+        kernels.linear(latents[:, : self.kv_rank], self.w_ukv, kv)
+        q_rot = ctx.buf("latent.q_rot", (n, H, 64), self.dtype)
+        kernels.latent_q_rows(q, ctx.positions, self.inv_freq, H, self.dim, self.rot_dim, self.rot_dims, q_rot, rot_mult=self.rot_mult)
+        blocks = sum(-(-length // kernels.LATENT_WIDE_ROWS) for length in ctx.host_q_len[nd:])
+        kernels.latent_attention_wide(q, q_rot, kv, latents, starts, ctx.positions, heads, self.dim, self.rot_dim, self.scale, rows, blocks,
+                                      ctx.status, gate=gate, sink=self.sink, window=self.window)
+
+    def _attend_latent(self, ctx, q, pages, tables, heads, gate) -> None:
+        """The batch's first ``q.shape[0]`` tokens in the latent space, to ``heads``."""
+        m, H, r, dr = q.shape[0], self.n_heads, self.kv_rank, self.rot_dim
+        q_lat = ctx.buf("latent.q", (m, H, r + dr), torch.float32)
+        kernels.latent_q_rotate(q, ctx.positions, self.inv_freq, H, self.dim, dr, r, self.rot_dims, q_lat, rot_mult=self.rot_mult)
+        kernels.linear_batched(q.as_strided((m, H, self.dim), (q.stride(0), self.dim + dr, 1)), self.w_uk_t, q_lat[:, :, :r])
+        o_lat = ctx.buf("latent.o", (m, H, r), self.dtype)
+        self._attend(ctx, q_lat, pages, tables, o_lat, gate)
+        kernels.linear_batched(o_lat, self.w_uv, heads)
 
     def _attend(self, ctx, q_lat, pages, tables, o_lat, gate) -> None:
         n, H, r = q_lat.shape[0], self.n_heads, self.kv_rank
@@ -168,16 +222,17 @@ class LatentAttention(Mixer):
             kernels.linear(q_latent, self.w_uq, q)
         else:
             q = proj[:, : self.q_width]
-        q_lat = ctx.buf("latent.q", (n, H, r + dr), torch.float32)
-        kernels.latent_q_rotate(q, ctx.positions, self.inv_freq, H, self.dim, dr, r, self.rot_dims, q_lat,
-                                rot_mult=self.rot_mult)
-        q_heads = q.as_strided((n, H, self.dim), (q.stride(0), self.dim + dr, 1))
-        kernels.linear_batched(q_heads, self.w_uk_t, q_lat[:, :, :r])
-        o_lat = ctx.buf("latent.o", (n, H, r), self.dtype)
         gate = proj[:, self.off_g: self.off_g + H] if self.gated and not self.gate_entries else None
-        self._attend(ctx, q_lat, pages, ctx.block_tables[group], o_lat, gate)
         heads = ctx.buf("latent.heads", (n, H, self.v_dim), self.dtype)
-        kernels.linear_batched(o_lat, self.w_uv, heads)
+        tables = ctx.block_tables[group]
+        rows = self._wide_rows(ctx) if self.wide and n > ctx.n_decode else 0
+        if rows:
+            self._attend_wide(ctx, q, pages, tables, heads, gate, rows)
+            m = ctx.n_decode                             # the tokens that attend in the latent space
+            if m:
+                self._attend_latent(ctx, q[:m], pages, tables, heads[:m], gate if gate is None else gate[:m])
+        else:
+            self._attend_latent(ctx, q, pages, tables, heads, gate)
         if self.gate_entries:
             kernels.sigmoid_gate(heads.view(n, H * self.v_dim), proj[:, self.off_g: self.off_g + self.gate_width])
         y = ctx.buf("mixer.out", (n, self.hidden), self.dtype)

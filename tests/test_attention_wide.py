@@ -61,3 +61,61 @@ def test_differential_portions(lens, past, page, window, cap, sharp):
             want = z / torch.sqrt((z * z).mean(-1, keepdim=True) + eps) * scale
             got = out[rows, h * dv: (h + 1) * dv].double()
             assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -10 * scale).all(), (s, h)
+
+
+@pytest.mark.parametrize("dim,rot,v,rank", [(64, 32, 64, 64), (128, 64, 128, 96), (64, 8, 128, 32), (128, 24, 64, 40)])
+@pytest.mark.parametrize("lens,past,page,window", [([2], 0, 16, 0), ([64], 0, 8, 0), ([129, 2], 63, 16, 0), ([257, 128, 300], 65, 32, 0),
+                                                   ([300], 200, 16, 50), ([2, 260], 400, 24, 64), ([256], 1, 16, 100)])
+def test_latent_portions_over_rows(dim, rot, v, rank, lens, past, page, window):
+    """Gather, turned queries and the attention over up-projected rows, from the second row of a batch on, with sinks and gates, against float64
+    on the rows that the product left: weights to 2^-17 and float sums, rounded once to bfloat16 (2^-8 of the value; 2^-13 of the
+    values' size where they cancel)."""
+    from edgerag_b200.ops import kernels
+
+    H, scale, first = 3, 0.11, 1
+    g = torch.Generator().manual_seed(sum(lens) + dim)
+    rand = lambda *shape: torch.randn(*shape, generator=g)      # noqa: E731
+    pages, table = _pages(lens, past, 1, page, rank + rot, g)
+    n = first + sum(lens)
+    for s, length in enumerate(lens):                           # pages that a window has left behind hold no numbers either
+        for pos in range(0, max(0, past - window + 1) // page * page if window else 0):
+            pages[table[s, pos // page].long(), :, pos % page] = float("nan")
+    starts = torch.tensor([first, *(first + torch.tensor(lens).cumsum(0)).tolist()], dtype=torch.int32).cuda()
+    positions = torch.cat([torch.zeros(first, dtype=torch.long)] + [torch.arange(past, past + length) for length in lens]).int().cuda()
+    q = (2.0 * rand(n, H * (dim + rot) + 8)).to(torch.bfloat16).cuda()[:, : H * (dim + rot)]
+    gate, sink = rand(n, H).to(torch.bfloat16).cuda(), (3.0 * rand(H)).cuda()
+    inv_freq = (10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64) * 2 / rot)).float().cuda()
+    rows = past + max(lens) if not window else min(past + max(lens), window + max(lens) + 63)
+    rows = -(-rows // 64) * 64
+    latents = torch.empty(len(lens) * rows, rank + rot, dtype=torch.bfloat16, device="cuda")
+    kernels.latent_gather(pages, table, starts, positions, latents, rows, window)
+    q_rot = torch.empty(n, H, 64, dtype=torch.bfloat16, device="cuda")
+    kernels.latent_q_rows(q, positions, inv_freq, H, dim, rot, rot, q_rot, rot_mult=1.1)
+    kv = torch.empty(len(lens) * rows, H * (dim + v), dtype=torch.bfloat16, device="cuda")
+    kernels.linear(latents[:, :rank], (rand(H * (dim + v), rank) / rank ** 0.5).to(torch.bfloat16).cuda(), kv)
+    out, status = torch.full((n, H, v), float("nan"), dtype=torch.bfloat16, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    kernels.latent_attention_wide(q, q_rot, kv, latents, starts, positions, out, dim, rot, scale, rows,
+                                  sum(-(-length // kernels.LATENT_WIDE_ROWS) for length in lens), status, gate=gate, sink=sink, window=window)
+    assert status.item() == 0 and torch.isnan(out[:first]).all()
+    angle = positions.double()[:, None] * inv_freq.double()
+    turned = q.reshape(n, H, dim + rot)[..., dim:].double()
+    pairs = torch.stack([turned[..., 0::2] * angle.cos()[:, None] - turned[..., 1::2] * angle.sin()[:, None],
+                         turned[..., 1::2] * angle.cos()[:, None] + turned[..., 0::2] * angle.sin()[:, None]], -1).flatten(-2) * 1.1
+    assert (q_rot[..., :rot].double() - pairs).abs().max() < 2.0 ** -8 * pairs.abs().max() and not q_rot[..., rot:].any()
+    at = first
+    for s, length in enumerate(lens):
+        lo = max(0, past - window + 1) if window else 0
+        base, n_keys, t = lo // 64 * 64, past + length - lo, slice(at, at + length)
+        keys = slice(s * rows + lo - base, s * rows + lo - base + n_keys)
+        flat = pages[table[s].long()].reshape(-1, rank + rot)[lo: past + length]
+        assert torch.equal(latents[keys], flat) and not latents[s * rows: keys.start].any() and not latents[keys.stop: (s + 1) * rows].any()
+        seen = _seen(length, past, window)[:, lo:]
+        for h in range(H):
+            k = torch.cat([kv[keys, h * (dim + v): h * (dim + v) + dim], latents[keys, rank:]], 1).double()
+            value = kv[keys, h * (dim + v) + dim: (h + 1) * (dim + v)].double()
+            query = torch.cat([q.reshape(n, H, dim + rot)[t, h, :dim], q_rot[t, h, :rot]], 1).double()
+            score = (query @ k.T * scale).masked_fill(~seen, float("-inf"))
+            weight = torch.softmax(torch.cat([score, sink[h].double().expand(length, 1)], 1), -1)[:, :-1]
+            want = weight @ value * torch.sigmoid(gate[t, h].double())[:, None]
+            assert ((out[t, h].double() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -13 * value.abs().max()).all(), (s, h)
+        at += length
