@@ -6,19 +6,23 @@
 // 128.  Both query tiles use the same key and value tiles, so every byte of K and V that reaches
 // shared memory serves 256 rows.
 //
-//   warp 17 (copy)    brings K(j) and V(j) from the cache pages into 128-byte-swizzled shared memory
+//   warp 18 (copy)    brings K(j) and V(j) from the cache pages into 128-byte-swizzled shared memory
 //                     with TMA tensor copies, one copy per page, up to four tiles of each in flight
-//   warp 16 (issue)   one thread issues S_t(j) = Q_t K(j)^T (M 128, N 128, K 64) and
-//                     O_t += P_t(j) V(j) (M 128, N 64, K 128) for t = A, B; accumulators in TMEM
+//   warps 16, 17      issue S_t(j) = Q_t K(j)^T (M 128, N 128, K 64) and
+//   (issue)           O_t += P_t(j) V(j) (M 128, N 64, K 128), one for t = A and one for t = B; accumulators in TMEM
 //   warps 0-7, 8-15   softmax of tile A and of tile B: two threads per query row, each with 64 of the
 //                     tile's 128 keys; a thread reads its scores from TMEM 32 at a time, exponentiates
 //                     them, and writes P rounded to bfloat16 back to TMEM, from where the second product
 //                     reads it as its A operand (P never passes through shared memory)
 //
-// The two softmax groups work on alternate products: while group A exponentiates S_A(j), the tensor
-// core computes S_B(j) and O_A += P_A(j-1) V(j-1).  Nobody but the copy warp touches addresses of
-// pages, and no block-wide barrier is taken inside the loop: every hand-over is an mbarrier
-// (K/V tile full, tile free again, S ready, P ready, product done).
+// The scores have three places in TMEM, taken in turn by A(0), B(0), A(1), B(1), ..., and P takes the place of the scores it was
+// made of.  So the scores of a group's next tile are there when it has finished one, whatever the other group does, and the
+// groups need not wait for products: S of turn u only waits for P V of turn u - 3.  (With one place per query tile, S_A(j + 1)
+// could start only when P_A(j) was written, and 1,800 of a step's 4,480 clocks went into waiting for it: 32 heads of 2,048 tokens
+// 52 us instead of 43 us, of 8,192 tokens 541 us instead of 432 us.)
+//
+// Nobody but the copy warp touches addresses of pages, and no block-wide barrier is taken inside the loop: every hand-over is an
+// mbarrier (K/V tile full, tile free again, S ready, P ready, product done).
 //
 // A row's reference maximum is set on the first tile and then only moves when a tile's sum of P shows
 // that it has become far too low (P is a floating-point number: a reference that is low by twenty powers
@@ -69,21 +73,23 @@ constexpr int kRowsPerBlock = 2 * BM;
 constexpr int kKStages = 4, kVStages = 4;   // key and value tiles in shared memory (powers of two)
 constexpr int kSoftmaxWarps = 16;           // per query tile 8 warps: two threads per row, 64 keys of a tile each
 constexpr int kGroupThreads = 2 * BM;       // threads of one softmax group
-constexpr int kIssueWarp = kSoftmaxWarps, kCopyWarp = kSoftmaxWarps + 1;
-constexpr int kThreads = (kSoftmaxWarps + 2) * 32;
+constexpr int kIssueWarp = kSoftmaxWarps, kCopyWarp = kSoftmaxWarps + 2;      // (two issuing warps)
+constexpr int kThreads = (kSoftmaxWarps + 3) * 32;
 constexpr uint32_t kQBytes = BM * HD * 2;               // 16 KB per query tile
 constexpr uint32_t kKvBytes = BN * HD * 2;              // 16 KB per key or value tile
 // barriers, in this order (8 bytes each)
 constexpr int kBarKFull = 0, kBarKEmpty = kBarKFull + kKStages, kBarVFull = kBarKEmpty + kKStages,
-              kBarVEmpty = kBarVFull + kVStages, kBarSFull = kBarVEmpty + kVStages, kBarPFull = kBarSFull + 2,
-              kBarPvDone = kBarPFull + 2, kNumBars = kBarPvDone + 2;
+              kBarVEmpty = kBarVFull + kVStages, kBarSFull = kBarVEmpty + kVStages, kBarPFull = kBarSFull + 4,
+              kBarPvTile = kBarPFull + 4, kBarPvPlace = kBarPvTile + 4, kNumBars = kBarPvPlace + 3;
+// S there, P written and P V done: one of each per query tile for its even and for its odd steps (the scores of step i + 2 are
+// issued behind P V of step i, so that who waits is never two phases behind); P V done once more per place of the scores
 constexpr uint32_t kSmemTiles = 2 * kQBytes + kKStages * kKvBytes + kVStages * kKvBytes;
 constexpr uint32_t kSmemExchange = 2 * 2 * BM * 2 * 4;  // two floats (maximum, sum) per (group, row, half of the row)
 constexpr uint32_t kSmemBytes = kSmemTiles + kSmemExchange + 8 * kNumBars + 16 + 1024;   // + abort flag, TMEM slot, alignment slack
-// TMEM columns: S_A 0..127, S_B 128..255, O_A 256..319, O_B 320..383, P_A 384..447, P_B 448..511
-// (P: two bfloat16 per 32-bit column, the row's keys in order: the A operand of the second product)
+// TMEM columns: three places of scores 0..383, O_A 384..447, O_B 448..511
+// (P in the first half of its scores' place, two bfloat16 per 32-bit column, the row's keys in order: the A operand of the second product)
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kColS = 0, kColO = 256, kColP = 384;
+constexpr uint32_t kColO = 384;
 // From this distance (in keys) on the penalty of 16 neighbouring keys is a series about their middle, at most 7.5 keys away:
 // the first term left out is below (7.5 / 71.5)^4 / 4 < 4e-5 of r1.
 constexpr int kPenaltyFar = 64;
@@ -136,13 +142,15 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   const int* bt = block_tables + (size_t)seq * max_pages;
 
   if (tid == 0) {
-    for (int s = 0; s < kKStages; ++s) { mbar_init(bar(kBarKFull + s), 1); mbar_init(bar(kBarKEmpty + s), 1); }
-    for (int s = 0; s < kVStages; ++s) { mbar_init(bar(kBarVFull + s), 1); mbar_init(bar(kBarVEmpty + s), 1); }
-    for (int t = 0; t < 2; ++t) {
-      mbar_init(bar(kBarSFull + t), 1);
-      mbar_init(bar(kBarPFull + t), kGroupThreads / 32);   // one arrival per warp of the group
-      mbar_init(bar(kBarPvDone + t), 1);
+    // (a tile is free again when both issuing warps say so)
+    for (int s = 0; s < kKStages; ++s) { mbar_init(bar(kBarKFull + s), 1); mbar_init(bar(kBarKEmpty + s), 2); }
+    for (int s = 0; s < kVStages; ++s) { mbar_init(bar(kBarVFull + s), 1); mbar_init(bar(kBarVEmpty + s), 2); }
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(bar(kBarSFull + i), 1);
+      mbar_init(bar(kBarPFull + i), kGroupThreads / 32);   // one arrival per warp of the group
+      mbar_init(bar(kBarPvTile + i), 1);
     }
+    for (int p = 0; p < 3; ++p) mbar_init(bar(kBarPvPlace + p), 1);
     *s_abort = 0;
     mbar_init_fence();
   }
@@ -178,6 +186,9 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   const int per_split = (n_kv + key_splits - 1) / key_splits;
   const int j0 = (int)blockIdx.z * per_split, j1 = min(n_kv, j0 + per_split);
   const int n_end[2] = {min(n_t[0], j1), min(n_t[1], j1)};
+  // The turn of step i (counted from j0) of query tile t: A and B alternate while both have steps.
+  const int n_both = max(0, min(n_end[0], n_end[1]) - j0);
+  auto turn_of = [&](int i, int t) { return i < n_both ? 2 * i + t : n_both + i; };
 
   if (warp < kSoftmaxWarps) {
     // Q tiles: each softmax thread copies its share (a warp covers whole 128-byte rows); rows past the
@@ -249,71 +260,93 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       bring(j, page, &map_v, sV + vs * kKvBytes, bar(kBarVFull + vs), true);
       copies_v = jj + 1;
     }
-  } else if (warp == kIssueWarp) {
-    // ---- one thread issues the products (a lone thread runs an instruction every few clocks: its code is kept short) ----
-    if (lane == 0 && j0 < j1) {
-      const uint64_t dq[2] = {make_desc(sQ), make_desc(sQ + kQBytes)};
-      const uint64_t dk0 = make_desc(sK), dv0 = make_desc(sV);
-      const uint32_t d_s[2] = {tmem + kColS, tmem + kColS + BN}, d_o[2] = {tmem + kColO, tmem + kColO + HD},
-                     a_p[2] = {tmem + kColP, tmem + kColP + BN / 2};
-      bool ok = true;
-      auto issue_s = [&](int t, int j) {                // S_t(j) = Q_t K(j)^T
-        const uint64_t dk = dk0 + (uint64_t)(((j - j0) & (kKStages - 1)) * (kKvBytes >> 4));
-#pragma unroll
-        for (int k = 0; k < HD / 16; ++k) mma_bf16(d_s[t], dq[t] + 2 * k, dk + 2 * k, kIdescS, k > 0);
-        mma_commit(bar(kBarSFull + t));
-      };
-      auto issue_pv = [&](int t, int j) {               // O_t += P_t(j) V(j): 16 keys per step, 8 columns of P, 2048 bytes of V
-        const uint64_t dv = dv0 + (uint64_t)(((j - j0) & (kVStages - 1)) * (kKvBytes >> 4));
-        if (j < n_kv - 1) {
-#pragma unroll
-          for (int k = 0; k < BN / 16; ++k)
-            mma_bf16_a_tmem(d_o[t], a_p[t] + k * 8, dv + (uint64_t)(k * (2048 >> 4)), kIdescO, (j > j0 || k > 0) ? 1u : 0u);
-        } else {
-          for (int k = 0; k < ksteps_last; ++k)
-            mma_bf16_a_tmem(d_o[t], a_p[t] + k * 8, dv + (uint64_t)(k * (2048 >> 4)), kIdescO, (j > j0 || k > 0) ? 1u : 0u);
-        }
-        mma_commit(bar(kBarPvDone + t));
-      };
-      ok = mbar_wait_or_abort(bar(kBarKFull + 0), 0, s_abort);
-      if (ok) {
-        if (j0 < n_end[0]) issue_s(0, j0);
-        if (j0 < n_end[1]) issue_s(1, j0);
-        mma_commit(bar(kBarKEmpty + 0));
-      }
-      for (int j = j0; j < j1 && ok; ++j) {
-        const int jj = j - j0;
-        for (int t = 0; t < 2 && ok; ++t) {
-          if (j >= n_end[t]) continue;
-          ok = mbar_wait_or_abort(bar(kBarPFull + t), jj & 1, s_abort);   // P_t(j) is written and S_t(j) has been read
-          if (!ok) break;
+  } else if (warp >= kIssueWarp) {
+    // ---- a warp per query tile; one elected lane issues, with what a product takes in uniform registers (a lone lane takes about
+    // 150 clocks a product to make its descriptors).  Whatever is ready first goes first: the scores of the next step, when their
+    // place and their keys are there, or P V of this one.
+    const bool elected = elect_one();
+    const int t = __shfl_sync(0xffffffffu, warp - kIssueWarp, 0), n = __shfl_sync(0xffffffffu, max(0, n_end[t] - j0), 0);
+    const int n_copied = __shfl_sync(0xffffffffu, max(0, j1 - j0), 0), n_rest = __shfl_sync(0xffffffffu, n_kv - j0, 0);
+    const int steps_last = __shfl_sync(0xffffffffu, ksteps_last, 0);
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), d_o = tm + kColO + t * HD;
+    const uint64_t dq = make_desc(sQ + t * kQBytes), dk0 = make_desc(sK), dv0 = make_desc(sV);
+    auto ready = [&](int which, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test(bar(which), parity)) != 0; };
+    bool ok = true;
+    uint32_t polls = 0;
+    int i_s = 0, i_pv = 0;                              // the next step whose scores, whose P V are to be issued
+    while (i_pv < n) {
+      bool idle = true;
+      if (i_s < n && i_s <= i_pv + 1) {                 // S_t = Q_t K^T; the key tile is free again behind it
+        const int u = turn_of(i_s, t), place = u % 3, st = i_s & (kKStages - 1);
+        // The place is free behind P V of turn u - 3.  (A test of its barrier means that turn only once turn u - 6 is done: while
+        // the groups alternate that is this tile's step i_s - 3, which P of step i_s - 1 implies, and else is looked at here.)
+        const bool early = i_s >= 3 && i_pv < i_s && !ready(kBarPvTile + 2 * t + ((i_s - 3) & 1), ((i_s - 3) >> 1) & 1);
+        if (!early && ready(kBarKFull + st, (i_s / kKStages) & 1) && (u < 3 || ready(kBarPvPlace + place, ((u / 3) - 1) & 1))) {
           fence_after_sync();
-          if (j + 1 < n_end[t]) {
-            const bool first_user = (t == 0) || (j + 1 >= n_end[0]);
-            const bool last_user = (t == 1) || (j + 1 >= n_end[1]);
-            if (first_user) ok = mbar_wait_or_abort(bar(kBarKFull + ((jj + 1) & (kKStages - 1))), ((jj + 1) / kKStages) & 1, s_abort);
-            if (!ok) break;
-            issue_s(t, j + 1);
-            if (last_user) mma_commit(bar(kBarKEmpty + ((jj + 1) & (kKStages - 1))));
+          const uint64_t dk = dk0 + (uint64_t)(st * (kKvBytes >> 4));
+          const uint32_t d_s = tm + place * BN;
+          if (elected) {
+#pragma unroll
+            for (int k = 0; k < HD / 16; ++k) mma_bf16(d_s, dq + 2 * k, dk + 2 * k, kIdescS, k > 0);
+            mma_commit(bar(kBarSFull + 2 * t + (i_s & 1)));
+            mma_commit(bar(kBarKEmpty + st));
           }
-          const bool first_user = (t == 0) || (j >= n_end[0]);
-          const bool last_user = (t == 1) || (j >= n_end[1]);
-          if (first_user) {
-            ok = mbar_wait_or_abort(bar(kBarVFull + (jj & (kVStages - 1))), (jj / kVStages) & 1, s_abort);
-            if (!ok) break;
-            if (j == n_kv - 1) {
-              // Rows behind the last key may hold anything (unwritten slots of the page, an earlier tile):
-              // their P is zero, but 0 * NaN would spoil the product, so they are made zero.
-              uint8_t* v_tile = smem + (sV - base) + (jj & (kVStages - 1)) * kKvBytes;
-              for (int idx = 0; idx < (ksteps_last * 16 - valid_last) * 8; ++idx)
-                *reinterpret_cast<uint4*>(v_tile + swz(valid_last + (idx >> 3), idx & 7)) = make_uint4(0, 0, 0, 0);
-              fence_async_proxy();
+          __syncwarp();
+          ++i_s;
+          idle = false;
+        }
+      }
+      if (i_pv < i_s) {                                 // O_t += P_t V: 16 keys per step, 8 columns of P, 2048 bytes of V
+        const int u = turn_of(i_pv, t), place = u % 3, st = i_pv & (kVStages - 1);
+        if (ready(kBarPFull + 2 * t + (i_pv & 1), (i_pv >> 1) & 1) && ready(kBarVFull + st, (i_pv / kVStages) & 1)) {
+          fence_after_sync();
+          const uint64_t dv = dv0 + (uint64_t)(st * (kKvBytes >> 4));
+          const uint32_t a_p = tm + place * BN, more = i_pv > 0 ? 1u : 0u;
+          if (i_pv < n_rest - 1) {
+            if (elected) {
+#pragma unroll
+              for (int k = 0; k < BN / 16; ++k) mma_bf16_a_tmem(d_o, a_p + k * 8, dv + (uint64_t)(k * (2048 >> 4)), kIdescO, k > 0 ? 1u : more);
+            }
+          } else {
+            // Rows behind the last key may hold anything (unwritten slots of the page, an earlier tile): their P is zero, but 0 * NaN
+            // would spoil the product, so they are made zero up to the last step's (by both warps, whichever comes first).
+            uint8_t* v_tile = smem + (sV - base) + st * kKvBytes;
+            for (int idx = lane; idx < (steps_last * 16 - valid_last) * 8; idx += 32)
+              *reinterpret_cast<uint4*>(v_tile + swz(valid_last + (idx >> 3), idx & 7)) = make_uint4(0, 0, 0, 0);
+            fence_async_proxy();
+            __syncwarp();
+            if (elected) {
+              for (int k = 0; k < steps_last; ++k) mma_bf16_a_tmem(d_o, a_p + k * 8, dv + (uint64_t)(k * (2048 >> 4)), kIdescO, k > 0 ? 1u : more);
             }
           }
-          issue_pv(t, j);
-          if (last_user) mma_commit(bar(kBarVEmpty + (jj & (kVStages - 1))));
+          if (elected) {
+            mma_commit(bar(kBarPvPlace + place));
+            mma_commit(bar(kBarPvTile + 2 * t + (i_pv & 1)));
+            mma_commit(bar(kBarVEmpty + st));
+          }
+          __syncwarp();
+          ++i_pv;
+          idle = false;
         }
       }
+      polls = idle ? polls + 1 : 0;
+      if (idle && __any_sync(0xffffffffu, *s_abort != 0 || polls > kSpinLimit)) {
+        if (lane == 0) *s_abort = 1;
+        ok = false;
+        break;
+      }
+    }
+    // tiles that only the other query tile uses are free for this one (each once it is there: the copies' phases stay in step)
+    auto wait = [&](int which, uint32_t parity) {
+      if (ok) ok = mbar_wait_or_abort(bar(which), parity, s_abort);
+      ok = __all_sync(0xffffffffu, ok) != 0;
+    };
+    for (int i = n; i < n_copied && ok; ++i) {
+      const int ks = i & (kKStages - 1), vs = i & (kVStages - 1);
+      wait(kBarKFull + ks, (i / kKStages) & 1);
+      if (ok && lane == 0) mbar_arrive(bar(kBarKEmpty + ks));
+      wait(kBarVFull + vs, (i / kVStages) & 1);
+      if (ok && lane == 0) mbar_arrive(bar(kBarVEmpty + vs));
     }
   } else {
     // ---- the softmax groups: two threads per query row, each with 64 of a tile's 128 keys ----
@@ -323,8 +356,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     const int row = quarter * 32 + lane;
     const int my_pos = pos0 + t * BM + row;
     const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16);      // this warp's 32 lanes of TMEM
-    const uint32_t t_s = t_lane + kColS + t * BN + half * 64, t_o = t_lane + kColO + t * HD + half * 32;
-    const uint32_t t_p = t_lane + kColP + t * (BN / 2) + half * 32;
+    const uint32_t t_o = t_lane + kColO + t * HD + half * 32;
     const int pair_barrier = 1 + t * 4 + quarter;                         // the two warps that share these rows
     float* mine = exchange + (t * BM + row) * 2 + half;
     const float* partners = exchange + (t * BM + row) * 2 + (half ^ 1);
@@ -338,9 +370,11 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     const float pen_r1 = PEN ? penalty[h] : 0.f, pen_r2 = PEN ? penalty[nq + h] : 0.f;
     auto hidden = [&](int key) { return key > my_pos || (key < win_lo && key >= keep_first); };
     for (int j = j0; j < n_end[t]; ++j) {
-      wait(kBarSFull + t, (j - j0) & 1);
+      const int place = turn_of(j - j0, t) % 3;
+      wait(kBarSFull + 2 * t + ((j - j0) & 1), ((j - j0) >> 1) & 1);
       if (!ok) break;
       fence_after_sync();
+      const uint32_t t_s = t_lane + place * BN + half * 64;
       const int tile_key0 = tile_of(j) * BN, key0 = tile_key0 + half * 64;
       // 1 + r2 * (distance to this thread's first key of the tile); the keys after it are r2 less each (a key behind the
       // row's own is masked: its logarithm, which may be no number, is never used)
@@ -388,7 +422,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           l_run *= alpha;
           if (j > j0) {
             // O is rescaled in TMEM: P V of tile j-1 must have landed first
-            wait(kBarPvDone + t, (j - 1 - j0) & 1);
+            wait(kBarPvTile + 2 * t + ((j - 1 - j0) & 1), ((j - 1 - j0) >> 1) & 1);
             if (!ok) break;
             fence_after_sync();
             float acc[32];
@@ -400,9 +434,8 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           }
         }
         float l4[4] = {0.f, 0.f, 0.f, 0.f};
-        // 16 keys at a time; the scores of the next 16 are on their way from TMEM while these are
-        // exponentiated.  P is collected in registers and stored once at the end, so that the wait for the
-        // second product of the tile before (whose P these stores overwrite) comes as late as possible.
+        // 16 keys at a time; the scores of the next 16 are on their way from TMEM while these are exponentiated.  P is collected in
+        // registers and stored once at the end, in the scores' place.
         float s[2][16];
         tmem_ld16(t_s, s[0]);
 #pragma unroll
@@ -464,23 +497,18 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           }
         }
         l_tile = (l4[0] + l4[1]) + (l4[2] + l4[3]);
-        // both threads of a row have to agree on the reference: the two warps decide together
-        if (search || !named_barrier_any(pair_barrier, 64, !(l_tile < kSumLimit))) break;
+        // both threads of a row have to agree on the reference: the two warps decide together (and behind this barrier both have
+        // read their scores, whose place P takes)
+        if (!named_barrier_any(pair_barrier, 64, !search && !(l_tile < kSumLimit))) break;
         search = true;
       }
       if (!ok) break;
-      if (j > j0) {
-        // P V of tile j-1 has to be done before its P is overwritten
-        wait(kBarPvDone + t, (j - 1 - j0) & 1);
-        if (!ok) break;
-        fence_after_sync();
-      }
-      tmem_st32(t_p, reinterpret_cast<const float*>(packed));
+      tmem_st32(t_lane + place * BN + half * 32, reinterpret_cast<const float*>(packed));
       tmem_st_wait();
       l_run += l_tile;
       fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(kBarPFull + t));
+      if (lane == 0) mbar_arrive(bar(kBarPFull + 2 * t + ((j - j0) & 1)));
     }
     // where this row's share of a split goes: [token][head][split] records of HD floats, and of (maximum, sum)
     const size_t record = ((size_t)(q0 + t * BM + row) * nq + h) * key_splits + blockIdx.z;
@@ -488,7 +516,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       // nothing of this range is visible to this query tile: an empty record for the merge
       if (key_splits > 1 && half == 0 && row < rows_t[t]) { part_ml[record * 2] = -INFINITY; part_ml[record * 2 + 1] = 0.f; }
     } else {
-      wait(kBarPvDone + t, (n_end[t] - 1 - j0) & 1);
+      wait(kBarPvTile + 2 * t + ((n_end[t] - 1 - j0) & 1), ((n_end[t] - 1 - j0) >> 1) & 1);
       fence_after_sync();
       mine[2 * 2 * BM] = l_run;                          // (a slot of its own: the partner may still be reading a maximum)
       named_barrier(pair_barrier, 64);
