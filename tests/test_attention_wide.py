@@ -119,3 +119,42 @@ def test_latent_portions_over_rows(dim, rot, v, rank, lens, past, page, window):
             want = weight @ value * torch.sigmoid(gate[t, h].double())[:, None]
             assert ((out[t, h].double() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -13 * value.abs().max()).all(), (s, h)
         at += length
+
+
+@pytest.mark.parametrize("lens", [[127], [128], [3, 1, 2, 130], [1] * 129])
+@pytest.mark.parametrize("rot_dims", [0, 32])
+def test_differential_rows_by_eight_channels(lens, rot_dims):
+    """The convolution, rotation and cache write around the line between the kernels (128 tokens), against float64: float sums of four
+    terms, turned in float, rounded once to bfloat16 (2^-8 of the value; angles of up to 200 in float: 2^-16 of the channel's size)."""
+    from edgerag_b200.ops import kernels
+
+    H, G, d, dv, page, n = 2, 1, 32, 24, 16, sum(lens)
+    channels = (H + G) * 2 * d + G * dv
+    g = torch.Generator().manual_seed(n + rot_dims)
+    rand = lambda *shape: torch.randn(*shape, generator=g)      # noqa: E731
+    proj, weight, record = rand(n, channels + 4).to(torch.bfloat16).cuda(), (0.4 * rand(channels, 4)).cuda(), rand(len(lens) + 1, 3, channels).cuda()
+    starts = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32).cuda()
+    seq = torch.tensor([s for s, length in enumerate(lens) for _ in range(length)], dtype=torch.int32).cuda()
+    positions = torch.cat([torch.arange(70, 70 + length) for length in lens]).int().cuda()
+    held, slots = torch.arange(len(lens), 0, -1, dtype=torch.int32).cuda(), torch.randperm(n + 8, generator=g)[:n].int()
+    slots[n // 2] = -1
+    k_pages = torch.zeros((n + 8) // page + 1, G, page, 2 * d, dtype=torch.bfloat16, device="cuda")
+    v_pages = torch.zeros(k_pages.shape[0], G, page, dv, dtype=torch.bfloat16, device="cuda")
+    q = torch.empty(n, H * 2 * d, dtype=torch.bfloat16, device="cuda")
+    freq = (1000.0 ** (-torch.arange(d // 2) / (d // 2))).float().cuda()
+    kernels.diff_prepare(proj, q, positions, H, G, d, dv, inv_freq=freq if rot_dims else None, rot_dims=rot_dims, conv_w=weight, conv_state=record,
+                         seq_of_token=seq, seq_starts=starts, state_slots=held, slots=slots.cuda(), k_pages=k_pages, v_pages=v_pages, page_size=page)
+    want = torch.cat([sum(torch.cat([record[held[s]].double(), proj[starts[s]: starts[s + 1], :channels].double()], 0)[j: j + length] * weight[:, j].double()
+                          for j in range(4)) for s, length in enumerate(lens)], 0)
+    maps = want[:, : (H + G) * 2 * d].reshape(n, -1, d)
+    if rot_dims:
+        a = (positions.double()[:, None] * freq.double())[:, None]
+        lo, hi = maps[..., : d // 2], maps[..., d // 2:]
+        maps = torch.cat([lo * a.cos() - hi * a.sin(), hi * a.cos() + lo * a.sin()], -1)
+    close = lambda got, exact: ((got.double() - exact).abs() <= exact.abs() * 2.0 ** -8 + 2.0 ** -14).all()      # noqa: E731
+    maps = maps.reshape(n, -1)
+    assert close(q, maps[:, : H * 2 * d])
+    kept = slots >= 0
+    at = slots[kept].long().cuda()
+    assert close(k_pages[at // page, 0, at % page], maps[kept.cuda(), H * 2 * d:]) and close(v_pages[at // page, 0, at % page], want[kept.cuda(), -dv:])
+    assert int((k_pages.abs().sum(-1) > 0).sum()) == int(kept.sum())
