@@ -188,54 +188,161 @@ moe_route_kernel(const T* __restrict__ x, int ld, const float* __restrict__ w_ro
                  normalise, weight);
 }
 
+#if ERB_ELEM == 1
+// Many tokens, rows of a multiple of 128 entries: a block takes kRouteMany tokens and a warp four experts at a time for half of them,
+// so that a router row is read once for eight tokens and a token's entries (kept as bfloat16 in shared memory) once for four experts.
+// Every sum is made in the order of moe_route_kernel: the same bits.  Bound by the reads of shared memory and the multiplications, about
+// alike.  2,048 tokens, 32 experts, rows of 2,048: 36 us by the kernel above, which read the whole router matrix for four
+// tokens, 21 here.  From 1,024 tokens: the router of 32 experts and the lists take 16.2 us above and 22.4 here for 512 tokens, 22.8 and
+// 24.9 here for 1,024 and 2,048 (58.7 above, with the earlier lists); a router of 160 experts 43 above and 67 here for 512, 68 and 74
+// here for 1,024 and 2,048 (87 and 171 above, with the earlier lists).  A block's time hardly depends on their number until every SM has one.
+constexpr int kRouteMany = 16, kRouteManyFrom = 1024;
+__global__ void __launch_bounds__(kRouteThreads, 1)
+moe_route_many_kernel(const __nv_bfloat16* __restrict__ x, int ld, const float* __restrict__ w_router, int n_tokens, int width, int n_experts,
+                      int top, int* __restrict__ choice, float* __restrict__ score, int score_kind, int n_groups, int keep_groups,
+                      const float* __restrict__ correction, int group_kind, int normalise, float weight, float* __restrict__ side_gate) {
+  chain_wait();
+  const int n_rows = n_experts + (side_gate != nullptr), e_pad = (n_rows + 3) & ~3;
+  extern __shared__ __align__(16) float z_s[];   // as in moe_route_kernel, then [kRouteMany][width] bfloat16
+  float* g_s = z_s + kRouteMany * e_pad;
+  float* c_s = g_s + kRouteMany * e_pad;
+  __nv_bfloat16* x_s = reinterpret_cast<__nv_bfloat16*>(c_s + kRouteMany * e_pad);
+  const int t0 = blockIdx.x * kRouteMany, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n_here = min(kRouteMany, n_tokens - t0), pieces = width / 8;
+  for (int idx = threadIdx.x; idx < kRouteMany * pieces; idx += kRouteThreads) {
+    const int j = idx / pieces, c = idx - j * pieces;
+    reinterpret_cast<uint4*>(x_s)[idx] = *reinterpret_cast<const uint4*>(x + (size_t)(t0 + min(j, n_here - 1)) * ld + 8 * c);
+  }
+  __syncthreads();
+  constexpr int kE = 4, kT = kRouteMany / 2;     // a warp's experts and tokens at a time
+  const int j0 = (warp & 1) * kT;
+  for (int e = kE * (warp >> 1); e < n_rows; e += kE * (kRouteThreads / 64)) {
+    const float* w[kE];
+    float acc[kE][kT];
+#pragma unroll
+    for (int i = 0; i < kE; ++i) {
+      w[i] = w_router + (size_t)min(e + i, n_rows - 1) * width;
+#pragma unroll
+      for (int j = 0; j < kT; ++j) acc[i][j] = 0.f;
+    }
+    float4 next[kE];
+#pragma unroll
+    for (int i = 0; i < kE; ++i) next[i] = *reinterpret_cast<const float4*>(w[i] + 4 * lane);
+    for (int k = 4 * lane; k < width; k += 128) {
+      float4 u[kE];
+#pragma unroll
+      for (int i = 0; i < kE; ++i) {
+        u[i] = next[i];
+        if (k + 128 < width) next[i] = *reinterpret_cast<const float4*>(w[i] + k + 128);     // (on its way while these are multiplied)
+      }
+#pragma unroll
+      for (int j = 0; j < kT; ++j) {
+        float xv[4];
+        Pack4<__nv_bfloat16>::load(x_s + (j0 + j) * width + k, xv);
+#pragma unroll
+        for (int i = 0; i < kE; ++i) {
+          acc[i][j] = fmaf(xv[0], u[i].x, acc[i][j]);
+          acc[i][j] = fmaf(xv[1], u[i].y, acc[i][j]);
+          acc[i][j] = fmaf(xv[2], u[i].z, acc[i][j]);
+          acc[i][j] = fmaf(xv[3], u[i].w, acc[i][j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kE; ++i)
+#pragma unroll
+      for (int j = 0; j < kT; ++j) {
+        const float total = warp_sum(acc[i][j]);
+        if (lane == 0 && e + i < n_rows) z_s[(j0 + j) * e_pad + e + i] = total;
+      }
+  }
+  __syncthreads();
+  if (warp >= n_here) return;
+  const int t = t0 + warp;
+  float* z = z_s + warp * e_pad;
+  if (side_gate && lane == 0) side_gate[t] = 1.f / (1.f + expf(-z[n_experts]));
+  choose_experts(z, reinterpret_cast<unsigned*>(c_s) + warp * e_pad, reinterpret_cast<unsigned*>(g_s) + warp * e_pad, n_experts, top,
+                 choice + (size_t)t * top, score + (size_t)t * top, nullptr, score_kind, n_groups, keep_groups, correction, group_kind,
+                 normalise, weight);
+}
+static_assert(kRouteMany == kRouteThreads / 32, "a warp per token picks");
+#endif
+
 // One block per expert e builds the expert's part of the lists on its own: a histogram of all choices in shared memory
 // gives offsets[e] (the pairs of the experts before e) and tiles[e] (their row tiles of `tile_rows` rows); then the pairs
 // that chose e are written behind the offset in rising order.  The last block also writes the totals at [n_experts].
-__global__ void __launch_bounds__(256) moe_lists_kernel(const int* __restrict__ choice, int n_pairs, int n_experts, int tile_rows,
-                                                        int* __restrict__ counts, int* __restrict__ offsets,
-                                                        int* __restrict__ tiles, int* __restrict__ order) {
+// A thread owns one run of consecutive pairs: it counts its own e while it adds to the histogram (with a copy of the histogram per
+// warp, so that warps do not queue for its words), a scan over the threads gives its place, and it walks its run once more.
+// (A walk of all pairs 256 at a time with three barriers each took 22 us for 8,192 pairs of 32 experts; this takes 4.)
+constexpr int kListThreads = 512;
+__global__ void __launch_bounds__(kListThreads) moe_lists_kernel(const int* __restrict__ choice, int n_pairs, int n_experts, int tile_rows, int copies,
+                                                                 int* __restrict__ counts, int* __restrict__ offsets,
+                                                                 int* __restrict__ tiles, int* __restrict__ order) {
   chain_wait();
-  extern __shared__ int hist[];                  // [n_experts]
-  __shared__ int warp_counts[8];
+  extern __shared__ int hist[];                  // [copies][n_experts]
+  __shared__ int warp_sums[kListThreads / 32];
   __shared__ int base_s;
   const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < n_experts; i += blockDim.x) hist[i] = 0;
+  for (int i = threadIdx.x; i < copies * n_experts; i += kListThreads) hist[i] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) atomicAdd(&hist[choice[i]], 1);
+  // runs of a multiple of four pairs, so that they are read 16 bytes at a time (the tail of the last one singly)
+  const int per = ((n_pairs + kListThreads - 1) / kListThreads + 3) & ~3;
+  const int begin = min(n_pairs, (int)threadIdx.x * per), end = min(n_pairs, begin + per), whole = begin + ((end - begin) & ~3);
+  int* mine = hist + (warp % copies) * n_experts;
+  int own = 0;
+  const bool wide = ((uintptr_t)choice & 15) == 0;
+  auto each = [&](auto f) {
+    int i = begin;
+    if (wide)
+      for (; i < whole; i += 4) {
+        const int4 c = *reinterpret_cast<const int4*>(choice + i);
+        f(i, c.x); f(i + 1, c.y); f(i + 2, c.z); f(i + 3, c.w);
+      }
+    for (; i < end; ++i) f(i, choice[i]);
+  };
+  each([&](int, int c) { atomicAdd(&mine[c], 1); own += c == e; });
+  // the threads' counts before this one
+  int before = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += v;
+  }
+  if (lane == 31) warp_sums[warp] = before;
+  before -= own;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int off = 0, tl = 0;
-    for (int i = 0; i < e; ++i) {
-      off += hist[i];
-      tl += (hist[i] + tile_rows - 1) / tile_rows;
+  for (int w = 0; w < warp; ++w) before += warp_sums[w];
+  // the experts before this one: a warp adds them up
+  if (warp == 0) {
+    int off = 0, tl = 0, here = 0;
+    for (int i = lane; i <= e; i += 32) {
+      int n = 0;
+      for (int c = 0; c < copies; ++c) n += hist[c * n_experts + i];
+      if (i < e) { off += n; tl += (n + tile_rows - 1) / tile_rows; }
+      else here = n;
     }
-    counts[e] = hist[e];
-    offsets[e] = off;
-    tiles[e] = tl;
-    base_s = off;
-    if (e == n_experts - 1) {
-      offsets[n_experts] = off + hist[e];
-      tiles[n_experts] = tl + (hist[e] + tile_rows - 1) / tile_rows;
-      counts[n_experts] = 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, o);
+      tl += __shfl_xor_sync(0xffffffffu, tl, o);
+      here += __shfl_xor_sync(0xffffffffu, here, o);
+    }
+    if (lane == 0) {
+      counts[e] = here;
+      offsets[e] = off;
+      tiles[e] = tl;
+      base_s = off;
+      if (e == n_experts - 1) {
+        offsets[n_experts] = off + here;
+        tiles[n_experts] = tl + (here + tile_rows - 1) / tile_rows;
+        counts[n_experts] = 0;
+      }
     }
   }
   __syncthreads();
-  for (int i0 = 0; i0 < n_pairs; i0 += 256) {
-    const int i = i0 + threadIdx.x;
-    const bool mine = i < n_pairs && choice[i] == e;
-    const unsigned ballot = __ballot_sync(0xffffffffu, mine);
-    if (lane == 0) warp_counts[warp] = __popc(ballot);
-    __syncthreads();
-    int before = 0;
-    for (int w = 0; w < warp; ++w) before += warp_counts[w];
-    if (mine) order[base_s + before + __popc(ballot & ((1u << lane) - 1))] = i;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int all = 0;
-      for (int w = 0; w < 8; ++w) all += warp_counts[w];
-      base_s += all;
-    }
-    __syncthreads();
+  if (own) {
+    int at = base_s + before;
+    each([&](int i, int c) { if (c == e) order[at++] = i; });
   }
 }
 
@@ -499,18 +606,33 @@ ERB_EXPORT int erb_moe_route(const void* x, int ld, const float* w_router, int n
     return check_launch("moe_choose_lists");
   }
   const size_t route_smem = sizeof(float) * kRouteTokens * (3 * (size_t)((n_rows + 3) & ~3) + width);
-  if (route_smem > 48 * 1024) {
+  bool routed = false;
+  int rc = ERB_OK;
+#if ERB_ELEM == 1
+  const size_t many_smem = sizeof(float) * kRouteMany * 3 * (size_t)((n_rows + 3) & ~3) + sizeof(elem_t) * kRouteMany * (size_t)width;
+  if (n_tokens >= kRouteManyFrom && width % 128 == 0 && ld % 8 == 0 && !(((uintptr_t)x | (uintptr_t)w_router) & 15) && many_smem <= 200 * 1024) {
+    cudaError_t err = cudaFuncSetAttribute(moe_route_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)many_smem);
+    if (err != cudaSuccess) return fail(ERB_ERR_CUDA, "moe_route: %s", cudaGetErrorString(err));
+    launch_chained(moe_route_many_kernel, dim3((n_tokens + kRouteMany - 1) / kRouteMany), dim3(kRouteThreads), many_smem, s, (const elem_t*)x,
+                   ld, w_router, n_tokens, width, n_experts, top, choice, score, score_kind, n_groups, keep_groups, correction, group_kind,
+                   normalise, weight, side_gate);
+    if ((rc = check_launch("moe_route"))) return rc;
+    routed = true;
+  }
+#endif
+  if (!routed && route_smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(moe_route_kernel<elem_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)route_smem);
     if (err != cudaSuccess) return fail(ERB_ERR_CUDA, "moe_route: %s", cudaGetErrorString(err));
   }
-  if (route_smem > 200 * 1024) return fail(ERB_ERR_UNSUPPORTED, "moe_route: rows of %d entries with %d experts", width, n_experts);
-  launch_chained(moe_route_kernel<elem_t>, dim3((n_tokens + kRouteTokens - 1) / kRouteTokens), dim3(kRouteThreads), route_smem, s,
+  if (!routed && route_smem > 200 * 1024) return fail(ERB_ERR_UNSUPPORTED, "moe_route: rows of %d entries with %d experts", width, n_experts);
+  if (!routed) launch_chained(moe_route_kernel<elem_t>, dim3((n_tokens + kRouteTokens - 1) / kRouteTokens), dim3(kRouteThreads), route_smem, s,
                  (const elem_t*)x, ld, w_router, n_tokens, width, n_experts, top, choice, score, score_kind, n_groups, keep_groups,
                  correction, group_kind, normalise, weight, side_gate);
-  int rc = check_launch("moe_route");
+  rc = check_launch("moe_route");
   if (rc) return rc;
-  launch_chained(moe_lists_kernel, dim3(n_experts), dim3(256), sizeof(int) * n_experts, s, (const int*)choice, n_pairs, n_experts,
-                 tile_rows > 0 ? tile_rows : kTM, counts, offsets, tiles, order);
+  const int copies = n_experts <= 512 ? kListThreads / 32 : 1;
+  launch_chained(moe_lists_kernel, dim3(n_experts), dim3(kListThreads), sizeof(int) * copies * n_experts, s, (const int*)choice, n_pairs,
+                 n_experts, tile_rows > 0 ? tile_rows : kTM, copies, counts, offsets, tiles, order);
   return check_launch("moe_lists");
 }
 
