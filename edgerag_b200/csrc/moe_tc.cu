@@ -8,9 +8,9 @@
 //               xs[list row] = round(score * x[token]), so that both products read their rows as plain 2-d tiles
 //   warp 0      one thread brings tiles of the weight (2 x 128 rows x 64 k) and of the rows (MT x 64 k) into
 //               128-byte-swizzled shared memory with TMA tensor copies, five stages deep (tiles of 128 rows: two, and two
-//               blocks share an SM)
-//   warp 1      one thread issues tcgen05.mma with the weight's rows as the M = 128 side and the list's rows as the N side,
-//               once per accumulator; the accumulators are 2 x MT columns of TMEM
+//               blocks share an SM; of 256: three)
+//   warp 1      one thread issues tcgen05.mma with the weight's rows as the M = 128 side and the list's rows as the N side
+//               (as many, up to a multiple of 16, as the tile holds), once per accumulator; the accumulators are 2 x MT columns of TMEM
 //   all warps   read the accumulators (a thread = a row of the weight in each) and finish from registers:
 //               gate/up: the first accumulator holds 128 gate rows, the second the 128 up rows that go with them:
 //                        act[list row][column] = silu(gate) * up;
@@ -19,10 +19,15 @@
 //                        (not its input) carries the weight;
 //               single:  one product without a gate branch, act[list row][column] = relu(sum)^2 for both accumulators
 //
-// A tile's rows past the end of its expert's list are rows of the next expert (or nothing): they are multiplied along and
+// A tile's rows past the end of its expert's list are rows of the next expert (or nothing): at most 15 are multiplied along and
 // never stored.  A tile of weight rows past the expert's last row reads the next expert's rows: not stored either.  k is
 // walked in one order whatever tile a row falls into, and a row is a column of the accumulator that no other row touches,
 // so a token's result does not depend on the other tokens of the step.
+//
+// Large tiles are bound by shared memory: 128 weight rows times 128 list rows read as many bytes for each k as they take clocks, and
+// the copies come on top; with 256 list rows the weight is read once for twice the products.  2,048 tokens, 4 of 32 experts, rows of
+// 2,048 and 1,024 within (about 256 pairs an expert, half of the experts with a short second tile): gate/up 107 us in tiles of 128, 91
+// in tiles of 256 (753 Tflop/s of the pairs' own work), down 63 and 55.
 //
 // Every wait is bounded; a thread that gives up raises a block-wide flag, the block lets its copies land, records
 // 5000000 + block in *status (if given), frees its TMEM and writes nothing.
@@ -41,14 +46,16 @@ namespace {
 
 constexpr int kTileN = 128;              // rows of the weight per block (the M side of the instruction)
 constexpr int kTileK = 64;               // k per stage: one 128-byte swizzle span
-constexpr int kThreads = 128;
 constexpr uint32_t kWBytes = kTileN * kTileK * 2;      // 16 KB
 
 template <int MT> struct Plan {
   static constexpr uint32_t kABytes = MT * kTileK * 2;
   static constexpr uint32_t kStageBytes = 2 * kWBytes + kABytes;
-  // tiles of 128 rows: two stages a block, so that two blocks share an SM and one's epilogue runs under the other's products
-  static constexpr int kStages = MT >= 128 ? 2 : 5;
+  // tiles of 128 rows: two stages a block, so that two blocks share an SM and one's epilogue runs under the other's products; tiles of
+  // 256 rows take all columns of TMEM, so that a block has its SM to itself: three stages, and eight warps to finish
+  static constexpr int kStages = MT >= 256 ? 3 : MT >= 128 ? 2 : 5;
+  static constexpr int kThreads = MT >= 256 ? 256 : 128;
+  static constexpr int kBoxRows = MT < 64 ? MT : 64;          // the list's rows come in boxes of this many, only those that hold some
   static constexpr uint32_t kSmemBytes = kStages * kStageBytes + 1024;
   static constexpr uint32_t kTmemCols = 2 * MT < 32 ? 32 : 2 * MT;
 };
@@ -84,14 +91,14 @@ moe_gather_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int* __res
 // gate rows and then n_out up rows, a tile takes 128 of each; else it takes 256 neighbouring rows.
 constexpr int kDown = 0, kGated = 1, kSingle = 2;
 template <int MT, int MODE>
-__global__ void __launch_bounds__(kThreads, MT >= 128 ? 2 : 1)
+__global__ void __launch_bounds__(Plan<MT>::kThreads, MT == 128 ? 2 : 1)
 moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
               const int* __restrict__ offsets, const int* __restrict__ tiles, const int* __restrict__ order, int n_experts,
               int top, int n_tokens, int n_out, int K, __nv_bfloat16* __restrict__ act, float* __restrict__ parts,
               const float* __restrict__ out_score, int* __restrict__ status) {
   constexpr bool GATED = MODE == kGated, PAIRS = MODE == kDown;
   using P = Plan<MT>;
-  constexpr int kStages = P::kStages;
+  constexpr int kStages = P::kStages, kThreads = P::kThreads;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * kStages + 1];      // full, empty, accumulator done
   __shared__ int s_abort;
@@ -120,14 +127,16 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   const int n0 = blockIdx.y * (GATED ? kTileN : 2 * kTileN);    // first output column of this block
   const int w_row0 = e * (GATED ? 2 : 1) * n_out + n0;          // its first row in the stacked weights
   const int n_kb = (K + kTileK - 1) / kTileK;
+  const int boxes = (n_rows + P::kBoxRows - 1) / P::kBoxRows;
 
   auto ask = [&](int i) {
     const int s = i % kStages;
-    mbar_expect(full0 + 8 * s, 2 * kWBytes + P::kABytes);
+    mbar_expect(full0 + 8 * s, 2 * kWBytes + boxes * P::kBoxRows * kTileK * 2);
     const uint32_t dst = base + s * P::kStageBytes;
     tma_load_2d(dst, &map_w, i * kTileK, w_row0, full0 + 8 * s);
     tma_load_2d(dst + kWBytes, &map_w, i * kTileK, w_row0 + (GATED ? n_out : kTileN), full0 + 8 * s);
-    tma_load_2d(dst + 2 * kWBytes, &map_a, i * kTileK, row0, full0 + 8 * s);
+    for (int b = 0; b < boxes; ++b)
+      tma_load_2d(dst + 2 * kWBytes + b * P::kBoxRows * kTileK * 2, &map_a, i * kTileK, row0 + b * P::kBoxRows, full0 + 8 * s);
   };
   const int ahead = min(kStages, n_kb);
   if (tid == 0) {
@@ -164,7 +173,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
       asked = i + 1;
     }
   } else if (warp == 1 && lane == 0) {
-    constexpr uint32_t idesc = mma_idesc(kTileN, MT, false);
+    const uint32_t idesc = mma_idesc(kTileN, (n_rows + 15) & ~15, false);   // (a short tile multiplies its own rows only)
     bool ok = true;
     for (int i = 0; i < n_kb && ok; ++i) {
       const int s = i % kStages;
@@ -199,11 +208,11 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   // ---- finishing, from registers: thread = a row of the weight in each accumulator = an output column ----
   fence_after_sync();
   {
-    const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16);
-    const int n_a = n0 + tid, n_b = n0 + kTileN + tid;          // (gated: one column n_a from both accumulators)
+    const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const int n_a = n0 + (tid & 127), n_b = n_a + kTileN;          // (gated: one column n_a from both accumulators)
 #pragma unroll 1
-    for (int c = 0; c < MT / 16; ++c) {
-      if (16 * c >= n_rows) break;                              // (the same for every thread: the loads are collective)
+    for (int c = tid >> 7; c < MT / 16; c += kThreads / 128) {
+      if (16 * c >= n_rows) break;                              // (the same for every thread of a warp: the loads are collective)
       float v0[16], v1[16];
       tmem_ld16(t_lane + 16 * c, v0);
       tmem_ld16(t_lane + MT + 16 * c, v1);
@@ -275,7 +284,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& ma, const int* offsets, con
   const int per_tile = GATED ? kTileN : 2 * kTileN;
   // an upper bound of the row tiles: every expert's last tile may be short
   const dim3 grid((unsigned)((pairs + MT - 1) / MT + n_experts), (unsigned)((n_out + per_tile - 1) / per_tile));
-  launch_chained(kern, grid, dim3(kThreads), Plan<MT>::kSmemBytes, stream, mw, ma, offsets, tiles, order, n_experts, top, n_tokens,
+  launch_chained(kern, grid, dim3(Plan<MT>::kThreads), Plan<MT>::kSmemBytes, stream, mw, ma, offsets, tiles, order, n_experts, top, n_tokens,
                  n_out, K, (__nv_bfloat16*)act, parts, out_score, status);
   return check_launch("moe_tc");
 }
@@ -292,7 +301,7 @@ int run(const void* a, const void* w, const int* offsets, const int* tiles, cons
   if (pairs > 0x7fffffffLL || w_rows > 0x7fffffffLL) return fail(ERB_ERR_UNSUPPORTED, "moe_tc: too many rows");
   CUtensorMap mw, ma;
   int rc;
-  if ((rc = matrix_map(&mw, w, w_rows, K, K, kTileN)) || (rc = matrix_map(&ma, a, pairs, K, K, tile_rows))) return rc;
+  if ((rc = matrix_map(&mw, w, w_rows, K, K, kTileN)) || (rc = matrix_map(&ma, a, pairs, K, K, tile_rows < 64 ? tile_rows : 64))) return rc;
 #define ERB_MOE_CASE(MT) \
   case MT: return launch<MT, MODE>(mw, ma, offsets, tiles, order, n_experts, top, n_tokens, n_out, K, act, parts, out_score, status, stream);
   switch (tile_rows) {
@@ -300,7 +309,8 @@ int run(const void* a, const void* w, const int* offsets, const int* tiles, cons
     ERB_MOE_CASE(32)
     ERB_MOE_CASE(64)
     ERB_MOE_CASE(128)
-    default: return fail(ERB_ERR_ARG, "moe_tc: tiles of %d rows (takes 16, 32, 64, 128)", tile_rows);
+    ERB_MOE_CASE(256)
+    default: return fail(ERB_ERR_ARG, "moe_tc: tiles of %d rows (takes 16, 32, 64, 128, 256)", tile_rows);
   }
 #undef ERB_MOE_CASE
 }
@@ -322,7 +332,7 @@ ERB_EXPORT int erb_moe_tc_gather(const void* x, int ldx, const int* order, const
 }
 
 // act[list row][ff] = silu(W_gate r) * (W_up r) for the rows r = xs[list row] of every expert's list; w [experts][2 ff][k]
-// (gate rows, then up rows).  tile_rows: what the lists' tile offsets were made for (16, 32, 64 or 128).
+// (gate rows, then up rows).  tile_rows: what the lists' tile offsets were made for (16, 32, 64, 128 or 256).
 ERB_EXPORT int erb_moe_tc_gate_up(const void* xs, const void* w, const int* offsets, const int* tiles, const int* order,
                                   int n_experts, int top, int n_tokens, int ff, int K, int tile_rows, void* act, int* status,
                                   void* stream) {

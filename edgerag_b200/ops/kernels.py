@@ -1630,11 +1630,17 @@ def moe_tc_supported(dtype: torch.dtype, width: int, ff: int) -> bool:
 
 
 def moe_tc_tile_rows(n_tokens: int, n_experts: int, top: int) -> int:
-    """Rows of a tile of the tensor-core products for this many tokens: 16 to 128, the smallest that holds an expert's
+    """Rows of a tile of the tensor-core products for this many tokens: 16 to 256, the smallest that holds an expert's
     even share of the (token, choice) pairs, so that few rows cost few columns of the accumulator and many rows re-read
-    the weight seldom."""
+    the weight seldom.  Beyond a share of 256 tiles of 128 rows again, two of whose blocks run on an SM: the experts' short
+    last tiles then matter less than an SM's idle end (both products, rows of 2,048 and 1,024 within, 128 | 256: 32 experts, shares of
+    130, 138, 200 and 256 119 | 103, 123 | 103, 130 | 118, 166 | 146 us; 16 experts, shares of 138 and 256 64 | 49, 98 | 86; a share
+    of 512 with 16 experts 124 | 130, with 32 and rows of 1,024 and 512 87 | 91, with 8 and rows of 2,048 and 4,096 215 | 224)."""
     share = -(-n_tokens * top // max(1, n_experts))
-    return 16 if share <= 16 else 32 if share <= 32 else 64 if share <= 64 else 128
+    for rows in (16, 32, 64, 128, 256):
+        if share <= rows:
+            return rows
+    return 128
 
 
 def moe_tc_gather(x: torch.Tensor, lists: torch.Tensor, score: torch.Tensor | None, n_experts: int, top: int, xs: torch.Tensor) -> None:

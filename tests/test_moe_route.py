@@ -1,5 +1,5 @@
 """The router over many tokens at once: its choices, weights and side gate against the router over fewer tokens (the same sums in the
-same order, so the same bits) and against float64, and the experts' lists against a count on the host."""
+same order, so the same bits) and against float64, the experts' lists against a count on the host, and the experts' products in tiles of 256 rows against smaller ones."""
 
 from __future__ import annotations
 
@@ -65,3 +65,40 @@ def test_lists_of_any_size(n, experts, top):
     for tile in (16, 128):
         parts, _, _ = _route(x, router, top, tile, False)
         _check_lists(parts, experts, tile)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("counts,width,ff", [
+    ((1, 16, 17, 64, 65, 128, 129, 0), 64, 128), ((255, 256, 257, 511), 136, 72), ((300, 0, 520), 512, 264), ((240,), 72, 8),
+])
+def test_products_in_tiles_of_256_rows(counts, width, ff):
+    """A row's product does not depend on the tile that it falls into: the same bits in tiles of 256 rows as in tiles of 32; and close to float64."""
+    g = torch.Generator().manual_seed(sum(counts))
+    n, experts = sum(counts), len(counts)
+    which = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts))[torch.randperm(n, generator=g)]
+    x = torch.zeros(n, 64)
+    x[torch.arange(n), which] = 1.0
+    xs = torch.randn(n, width, generator=g).to(torch.bfloat16).cuda()
+    w_in = (torch.randn(experts, 2 * ff, width, generator=g) * width ** -0.5).to(torch.bfloat16).cuda()
+    w_out = (torch.randn(experts, width, ff, generator=g) * ff ** -0.5).to(torch.bfloat16).cuda()
+    single = w_in[:, :ff].contiguous()
+    got = {}
+    for tile in (32, 256):
+        lists = torch.zeros(K.moe_lists_ints(n, experts, 1), dtype=torch.int32, device="cuda")
+        score = torch.empty(n, device="cuda")
+        K.moe_route(x.to(torch.bfloat16).cuda(), 20.0 * torch.eye(experts, 64, device="cuda"), 1, lists, score, tile)
+        act, act1 = (torch.full((n, ff), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        parts = torch.full((1, n, width), float("nan"), device="cuda")
+        K.moe_tc_gate_up(xs, w_in, lists, 1, tile, act)
+        K.moe_tc_up_act(xs, single, lists, 1, tile, act1)
+        K.moe_tc_down(act, w_out, lists, 1, tile, parts)
+        got[tile] = (act.cpu(), act1.cpu(), parts.cpu())
+        order = K._moe_lists(lists, n, experts, 1)[1].long().cpu()
+    assert all(torch.equal(a, b) for a, b in zip(got[32], got[256]))
+    act, _, parts = (v.double() for v in got[256])
+    rows = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts))          # (the lists' rows stand in the experts' order)
+    w = w_out.cpu().double()[rows]
+    want = torch.einsum("nf,nhf->nh", act, w)
+    # float sums of ff products: their error is at most ff * 2^-24 * sum |act w| (the unit may cut instead of rounding: twice that)
+    bound = 2 * ff * 2.0 ** -24 * torch.einsum("nf,nhf->nh", act.abs(), w.abs()).max() + 1e-30
+    assert (parts[0][order] - want).abs().max() <= bound
