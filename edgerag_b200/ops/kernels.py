@@ -58,7 +58,7 @@ _SIGNATURES = {
                            c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
     "erb_attention_rows": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                            c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_float,
-                           c_void_p, c_int, c_void_p],
+                           c_void_p, c_int, c_int, c_void_p],
     "erb_attention_decode": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                              c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                              c_int, c_int, c_int, c_float, c_void_p, c_float, c_void_p, c_int, c_void_p],
@@ -1776,8 +1776,10 @@ def _gate(gate: torch.Tensor | None, out: torch.Tensor, width: int) -> tuple[int
 def attention_rows(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, block_tables: torch.Tensor,
                    seq_of_token: torch.Tensor, positions: torch.Tensor, out: torch.Tensor, n_q_heads: int,
                    scale: float, window: int = 0, keep_first: int = 0, chunk: int = 0,
-                   penalty: torch.Tensor | None = None, softcap: float = 0.0, gate: torch.Tensor | None = None) -> None:
+                   penalty: torch.Tensor | None = None, softcap: float = 0.0, gate: torch.Tensor | None = None,
+                   tiled: bool = False) -> None:
     """Causal attention of every token over its sequence's pages (general kernel, any portion sizes).
+    ``tiled``: the tokens are portions of prompts and may be taken 32 neighbouring ones together (float32, heads of 64 and 128).
     ``window`` > 0: a query sees the last ``window`` keys (its own included) and the first ``keep_first`` of the sequence.
     ``chunk`` > 0 (instead of a window): a query sees the earlier keys of its own run of ``chunk`` positions, runs
     counted from position 0 of the sequence.  ``penalty`` float ``[2, n_q_heads]`` (``r1``, then ``r2`` of every query
@@ -1799,7 +1801,8 @@ def attention_rows(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor
     _call(_fn("attention", _elem(q), "erb_attention_rows"), q.data_ptr(), q.stride(0), k_pages.data_ptr(),
           v_pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1], seq_of_token.data_ptr(),
           positions.data_ptr(), out.data_ptr(), out.stride(0), n, n_q_heads, nkv, d, page_size, mask_reach(window, chunk),
-          int(keep_first), float(scale), _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d), _stream())
+          int(keep_first), float(scale), _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d),
+          int(tiled), _stream())
 
 
 _sm_counts: dict[int, int] = {}

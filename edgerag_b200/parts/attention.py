@@ -335,8 +335,16 @@ class Attention(Mixer):
         elif n > nd:
             kernels.attention_rows(qkv[nd:], k_pages, v_pages, tables, ctx.seq_of_token[nd:], ctx.positions[nd:],
                                    out[nd:], self.n_q, self.scale, window=self.window, keep_first=self.keep_first, chunk=self.chunk,
-                                   gate=gate if gate is None else gate[nd:], **score)
+                                   gate=gate if gate is None else gate[nd:], tiled=self._tiled(ctx), **score)
         return self._project_out(out, ctx)
+
+    def _tiled(self, ctx) -> bool:
+        """Whether the step's portions are long enough that the 32-bit kernel for 32 tokens at a time takes them: 9 heads of 64, a
+        portion without a past, by rows | by tiles: 64 tokens 9.1 | 10.3 us, 96 tokens 16.1 | 14.8, 333 tokens 93 | 34; behind 7,000
+        tokens from the first; several portions share a block one after the other (512 tokens in portions of 17 15.6 | 19.6, of 32
+        20.8 | 9.6)."""
+        lens = ctx.host_q_len[ctx.n_decode:]
+        return not ctx.batch_invariant and sum(lens) >= 96 and sum(lens) >= 32 * len(lens)
 
     def _project_out(self, out: torch.Tensor, ctx) -> torch.Tensor:
         n = out.shape[0]
