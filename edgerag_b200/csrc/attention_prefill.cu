@@ -51,13 +51,15 @@
 //
 // Every wait is bounded: a thread that gives up raises a block-wide flag, every other wait of the
 // block then ends too, the block records a code in *status, lets its copies land, frees its TMEM
-// and returns.
+// and returns.  The barriers between two softmax warps have no limit; both come to each of them, whatever their waits give
+// (pair_rounds.h).
 #include <limits.h>
 #include <stdarg.h>
 #include <stdio.h>
 
 #undef ERB_ELEM
 #define ERB_ELEM 1
+#include "pair_rounds.h"
 #include "tc_common.cuh"
 
 using namespace erb;
@@ -361,9 +363,8 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     float* mine = exchange + (t * BM + row) * 2 + half;
     const float* partners = exchange + (t * BM + row) * 2 + (half ^ 1);
     bool ok = true;
-    auto wait = [&](int which, uint32_t parity) {
-      if (ok) ok = mbar_wait_or_abort(bar(which), parity, s_abort);
-      ok = __all_sync(0xffffffffu, ok) != 0;             // the same answer for every lane: TMEM loads are collective
+    auto wait = [&](int which, uint32_t parity) {        // the same answer for every lane: TMEM loads are collective
+      return __all_sync(0xffffffffu, mbar_wait_or_abort(bar(which), parity, s_abort)) != 0;
     };
     float m_ref = -INFINITY, l_run = 0.f;                // l_run: this thread's half of the row's sum
     const int win_lo = first_visible_key(my_pos, window);               // first key of this row's window or chunk
@@ -371,8 +372,16 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
     auto hidden = [&](int key) { return key > my_pos || (key < win_lo && key >= keep_first); };
     for (int j = j0; j < n_end[t]; ++j) {
       const int place = turn_of(j - j0, t) % 3;
-      wait(kBarSFull + 2 * t + ((j - j0) & 1), ((j - j0) >> 1) & 1);
-      if (!ok) break;
+      PairRounds pair(j == j0);
+      if (!wait(kBarSFull + 2 * t + ((j - j0) & 1), ((j - j0) >> 1) & 1)) {
+        // the partner may have found the scores there: to its barriers, then out with it
+        do {
+          if (pair.search()) named_barrier(pair_barrier, 64);
+          named_barrier_any(pair_barrier, 64, true);
+        } while (pair.again());
+        ok = false;
+        break;
+      }
       fence_after_sync();
       const uint32_t t_s = t_lane + place * BN + half * 64;
       const int tile_key0 = tile_of(j) * BN, key0 = tile_key0 + half * 64;
@@ -390,9 +399,8 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       // O and the running sum rescaled, and the tile's P computed again.
       float l_tile = 0.f;
       uint32_t packed[32];
-      bool search = j == j0;
       for (;;) {
-        if (search) {
+        if (pair.search()) {
           float m_half = -INFINITY;
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
@@ -422,15 +430,15 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
           l_run *= alpha;
           if (j > j0) {
             // O is rescaled in TMEM: P V of tile j-1 must have landed first
-            wait(kBarPvTile + 2 * t + ((j - 1 - j0) & 1), ((j - 1 - j0) >> 1) & 1);
-            if (!ok) break;
-            fence_after_sync();
-            float acc[32];
-            tmem_ld32(t_o, acc);
-            tmem_ld_wait();
+            if (wait(kBarPvTile + 2 * t + ((j - 1 - j0) & 1), ((j - 1 - j0) >> 1) & 1)) {
+              fence_after_sync();
+              float acc[32];
+              tmem_ld32(t_o, acc);
+              tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] *= alpha;
-            tmem_st32(t_o, acc);
+              for (int i = 0; i < 32; ++i) acc[i] *= alpha;
+              tmem_st32(t_o, acc);
+            }
           }
         }
         float l4[4] = {0.f, 0.f, 0.f, 0.f};
@@ -499,8 +507,8 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         l_tile = (l4[0] + l4[1]) + (l4[2] + l4[3]);
         // both threads of a row have to agree on the reference: the two warps decide together (and behind this barrier both have
         // read their scores, whose place P takes)
-        if (!named_barrier_any(pair_barrier, 64, !search && !(l_tile < kSumLimit))) break;
-        search = true;
+        if (!named_barrier_any(pair_barrier, 64, pair.vote(!(l_tile < kSumLimit), s_abort))) break;
+        if (!pair.again()) { ok = false; break; }
       }
       if (!ok) break;
       tmem_st32(t_lane + place * BN + half * 32, reinterpret_cast<const float*>(packed));
@@ -516,7 +524,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       // nothing of this range is visible to this query tile: an empty record for the merge
       if (key_splits > 1 && half == 0 && row < rows_t[t]) { part_ml[record * 2] = -INFINITY; part_ml[record * 2 + 1] = 0.f; }
     } else {
-      wait(kBarPvTile + 2 * t + ((n_end[t] - 1 - j0) & 1), ((n_end[t] - 1 - j0) >> 1) & 1);
+      if (ok) ok = wait(kBarPvTile + 2 * t + ((n_end[t] - 1 - j0) & 1), ((n_end[t] - 1 - j0) >> 1) & 1);
       fence_after_sync();
       mine[2 * 2 * BM] = l_run;                          // (a slot of its own: the partner may still be reading a maximum)
       named_barrier(pair_barrier, 64);

@@ -17,8 +17,9 @@
 //
 // A tile's scores have two places in TMEM, and P takes the place of the scores that it was made of: S_t(j + 1) is there when the
 // softmax of S_t(j) ends, and the softmax warps need not wait for a product in a step.  The place of S_t(j) is taken by
-// S_t(j + 2) only once P_t(j) V(j) has been seen to end.  Every hand-over is an mbarrier, every wait is bounded: a thread that
-// gives up raises a block-wide flag, the block records a code in *status, lets its copies land, frees its TMEM and returns.
+// S_t(j + 2) only once P_t(j) V(j) has been seen to end.  Every hand-over is an mbarrier, every wait for one is bounded: a thread that
+// gives up raises a block-wide flag, the block records a code in *status, lets its copies land, frees its TMEM and returns.  The
+// barriers between softmax warps have no limit; all their warps come to each of them, whatever their waits give (pair_rounds.h).
 //
 // P goes into the second product as two bfloat16 pieces, its rounding and what that leaves: the reference maximum moves seldom, so
 // the largest weight of a row is no longer exactly 1, and rounding it once would lose 4 % of accuracy against a kernel that
@@ -36,6 +37,7 @@
 
 #undef ERB_ELEM
 #define ERB_ELEM 1
+#include "pair_rounds.h"
 #include "tc_common.cuh"
 
 using namespace erb;
@@ -313,17 +315,24 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     float* mine = shared_rows + (t * BM + row) * 2 + half;
     const float* partners = shared_rows + (t * BM + row) * 2 + (half ^ 1);
     bool ok = true;
-    auto wait = [&](int which, uint32_t parity) {
-      if (ok) ok = mbar_wait_or_abort(bar(which), parity, s_abort);
-      ok = __all_sync(0xffffffffu, ok) != 0;             // the same answer for every lane: TMEM loads are collective
+    auto wait = [&](int which, uint32_t parity) {        // the same answer for every lane: TMEM loads are collective
+      return __all_sync(0xffffffffu, mbar_wait_or_abort(bar(which), parity, s_abort)) != 0;
     };
     float m_ref = -INFINITY, l_run = 0.f;                // l_run: this thread's half of the row's sum
     const int win_lo = first_visible_key(my_pos, a.window);
     auto hidden = [&](int key) { return key > my_pos || key < win_lo; };
     const int n_mine = n_end[t];
     for (int j = 0; j < n_mine; ++j) {
-      wait(kBarS + 2 * t + (j & 1), (j >> 1) & 1);
-      if (!ok) break;
+      PairRounds pair(j == 0);
+      if (!wait(kBarS + 2 * t + (j & 1), (j >> 1) & 1)) {
+        // the partner may have found the scores there: to its barriers, then out with it
+        do {
+          if (pair.search()) named_barrier(pair_barrier, 64);
+          named_barrier_any(pair_barrier, 64, true);
+        } while (pair.again());
+        ok = false;
+        break;
+      }
       fence_after_sync();
       const uint32_t t_s = t_lane + col_s(t, j);
       const int tile_key0 = key_first + j * BN, key0 = tile_key0 + 32 * half;
@@ -333,10 +342,9 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
       // the tile's P made again (P is a floating-point number: a reference that is low by twenty powers of two costs no precision).
       float l_tile = 0.f;
       uint32_t high[16], low[16];                        // P in two pieces, pairs of neighbouring keys
-      bool search = j == 0, searched = false, capped = false;      // capped: the scores have been replaced by capped ones in the log2 domain
+      bool capped = false;                               // the scores have been replaced by capped ones in the log2 domain
       for (;;) {
-        if (search) {
-          searched = true;
+        if (pair.search()) {
           float m_raw = -INFINITY;
           {
             float s[32];
@@ -357,17 +365,17 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
           }
           l_run *= alpha;
           if (j > 0) {
-            wait(kBarPv + 2 * t + ((j - 1) & 1), ((j - 1) >> 1) & 1);      // P V of the tile before must have landed
-            if (!ok) break;
-            fence_after_sync();
+            if (wait(kBarPv + 2 * t + ((j - 1) & 1), ((j - 1) >> 1) & 1)) {      // P V of the tile before must have landed
+              fence_after_sync();
 #pragma unroll 1
-            for (int c = 0; c < VB; ++c) {
-              float acc[32];
-              tmem_ld32(t_o + 32 * c, acc);
-              tmem_ld_wait();
+              for (int c = 0; c < VB; ++c) {
+                float acc[32];
+                tmem_ld32(t_o + 32 * c, acc);
+                tmem_ld_wait();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) acc[i] *= alpha;
-              tmem_st32(t_o + 32 * c, acc);
+                for (int i = 0; i < 32; ++i) acc[i] *= alpha;
+                tmem_st32(t_o + 32 * c, acc);
+              }
             }
           }
         }
@@ -437,8 +445,8 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
         }
         l_tile = even + odd;
         // both threads of a row have to agree on the reference (and behind this barrier both have read their scores)
-        if (!named_barrier_any(pair_barrier, 64, !searched && !(l_tile < kSumLimit))) break;
-        search = true;
+        if (!named_barrier_any(pair_barrier, 64, pair.vote(!(l_tile < kSumLimit), s_abort))) break;
+        if (!pair.again()) { ok = false; break; }
       }
       if (!ok) break;
       tmem_st16(t_s + 16 * half, high);                  // (in the scores' place: 32 columns of pairs of each piece)
@@ -449,8 +457,8 @@ attention_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(kBarP + 2 * t + (j & 1)));
     }
-    if (n_mine > 0) {
-      wait(kBarPv + 2 * t + ((n_mine - 1) & 1), ((n_mine - 1) >> 1) & 1);
+    if (n_mine > 0 && ok) {
+      ok = wait(kBarPv + 2 * t + ((n_mine - 1) & 1), ((n_mine - 1) >> 1) & 1);
       fence_after_sync();
     }
     *mine = l_run;                                       // (behind the last vote: the partner has read the maximum)
