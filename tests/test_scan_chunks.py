@@ -52,6 +52,50 @@ def test_state_space_chunks(H, P, N, G, lens, pace):
         assert torch.equal(state[0], before[0])     # the slot nobody holds
 
 
+def _same_as_walked(got, walked, what):
+    """Numbers that are not finite lie where the walk has them and are the same; the others are within the band of the tests above."""
+    assert torch.equal(torch.isfinite(got), torch.isfinite(walked)), what
+    assert torch.equal(torch.nan_to_num(got[~torch.isfinite(got)]), torch.nan_to_num(walked[~torch.isfinite(walked)])), what
+    fine = torch.isfinite(walked)
+    assert (got[fine].double() - walked[fine].double()).abs().max() < 6e-5 * max(1.0, walked[fine].abs().max().item()), what
+
+
+@pytest.mark.parametrize("P,N", [(32, 32), (64, 64), (64, 128)])
+@pytest.mark.parametrize("what", ["x", "x nan", "B", "C", "step", "state", "decay"])
+def test_state_space_chunks_keep_numbers_that_are_not_finite_to_the_later_tokens(P, N, what):
+    """One number that is not finite at token 37 of a portion of 130 (or in its state, or a decay of exactly zero): the tokens before it
+    are what they are without it, and everything is what the walk gives."""
+    from edgerag_b200.ops import kernels
+
+    H, G, lens, at = 4, 2, [1, 130, 64], 1 + 37
+    n, inner, m = sum(lens), H * P, len(lens)
+    g = torch.Generator().manual_seed(N)
+    xbc = torch.randn(n, inner + 2 * G * N, generator=g) * 0.5
+    proj, a_log = torch.randn(n, 8, generator=g), torch.randn(H, generator=g) * 0.3
+    before = torch.randn(m + 1, H, N, P, generator=g)
+    if what[0] in "xBC":
+        xbc[at, {"x": P + 3, "B": inner + 5, "C": inner + G * N + N + 7}[what[0]]] = float("nan" if "nan" in what else "inf")
+    elif what == "step":
+        proj[at, 1 + 2] = float("inf")
+    elif what == "state":
+        before[2, 1, 9, 4] = float("inf")
+    else:
+        a_log[1] = 100.0
+    xbc, proj = xbc.to(torch.bfloat16).cuda(), proj.to(torch.bfloat16).cuda()
+    dt_bias, skip = torch.randn(H, generator=g).cuda() - 1.0, torch.randn(H, generator=g).cuda()
+    starts, slots = torch.tensor([0, 1, 131, 195], dtype=torch.int32).cuda(), torch.tensor([1, 2, 0], dtype=torch.int32).cuda()
+    done = []
+    for longest in (1 << 20, 1):
+        state, y = before.clone().cuda(), torch.full((n, inner), 7.0, device="cuda")
+        kernels.ssm_scan(xbc, proj, 1, dt_bias, a_log.cuda(), skip, state, m, starts, slots, y, G, longest=longest)
+        done.append((y, state))
+    _same_as_walked(done[0][0], done[1][0], "y")
+    _same_as_walked(done[0][1], done[1][1], "state")
+    y = done[0][0]
+    assert torch.isfinite(y[131:]).all() and (what == "state" or torch.isfinite(y[:at]).all())
+    assert torch.isfinite(y).all() == (what == "decay")
+
+
 def _delta_reference(qkv, b, a, dt_bias, a_log, state, H, G, d, dv):
     n, x = qkv.shape[0], qkv.double()
     unit = lambda z: z / torch.sqrt((z * z).sum(-1, keepdim=True) + 1e-6)      # noqa: E731
