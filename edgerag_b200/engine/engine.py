@@ -84,9 +84,11 @@ class EngineOptions:
     lookahead: bool = True
     poison_freed_pages: bool = False    # tests: NaN in free pages, so a stale read shows
     #: launch shapes that do not depend on the batch (decode attention always in splits of 512 keys with
-    #: the default grouping of heads): up to 16 single-token rows a request's logits are then the same
-    #: bits whatever shares its step; off, the attention kernel's shape follows the batch, which is
-    #: faster for small batches and short contexts
+    #: the default grouping of heads; the recurrent mixers walk every token, where a step's longest portion
+    #: would otherwise choose between a walk and chunks; portions of differential, latent and 32-bit attention by
+    #: the kernels that take a row the same way in any step): up to 16 single-token rows a request's logits are
+    #: then the same bits whatever shares its step; off, the kernels follow the batch, which is
+    #: faster for small batches, short contexts and portions of prompts
     batch_invariant: bool = False
     #: captured steps fill their single-token rows up to the next of a few sizes (1, 2, 4, 8, 16, 24, ...), so
     #: that a change in the number of running requests seldom needs another graph

@@ -89,11 +89,12 @@ class GatedDeltaRule(Mixer):
             kernels.conv_silu(proj, 0, self.w_conv, None, ctx.buf("delta.no_conv_state", (1, 0, self.channels), torch.float32),
                               ctx.seq_of_token, ctx.seq_starts, ctx.state_slots, qkv)
         o = ctx.buf("delta.o", (n, self.inner), torch.float32)
+        # portions in chunks, where that is the faster form for the step; all walked where nothing may depend on what shares the step
+        chunks = self.dtype == torch.bfloat16 and not ctx.batch_invariant
+        scratch = kernels.delta_scratch_floats(n, self.n_heads, self.n_key_heads, self.key_dim, self.v_dim, ctx.n_seqs if chunks else 0)
         kernels.delta_scan(qkv, proj, self.off_b, self.off_a, self.dt_bias, self.a_log, ctx.state("delta", call.cache_layer),
                            ctx.n_seqs, ctx.seq_starts, ctx.state_slots, o, self.n_key_heads, self.key_dim,
-                           ctx.buf("delta.scratch", (kernels.delta_scratch_floats(n, self.n_heads, self.n_key_heads, self.key_dim, self.v_dim,
-                                                                                  ctx.n_seqs if self.dtype == torch.bfloat16 else 0),),
-                                   torch.float32), longest=max(ctx.host_q_len))
+                           ctx.buf("delta.scratch", (scratch,), torch.float32), longest=max(ctx.host_q_len) if chunks else 1)
         gated = ctx.buf("delta.gated", (n, self.inner), self.dtype)
         kernels.head_norm_gate(o, proj[:, self.off_gate: self.off_gate + self.inner], self.norm_w, gated, self.n_heads, self.eps)
         n_parts = kernels.linear_parts_count(gated, self.w_o)

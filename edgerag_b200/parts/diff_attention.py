@@ -101,7 +101,10 @@ class DiffAttention(Mixer):
         self.lam = float(torch.exp((f64("lq1") * f64("lk1")).sum()) - torch.exp((f64("lq2") * f64("lk2")).sum()) + self.diff)
 
     def _wide_blocks(self, ctx, n: int) -> int:
-        """Blocks per head of the tcgen05 kernel for the step's ``n`` tokens of portions; 0: another kernel takes them."""
+        """Blocks per head of the tcgen05 kernel for the step's ``n`` tokens of portions; 0: another kernel takes them (as always where
+        nothing may depend on what shares the step: the line between the kernels is one on the whole step)."""
+        if ctx.batch_invariant:
+            return 0
         if n < self.MMA_FROM_TOKENS or not kernels.diff_wide_supported(self.dtype, self.dim, self.v_dim, ctx.page_size):
             return 0
         if 0 < self.window < self.WIDE_FROM_WINDOW or not self.scale > 0:

@@ -146,6 +146,27 @@ def test_delta_chunks(H, G, d, dv, lens, pace, alike):
         assert torch.equal(state[0], before[0])
 
 
+def test_walked_portions_do_not_depend_on_what_shares_the_step():
+    """The form that ``batch_invariant`` pins (``longest`` 1): the bits of a portion alone and beside others are the same, and so is its record."""
+    from edgerag_b200.ops import kernels
+
+    g = torch.Generator().manual_seed(3)
+    H, P, N, G, d, dv, lens = 4, 64, 128, 2, 128, 64, [30] + [8] * 31
+    n = sum(lens)
+    xbc, qkv = ((0.5 * torch.randn(n, w, generator=g)).to(torch.bfloat16).cuda() for w in (H * P + 2 * G * N, 2 * G * d + H * dv))
+    proj, vec = torch.randn(n, 2 * H, generator=g).to(torch.bfloat16).cuda(), torch.randn(3, H, generator=g).cuda()
+    ssm, delta = torch.randn(32, H, N, P, generator=g).cuda(), 0.3 * torch.randn(32, H, dv, d, generator=g).cuda()
+    results = []
+    for m in (1, 32):
+        rows, starts = sum(lens[:m]), torch.tensor([0, *torch.tensor(lens[:m]).cumsum(0).tolist()], dtype=torch.int32).cuda()
+        slots, states = torch.arange(m, dtype=torch.int32).cuda(), (ssm.clone(), delta.clone())
+        y, o = torch.empty(rows, H * P, device="cuda"), torch.empty(rows, H * dv, device="cuda")
+        kernels.ssm_scan(xbc[:rows], proj[:rows], 0, vec[0], vec[1], vec[2], states[0], m, starts, slots, y, G, longest=1)
+        kernels.delta_scan(qkv[:rows], proj[:rows], 0, H, vec[0], vec[1], states[1], m, starts, slots, o, G, d, longest=1)
+        results.append((y[:30], o[:30], states[0][0], states[1][0]))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
 @pytest.mark.parametrize("lens", [[7], [8], [1] * 9, [255], [3, 1, 2, 250, 1], [9, 300]])
 def test_short_convolution_by_eight_channels(lens):
     """Rows of four taps, with and without a bias, at counts around the lines between the kernels: float sums of five terms
