@@ -1149,10 +1149,12 @@ LATENT_WIDE_KEYS = 64      # ... and keys of its tiles: a portion's rows are a m
 
 
 def latent_wide_supported(dtype: torch.dtype, dim: int, rot_dim: int, v_dim: int, rank: int) -> bool:
-    """Whether the tcgen05 form over up-projected keys and values takes these sizes: bfloat16, unrotated parts and values of 64 or
-    128, a rotated part of at most 64 and latents in multiples of 8."""
+    """Whether the tcgen05 form over up-projected keys and values takes these sizes: unrotated parts and values of 64 or 128, a rotated
+    part of at most 64, and what the tensor-core form in the latent space takes.  Beside that form the roundings to bfloat16 only
+    change places (keys and values instead of the absorbed query and the latent result); sizes beyond it (latents of more than
+    512) keep their queries and weights in float32, in the general kernel."""
     return (dtype == torch.bfloat16 and dim in (64, 128) and v_dim in (64, 128) and 0 < rot_dim <= 64 and rot_dim % 8 == 0
-            and rank > 0 and rank % 8 == 0)
+            and latent_mma_supported(dtype, rank, rot_dim))
 
 
 def latent_gather(pages: torch.Tensor, block_tables: torch.Tensor, seq_starts: torch.Tensor, positions: torch.Tensor, out: torch.Tensor,
