@@ -20,8 +20,8 @@ window go back to the pool, and ``gated=False`` leaves the sigmoid gate out.
 
 Portions of prompts are worth the opposite: with many new tokens per cached one it is cheaper to up-project the context once and to
 attend with heads of ``dim + rot_dim`` and values of ``v_dim`` than over rows of ``kv_rank + rot_dim``.  Where the sizes allow it
-(``kernels.latent_wide_supported``) a portion's cache rows are gathered, one product makes every head's keys and values of them,
-and a tcgen05 kernel attends; single tokens stay in the latent space.
+(``kernels.latent_wide_supported``) and it pays (``_wide_pays``) a portion's cache rows are gathered, one product makes every head's
+keys and values of them, and a tcgen05 kernel attends; single tokens, and many short portions, stay in the latent space.
 
 The first product reads the mixer's input once for everything that is made from it: queries (or
 their latent), the down-projection of ``[c | kr]`` and the gate logits.
@@ -146,10 +146,31 @@ class LatentAttention(Mixer):
         total = rows * len(lens)
         if 2 * total * self.n_heads * (self.dim + self.v_dim) > self.WIDE_MAX_BYTES:
             return 0
-        # The form is the faster one for every portion measured, of 2 tokens to 2,048 behind 0 to 8,000 (2,048 tokens of 16 heads of
-        # 128 + 64 over latents of 512: the sublayer 800 us in the latent space, 129 us; 2 tokens behind 2,048: 190 us, 73 us; 17 behind
-        # none: 40 us, 32 us).  But beside single tokens the bound may be theirs, with rows that no portion needs, at 6 us a thousand.
-        return rows if not ctx.n_decode or total <= 32 * sum(lens) + 2048 else 0
+        # (beside single tokens the bound may be theirs, with rows that no portion needs)
+        if ctx.n_decode and total > 32 * sum(lens) + 2048:
+            return 0
+        return rows if self._wide_pays(lens, rows) else 0
+
+    def _wide_pays(self, lens, rows: int) -> bool:
+        """Whether the up-projected form is the faster one for portions of these lengths, the longest of which is taken for the one with the
+        longest context (of up to ``rows`` keys).  Both forms' device times in us, fitted to the sublayer's over 1 to 32 portions of 2 to
+        512 tokens behind up to 8,000 (16 heads of 128 + 64 and 128 over latents of 512; 8 heads of 64 + 32 and 64 over 256):
+
+        * up-projected, a share for every row of every portion (gather, product), and waves of a block an SM that walk the context in
+          tiles of 64 keys: 2 tokens behind 2,000 68 us (185 in the latent space), behind 8,000 204 (645); with a context of 2,000
+          beside seven portions of 2 tokens 125 (189), beside fifteen 187 (189);
+        * in the latent space, a slow walk of the longest context, whose blocks the others' run beside: 32 portions of 2 tokens behind 60
+          41 us (up-projected 62), 16 behind 500 74 (96), 16 behind 2,000 191 (232)."""
+        H, sms, tile = self.n_heads, kernels._sms(self.device), kernels.LATENT_WIDE_KEYS
+        tiles = rows / tile
+        per_row = 0.0005 + 0.003 * H * (self.dim + self.v_dim) * self.kv_rank / 2 ** 21
+        per_tile = 0.35 + 0.15 * ((self.dim + self.v_dim) // 64 + 1)
+        blocks = H * sum(-(-n // kernels.LATENT_WIDE_ROWS) for n in lens)
+        wide = 10.0 + per_row * rows * len(lens) + max(1.0, blocks / sms) * (10.0 + per_tile * tiles)
+        width = (2 * self.kv_rank + self.rot_dim) / 1088
+        longest = max(lens)
+        walked = sum(-(-n * H // 32) * -(-n // tile) for n in lens) + -(-longest * H // 32) * (tiles - -(-longest // tile))
+        return wide < 8.0 + 22.0 * width + (2.0 + 3.0 * width) * max(tiles, walked / sms)
 
     def _attend_wide(self, ctx, q, pages, tables, heads, gate, rows: int) -> None:
         """The portions' tokens over up-projected keys and values; ``q``, ``gate`` and ``heads`` hold the whole batch's rows."""
