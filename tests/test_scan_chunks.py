@@ -167,6 +167,40 @@ def test_walked_portions_do_not_depend_on_what_shares_the_step():
     assert all(torch.equal(a, b) for a, b in zip(*results))
 
 
+@pytest.mark.parametrize("d,dv", [(64, 16), (128, 128)])
+@pytest.mark.parametrize("what", ["q", "k", "v", "v nan", "strength", "decay", "state"])
+def test_delta_chunks_keep_numbers_that_are_not_finite_to_the_later_tokens(d, dv, what):
+    """As for the state-space chunks; a decay input of infinity is a decay of exactly zero."""
+    from edgerag_b200.ops import kernels
+
+    H, G, lens, at = 4, 2, [1, 130, 64], 1 + 37
+    n, m = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(d + dv)
+    qkv, proj = torch.randn(n, 2 * G * d + H * dv, generator=g) * 0.5, torch.randn(n, 2 * H + 3, generator=g)
+    before = 0.3 * torch.randn(m + 1, H, dv, d, generator=g)
+    if what[0] in "qkv":
+        qkv[at, {"q": 5, "k": G * d + d + 6, "v": 2 * G * d + 3 * dv + 2}[what[0]]] = float("nan" if "nan" in what else "inf")
+    elif what == "strength":
+        proj[at, 1 + 2] = float("nan")
+    elif what == "decay":
+        proj[at, 2 + H + 1] = float("inf")
+    else:
+        before[2, 1, 9, 4] = float("inf")
+    qkv, proj = qkv.to(torch.bfloat16).cuda(), proj.to(torch.bfloat16).cuda()
+    dt_bias, a_log = torch.randn(H, generator=g).cuda() - 1.0, torch.randn(H, generator=g).cuda() * 0.3
+    starts, slots = torch.tensor([0, 1, 131, 195], dtype=torch.int32).cuda(), torch.tensor([1, 2, 0], dtype=torch.int32).cuda()
+    done = []
+    for longest in (1 << 20, 1):
+        state, out = before.clone().cuda(), torch.full((n, H * dv), 7.0, device="cuda")
+        kernels.delta_scan(qkv, proj, 1, 2 + H, dt_bias, a_log, state, m, starts, slots, out, G, d, longest=longest)
+        done.append((out, state))
+    _same_as_walked(done[0][0], done[1][0], "out")
+    _same_as_walked(done[0][1], done[1][1], "state")
+    out = done[0][0]
+    assert torch.isfinite(out[131:]).all() and (what == "state" or torch.isfinite(out[:at]).all())
+    assert torch.isfinite(out).all() == (what == "decay")
+
+
 @pytest.mark.parametrize("lens", [[7], [8], [1] * 9, [255], [3, 1, 2, 250, 1], [9, 300]])
 def test_short_convolution_by_eight_channels(lens):
     """Rows of four taps, with and without a bias, at counts around the lines between the kernels: float sums of five terms
