@@ -158,3 +158,30 @@ def test_differential_rows_by_eight_channels(lens, rot_dims):
     at = slots[kept].long().cuda()
     assert close(k_pages[at // page, 0, at % page], maps[kept.cuda(), H * 2 * d:]) and close(v_pages[at // page, 0, at % page], want[kept.cuda(), -dv:])
     assert int((k_pages.abs().sum(-1) > 0).sum()) == int(kept.sum())
+
+
+@pytest.mark.parametrize("lens", [[128], [3, 1, 2, 250]])
+@pytest.mark.parametrize("rot_dims", [0, 64])
+def test_differential_rows_have_the_bits_of_the_general_kernel(lens, rot_dims):
+    """Rows whose length is no multiple of four take the general kernel: the same numbers in such rows give the same bits."""
+    from edgerag_b200.ops import kernels
+
+    H, G, d, dv, page, n = 4, 2, 64, 128, 16, sum(lens)
+    channels = (H + G) * 2 * d + G * dv
+    g = torch.Generator().manual_seed(n + rot_dims)
+    rand = lambda *shape: torch.randn(*shape, generator=g)      # noqa: E731
+    proj, weight, record = rand(n, channels + 6).to(torch.bfloat16).cuda(), (0.4 * rand(channels, 4)).cuda(), rand(len(lens), 3, channels).cuda()
+    starts = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32).cuda()
+    seq = torch.tensor([s for s, length in enumerate(lens) for _ in range(length)], dtype=torch.int32).cuda()
+    positions = torch.cat([torch.arange(70, 70 + length) for length in lens]).int().cuda()
+    freq = (1000.0 ** (-torch.arange(d // 2) / (d // 2))).float().cuda()
+    results = []
+    for rows in (proj[:, :channels].contiguous(), proj):
+        k_pages = torch.zeros(n // page + 1, G, page, 2 * d, dtype=torch.bfloat16, device="cuda")
+        v_pages = torch.zeros(n // page + 1, G, page, dv, dtype=torch.bfloat16, device="cuda")
+        q = torch.empty(n, H * 2 * d, dtype=torch.bfloat16, device="cuda")
+        kernels.diff_prepare(rows, q, positions, H, G, d, dv, inv_freq=freq if rot_dims else None, rot_dims=rot_dims, conv_w=weight, conv_state=record,
+                             seq_of_token=seq, seq_starts=starts, state_slots=torch.arange(len(lens), dtype=torch.int32).cuda(),
+                             slots=torch.arange(n, dtype=torch.int32).cuda(), k_pages=k_pages, v_pages=v_pages, page_size=page)
+        results.append((q, k_pages, v_pages))
+    assert all(torch.equal(a, b) for a, b in zip(*results))

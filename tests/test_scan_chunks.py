@@ -228,6 +228,26 @@ def test_short_convolution_by_eight_channels(lens):
             at += length
 
 
+@pytest.mark.parametrize("lens", [[8], [255, 3], [1] * 9, [9, 300]])
+def test_short_convolution_has_the_bits_of_the_general_kernel(lens):
+    """Rows whose length is no multiple of eight take the general kernel: the same numbers in such rows give the same bits."""
+    from edgerag_b200.ops import kernels
+
+    n, channels, off = sum(lens), 72, 16
+    g = torch.Generator().manual_seed(n)
+    proj = torch.randn(n, 100, generator=g).to(torch.bfloat16).cuda()
+    weight, bias = torch.randn(channels, 4, generator=g).to(torch.bfloat16).cuda(), torch.randn(channels, generator=g).to(torch.bfloat16).cuda()
+    record = torch.randn(len(lens), 3, channels, generator=g).cuda()
+    starts = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32).cuda()
+    seq = torch.tensor([s for s, length in enumerate(lens) for _ in range(length)], dtype=torch.int32).cuda()
+    held = torch.arange(len(lens), dtype=torch.int32).cuda()
+    for b in (bias, None):
+        outs = [torch.empty(n, channels, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+        for rows, out in zip((proj[:, :96].contiguous(), proj), outs):
+            kernels.conv_silu(rows, off, weight, b, record, seq, starts, held, out)
+        assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("n,parts,per", [(1, 1, 128), (5, 3, 256), (33, 2, 512), (3, 1, 1024)])
 @pytest.mark.parametrize("gated", [False, True])
 def test_group_norm_by_warps(n, parts, per, gated):
