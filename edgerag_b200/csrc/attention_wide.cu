@@ -27,7 +27,8 @@
 //
 // What bounds it: the exponentials and what is done to a score besides (about 12 instructions with a cap of the scores); the tensor
 // cores wait for them.  Tiles of 64 keys leave room in TMEM for two accumulators of 128 columns beside the scores, and in shared
-// memory for three to four tiles beside the queries.  Differential, 2,048 tokens of 16 heads, capped: 240 us by the mma.sync
+// memory for three to four tiles beside the queries; that, and boxes of 64 columns, is why heads and values are of 64 or 128 (the
+// differential form of 64 and 128: other sizes are diff_attention.cu's).  Differential, 2,048 tokens of 16 heads, capped: 240 us by the mma.sync
 // kernel of diff_attention.cu, 74 us by this; without a cap 185 us and 58 us.
 // Rows, 2,048 tokens of 16 heads of 128 + 64 and 128: about 50 us beside 20 us of gathering and up-projecting, where the kernel over
 // latents of 512 took 705 us.
@@ -617,9 +618,6 @@ int launch(const CUtensorMap& mk, const CUtensorMap& mv, const WideArgs& a, int 
 
 }  // namespace
 
-// Tokens of one (sequence, head) that a block of the differential form takes.
-ERB_EXPORT int erb_attention_wide_diff_rows() { return BM; }
-
 // Differential attention over portions (maps of 64, values of 128, pages of 8 to 128 tokens, a power of two).  q: [token][head][2][64],
 // rotated, not scaled; seq_starts: int32 [n_seqs + 1] offsets of the sequences to process (consecutive rows of block_tables);
 // n_blocks: sum over them of ceil(length / 128) (an upper bound is fine).  window > 0: a row sees its last `window` keys.
@@ -680,11 +678,6 @@ ERB_EXPORT int erb_latent_q_rows(const void* q, int n_tokens, int ld, int heads,
   return check_launch("latent_q_rows");
 }
 
-// Whether erb_attention_wide_rows takes these sizes.
-ERB_EXPORT int erb_attention_wide_rows_supported(int dim, int rot, int v_dim, int rank) {
-  return (dim == 64 || dim == 128) && (v_dim == 64 || v_dim == 128) && rot > 0 && rot <= 64 && rot % 8 == 0 && rank > 0 && rank % 8 == 0;
-}
-
 // Attention over rows: keys of a head are [dim | shared rot], values v_dim.  q: [token][head][dim + rot] (rows q_ld apart, the first
 // `dim` entries of a head are read), q_rot: [token][head][64] from erb_latent_q_rows; kv: [n_seqs * kv_rows][heads][dim + v_dim];
 // latents: [n_seqs * kv_rows][rank + rot] from erb_latent_gather, whose last `rot` columns are the keys' shared part.  All token rows
@@ -695,7 +688,7 @@ ERB_EXPORT int erb_attention_wide_rows(const void* q, int q_ld, const void* q_ro
                                        int v_dim, int rank, int window, float scale, const float* sink, const void* gate, int gate_ld,
                                        int* status, void* stream) {
   if (n_seqs <= 0 || n_blocks <= 0) return ERB_OK;
-  if (!erb_attention_wide_rows_supported(dim, rot, v_dim, rank))
+  if ((dim != 64 && dim != 128) || (v_dim != 64 && v_dim != 128) || rot <= 0 || rot > 64 || rot % 8 || rank <= 0 || rank % 8)
     return fail(ERB_ERR_UNSUPPORTED, "attention_wide_rows: heads of %d + %d and %d over latents of %d", dim, rot, v_dim, rank);
   if (heads <= 0 || n_blocks > 65535 || kv_rows <= 0 || kv_rows % BN || !status || window < 0 || !(scale > 0.f) ||
       (long long)n_seqs * kv_rows > 0x7fffffffLL)

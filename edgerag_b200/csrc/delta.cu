@@ -18,11 +18,12 @@
 // way while these are walked.
 //
 // A request's tokens of one step are neighbours in the batch (rows seq_starts[s] .. seq_starts[s+1]), its slot is
-// state_slots[s]; every (request, head, column) is walked by exactly one thread group, token after token, so the
-// arithmetic of a token does not depend on how the sequence was cut into steps.
+// state_slots[s].  Walked, every (request, head, column) is one thread group's, token after token, and the arithmetic of a
+// token does not depend on how the sequence was cut into steps or on what else the step holds.
 //
-// Portions of prompts (bfloat16 rows, keys of 64 or 128, values of a multiple of 16) are not walked but taken 64 tokens at a
-// time, as products of matrices: see delta_chunk_kernel.  The two forms differ by rounding.
+// Portions of prompts (bfloat16 rows, keys of 64 or 128, values of a multiple of 16) are taken 64 tokens at a time, as products
+// of matrices, where chunks_pay says so: see delta_chunk_kernel.  The two forms differ by rounding, and which of them a portion
+// gets depends on the step; a caller for whom that matters gives `longest` as 1.
 #include <limits.h>
 #include <math.h>
 
@@ -505,8 +506,8 @@ delta_chunk_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, 
   }
   __syncthreads();
   // T = (I + A)^-1 in place of A, by blocks of 16: the diagonal ones column by column, then the others by rising distance from
-  // the diagonal, T_ij = -T_ii sum_k A_ik T_kj (k from j to i - 1).  A tile of A is read for the last time before its place is
-  // taken: A_ik is needed for the T_ij with j <= k, at distances >= that of (i, k); X holds a distance's sums.
+  // the diagonal, T_ij = -T_ii sum_k A_ik T_kj (k from j to i - 1).  The tiles of A at distances 1 and 2 are used again after T has
+  // taken their places, so each thread keeps its rows of them in registers; only (3, 0) is read where it was.  X holds a distance's sums.
   float tcol[16];
   if (warp < 4 && lane < 16) {
     const int b = 16 * warp;
@@ -526,9 +527,6 @@ delta_chunk_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, 
   __syncthreads();
   {
     const int er = threadIdx.x >> 4, ec = threadIdx.x & 15;    // a thread's entry of a tile
-    // Distances 1 to 3; the tiles of A at larger distances than the current one are still A.  T_kj for k > j lies at a smaller
-    // distance and has been made.  A_ik with i - k < distance has been overwritten, so the sums use copies: x = T_ii^-1 parts
-    // are avoided by multiplying with A from registers saved before.
     float a_keep[3][16];                                       // this thread's rows of A at distance 1 (tiles (1,0), (2,1), (3,2)): row er
     float a_keep2[2][16];                                      // and at distance 2 (tiles (2,0), (3,1))
 #pragma unroll
@@ -828,6 +826,11 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
 inline bool chunk_sizes(int d, int dv) { return (d == 64 || d == 128) && dv % kChunkCols == 0; }
 inline long long chunk_records(int n_tokens, int n_seqs, int H) { return (long long)(n_tokens / kChunk + n_seqs) * H; }
 
+// Floats that portions in chunks need: the chunks' records, and the walk's scratch for requests of one token.
+inline long long chunk_scratch_floats(int n_tokens, int n_seqs, int H, int G, int d, int dv) {
+  return chunk_records(n_tokens, n_seqs, H) * (long long)(sizeof(ChunkRecord) / 4) + (long long)delta_scratch_floats(n_seqs, H, G, d, dv);
+}
+
 // Whether the chunks are the faster form: both costs in microseconds, fitted to the times of 1 to 64 requests of 2 to 500 tokens
 // (4 to 16 heads of 64 x 48 and 128 x 128).  The walk costs 0.49 us a token of the longest portion or, when the GPU is full,
 // its blocks' tokens and states; the chunks cost two more launches, 3.7 us a chunk of the longest portion or, when the GPU is
@@ -841,27 +844,9 @@ inline bool chunks_pay(int blocks, int n_tokens, int n_seqs, int longest) {
   const double walk = fmax(6.0 + 0.49 * longest, blocks * (0.00086 * n_tokens + 0.0024 * n_seqs));
   return 15.0 + fmax(3.7 * own, 0.0384 * blocks * chunks) + 0.003 * blocks * singles < walk;
 }
-
-#define ERB_DELTA_CHUNKS 1
-#else
-inline bool chunk_sizes(int, int) { return false; }
-#define ERB_DELTA_CHUNKS 0
 #endif  // ERB_ELEM == 1
 
 }  // namespace
-
-// Floats of the scratch that erb_delta_scan needs for a step of n_tokens tokens, and (n_seqs > 0) what it needs to take portions
-// of prompts in chunks: the chunks' records, and the walk's scratch for requests of one token.
-ERB_EXPORT long long erb_delta_scratch_floats(int n_tokens, int n_seqs, int H, int G, int d, int dv) {
-  long long need = (long long)delta_scratch_floats(n_tokens, H, G, d, dv);
-#if ERB_DELTA_CHUNKS
-  if (n_seqs > 0 && n_tokens > n_seqs && chunk_sizes(d, dv)) {
-    const long long chunks = chunk_records(n_tokens, n_seqs, H) * (long long)(sizeof(ChunkRecord) / 4) + (long long)delta_scratch_floats(n_seqs, H, G, d, dv);
-    if (chunks > need) need = chunks;
-  }
-#endif
-  return need;
-}
 
 ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, int ld, int off_b, int off_a,
                               const float* dt_bias, const float* a_log, float* state, const int* seq_starts,
@@ -874,10 +859,10 @@ ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, i
   if (!scratch || ((uintptr_t)scratch & 15)) return fail(ERB_ERR_ARG, "delta_scan: the scratch must be 16-byte aligned");
   bool singles = false;                  // whether the walk is left with the requests of one token
   int walk_tokens = n_tokens;
-#if ERB_DELTA_CHUNKS
+#if ERB_ELEM == 1
   if (chunk_sizes(d, dv) && n_tokens > n_seqs && chunks_pay(H * (dv / kChunkCols), n_tokens, n_seqs, longest) && channels % 8 == 0 &&
       !(((uintptr_t)qkv | (uintptr_t)scratch) & 15) && !((uintptr_t)out & 7) && n_tokens / kChunk + n_seqs <= 65535 &&
-      scratch_floats >= erb_delta_scratch_floats(n_tokens, n_seqs, H, G, d, dv)) {
+      scratch_floats >= chunk_scratch_floats(n_tokens, n_seqs, H, G, d, dv)) {
     ChunkRecord* records = reinterpret_cast<ChunkRecord*>(scratch);
     auto prep = d == 64 ? delta_chunk_prepare_kernel<64> : delta_chunk_prepare_kernel<128>;
     const size_t prep_bytes = d == 64 ? sizeof(DeltaPrepSmem<64>) : sizeof(DeltaPrepSmem<128>);

@@ -126,6 +126,7 @@ diff_prepare_kernel(const T* __restrict__ proj, int ld, const float* __restrict_
 // map that turn together or eight neighbours of a value row.  Weights are read once for the tokens and inputs once for all taps, 16
 // and 8 bytes at a time, the angles are made once per token.  The sums are made in the same order: the same bits.
 // 2,048 tokens of 16 heads: 44 us by the kernel above, 18.6 us; 256 tokens 13.2 us and 6.3 us; 64 tokens 5.6 us by both (the line: 128).
+// Four taps are what the benchmarked sizes have; others take the kernel above.
 template <int TT>
 __global__ void __launch_bounds__(128)
 diff_prepare_vec_kernel(const __nv_bfloat16* __restrict__ proj, int ld, const float* __restrict__ conv_w, const float* __restrict__ conv_state,

@@ -58,7 +58,8 @@ conv_silu_kernel(const T* __restrict__ proj, int ld, int off, int channels, int 
 // The same for TAPS taps and rows whose channels come in aligned runs of eight (bfloat16 build): a thread owns eight channels
 // of TT neighbouring tokens, keeps its weights in registers and reads every input once with 16-byte loads instead of TAPS
 // times with 2-byte ones.  Same arithmetic in the same order: the same bits.  2,048 tokens of 6,144 channels:
-// 70 us before, 26 us; 64 single tokens 16 us before, 3.6 us.  What is left is the arithmetic of silu.
+// 70 us before, 26 us; 64 single tokens 16 us before, 3.6 us.  What is left is the arithmetic of silu.  (Built for four taps, what the
+// benchmarked sizes have; the eight channels' weights are then 16-byte pieces.  Others take the kernel above.)
 template <int TAPS, int TT>
 __global__ void __launch_bounds__(128)
 conv_silu_vec_kernel(const __nv_bfloat16* __restrict__ proj, int ld, int off, int channels, const __nv_bfloat16* __restrict__ weight,
