@@ -172,14 +172,20 @@ class LatentAttention(Mixer):
         walked = sum(-(-n * H // 32) * -(-n // tile) for n in lens) + -(-longest * H // 32) * (tiles - -(-longest // tile))
         return wide < 8.0 + 22.0 * width + (2.0 + 3.0 * width) * max(tiles, walked / sms)
 
+    def _wide_room(self, rows: int) -> int:
+        """Rows that the scratch of ``rows`` rows is asked for: the next power of two within the limit of bytes.  The rows follow the context,
+        and a buffer that grows drops the captured steps, so it should not grow with every portion of a long prompt."""
+        return max(rows, min(1 << (rows - 1).bit_length(), self.WIDE_MAX_BYTES // (2 * self.n_heads * (self.dim + self.v_dim))))
+
     def _attend_wide(self, ctx, q, pages, tables, heads, gate, rows: int) -> None:
         """The portions' tokens over up-projected keys and values; ``q``, ``gate`` and ``heads`` hold the whole batch's rows."""
         nd, n, H = ctx.n_decode, q.shape[0], self.n_heads
         starts = ctx.seq_starts[nd: ctx.n_seqs + 1]
         seqs = ctx.n_seqs - nd
-        latents = ctx.buf("latent.rows", (seqs * rows, self.kv_rank + self.rot_dim), self.dtype)
+        room = self._wide_room(seqs * rows)
+        latents = ctx.buf("latent.rows", (room, self.kv_rank + self.rot_dim), self.dtype)[: seqs * rows]
         kernels.latent_gather(pages, tables[nd:], starts, ctx.positions, latents, rows, self.window)
-        kv = ctx.buf("latent.kv", (seqs * rows, H * (self.dim + self.v_dim)), self.dtype)
+        kv = ctx.buf("latent.kv", (room, H * (self.dim + self.v_dim)), self.dtype)[: seqs * rows]
         kernels.linear(latents[:, : self.kv_rank], self.w_ukv, kv)
         q_rot = ctx.buf("latent.q_rot", (n, H, 64), self.dtype)
         kernels.latent_q_rows(q, ctx.positions, self.inv_freq, H, self.dim, self.rot_dim, self.rot_dims, q_rot, rot_mult=self.rot_mult)

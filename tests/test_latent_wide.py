@@ -63,6 +63,16 @@ def test_rows_follow_the_window_and_the_limit_of_bytes(monkeypatch):
     assert mixer._wide_rows(step) == 0
 
 
+def test_scratch_grows_seldom_while_a_prompt_is_read():
+    """Portions of 512 tokens up to a context of 32,768, whose bounds are quarters of a power of two: seven sizes, all within the limit."""
+    mixer = _mixer(16, 128, 64, 128, 512)
+    most = mixer.WIDE_MAX_BYTES // (2 * 16 * 256)
+    bounds = [kernels.context_bound(past // 16)[0] * 16 for past in range(512, 32769, 512)]
+    rooms = [mixer._wide_room(rows) for rows in bounds]
+    assert all(rows <= room <= most for rows, room in zip(bounds, rooms)) and len(set(rooms)) == 7 < len(set(bounds))
+    assert mixer._wide_room(most - 64) == most and mixer._wide_room(64) == 64
+
+
 # --- through the engine ------------------------------------------------------------------------------------------------
 
 def _models():
