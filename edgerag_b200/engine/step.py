@@ -17,6 +17,7 @@ and the row kernel each see a contiguous range; the caller's order is restored i
 from __future__ import annotations
 
 import gc
+import weakref
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -173,7 +174,13 @@ class ModelRunner:
         self.max_step_tokens = max_step_tokens
         self.check_status = check_status
         self.workspace = Workspace(self.device)
-        self.workspace.on_move = self.drop_graphs
+        runner = weakref.ref(self)     # (no cycle: a runner that is dropped gives its memory back at once)
+
+        def moving() -> None:
+            if runner() is not None:
+                runner().drop_graphs()
+
+        self.workspace.on_move = moving
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
         #: int32 device tensor that entries with ``fed_back`` take their token from (set by the caller)
         self.feedback: torch.Tensor | None = None
