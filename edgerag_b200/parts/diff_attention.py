@@ -39,12 +39,9 @@ class DiffAttention(Mixer):
     graph_safe = True
     #: prompt tokens of a step from which the tensor-core kernel (tiles of 64 tokens) takes the portions
     MMA_FROM_TOKENS = 32
-    #: windows from which on the tcgen05 kernel (tiles of 128 tokens and 64 keys) takes them, and how many of its rows a token may
-    #: cost.  700 tokens with a window of 128, 256, 512: 22.7, 26.5, 33.3 us against 23.7, 33.7, 50.9 us by the tensor-core kernel of
-    #: 64 rows (a window of 64: 16.2 against 14.5 us); 16 portions of 8 tokens behind 1,024: 80 us against 75 us, 8 portions of 32
-    #: behind 512: 25 us against 46 us, 17 tokens behind 2,048: 69 us against 133 us.
-    WIDE_FROM_WINDOW = 128
-    WIDE_ROWS_PER_TOKEN = 8
+    #: windows from which on the tcgen05 kernel (blocks of 128 tokens and tiles of 64 keys) may take them.  With a window of 128 a block
+    #: walks five tiles for two of its own: 300 tokens of 16 heads behind 500, capped, 25.8 us against 20.9 us by the kernel of 64 rows.
+    WIDE_FROM_WINDOW = 256
 
     def __init__(self, hidden: int, n_q_heads: int, n_kv_heads: int, dim: int, v_dim: int, scale: float, diff: float,
                  eps: float, dtype: torch.dtype, device: torch.device, window: int = 0, softcap: float = 0.0, conv: int = 0,
@@ -107,10 +104,47 @@ class DiffAttention(Mixer):
             return 0
         if n < self.MMA_FROM_TOKENS or not kernels.diff_wide_supported(self.dtype, self.dim, self.v_dim, ctx.page_size):
             return 0
-        if 0 < self.window < self.WIDE_FROM_WINDOW or not self.scale > 0:
+        lens = ctx.host_q_len[ctx.n_decode:]
+        if 0 < self.window < self.WIDE_FROM_WINDOW or not self.scale > 0 or not self._wide_pays(lens, ctx.max_keys_bound()):
             return 0
-        blocks = sum(-(-length // kernels.DIFF_WIDE_ROWS) for length in ctx.host_q_len[ctx.n_decode:])
-        return blocks if blocks * kernels.DIFF_WIDE_ROWS <= self.WIDE_ROWS_PER_TOKEN * n else 0
+        return sum(-(-length // kernels.DIFF_WIDE_ROWS) for length in lens)
+
+    def _wide_pays(self, lens, bound: int) -> bool:
+        """Whether the tcgen05 kernel is the faster one for portions of these lengths in contexts of up to ``bound`` keys.  Both kernels' times
+        in us, fitted to 2,660 pairs (4 to 32 heads, windows from 128 on and none, with and without a cap, 1 to 32 portions of 2 to 2,048
+        tokens behind up to 4,000):
+
+        * tcgen05, a block an SM, so in whole waves: 8 us a block and 1.36 a tile of 64 keys (0.57 more with a cap);
+        * 64 rows of a kv head's heads, 1.36 blocks an SM at a time: 5 us a block and 2.78 a tile (1.09 more).
+
+        2,048 tokens of 16 heads over 4 kv heads, capped, 71 | 240 us; one portion of 33 behind 1,000 32 | 57; 32 portions of 17, whose blocks of
+        128 rows are mostly empty, 36 | 15.  Which portion has the longest context is not part of a captured step's layout, so the two are
+        compared for the longest portion and for all of them, and the ratios averaged; 8 % have to be gained.  Of the pairs with windows
+        from 256 on, 67 of 2,080 are slower by more than 5 % than with 64 rows, 1.6 times at most."""
+        H, G, sms = self.n_q, self.n_kv, kernels._sms(self.device)
+        longest = lens.index(max(lens))
+
+        def walk(rows: int, columns: int, everyone: bool) -> tuple[int, float, float]:
+            """Blocks of ``rows`` tokens, their tiles, the tiles of the longest."""
+            most = (self.window + rows) / 64 + 1 if self.window else float("inf")
+            blocks, tiles, deepest = 0, 0.0, 0.0
+            for i, n in enumerate(lens):
+                past = max(0, bound - n) if everyone or i == longest else 0
+                b = -(-n // rows) * columns
+                blocks += b
+                tiles += b * min(most, (past + (n + min(rows, n)) / 2) / 64 + 0.5)
+                deepest = max(deepest, min(most, (past + n) / 64 + 0.5))
+            return blocks, tiles, deepest
+
+        gain = 1.0
+        for everyone in (False, True):
+            per = 1.36 + (0.57 if self.softcap > 0 else 0.0)
+            blocks, tiles, deepest = walk(kernels.DIFF_WIDE_ROWS, H, everyone)
+            wide = 1.09 + max(8.0 + deepest * per, -(-blocks // sms) * (8.0 + tiles / blocks * per))
+            per = 2.78 + (1.09 if self.softcap > 0 else 0.0)
+            blocks, tiles, deepest = walk(max(1, kernels.DIFF_MMA_ROWS * G // H), G, everyone)
+            gain *= (3.59 + max(5.05 + deepest * per, (5.05 * blocks + tiles * per) / (1.36 * sms))) / wide
+        return gain > 1.08 ** 2
 
     def _decode_plan(self, ctx, n_rows: int) -> tuple[int, int]:
         """(keys per split, splits) for the single-token rows: enough blocks for two per SM, splits of a multiple of 64

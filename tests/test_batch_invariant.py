@@ -30,7 +30,7 @@ class Recorder:
 def step(lens, batch_invariant):
     return SimpleNamespace(batch_invariant=batch_invariant, host_q_len=lens, n_seqs=len(lens), n_decode=sum(n == 1 for n in lens), page_size=16,
                            seq_of_token=None, seq_starts=None, state_slots=None, state=lambda name, layer: None,
-                           buf=lambda name, shape, dtype: torch.empty(shape, dtype=dtype))
+                           max_keys_bound=lambda: 4096, buf=lambda name, shape, dtype: torch.empty(shape, dtype=dtype))
 
 
 @pytest.mark.parametrize("lens", [[30], [1, 30], [30] + [8] * 31, [500, 64]])
@@ -49,7 +49,8 @@ def test_scans_walk_every_token(lens, monkeypatch):
                 assert args[-1].numel() == kernels.delta_scratch_floats(n, 4, 2, 64, 32, 0 if pinned else len(lens))
 
 
-def test_differential_portions_keep_their_kernel():
+def test_differential_portions_keep_their_kernel(monkeypatch):
+    monkeypatch.setattr(kernels, "_sms", lambda device: 148)
     mixer = DiffAttention(64, 4, 2, 64, 128, 0.125, 0.4, 1e-5, torch.bfloat16, torch.device("cpu"))
     assert mixer._wide_blocks(step([300], False), 300) == 3
     assert mixer._wide_blocks(step([300], True), 300) == 0
