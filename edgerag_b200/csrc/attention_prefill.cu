@@ -19,7 +19,7 @@
 // made of.  So the scores of a group's next tile are there when it has finished one, whatever the other group does, and the
 // groups need not wait for products: S of turn u only waits for P V of turn u - 3.  (With one place per query tile, S_A(j + 1)
 // could start only when P_A(j) was written, and 1,800 of a step's 4,480 clocks went into waiting for it: 32 heads of 2,048 tokens
-// 52 us instead of 43 us, of 8,192 tokens 541 us instead of 432 us.)
+// 52 us instead of 44 us, of 8,192 tokens 541 us instead of 440 us.)
 //
 // Nobody but the copy warp touches addresses of pages, and no block-wide barrier is taken inside the loop: every hand-over is an
 // mbarrier (K/V tile full, tile free again, S ready, P ready, product done).

@@ -29,7 +29,7 @@
 // cores wait for them.  Tiles of 64 keys leave room in TMEM for two accumulators of 128 columns beside the scores, and in shared
 // memory for three to four tiles beside the queries; that, and boxes of 64 columns, is why heads and values are of 64 or 128 (the
 // differential form of 64 and 128: other sizes are diff_attention.cu's).  Differential, 2,048 tokens of 16 heads, capped: 240 us by the mma.sync
-// kernel of diff_attention.cu, 74 us by this; without a cap 185 us and 58 us.
+// kernel of diff_attention.cu, 71 us by this; without a cap 185 us and 56 us.
 // Rows, 2,048 tokens of 16 heads of 128 + 64 and 128: about 50 us beside 20 us of gathering and up-projecting, where the kernel over
 // latents of 512 took 705 us.
 #include <limits.h>

@@ -835,9 +835,10 @@ inline long long chunk_scratch_floats(int n_tokens, int n_seqs, int H, int G, in
 // (4 to 16 heads of 64 x 48 and 128 x 128).  The walk costs 0.49 us a token of the longest portion or, when the GPU is full,
 // its blocks' tokens and states; the chunks cost two more launches, 3.7 us a chunk of the longest portion or, when the GPU is
 // full, a share of an SM for every chunk, be it full or not, and requests of one token are then walked by themselves.  One
-// request: from 32 tokens on; 32 requests of equal length: from about 50.
+// request: from 34 tokens on (8 heads of 128 x 128: 28 tokens 16.3 us walked, 20.0 in a chunk; 32 17.3 | 20.0; 36 18.8 | 20.1;
+// 44 21.3 | 20.1); 32 requests of equal length: from about 50.
 inline bool chunks_pay(int blocks, int n_tokens, int n_seqs, int longest) {
-  if (longest <= 1) return false;
+  if (longest < 34) return false;
   const double extra = (double)n_tokens - n_seqs - (longest - 1);      // tokens beyond one of the other requests
   const double others = fmax(0.0, fmin(extra, n_seqs - 1.0)), singles = n_seqs - 1.0 - others;
   const double own = (longest + 63) / 64, chunks = own + (others > 0.0 ? others + extra / 64.0 : 0.0);

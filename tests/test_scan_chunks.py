@@ -146,6 +146,24 @@ def test_delta_chunks(H, G, d, dv, lens, pace, alike):
         assert torch.equal(state[0], before[0])
 
 
+@pytest.mark.parametrize("length,walked", [(2, True), (28, True), (33, True), (300, False)])
+def test_short_portions_of_the_delta_rule_are_walked(length, walked):
+    """A chunk costs what 34 tokens of the walk cost: shorter portions have the walk's bits, longer ones differ from it by rounding."""
+    from edgerag_b200.ops import kernels
+
+    H, G, d, dv = 4, 4, 64, 48
+    g = torch.Generator().manual_seed(length)
+    qkv, proj = (torch.randn(length, w, generator=g).to(torch.bfloat16).cuda() for w in (2 * G * d + H * dv, 2 * H))
+    dt_bias, a_log = torch.randn(H, generator=g).cuda() - 1.0, torch.randn(H, generator=g).cuda() * 0.3
+    starts, slots = torch.tensor([0, length], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda()
+    outs = []
+    for longest in (None, 1):
+        out = torch.empty(length, H * dv, device="cuda")
+        kernels.delta_scan(qkv, proj, 0, H, dt_bias, a_log, torch.zeros(1, H, dv, d, device="cuda"), 1, starts, slots, out, G, d, longest=longest)
+        outs.append(out)
+    assert torch.equal(*outs) == walked
+
+
 def test_walked_portions_do_not_depend_on_what_shares_the_step():
     """The form that ``batch_invariant`` pins (``longest`` 1): the bits of a portion alone and beside others are the same, and so is its record."""
     from edgerag_b200.ops import kernels
