@@ -777,11 +777,14 @@ ERB_EXPORT int erb_conv_silu(const void* proj, int n_tokens, int ld, int off, in
   if (n_tokens <= 0) return ERB_OK;
   if (channels <= 0 || taps < 1 || (taps > 1 && !conv_state)) return fail(ERB_ERR_ARG, "conv_silu: bad sizes");
 #if ERB_ELEM == 1
-  // (from eight tokens on: a lone token has too few such threads to hide its loads, 2.3 us by the kernel above, 2.9 us by this)
-  if (n_tokens >= 8 && taps == 4 && channels % 8 == 0 && ld % 8 == 0 && off % 8 == 0 &&
+  // Few channels of few tokens: the kernel above, whose threads have less to do one after the other (8 tokens of 6,144 channels 1.9 us
+  // there, 2.5 here; 256 of 72 1.8 | 2.5); from 64 tokens on it gives a token's channels to one block (64 of 1,024 3.1 | 2.5, of
+  // 6,144 12.6 | 2.9).  Eight tokens a thread read the weights seldom, but take 7 us whatever they do: from about 2,048 tokens of
+  // 2,048 channels on (256 of 1,024 2.6 us with one token a thread, 7.4 with eight; 768 of 6,144 11.9 | 10.1).
+  const long long sums = (long long)n_tokens * channels;
+  if ((sums >= 100000 || (n_tokens >= 64 && channels >= 1024)) && taps == 4 && channels % 8 == 0 && ld % 8 == 0 && off % 8 == 0 &&
       !(((uintptr_t)proj | (uintptr_t)weight | (uintptr_t)bias | (uintptr_t)conv_state | (uintptr_t)out) & 15)) {
-    // (few tokens: a token a thread, more blocks)
-    const int per = n_tokens >= 256 ? 8 : 1;
+    const int per = sums >= 4000000 ? 8 : 1;
     launch_chained(per == 8 ? conv_silu_vec_kernel<4, 8> : conv_silu_vec_kernel<4, 1>,
                    dim3((n_tokens + per - 1) / per, (channels / 8 + 127) / 128), dim3(128), 0, (cudaStream_t)stream, (const elem_t*)proj,
                    ld, off, channels, (const elem_t*)weight, (const elem_t*)bias, conv_state, seq_of_token, seq_starts, state_slots,

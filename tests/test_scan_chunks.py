@@ -246,14 +246,16 @@ def test_short_convolution_by_eight_channels(lens):
             at += length
 
 
-@pytest.mark.parametrize("lens", [[8], [255, 3], [1] * 9, [9, 300]])
-def test_short_convolution_has_the_bits_of_the_general_kernel(lens):
-    """Rows whose length is no multiple of eight take the general kernel: the same numbers in such rows give the same bits."""
+@pytest.mark.parametrize("lens,channels", [([64], 1024), ([255, 3, 1], 1024), ([1] * 65, 1536), ([9, 300, 1], 2048), ([3, 15], 6144),
+                                           ([1000, 1, 2, 997, 50], 2048), ([301, 1, 350], 6152)])
+def test_short_convolution_has_the_bits_of_the_general_kernel(lens, channels):
+    """Rows whose length is no multiple of eight take the general kernel: the same numbers in such rows give the same bits, with one token a
+    thread and (from four million sums on) with eight."""
     from edgerag_b200.ops import kernels
 
-    n, channels, off = sum(lens), 72, 16
+    n, off = sum(lens), 16
     g = torch.Generator().manual_seed(n)
-    proj = torch.randn(n, 100, generator=g).to(torch.bfloat16).cuda()
+    proj = torch.randn(n, channels + 28, generator=g).to(torch.bfloat16).cuda()
     weight, bias = torch.randn(channels, 4, generator=g).to(torch.bfloat16).cuda(), torch.randn(channels, generator=g).to(torch.bfloat16).cuda()
     record = torch.randn(len(lens), 3, channels, generator=g).cuda()
     starts = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32).cuda()
@@ -261,7 +263,7 @@ def test_short_convolution_has_the_bits_of_the_general_kernel(lens):
     held = torch.arange(len(lens), dtype=torch.int32).cuda()
     for b in (bias, None):
         outs = [torch.empty(n, channels, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
-        for rows, out in zip((proj[:, :96].contiguous(), proj), outs):
+        for rows, out in zip((proj[:, : channels + 24].contiguous(), proj), outs):
             kernels.conv_silu(rows, off, weight, b, record, seq, starts, held, out)
         assert torch.equal(*outs)
 
