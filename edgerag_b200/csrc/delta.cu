@@ -340,9 +340,9 @@ head_norm_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ gat
 // are (their lengths are factors of rows and columns); every other operand goes in as three bfloat16 pieces (mma_split.cuh), so
 // that nothing is rounded to 16 bits.  c is summed in double and kept as two floats.
 //
-// What bounds it: the three dependent phases of a chunk, and the 64 KB of operands a block reads of it.  The walk took 0.49 us
-// a token (2,048 tokens of 16 heads of 128 x 128: 1,011 us
-// behind 24 us of preparing); the chunks 3.7 us for 64 tokens (142 us for both kernels).  Error against float64: 1.7e-7, as the walk's.
+// What bounds it: the three dependent phases of a chunk, and the 64 KB of operands a block reads of it.  The walk takes 0.46 us
+// a token (2,048 tokens of 16 heads of 128 x 128: 971 us with its preparing); the chunks 3.5 us for 64 tokens (144 us for both
+// kernels).  Error against float64: 1.7e-7, as the walk's.
 constexpr int kChunk = 64, kChunkCols = 16, kChunkWarps = 16, kChunkPrepWarps = 8;
 constexpr int kPieceElems = kChunk * kChunk;
 
@@ -832,7 +832,7 @@ inline long long chunk_scratch_floats(int n_tokens, int n_seqs, int H, int G, in
 }
 
 // Whether the chunks are the faster form: both costs in microseconds, fitted to the times of 1 to 64 requests of 2 to 500 tokens
-// (4 to 16 heads of 64 x 48 and 128 x 128).  The walk costs 0.49 us a token of the longest portion or, when the GPU is full,
+// (4 to 16 heads of 64 x 48 and 128 x 128).  The walk is taken for 0.49 us a token of the longest portion (0.46 now) or, when the GPU is full,
 // its blocks' tokens and states; the chunks cost two more launches, 3.7 us a chunk of the longest portion or, when the GPU is
 // full, a share of an SM for every chunk, be it full or not, and requests of one token are then walked by themselves.  One
 // request: from 34 tokens on (8 heads of 128 x 128: 28 tokens 16.3 us walked, 20.0 in a chunk; 32 17.3 | 20.0; 36 18.8 | 20.1;
