@@ -1,12 +1,13 @@
 // Decode attention (one new token per sequence) for bfloat16: keys and values streamed from the cache
 // pages by the asynchronous copy engines.  Two kernels share the split-KV scheme and the scratch layout
-// of the general kernel: one for a single query head per kv head (CUDA cores, bulk copies), one for
-// grouped query heads (tensor cores, TMA tensor copies).
+// of the general kernel: one on CUDA cores (bulk copies; any number of query heads per kv head), one on tensor cores for heads
+// of 64 (TMA tensor copies).
 #include <stdarg.h>
 #include <stdio.h>
 
 #undef ERB_ELEM
 #define ERB_ELEM 1
+#include "mma_split.cuh"
 #include "tc_common.cuh"
 
 using namespace erb;
@@ -19,8 +20,9 @@ ERB_DEFINE_LAST_ERROR(erb_last_error)
 // A block owns one (split of keys, kv head, sequence) and all query heads of that kv head's group.
 // The keys and values of its split arrive in shared memory through cp.async.bulk copies of whole
 // page segments (one contiguous run of rows per page), kStages stages deep, each stage signalled by
-// an mbarrier with a transaction count; four warps consume a stage while the next ones are in
-// flight, so the bytes in flight per SM are set by the pipeline depth, not by registers.
+// an mbarrier with a transaction count; eight warps consume a stage while the next ones are in
+// flight, so the bytes in flight per SM are set by the pipeline depth, not by registers.  The first warp asks for the copies, a page
+// a lane, once the stage's eight warps have left it.
 // Inside a stage a key is handled by D/8 lanes (16 bytes each); the dot product is finished with
 // shuffles and every lane keeps the running max, denominator and 8 accumulators of its slice.
 // Partial results go to the same scratch layout as the general kernel; a combine kernel merges the
@@ -84,48 +86,62 @@ __device__ __forceinline__ void merge_splits_if_last(int* counter, const float* 
                                                      __nv_bfloat16* o, const __nv_bfloat16* gate) {
   __shared__ int s_last;
   __shared__ float s_w[kMergeWarps][kCombineMaxSplits];     // the splits' weights, per warp
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0) {                                   // (the barrier has ordered the block's results before this fence)
+    __threadfence();
     const int last = atomicAdd(counter, 1) == n_splits - 1;
     if (last) atomicExch(counter, 0);
+    __threadfence();
     s_last = last;
   }
   __syncthreads();
   if (!s_last) return;
-  __threadfence();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
   if (warp >= kMergeWarps) return;
   float* w = s_w[warp];
+  // A lane owns D / 32 neighbouring elements, so that a split costs it one load and many are in flight; the first kAhead
+  // splits' are asked for before the weights are there.
+  constexpr int V = D / 32, kAhead = 8;
+  auto load = [&](const float* src, float* x) {
+    if constexpr (V == 4) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(src));
+      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    } else if constexpr (V == 2) {
+      const float2 v = __ldcg(reinterpret_cast<const float2*>(src));
+      x[0] = v.x; x[1] = v.y;
+    } else {
+      x[0] = __ldcg(src);
+    }
+  };
   for (int h = warp; h < n_heads; h += min(n_warps, kMergeWarps)) {
     const size_t base = (head0 + h) * max_splits;
+    const float* src = part_acc + base * D + lane * V;
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
     if (lane < n_splits) { m0 = __ldcg(part_ml + (base + lane) * 2); l0 = __ldcg(part_ml + (base + lane) * 2 + 1); }
     if (lane + 32 < n_splits) { m1 = __ldcg(part_ml + (base + lane + 32) * 2); l1 = __ldcg(part_ml + (base + lane + 32) * 2 + 1); }
+    float first[kAhead][V];
+#pragma unroll
+    for (int sp = 0; sp < kAhead; ++sp)
+      if (sp < n_splits) load(src + (size_t)sp * D, first[sp]);
     const float m = warp_max(fmaxf(m0, m1));
     const float w0 = lane < n_splits ? exp2f(m0 - m) : 0.f, w1 = lane + 32 < n_splits ? exp2f(m1 - m) : 0.f;
     w[lane] = w0;
     w[lane + 32] = w1;
     const float inv = 1.f / warp_sum(l0 * w0 + l1 * w1);
     __syncwarp();
-    // A lane owns D / 32 neighbouring elements, so that a split costs it one load and many are in flight.
-    constexpr int V = D / 32;
     float sum[V];
 #pragma unroll
     for (int i = 0; i < V; ++i) sum[i] = 0.f;
-    const float* src = part_acc + base * D + lane * V;
-#pragma unroll 8
-    for (int sp = 0; sp < n_splits; ++sp) {
-      float x[V];
-      if constexpr (V == 4) {
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(src + (size_t)sp * D));
-        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-      } else if constexpr (V == 2) {
-        const float2 v = __ldcg(reinterpret_cast<const float2*>(src + (size_t)sp * D));
-        x[0] = v.x; x[1] = v.y;
-      } else {
-        x[0] = __ldcg(src + (size_t)sp * D);
+#pragma unroll
+    for (int sp = 0; sp < kAhead; ++sp)
+      if (sp < n_splits) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) sum[i] += first[sp][i] * w[sp];
       }
+#pragma unroll 8
+    for (int sp = kAhead; sp < n_splits; ++sp) {
+      float x[V];
+      load(src + (size_t)sp * D, x);
 #pragma unroll
       for (int i = 0; i < V; ++i) sum[i] += x[i] * w[sp];
     }
@@ -143,7 +159,7 @@ attention_decode_bulk_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stri
                              const int* __restrict__ block_tables, int max_pages,
                              const int* __restrict__ token_of_seq, const int* __restrict__ positions,
                              float* __restrict__ part_acc, float* __restrict__ part_ml, int max_splits, int nq,
-                             int nkv, int page_size, int split_keys, float scale_log2, int hg,
+                             int nkv, int page_size, int page_shift, int split_keys, float scale_log2, int hg,
                              __nv_bfloat16* __restrict__ out, int out_row_stride, int* __restrict__ status,
                              int* __restrict__ counters, int window, int keep_first, const float* __restrict__ penalty, float softcap,
                              const __nv_bfloat16* __restrict__ gate, int gate_stride) {
@@ -163,8 +179,9 @@ attention_decode_bulk_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stri
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 127u) & ~127u;
   uint8_t* smem = smem_raw + (base - raw);
-  // layout: K stages | V stages | barriers | merge area | page ids
-  const uint32_t sK = base, sV = base + kStages * STAGE_BYTES, sBar = sV + kStages * STAGE_BYTES;
+  // layout: K stages | V stages | barriers (stage there, stage free again), abort flag | merge area | page ids
+  const uint32_t sK = base, sV = base + kStages * STAGE_BYTES, sBar = sV + kStages * STAGE_BYTES, sEmpty = sBar + 8 * kStages;
+  volatile int* s_abort = reinterpret_cast<volatile int*>(smem + 2 * kStages * STAGE_BYTES + 56);
   float* merge = reinterpret_cast<float*>(smem + 2 * kStages * STAGE_BYTES + 64);   // [warps][R][D + 2]
   int* s_pages = reinterpret_cast<int*>(merge + kDecWarps * R * (D + 2));
 
@@ -201,61 +218,57 @@ attention_decode_bulk_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stri
 
   if (tid == 0) {
 #pragma unroll
-    for (int s = 0; s < kStages; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sBar + 8 * s));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(sBar + 8 * s, 1);
+      mbar_init(sEmpty + 8 * s, kDecWarps);
+    }
+    *s_abort = 0;
+    mbar_init_fence();
   }
-  // The block table entries of the split, fetched by all threads at once: the thread that issues
+  // The block table entries of the split, fetched by all threads at once: the warp that issues
   // the copies must not wait on a global load per page.
-  const int first_page = begin / page_size;
-  const int n_pages = (end - 1) / page_size - first_page + 1;
+  auto page_of = [&](int key) { return page_shift >= 0 ? key >> page_shift : key / page_size; };
+  const int first_page = page_of(begin);
+  const int n_pages = page_of(end - 1) - first_page + 1;
   for (int i = tid; i < n_pages; i += kDecThreads) s_pages[i] = bt[first_page + i];
   int* s_kept = s_pages + split_keys / page_size + 2;     // the pages of the kept keys
   for (int i = tid; i * page_size < kept; i += kDecThreads) s_kept[i] = bt[i];
   __syncthreads();
 
-  auto issue = [&](int tile) {   // thread 0 only
+  // The whole first warp: every lane asks for a page's keys or values of its own (one thread took 250 clocks a copy).
+  auto issue = [&](int tile) {
     const int s = tile % kStages;
     const int kb = tile_begin(tile), ke = tile_end(tile);
     const int* pages_of_tile = tile < kept_tiles ? s_kept : s_pages - first_page;
-    const uint32_t bar = sBar + 8 * s;
-    if (hg == 1) {
-      // one head: copy exactly the visible keys, one run per page
-      mbar_expect(bar, (uint32_t)(ke - kb) * ROW * 2);
-      int k = kb;
-      while (k < ke) {
-        const int page = pages_of_tile[k / page_size], off = k % page_size;
-        const int n = min(page_size - off, ke - k);
-        const size_t src = (((size_t)page * nkv + kvh0) * page_size + off) * D;
-        const uint32_t dst = (uint32_t)(s * STAGE_BYTES + (k - kb) * ROW);
-        bulk_copy(sK + dst, k_pages + src, (uint32_t)n * ROW, bar);
-        bulk_copy(sV + dst, v_pages + src, (uint32_t)n * ROW, bar);
-        k += n;
-      }
-    } else {
-      // hg heads: whole pages (kb is a multiple of page_size), hg * page_size rows per copy
-      const int n_pg = (ke - kb + page_size - 1) / page_size;
-      const uint32_t slot_bytes = (uint32_t)(hg * page_size) * ROW;         // room of one page in the stage
-      const uint32_t chunk_bytes = (uint32_t)(hg_here * page_size) * ROW;   // what one page brings
-      mbar_expect(bar, (uint32_t)n_pg * chunk_bytes * 2);
-      for (int j = 0; j < n_pg; ++j) {
-        const int page = pages_of_tile[kb / page_size + j];
-        const size_t src = ((size_t)page * nkv + kvh0) * page_size * D;
-        const uint32_t dst = (uint32_t)(s * STAGE_BYTES) + (uint32_t)j * slot_bytes;
-        bulk_copy(sK + dst, k_pages + src, chunk_bytes, bar);
-        bulk_copy(sV + dst, v_pages + src, chunk_bytes, bar);
+    const uint32_t bar = sBar + 8 * s, stage = (uint32_t)(s * STAGE_BYTES);
+    const int page0 = page_of(kb), n_copies = 2 * (page_of(ke - 1) - page0 + 1);
+    // one head: exactly the visible keys, one run per page; hg heads: whole pages (kb is a multiple of page_size), hg * page_size
+    // rows per copy, of which there are hg_here
+    const uint32_t slot_bytes = (uint32_t)(hg * page_size) * ROW, chunk_bytes = (uint32_t)(hg_here * page_size) * ROW;
+    if (lane == 0) mbar_expect(bar, hg == 1 ? (uint32_t)(ke - kb) * ROW * 2 : (uint32_t)n_copies * chunk_bytes);
+    __syncwarp();
+    for (int c = lane; c < n_copies; c += 32) {
+      const int j = c >> 1, page = pages_of_tile[page0 + j];
+      const __nv_bfloat16* pool = c & 1 ? v_pages : k_pages;
+      const uint32_t to = (c & 1 ? sV : sK) + stage;
+      const size_t rows0 = ((size_t)page * nkv + kvh0) * page_size;
+      if (hg == 1) {
+        const int page_key = (page0 + j) * page_size, k0 = max(kb, page_key), k1 = min(ke, page_key + page_size);
+        bulk_copy(to + (uint32_t)(k0 - kb) * ROW, pool + (rows0 + (k0 - page_key)) * D, (uint32_t)(k1 - k0) * ROW, bar);
+      } else {
+        bulk_copy(to + (uint32_t)j * slot_bytes, pool + rows0 * D, chunk_bytes, bar);
       }
     }
+    __syncwarp();
   };
   // Tiles that end before the page of the new token hold nothing this step has written.
-  const int old_end = (pos / page_size) * page_size;
+  const int old_end = page_of(pos) * page_size;
   int issued = 0;
-  if (tid == 0) {
+  if (warp == 0)
     while (issued < kStages && issued < n_tiles && tile_end(issued) <= old_end) issue(issued++);
-  }
   chain_wait();
-  if (tid == 0) {
-    for (int i = issued; i < kStages && i < n_tiles; ++i) issue(i);
-  }
+  if (warp == 0)
+    for (; issued < kStages && issued < n_tiles; ++issued) issue(issued);
 
   // This lane's slice of every query head of the group, pre-multiplied by scale * log2(e).
   const int sub = lane / LPK, chunk = lane % LPK;
@@ -281,7 +294,6 @@ attention_decode_bulk_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stri
     for (int i = 0; i < 8; ++i) acc[g][i] = 0.f;
   }
 
-  bool ok = true;
   // this lane group's first key (of its head) inside a stage, and where that row sits in the stage:
   // with hg > 1 a stage holds pages one after the other, each page holding its hg heads in turn
   const int key_in_stage = ((warp % warps_per_head) * GPW + sub) * kKeysPerGroup;
@@ -291,14 +303,17 @@ attention_decode_bulk_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stri
   const uint32_t group_mask = (LPK == 32 ? 0xffffffffu : ((1u << LPK) - 1u)) << (sub * LPK);   // lanes of this key group
   for (int tile = 0; tile < n_tiles; ++tile) {
     const int s = tile % kStages;
-    if (ok && !mbar_wait(sBar + 8 * s, (tile / kStages) & 1)) ok = false;
-    const int n_here = tile_end(tile) - tile_begin(tile);
-    if (ok && serves && key_in_stage < n_here) {
-      // keys of the first page that lie before the window and are not kept (only where whole pages are copied)
-      const int key0 = tile_begin(tile) + key_in_stage;
+    if (!__all_sync(0xffffffffu, mbar_wait_or_abort(sBar + 8 * s, (tile / kStages) & 1, s_abort))) break;
+    const int tile0 = tile_begin(tile), n_here = tile_end(tile) - tile0;
+    if (serves && key_in_stage < n_here) {
+      const int key0 = tile0 + key_in_stage;
+      // a tile with keys that are not seen: past its end, or of the window's first page before the window and not kept (only where
+      // whole pages are copied)
+      const bool partial = n_here < STAGE_KEYS || tile0 < k_lo;
       bool hidden[kKeysPerGroup];
 #pragma unroll
-      for (int u = 0; u < kKeysPerGroup; ++u) hidden[u] = key_in_stage + u >= n_here || (key0 + u < k_lo && key0 + u >= keep_first);
+      for (int u = 0; u < kKeysPerGroup; ++u)
+        hidden[u] = partial && (key_in_stage + u >= n_here || (key0 + u < k_lo && key0 + u >= keep_first));
       const uint8_t* kt = smem + s * STAGE_BYTES + row_offset + chunk * 16;
       const uint8_t* vt = kt + kStages * STAGE_BYTES;
       uint4 kraw[kKeysPerGroup];
@@ -340,10 +355,10 @@ attention_decode_bulk_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stri
         }
         // (all of the group's keys may be hidden so far: exponentials are then taken against 0 and are 0)
         const float m_ref = m_new == -INFINITY ? 0.f : m_new;
-        const float a = exp2f(m_run[g] - m_ref);
+        const float a = fast_exp2(m_run[g] - m_ref);
         float sum = 0.f;
 #pragma unroll
-        for (int u = 0; u < kKeysPerGroup; ++u) { p[g][u] = exp2f(sc[g][u] - m_ref); sum += p[g][u]; }
+        for (int u = 0; u < kKeysPerGroup; ++u) { p[g][u] = fast_exp2(sc[g][u] - m_ref); sum += p[g][u]; }
         l_run[g] = l_run[g] * a + sum;
         m_run[g] = m_new;
 #pragma unroll
@@ -364,8 +379,12 @@ attention_decode_bulk_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stri
         }
       }
     }
-    __syncthreads();                                        // everyone is done with stage s
-    if (tid == 0 && ok && tile + kStages < n_tiles) issue(tile + kStages);
+    __syncwarp();                                           // this warp is done with stage s
+    if (lane == 0) mbar_arrive(sEmpty + 8 * s);
+    if (warp == 0 && tile + kStages < n_tiles) {            // (the other warps run ahead as far as the stages reach)
+      if (!__all_sync(0xffffffffu, mbar_wait_or_abort(sEmpty + 8 * s, (tile / kStages) & 1, s_abort))) break;
+      issue(issued++);
+    }
   }
 
   // Merge the lane groups of each warp (lanes that share `chunk`), then the warps.
@@ -394,7 +413,9 @@ attention_decode_bulk_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stri
   }
   const __nv_bfloat16* gate_row = SHAPED && gate ? gate + (size_t)t * gate_stride : nullptr;
   __syncthreads();
-  if (!ok) {
+  if (*s_abort) {
+    if (tid == 0)                                           // copies under way land before the block leaves
+      for (int i = max(0, issued - kStages); i < issued; ++i) mbar_wait(sBar + 8 * (i % kStages), (i / kStages) & 1);
     if (tid == 0) atomicCAS(status, 0, 2000000 + (int)blockIdx.x);
     return;
   }
@@ -488,6 +509,13 @@ int decode_head_group(int nkv, int head_dim, int page_size, int split_keys, int 
   return hg;
 }
 
+// log2 of a page size that is a power of two, else -1.
+inline int page_shift(int page_size) {
+  int s = 0;
+  while ((1 << s) < page_size) ++s;
+  return (1 << s) == page_size ? s : -1;
+}
+
 template <int D, int R>
 int launch_decode_bulk(const void* q, int q_row_stride, const void* k_pages, const void* v_pages,
                        const int* block_tables, int max_pages, const int* token_of_seq, const int* positions,
@@ -512,8 +540,8 @@ int launch_decode_bulk(const void* q, int q_row_stride, const void* k_pages, con
   }
   launch_chained(kern, dim3(dim3(max_splits, (nkv + hg - 1) / hg, n_seqs)), dim3(kDecThreads), smem, s, (const __nv_bfloat16*)q, q_row_stride,
       (const __nv_bfloat16*)k_pages, (const __nv_bfloat16*)v_pages, block_tables, max_pages, token_of_seq, positions,
-      part_acc, part_ml, max_splits, nq, nkv, page_size, split_keys, scale_log2, hg, (__nv_bfloat16*)out, out_row_stride, status, counters,
-      window, keep_first, penalty, softcap, (const __nv_bfloat16*)gate, gate_stride);
+      part_acc, part_ml, max_splits, nq, nkv, page_size, page_shift(page_size), split_keys, scale_log2, hg, (__nv_bfloat16*)out, out_row_stride,
+      status, counters, window, keep_first, penalty, softcap, (const __nv_bfloat16*)gate, gate_stride);
   return check_launch("attention_decode_bulk");
 }
 
@@ -537,12 +565,11 @@ int dispatch_group(int r, const void* q, int q_row_stride, const void* k_pages, 
 }  // namespace
 
 // =============================================================================================
-// Decode attention for grouped query heads (2 to 8 query heads per kv head) on tensor cores.
+// Decode attention for heads of 64 (1 to 8 query heads per kv head) on tensor cores.
 //
-// With several query heads per kv head the CUDA-core kernel above does its arithmetic once per
-// query head and key and falls behind the memory (3.4 TB/s at three heads per kv head).  Here the
-// query heads of a kv head are the rows of an mma.sync.m16n8k16 tile, so a key costs the same
-// whatever their number:
+// The CUDA-core kernel above does its arithmetic once per query head and key: with three heads per kv head it reaches 3.4 TB/s, and
+// with one a tile of 16 keys a warp takes 1,250 clocks where its bytes take 700 (8 sequences of 520 tokens, traced in place).  Here the
+// query heads of a kv head are the rows of an mma.sync.m16n8k16 tile, so a key costs the same whatever their number:
 //
 //   S[heads x 8 keys]   = Q[heads x 64] K^T       A = Q from registers, B = K rows via ldmatrix
 //   O[heads x 64]      += P[heads x 16 keys] V    A = P from the S registers, B = V via ldmatrix.trans
@@ -554,6 +581,10 @@ int dispatch_group(int r, const void* q, int q_row_stride, const void* k_pages, 
 // path: pages are brought in by TMA tensor copies (cp.async.bulk.tensor.2d) through tensor maps
 // over the page pools with the 128-byte swizzle, so that the ldmatrix reads of 8 rows x 16 bytes
 // touch all banks.  bfloat16, head size 64, pages of a multiple of 8 tokens.
+//
+// Measured with equal splits (one layer with its projections and norm): 8 sequences of 8,192 tokens of 32 heads 103 us by the kernel
+// above in splits at multiples of 2,048, 93.7 us here (a decode step at 520 tokens 1,162 | 1,139 us); 64 of 7,531 tokens of 15 heads
+// over 5 132 | 122 us here with splits at multiples of 2,048 | equal splits.
 // =============================================================================================
 namespace {
 
@@ -584,7 +615,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-template <bool SHAPED>
+// SINGLE: one query head per kv head.  Its weights go into the second product as three bfloat16 pieces, which lose nothing, in three
+// rows of the tile (a tile of one row costs as much); the rows of the result are added at the end.
+template <bool SHAPED, bool SINGLE>
 __global__ void __launch_bounds__(kGqaThreads, 2)
 attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                             const __grid_constant__ CUtensorMap map_k_last, const __grid_constant__ CUtensorMap map_v_last,
@@ -592,12 +625,12 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                             const int* __restrict__ block_tables, int max_pages,
                             const int* __restrict__ token_of_seq, const int* __restrict__ positions,
                             float* __restrict__ part_acc, float* __restrict__ part_ml, int max_splits, int nq,
-                            int nkv, int page_size, int split_keys, float scale_log2, int hg,
+                            int nkv, int page_size, int split_most, int even_splits, float scale_log2, int hg,
                             __nv_bfloat16* __restrict__ out, int out_row_stride, int* __restrict__ status,
                             int* __restrict__ counters, int window, int keep_first, const float* __restrict__ penalty, float softcap,
                             const __nv_bfloat16* __restrict__ gate, int gate_stride) {
   constexpr int D = 64;
-  const int R = nq / nkv;
+  const int R = SINGLE ? 1 : nq / nkv;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;            // the swizzle repeats every 1024 bytes
@@ -620,6 +653,9 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   const int pos = positions[t];
   // A window: as in the kernel above (whole pages are copied, so the first split starts at the page of the window's
   // first key, the keys before it are masked, and the first split walks the kept keys first).
+  // even_splits: a sequence's keys are cut into max_splits equal parts (whole pages, split_most keys at most), else at multiples of
+  // split_most.
+  const int split_keys = even_splits ? ((pos + max_splits) / max_splits + page_size - 1) / page_size * page_size : split_most;
   const int k_lo = first_visible_key(pos, window);   // (a negative window: a mask of chunks of -window positions)
   const int first_split = k_lo / split_keys;
   const int k_first = (k_lo / page_size) * page_size;
@@ -647,7 +683,7 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   const int first_page = begin / page_size;
   const int n_pages = (end - 1) / page_size - first_page + 1;
   for (int i = tid; i < n_pages; i += kGqaThreads) s_pages[i] = bt[first_page + i];
-  int* s_kept = s_pages + split_keys / page_size + 2;     // the pages of the kept keys
+  int* s_kept = s_pages + split_most / page_size + 2;     // the pages of the kept keys
   for (int i = tid; i * page_size < kept; i += kGqaThreads) s_kept[i] = bt[i];
   __syncthreads();
   // A wait that gives up when its own limit runs out or when another thread of the block has given up.
@@ -702,12 +738,13 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   }
   chain_wait();
 
-  // Q of this warp's kv head as the A operand: row g = lane / 4 is query head g of the group.
+  // Q of this warp's kv head as the A operand: row g = lane / 4 is query head g of the group (SINGLE: piece g of the one head).
   const int g = lane >> 2, j = lane & 3;
+  const int q_head = (kvh0 + hh) * R + (SINGLE ? 0 : g);
+  const bool real = serves && g < (SINGLE ? 3 : R);
   uint32_t qa[4][2];
   {
-    const bool real = serves && g < R;
-    const __nv_bfloat16* qp = q + (size_t)t * q_row_stride + (size_t)((real ? (kvh0 + hh) * R + g : 0)) * D;
+    const __nv_bfloat16* qp = q + (size_t)t * q_row_stride + (size_t)(real ? q_head : 0) * D;
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       qa[ks][0] = real ? *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 2 * j) : 0u;
@@ -717,7 +754,7 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   const bool shaped = SHAPED && (penalty || softcap > 0.f), capped = softcap > 0.f;      // something is done to the scores
   Penalty2 pen;                               // (a cap keeps its two numbers in the penalty's place)
   if (SHAPED && capped) { pen.r1 = softcap * 1.4426950408889634f; pen.r2 = 2.f / softcap; }
-  else if (SHAPED && serves && g < R) pen.load(penalty, (kvh0 + hh) * R + g, nq);
+  else if (SHAPED && real) pen.load(penalty, q_head, nq);
   float o[8][4];
 #pragma unroll
   for (int nb = 0; nb < 8; ++nb)
@@ -765,14 +802,15 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         }
       }
       // this lane: row g, keys key0 + 8 b + 2 j, + 1
+      // (hidden: keys past the split's end, and keys of the window's first page that lie before the window and are not kept)
+      const bool partial = n_here < stage_keys || key_abs0 < k_lo;
       float m_new = m_run;
 #pragma unroll
       for (int b = 0; b < 2; ++b)
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const int key = key0 + 8 * b + 2 * j + i;
-          // (keys past the split's end, and keys of the window's first page that lie before the window and are not kept)
-          const bool seen = key < n_here && !(key_abs0 + key < k_lo && key_abs0 + key >= keep_first);
+          const bool seen = !partial || (key < n_here && !(key_abs0 + key < k_lo && key_abs0 + key >= keep_first));
           sc[b][i] *= scale_log2;
           if (shaped) sc[b][i] = capped ? capped_score(sc[b][i] * pen.r2, pen.r1) : sc[b][i] - pen.at(pos - (key_abs0 + key));
           if (!seen) sc[b][i] = -INFINITY;
@@ -782,15 +820,25 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
       m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 2));
       // (all of the row's keys may be hidden so far: exponentials are then taken against 0 and are 0)
       const float m_ref = m_new == -INFINITY ? 0.f : m_new;
-      const float a = exp2f(m_run - m_ref);
+      const float a = fast_exp2(m_run - m_ref);
       float p[2][2], sum = 0.f;
 #pragma unroll
       for (int b = 0; b < 2; ++b)
 #pragma unroll
-        for (int i = 0; i < 2; ++i) { p[b][i] = exp2f(sc[b][i] - m_ref); sum += p[b][i]; }
+        for (int i = 0; i < 2; ++i) { p[b][i] = fast_exp2(sc[b][i] - m_ref); sum += p[b][i]; }
       l_run = l_run * a + sum;
       m_run = m_new;
-      const uint32_t pa0 = pack_bf16(p[0][0], p[0][1]), pa2 = pack_bf16(p[1][0], p[1][1]);
+      uint32_t pa0, pa2;
+      if (SINGLE) {                                         // (the rows behind the pieces are never looked at)
+        uint32_t piece[2][3];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) split_pair(p[b][0], p[b][1], piece[b]);
+        pa0 = g == 0 ? piece[0][0] : g == 1 ? piece[0][1] : piece[0][2];
+        pa2 = g == 0 ? piece[1][0] : g == 1 ? piece[1][1] : piece[1][2];
+      } else {
+        pa0 = pack_bf16(p[0][0], p[0][1]);
+        pa2 = pack_bf16(p[1][0], p[1][1]);
+      }
 #pragma unroll
       for (int nb = 0; nb < 8; ++nb) { o[nb][0] *= a; o[nb][1] *= a; }
       // O += P V over the 16 keys: matrices (keys 0..7 | 8..15) x (8 values of chunk nb | nb + 1)
@@ -810,6 +858,16 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   // The row's sum over its four lanes; then this warp's result for its query heads.
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
+  if (SINGLE) {
+#pragma unroll
+    for (int nb = 0; nb < 8; ++nb)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float first = o[nb][i];
+        const float sum = (__shfl_down_sync(0xffffffffu, first, 8) + __shfl_down_sync(0xffffffffu, first, 4)) + first;
+        o[nb][i] = fabsf(first) < INFINITY ? sum : first;   // (the first piece is zero only where the weight is: its sum alone has the value's kind)
+      }
+  }
   if (warp < kDecWarps && g < R) {
     float* w = merge + (warp * R + g) * (D + 2);
 #pragma unroll
@@ -822,31 +880,76 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     if (tid == 0) atomicCAS(status, 0, 2000000 + (int)blockIdx.x);
     return;
   }
-  for (int idx = tid; idx < hg_here * R * D; idx += kGqaThreads) {
-    const int head = idx / (R * D), gq = (idx / D) % R, d = idx % D;
-    const int w0 = head * warps_per_head;
+  // a warp per (kv head, query head), two values a lane
+  for (int row = warp; row < hg_here * R; row += kGqaThreads / 32) {
+    const int head = row / R, gq = row - head * R;
+    const float* from = merge + (head * warps_per_head * R + gq) * (D + 2);     // one of the head's warps, R * (D + 2) floats before the next
     float m = -INFINITY;
-    for (int w = w0; w < w0 + warps_per_head; ++w) m = fmaxf(m, merge[(w * R + gq) * (D + 2) + D]);
-    float sum = 0.f, l = 0.f;
-    for (int w = w0; w < w0 + warps_per_head; ++w) {
-      const float mw = merge[(w * R + gq) * (D + 2) + D];
-      const float f = (mw == -INFINITY) ? 0.f : exp2f(mw - m);
-      sum += merge[(w * R + gq) * (D + 2) + d] * f;
-      l += merge[(w * R + gq) * (D + 2) + D + 1] * f;
+    for (int w = 0; w < warps_per_head; ++w) m = fmaxf(m, from[w * R * (D + 2) + D]);
+    float2 sum = make_float2(0.f, 0.f);
+    float l = 0.f;
+    for (int w = 0; w < warps_per_head; ++w) {
+      const float* x = from + w * R * (D + 2);
+      const float f = (x[D] == -INFINITY) ? 0.f : exp2f(x[D] - m);
+      sum.x += x[2 * lane] * f;
+      sum.y += x[2 * lane + 1] * f;
+      l += x[D + 1] * f;
     }
+    const int col = (kvh0 * R + row) * D + 2 * lane;
     if (max_splits == 1) {      // the only split: this is the result (what the combine kernel would make of it)
-      const int col = ((kvh0 + head) * R + gq) * D + d;
-      out[(size_t)t * out_row_stride + col] = gated(sum * (1.f / l), gate_row, col);
+      const float inv = 1.f / l;
+      __nv_bfloat16* to = out + (size_t)t * out_row_stride + col;
+      to[0] = gated(sum.x * inv, gate_row, col);
+      to[1] = gated(sum.y * inv, gate_row, col + 1);
       continue;
     }
-    const size_t slot = ((size_t)seq * nq + (kvh0 + head) * R + gq) * max_splits + split;
-    part_acc[slot * D + d] = sum;
-    if (d == 0) { part_ml[slot * 2] = m; part_ml[slot * 2 + 1] = l; }
+    const size_t slot = ((size_t)seq * nq + kvh0 * R + row) * max_splits + split;
+    *reinterpret_cast<float2*>(part_acc + slot * D + 2 * lane) = sum;
+    if (lane == 0) *reinterpret_cast<float2*>(part_ml + slot * 2) = make_float2(m, l);
   }
   if (max_splits > 1 && counters)
     merge_splits_if_last<D>(counters + (size_t)seq * gridDim.y + blockIdx.y, part_acc, part_ml,
                             (size_t)seq * nq + (size_t)kvh0 * R, hg_here * R, min(pos / split_keys - first_split + 1, max_splits), max_splits,
                             out + (size_t)t * out_row_stride + (size_t)kvh0 * R * D, gate_row ? gate_row + kvh0 * R * D : nullptr);
+}
+
+// Whether the kernel above takes these sizes with hg kv heads per block.
+bool decode_mma_fits(int nkv, int page_size, int split_keys, int hg) {
+  return page_size > 0 && page_size % 8 == 0 && split_keys > 0 && split_keys % page_size == 0 && hg > 0 && hg <= kDecWarps &&
+         (kGqaStageRows / hg) % page_size == 0 && hg * page_size <= 256;
+}
+
+int launch_decode_mma(const void* q, int q_row_stride, const void* k_pages, const void* v_pages, int n_pool_pages,
+                      const int* block_tables, int max_pages, const int* token_of_seq, const int* positions, void* out,
+                      int out_row_stride, float* part_acc, float* part_ml, int max_splits, int n_seqs, int nq, int nkv, int page_size,
+                      int split_keys, int even_splits, float scale_log2, int hg, int* status, int* counters, int window, int keep_first,
+                      const float* penalty, float softcap, const void* gate, int gate_stride, cudaStream_t s) {
+  const int last = nkv % hg ? nkv % hg : hg, r = nq / nkv;
+  if (window || !counters) even_splits = 0;
+  const unsigned long long rows = (unsigned long long)n_pool_pages * nkv * page_size;
+  CUtensorMap mk, mv, mkl, mvl;
+  int rc;
+  if ((rc = pool_map(&mk, k_pages, rows, (unsigned)(hg * page_size), "attention_decode")) || (rc = pool_map(&mv, v_pages, rows, (unsigned)(hg * page_size), "attention_decode")) ||
+      (rc = pool_map(&mkl, k_pages, rows, (unsigned)(last * page_size), "attention_decode")) || (rc = pool_map(&mvl, v_pages, rows, (unsigned)(last * page_size), "attention_decode")))
+    return rc;
+  const size_t smem = 1024 + 2 * kGqaStages * kGqaStageBytes + 64 + (size_t)kDecWarps * r * (64 + 2) * sizeof(float) + 128 +
+                      (size_t)(split_keys / page_size + 2 + (window > 0 ? keep_first / page_size + 1 : 0)) * sizeof(int);
+  if (smem > 200 * 1024) return fail(ERB_ERR_UNSUPPORTED, "attention_decode: split of %d keys in pages of %d", split_keys, page_size);
+  const int shaped = penalty || softcap > 0.f || gate, which = 2 * shaped + (r == 1);
+  auto kern = which == 0 ? attention_decode_gqa_kernel<false, false> : which == 1 ? attention_decode_gqa_kernel<false, true>
+            : which == 2 ? attention_decode_gqa_kernel<true, false> : attention_decode_gqa_kernel<true, true>;
+  static size_t configured_for[4] = {0, 0, 0, 0};
+  size_t& configured = configured_for[which];
+  if (smem > configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "attention_decode: %s", cudaGetErrorString(e));
+    configured = smem;
+  }
+  launch_chained(kern, dim3(dim3(max_splits, (nkv + hg - 1) / hg, n_seqs)), dim3(kGqaThreads), smem, s,
+                 mk, mv, mkl, mvl, (const __nv_bfloat16*)q, q_row_stride, block_tables, max_pages, token_of_seq, positions,
+                 part_acc, part_ml, max_splits, nq, nkv, page_size, split_keys, even_splits, scale_log2, hg, (__nv_bfloat16*)out,
+                 out_row_stride, status, counters, window, keep_first, penalty, softcap, (const __nv_bfloat16*)gate, gate_stride);
+  return check_launch("attention_decode");
 }
 
 }  // namespace
@@ -855,9 +958,8 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
 ERB_EXPORT int erb_attention_decode_gqa_supported(int nq, int nkv, int head_dim, int page_size, int split_keys) {
   if (head_dim != 64 || nq <= 0 || nkv <= 0 || nq % nkv) return 0;
   const int r = nq / nkv;
-  if (r < 2 || r > kGqaMaxHeads || page_size <= 0 || page_size % 8 || split_keys <= 0 || split_keys % page_size) return 0;
-  const int hg = decode_head_group(nkv, 64, page_size, split_keys);
-  return (kGqaStageRows / hg) % page_size == 0 && hg * page_size <= 256 && min(hg, nkv) * page_size <= 256;
+  if (r < 2 || r > kGqaMaxHeads || page_size <= 0 || split_keys <= 0) return 0;
+  return decode_mma_fits(nkv, page_size, split_keys, decode_head_group(nkv, 64, page_size, split_keys));
 }
 
 // Same contract as erb_attention_decode_bulk, for 2 to 8 query heads per kv head of size 64;
@@ -868,7 +970,7 @@ ERB_EXPORT int erb_attention_decode_gqa(const void* q, int q_row_stride, const v
                                         float* part_acc, float* part_ml, int max_splits, int n_seqs, int nq, int nkv,
                                         int head_dim, int page_size, int split_keys, float scale, int* status,
                                         int* counters, int window, int keep_first, const float* penalty, float softcap,
-                                        const void* gate, int gate_stride, void* stream) {
+                                        const void* gate, int gate_stride, int even_splits, void* stream) {
   if (n_seqs <= 0) return ERB_OK;
   if (penalty && softcap > 0.f) return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: a penalty and a cap of the scores exclude each other");
   keep_first = window > 0 && keep_first > 0 ? keep_first : 0;
@@ -884,38 +986,22 @@ ERB_EXPORT int erb_attention_decode_gqa(const void* q, int q_row_stride, const v
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: %d splits (at most %d)", max_splits, kCombineMaxSplits);
   if ((unsigned long long)n_pool_pages * nkv * page_size > 0x7fffffffull)
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: pool too large for 32-bit row coordinates");
-  const int hg = decode_head_group(nkv, 64, page_size, split_keys);
-  const int last = nkv % hg ? nkv % hg : hg;
-  const unsigned long long rows = (unsigned long long)n_pool_pages * nkv * page_size;
-  CUtensorMap mk, mv, mkl, mvl;
-  int rc;
-  if ((rc = pool_map(&mk, k_pages, rows, (unsigned)(hg * page_size), "attention_decode_gqa")) || (rc = pool_map(&mv, v_pages, rows, (unsigned)(hg * page_size), "attention_decode_gqa")) ||
-      (rc = pool_map(&mkl, k_pages, rows, (unsigned)(last * page_size), "attention_decode_gqa")) || (rc = pool_map(&mvl, v_pages, rows, (unsigned)(last * page_size), "attention_decode_gqa")))
-    return rc;
-  const int r = nq / nkv;
-  const size_t smem = 1024 + 2 * kGqaStages * kGqaStageBytes + 64 + (size_t)kDecWarps * r * (64 + 2) * sizeof(float) + 128 +
-                      (size_t)(split_keys / page_size + 2 + (window > 0 ? keep_first / page_size + 1 : 0)) * sizeof(int);
-  if (smem > 200 * 1024) return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: split of %d keys in pages of %d", split_keys, page_size);
-  const bool shaped = penalty || softcap > 0.f || gate;
-  auto kern = shaped ? attention_decode_gqa_kernel<true> : attention_decode_gqa_kernel<false>;
-  static size_t configured_for[2] = {0, 0};
-  size_t& configured = configured_for[shaped];
-  if (smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "attention_decode_gqa: %s", cudaGetErrorString(e));
-    configured = smem;
-  }
   cudaStream_t s = (cudaStream_t)stream;
-  const float scale_log2 = scale * 1.4426950408889634f;
-  launch_chained(kern, dim3(dim3(max_splits, (nkv + hg - 1) / hg, n_seqs)), dim3(kGqaThreads), smem, s,
-                 mk, mv, mkl, mvl, (const __nv_bfloat16*)q, q_row_stride, block_tables, max_pages, token_of_seq, positions,
-                 part_acc, part_ml, max_splits, nq, nkv, page_size, split_keys, scale_log2, hg, (__nv_bfloat16*)out, out_row_stride,
-                 status, counters, window, keep_first, penalty, softcap, (const __nv_bfloat16*)gate, gate_stride);
+  const int rc = launch_decode_mma(q, q_row_stride, k_pages, v_pages, n_pool_pages, block_tables, max_pages, token_of_seq, positions, out,
+                                   out_row_stride, part_acc, part_ml, max_splits, n_seqs, nq, nkv, page_size, split_keys, even_splits,
+                                   scale * 1.4426950408889634f, decode_head_group(nkv, 64, page_size, split_keys), status, counters, window,
+                                   keep_first, penalty, softcap, gate, gate_stride, s);
   // a single split wrote the result itself; with counters the block that finishes last merges the splits
-  if ((rc = check_launch("attention_decode_gqa")) || max_splits == 1 || counters) return rc;
+  if (rc || max_splits == 1 || counters) return rc;
   launch_chained(attention_decode_bulk_combine_kernel, dim3(dim3(nq, n_seqs)), dim3(64), 0, s, part_acc, part_ml, token_of_seq, positions,
       (__nv_bfloat16*)out, out_row_stride, max_splits, nq, head_dim, split_keys, window, (const __nv_bfloat16*)gate, gate_stride);
   return check_launch("attention_decode_bulk_combine");
+}
+
+// Whether a decode entry given `even_splits` cuts by it: heads of 64 on the kernel above, with hg kv heads per block (0: its own choice).
+ERB_EXPORT int erb_attention_decode_even_supported(int nq, int nkv, int head_dim, int page_size, int split_keys, int hg) {
+  if (head_dim != 64 || nq <= 0 || nkv <= 0 || nq % nkv || nq / nkv > kGqaMaxHeads || page_size <= 0 || split_keys <= 0) return 0;
+  return decode_mma_fits(nkv, page_size, split_keys, decode_head_group(nkv, 64, page_size, split_keys, hg));
 }
 
 // Blocks per sequence and split of erb_attention_decode_bulk (groups of kv heads), for sizing decisions.
@@ -938,12 +1024,12 @@ ERB_EXPORT int erb_attention_decode_bulk_head_group(int nkv, int head_dim, int p
 // window > 0: the token sees its last `window` keys (its own included) and the first `keep_first` ones;
 // window < 0: the keys of its own run of -window positions (runs counted from position 0) up to itself.
 ERB_EXPORT int erb_attention_decode_bulk(const void* q, int q_row_stride, const void* k_pages, const void* v_pages,
-                                         const int* block_tables, int max_pages, const int* token_of_seq,
+                                         int n_pool_pages, const int* block_tables, int max_pages, const int* token_of_seq,
                                          const int* positions, void* out, int out_row_stride, float* part_acc,
                                          float* part_ml, int max_splits, int n_seqs, int nq, int nkv, int head_dim,
                                          int page_size, int split_keys, float scale, int* status, int* counters,
                                          int head_group, int window, int keep_first, const float* penalty, float softcap,
-                                         const void* gate, int gate_stride, void* stream) {
+                                         const void* gate, int gate_stride, int even_splits, void* stream) {
   if (n_seqs <= 0) return ERB_OK;
   if (penalty && softcap > 0.f) return fail(ERB_ERR_UNSUPPORTED, "attention_decode_bulk: a penalty and a cap of the scores exclude each other");
   if (nq <= 0 || nkv <= 0 || nq % nkv) return fail(ERB_ERR_ARG, "attention_decode_bulk: bad head counts");
@@ -958,8 +1044,15 @@ ERB_EXPORT int erb_attention_decode_bulk(const void* q, int q_row_stride, const 
   const float scale_log2 = scale * 1.4426950408889634f;
   cudaStream_t s = (cudaStream_t)stream;
   const int r = nq / nkv;
+  // Heads of 64 with one query head per kv head: the tensor-core kernel, wherever whole pages make its stages.
+  const int hg = r == 1 && head_dim == 64 ? decode_head_group(nkv, 64, page_size, split_keys, head_group) : 0;
+  const bool mma = hg > 0 && decode_mma_fits(nkv, page_size, split_keys, hg) && n_pool_pages > 0 && !((uintptr_t)k_pages & 127) &&
+                   !((uintptr_t)v_pages & 127) && (unsigned long long)n_pool_pages * nkv * page_size <= 0x7fffffffull;
   int rc;
-  switch (head_dim) {
+  if (mma) rc = launch_decode_mma(q, q_row_stride, k_pages, v_pages, n_pool_pages, block_tables, max_pages, token_of_seq, positions, out,
+                                  out_row_stride, part_acc, part_ml, max_splits, n_seqs, nq, nkv, page_size, split_keys, even_splits, scale_log2, hg,
+                                  status, counters, window, keep_first, penalty, softcap, gate, gate_stride, s);
+  else switch (head_dim) {
     case 32: rc = dispatch_group<32>(r, q, q_row_stride, k_pages, v_pages, block_tables, max_pages, token_of_seq,
                                      positions, part_acc, part_ml, max_splits, n_seqs, nq, nkv, page_size, split_keys,
                                      scale_log2, out, out_row_stride, status, counters, head_group, window, keep_first, penalty, softcap, gate, gate_stride, s); break;

@@ -66,13 +66,13 @@ _SIGNATURES = {
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
                                  c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_float, c_void_p, c_int,
                                  c_void_p],
-    "erb_attention_decode_bulk": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
+    "erb_attention_decode_bulk": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                   c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                   c_int, c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_int,
-                                  c_void_p],
+                                  c_int, c_void_p],
     "erb_attention_decode_gqa": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                  c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                 c_float, c_void_p, c_void_p, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_void_p],
+                                 c_float, c_void_p, c_void_p, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int, c_void_p],
     "erb_glu_bounded": [c_void_p, c_void_p, c_int, c_int, c_float, c_float, c_float, c_int, c_void_p, c_void_p],
     "erb_add_layernorm": [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_float,
                           c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p],
@@ -1915,6 +1915,53 @@ def _choose_decode_plan(device: int, n_seqs: int, n_kv_heads: int, max_keys: int
     return split, 0
 
 
+def choose_even_plan(n_seqs: int, n_q_heads: int, n_kv_heads: int, max_keys: int, page_size: int, head_dim: int) -> tuple[int, int, int] | None:
+    """(bound on the keys per split, kv heads per block, splits) for a decode step in which every sequence's keys are cut into as many
+    equal splits, or None where the tensor-core decode kernel does not run or such splits leave the GPU half empty
+    (``choose_decode_plan`` then stands).  A function of the batch's size and of the bound on the longest context only."""
+    return _choose_even_plan(torch._C._cuda_getDevice(), n_seqs, n_q_heads, n_kv_heads, max_keys, page_size, head_dim)
+
+
+@functools.lru_cache(maxsize=4096)
+def _choose_even_plan(device: int, n_seqs: int, n_q_heads: int, n_kv_heads: int, max_keys: int, page_size: int,
+                      head_dim: int) -> tuple[int, int, int] | None:
+    """One wave of blocks, two an SM, whatever the contexts' lengths: splits at multiples of a power of two gave 64 sequences of
+    7,531 tokens three full splits and a short one.  The lines lie where whole decode steps (captured, the three decoders of 9 over 3,
+    15 over 5 and 32 heads) and, for long contexts, layers of attention alone, caches from DRAM, were fastest.
+
+    Several query heads per kv head: up to 128 keys one split (9 over 3, 90 keys: a step of 452 us in one split, 519 in two), so the
+    other plan; then splits of 48 to 96 keys as far as a wave reaches (15 over 5, steps with splits of 128 | these: 200 keys 8 sequences
+    829 | 720 us, 400 keys 847 | 785; attention of 64 x 7,531 116 | 109, of 8 x 7,531 26.1 | 22.7).
+
+    One query head per kv head: the fewest kv heads per block whose blocks fit into one wave, and where they fill a third of it up to 768
+    keys in one split, which nobody has to merge (8 sequences, a step: 200 keys 1,075 -> 1,017 us, 520 keys 1,162 -> 1,139; attention of
+    64 x 1,000 87 -> 82).  Fewer blocks and short contexts keep the other plan (4 x 520: 1,056 us, equal splits 1,063 to 1,080).
+
+    A wave is filled to 0.9: with 288 of 296 places some blocks waited for the kernel before."""
+    if head_dim != 64 or n_q_heads % n_kv_heads:
+        return None
+    lib = native.load("attention_tc", None)
+    slots = 2 * (_sm_counts.get(device) or _sm_counts.setdefault(device, torch.cuda.get_device_properties(device).multi_processor_count))
+    grouped = n_q_heads != n_kv_heads
+    if grouped and max_keys <= 128:
+        return None
+    for heads in (0,) if grouped else (2, 4, 8):
+        groups = lib.erb_attention_decode_bulk_groups(n_kv_heads, head_dim, page_size, page_size) if grouped else -(-n_kv_heads // heads)
+        blocks = n_seqs * groups
+        if blocks > slots or not lib.erb_attention_decode_even_supported(n_q_heads, n_kv_heads, head_dim, page_size, page_size, heads):
+            continue
+        if not grouped and max_keys <= 768:
+            return (-(-max_keys // page_size) * page_size, heads, 1) if blocks >= 0.3 * slots else None
+        fewest_keys = 128 if not grouped else 48 if max_keys <= 256 else 96 if 512 < max_keys <= 768 else 64
+        by_keys = -(-max_keys // fewest_keys)
+        splits = max(1, min(int(0.9 * slots / blocks), by_keys, 64))
+        if splits < by_keys and blocks * splits < 0.6 * slots:
+            continue
+        split = -(-max_keys // (splits * page_size)) * page_size
+        return split, heads, -(-max_keys // split)
+    return None
+
+
 def decode_scratch_floats(n_seqs: int, n_q_heads: int, head_dim: int, max_splits: int) -> tuple[int, int]:
     return n_seqs * n_q_heads * max_splits * head_dim, n_seqs * n_q_heads * max_splits * 2
 
@@ -1986,7 +2033,7 @@ def attention_decode_bulk(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch
                           scale: float, part_acc: torch.Tensor, part_ml: torch.Tensor, max_splits: int,
                           status: torch.Tensor, split_keys: int = DECODE_SPLIT_KEYS, head_group: int = 0, window: int = 0,
                           keep_first: int = 0, chunk: int = 0, penalty: torch.Tensor | None = None, softcap: float = 0.0,
-                          gate: torch.Tensor | None = None) -> None:
+                          gate: torch.Tensor | None = None, even: bool = False) -> None:
     """``attention_decode`` for bfloat16 with keys and values streamed by bulk asynchronous copies.
     ``chunk`` > 0 (instead of a window): the mask of chunks of ``attention_rows``.
     ``window`` > 0: the last ``window`` keys and the first ``keep_first``; the splits are counted from the one
@@ -2000,18 +2047,18 @@ def attention_decode_bulk(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch
     _need(out, "out", torch.bfloat16, contiguous=False); _need(part_acc, "part_acc", torch.float32)
     _need(part_ml, "part_ml", torch.float32); _need(status, "status", torch.int32)
     n_seqs = token_of_seq.numel()
-    _, nkv, page_size, d = k_pages.shape
+    n_pages, nkv, page_size, d = k_pages.shape
     need_acc, need_ml = decode_scratch_floats(n_seqs, n_q_heads, d, max_splits)
     if part_acc.numel() < need_acc or part_ml.numel() < need_ml:
         raise KernelError("attention_decode_bulk: scratch too small")
     if q.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("attention_decode_bulk: q/out inner stride must be 1")
     _call(_fn("attention_tc", None, "erb_attention_decode_bulk"), q.data_ptr(), q.stride(0), k_pages.data_ptr(),
-          v_pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1], token_of_seq.data_ptr(),
+          v_pages.data_ptr(), n_pages, block_tables.data_ptr(), block_tables.shape[1], token_of_seq.data_ptr(),
           positions.data_ptr(), out.data_ptr(), out.stride(0), part_acc.data_ptr(), part_ml.data_ptr(), max_splits,
           n_seqs, n_q_heads, nkv, d, page_size, int(split_keys), float(scale), status.data_ptr(),
           split_counters(q.device, n_seqs * nkv).data_ptr(), int(head_group), mask_reach(window, chunk), int(keep_first),
-          _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d), _stream())
+          _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d), int(bool(even)), _stream())
 
 
 @functools.lru_cache(maxsize=4096)
@@ -2030,7 +2077,7 @@ def attention_decode_gqa(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.
                          scale: float, part_acc: torch.Tensor, part_ml: torch.Tensor, max_splits: int,
                          status: torch.Tensor, split_keys: int = DECODE_SPLIT_KEYS, window: int = 0, keep_first: int = 0,
                          chunk: int = 0, penalty: torch.Tensor | None = None, softcap: float = 0.0,
-                         gate: torch.Tensor | None = None) -> None:
+                         gate: torch.Tensor | None = None, even: bool = False) -> None:
     """``attention_decode`` for several query heads per kv head on tensor cores (``window`` and ``keep_first`` as in
     ``attention_decode_bulk``): the query heads of a
     kv head are the rows of one matrix tile, pages arrive by TMA tensor copies."""
@@ -2051,7 +2098,7 @@ def attention_decode_gqa(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.
           positions.data_ptr(), out.data_ptr(), out.stride(0), part_acc.data_ptr(), part_ml.data_ptr(), max_splits,
           n_seqs, n_q_heads, nkv, d, page_size, int(split_keys), float(scale), status.data_ptr(),
           split_counters(q.device, n_seqs * nkv).data_ptr(), mask_reach(window, chunk), int(keep_first),
-          _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d), _stream())
+          _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d), int(bool(even)), _stream())
 
 
 #: query rows of one (sequence, head) that a block of the tensor-core prefill kernel takes

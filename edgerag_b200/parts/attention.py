@@ -290,7 +290,12 @@ class Attention(Mixer):
             may_group = reach_mask <= 0 or nd * self.n_kv >= 64
             grouped = may_group and self.n_q != self.n_kv and kernels.decode_gqa_supported(
                 self.dtype, d, self.window, self.n_q, self.n_kv, ctx.page_size, kernels.DECODE_SPLIT_KEYS)
-            if ctx.batch_invariant:     # one plan for every batch: a sequence's sums are then added in one order
+            even = None                 # every sequence in equal splits
+            if not ctx.batch_invariant and reach_mask <= 0 and self.dtype == torch.bfloat16:
+                even = kernels.choose_even_plan(nd, self.n_q, self.n_kv, ctx.max_keys_bound(), ctx.page_size, d)
+            if even is not None:
+                split, heads_per_block, max_splits = even
+            elif ctx.batch_invariant:   # one plan for every batch: a sequence's sums are then added in one order
                 split, heads_per_block = kernels.DECODE_SPLIT_KEYS, 0
             elif reach_mask > 0:        # a token reads its window (or chunk) and the kept keys, however long its context is
                 reach = min(ctx.max_keys_bound(), -(-(reach_mask + self.keep_first) // ctx.page_size) * ctx.page_size)
@@ -299,19 +304,21 @@ class Attention(Mixer):
             else:
                 split, heads_per_block = kernels.choose_decode_plan(nd, self.n_kv, ctx.max_keys_bound(), ctx.page_size, d,
                                                                     grouped or self.dtype != torch.bfloat16, ctx.keys_granule())
-            max_splits = ctx.decode_splits(mask, split)
+            if even is None:
+                max_splits = ctx.decode_splits(mask, split)
             need_acc, need_ml = kernels.decode_scratch_floats(nd, self.n_q, d, max_splits)
             part_acc = ctx.buf("attn.part_acc", (need_acc,), torch.float32)
             part_ml = ctx.buf("attn.part_ml", (need_ml,), torch.float32)
             if may_group and kernels.decode_gqa_supported(self.dtype, d, self.window, self.n_q, self.n_kv, ctx.page_size, split, max_splits):
                 kernels.attention_decode_gqa(qkv[:nd], k_pages, v_pages, tables, ctx.token_of_seq[:nd], ctx.positions,
                                              out[:nd], self.n_q, self.scale, part_acc, part_ml, max_splits, ctx.status,
-                                             split_keys=split, window=self.window, keep_first=self.keep_first, chunk=self.chunk, gate=head_gate, **score)
+                                             split_keys=split, window=self.window, keep_first=self.keep_first, chunk=self.chunk, gate=head_gate,
+                                             even=even is not None, **score)
             elif kernels.decode_bulk_supported(self.dtype, d, self.window, self.n_q, self.n_kv, max_splits):
                 kernels.attention_decode_bulk(qkv[:nd], k_pages, v_pages, tables, ctx.token_of_seq[:nd], ctx.positions,
                                               out[:nd], self.n_q, self.scale, part_acc, part_ml, max_splits, ctx.status,
                                               split_keys=split, head_group=heads_per_block, window=self.window,
-                                              keep_first=self.keep_first, chunk=self.chunk, gate=head_gate, **score)
+                                              keep_first=self.keep_first, chunk=self.chunk, gate=head_gate, even=even is not None, **score)
             else:
                 kernels.attention_decode(qkv[:nd], k_pages, v_pages, tables, ctx.token_of_seq[:nd], ctx.positions,
                                          out[:nd], self.n_q, self.scale, part_acc, part_ml, max_splits,

@@ -1,0 +1,69 @@
+"""Decode attention whose sequences are cut into equally many splits each, and the tensor-core kernel with one query head per kv head
+(its weights in three pieces): against the reference, over the edges of pages, splits and stages."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from edgerag_b200.ops import kernels as K
+from test_kernels import attention_reference, paged_case, tol
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(case, nq, nkv, d, splits, split, heads, even=True):
+    dev = {n: case[n].cuda() for n in ("q", "kp", "vp", "tables", "pos")}
+    n = case["pos"].numel()
+    acc, ml = K.decode_scratch_floats(n, nq, d, splits)
+    part_acc, part_ml = (torch.full((m,), float("nan"), device="cuda") for m in (acc, ml))
+    out = torch.full((n, nq * d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    tok = torch.arange(n, dtype=torch.int32, device="cuda")
+    args = (dev["q"], dev["kp"], dev["vp"], dev["tables"], tok, dev["pos"], out, nq, d ** -0.5, part_acc, part_ml, splits, status)
+    if nq == nkv:
+        K.attention_decode_bulk(*args, split_keys=split, head_group=heads, even=even)
+    else:
+        K.attention_decode_gqa(*args, split_keys=split, even=even)
+    torch.cuda.synchronize()
+    assert int(status) == 0 and int(K.split_counters(out.device, 1).abs().sum()) == 0
+    return out
+
+
+@pytest.mark.parametrize("nq,nkv,ps,heads", [(8, 8, 16, 2), (5, 5, 16, 4), (9, 9, 8, 8), (3, 3, 128, 1), (15, 5, 16, 0), (6, 3, 64, 0)])
+@pytest.mark.parametrize("splits", [1, 2, 7, 64])
+def test_equal_splits(nq, nkv, ps, heads, splits):
+    ctx_lens = [1, 2, 15, 16, 17, 127, 128, 129, 500, 1300]
+    case = paged_case(torch.bfloat16, 7 + ps + splits, nq, nkv, 64, ps, ctx_lens, [1] * len(ctx_lens))
+    most = -(-max(ctx_lens) // (splits * ps)) * ps
+    got = _run(case, nq, nkv, 64, splits, most, heads)
+    torch.testing.assert_close(got.float().cpu(), attention_reference(case, nq, nkv, 64, 0.125), **tol(torch.bfloat16))
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_a_value_that_is_not_finite_stays_in_its_entry(bad):
+    """One query head per kv head: an infinity in the values gives an infinity (the pieces of its weight do not cancel), elsewhere nothing changes."""
+    case = paged_case(torch.bfloat16, 3, 4, 4, 64, 16, [200], [1])
+    clean = _run(case, 4, 4, 64, 3, 80, 2).float().cpu()
+    row = int(case["tables"][0, 2])
+    case["vp"][row, 1, 5, 9] = bad
+    got = _run(case, 4, 4, 64, 3, 80, 2).float().cpu()
+    at = 1 * 64 + 9
+    assert torch.equal(torch.isfinite(got[0]), torch.arange(256) != at)
+    assert torch.equal(got[0, at], torch.tensor(bad)) or bad != bad
+    keep = torch.arange(256) != at
+    assert torch.equal(got[0, keep], clean[0, keep])
+
+
+@pytest.mark.parametrize("nq,nkv", [(32, 32), (15, 5), (9, 3), (6, 6)])
+def test_the_plan_of_equal_splits(nq, nkv):
+    """Never more than one wave of blocks or 64 splits, whole pages, the bound covered; nothing for sizes that the kernel does not take."""
+    slots = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    for n in (1, 3, 8, 17, 64, 200, 1000):
+        for bound in (16, 128, 384, 768, 8192, 65536):
+            plan = K.choose_even_plan(n, nq, nkv, bound, 16, 64)
+            if plan is not None:
+                split, heads, splits = plan
+                groups = -(-nkv // (heads or 8))
+                assert split % 16 == 0 and split * splits >= bound and splits <= 64 and n * groups * splits <= slots
+    assert K.choose_even_plan(8, nq, nkv, 1024, 16, 128) is None and K.choose_even_plan(8, nq, nkv, 1024, 12, 64) is None
