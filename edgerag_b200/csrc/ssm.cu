@@ -12,13 +12,15 @@
 //
 // A request's tokens of one step are neighbours in the batch (rows seq_starts[s] .. seq_starts[s+1]),
 // its slot is state_slots[s].  Every (request, head, block of columns) is scanned by exactly one block: token after token, or
-// (bfloat16, the sizes of ssm_chunk_kernel) 64 tokens at a time as products of matrices.
+// (bfloat16, the sizes of ssm_chunk_kernel) 128 tokens at a time as products of matrices.
 #include <limits.h>
 #include <math.h>
+#include <stddef.h>
 
 #include "common.cuh"
 #if ERB_ELEM == 1
 #include "mma_split.cuh"
+#include "tc_common.cuh"
 #endif
 
 using namespace erb;
@@ -402,285 +404,439 @@ ssm_scan16_kernel(const T* __restrict__ xbc, int channels, const T* __restrict__
 }
 
 #if ERB_ELEM == 1
-// The scan of portions of prompts, 64 tokens at a time.  With c_t the sum of the logarithms of the chunk's decays up to and
+// The scan of portions of prompts, 128 tokens at a time.  With c_t the sum of the logarithms of the chunk's decays up to and
 // with token t, and S the state before the chunk,
 //     y_t = exp(c_t) S^T C_t + sum_{s <= t} (C_t . B_s) dt_s exp(c_t - c_s) x_s + D x_t
-//     S  <- exp(c_64) S + sum_s B_s (dt_s exp(c_64 - c_s) x_s)^T
-// which are products of matrices.  C, B and x are bfloat16 as they are; every operand that is not (the weights of the second
-// sum, the state, the weighted x of the third) goes in as three bfloat16 pieces (mma_split.cuh), so nothing is rounded to 16
-// bits.  c is summed in double and kept as two floats, since its differences, not its values, matter.
+//     S  <- exp(c_128) S + sum_s B_s (dt_s exp(c_128 - c_s) x_s)^T
+// which are products of matrices, here on tcgen05 with their sums in TMEM.  C, B and x are bfloat16 as they are; every operand that is
+// not (the weights of the second sum, the state, the weighted x of the third) goes in as three bfloat16 pieces (mma_split.cuh), so
+// nothing is rounded to 16 bits.  c is summed in double and kept as two floats, since its differences, not its values, matter.
 //
-// What bounds it: the dependent steps of a chunk (two barriers, the products between them), as the walk was bound by the
-// steps of a token.  Block: one (head, request, 32 columns), 16 warps of products and one that makes the next chunk's steps
-// and decays; the state stays in the accumulators' registers.  Between the barriers the work of a chunk is cut into pieces
-// of about the same length: first 10 of the warps make a tile of the weights (C B^T below the diagonal) each, the others the
-// weighted x, and every warp 16 rows x 8 columns of the part of y that comes from the state; then the same 16 x 8 of the
-// part within the chunk, and 16 rows of the state.  (With 8 warps that made their weights in registers, twice over, a chunk
-// took 5.0 us instead of 3.9.)
+// Block: one (head, request, 32 columns).  Sixteen warps do what is between the products, an issuing warp asks for the products, four warps
+// make the next chunk's steps and decays, one of their lanes brings the next chunk's rows by TMA tensor copies.  Per chunk c:
+//   G = C B^T                       as two sums over half of the state's rows each (the unit cuts its sums; one sum of 128 was a third
+//                                   further from float64), issued while the chunk before is finished
+//   the weighted x's pieces in shared memory; the weights' pieces from G, as the left operand in TMEM
+//   Y0 = C S, dS = B^T (weighted x) while the weights are made; Y1 = (weights) x, its first half of the tokens as soon as those weights are there
+//   the state in registers, S <- exp(c_128) S + dS, and its pieces; y = exp(c_t) Y0 + Y1 + D x
+// The pieces of the state and of the weighted x are neighbouring columns of one product: a product of 32 columns costs as much as one
+// of 96 (54 clocks, the left operand's reads).  Only the state's own line waits for the chunk before.
+//
+// What bounds it: a chunk's line, 6,500 clocks: the weighted x 900, G 500, the weights 3,200 (those of the last 32 tokens are all made by one
+// scheduler's warps, which alone reach their lanes of TMEM), the second half of Y1 700, outputs 850.  The products take 2,900 beside it.  2,048 tokens of 64 heads of 64 x 128: 64.5 us; 132 us
+// in chunks of 64 by mma.sync, 566 us walked.  Error against float64 1.2e-7 for y, 7.4e-8 for the state, as those.
 //
 // The products are causal for finite numbers only: above the diagonal the weights are zeros, and 0 * inf is no number; nor are the
-// pieces of an infinity, or the differences of c where a decay is exactly zero.  Whatever is not finite makes a y of its own token or
-// the last state not finite, so both are looked at (one multiplication an output), and a block that finds one walks its portion once
-// more from the state as it was, token after token like ssm_scan16_kernel and with its bits.  (2,048 tokens of 64 heads of 64 x 128:
-// 128.5 us without the look, 131.8 us with it.)
-constexpr int kChunk = 64, kChunkCols = 32, kChunkWarps = 16;
+// pieces of an infinity, or the differences of c where a decay is exactly zero; and a chunk's last rows may be another request's.
+// Whatever is not finite makes a y of its own token or the last state not finite, so both are looked at (one multiplication an output),
+// and a block that finds one walks its portion once more from the state as it was, token after token like ssm_scan16_kernel and with
+// its bits.
+//
+// Every wait for a product, a copy or warps is bounded; a thread that gives up raises a block-wide flag, all warps still come to the
+// barriers of the remaining chunks, the block records 7000000 in *status, lets its copies land, frees its TMEM and returns.
+constexpr int kChunk = 128, kChunkCols = 32, kChunkWarps = 16, kIssueWarp = 16, kStepWarp = 17, kStepWarps = 4,
+              kChunkThreads = 32 * (kStepWarp + kStepWarps);
 
-template <int N>
 struct ChunkSmem {
-  static constexpr int LdN = N + 8, LdP = kChunkCols + 8, LdM = kChunk + 8;   // rows 16 bytes longer than a power of two: no bank conflicts
-  __nv_bfloat16 c[2][kChunk][LdN];
-  __nv_bfloat16 b[2][kChunk][LdN];
-  __nv_bfloat16 x[2][kChunk][LdP];
-  __nv_bfloat16 s[3][N][LdP];                                  // the state before the chunk, in pieces
-  __nv_bfloat16 w[3][kChunk][LdP];                             // the weighted x, in pieces
-  __nv_bfloat16 m[3][kChunk][LdM];                             // the weights of the sum within the chunk, in pieces (tiles above the diagonal unused)
+  uint8_t c[2][2][kChunk * 128];             // two stages; blocks of 64 state rows, 128-byte rows of a token, 128-byte swizzle
+  uint8_t b[2][2][kChunk * 128];
+  uint8_t x[2][kChunk * 64];                 // 64-byte rows of a token, 64-byte swizzle; so are the pieces
+  uint8_t w[3][kChunk * 64];                 // the weighted x
+  uint8_t s[3][kChunk * 64];                 // the state before the chunk: a row per state row
   float dt[2][kChunk], hi[2][kChunk], lo[2][kChunk];           // step, c_t / ln 2 in two floats
-  float grown[2][kChunk], weight[2][kChunk];                   // exp(c_t), dt_t exp(c_64 - c_t)
-  float total[2];                                              // exp(c_64)
+  float grown[2][kChunk], weight[2][kChunk];                   // exp(c_t), dt_t exp(c_128 - c_t)
+  alignas(16) float out[kChunk][kChunkCols + 4];               // a chunk's y on its way to whole lines
+  double sums[kStepWarps];                                     // the sums of 32 logarithms each
+  uint64_t bars[9];
+  float total[2];                                              // exp(c_128)
+  int abort;
+  uint32_t tmem;
 };
+static_assert(offsetof(ChunkSmem, dt) % 16 == 0 && offsetof(ChunkSmem, hi) % 16 == 0 && offsetof(ChunkSmem, lo) % 16 == 0 &&
+                  offsetof(ChunkSmem, out) % 16 == 0 && (kChunkCols + 4) % 4 == 0 && offsetof(ChunkSmem, bars) % 8 == 0 &&
+                  offsetof(ChunkSmem, sums) % 8 == 0 && offsetof(ChunkSmem, b) % 1024 == 0 && offsetof(ChunkSmem, x) % 1024 == 0 &&
+                  offsetof(ChunkSmem, w) % 1024 == 0 && offsetof(ChunkSmem, s) % 1024 == 0, "read 16 bytes at a time; tiles start where their swizzle does");
+// byte offset of 16-byte piece c of row r in a tile of 64-byte rows with the 64-byte swizzle
+__device__ __forceinline__ uint32_t swz64(int r, int c) { return (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); }
+// Tiles of 64-byte rows as an operand whose columns are its outer side: 512 bytes between groups of 8 rows, a tile from 32 columns to the next.
+__device__ __forceinline__ uint64_t desc_rows64(uint32_t saddr) {
+  return (uint64_t)((saddr & 0x3FFFF) >> 4) | (uint64_t)((kChunk * 64) >> 4) << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 |
+         (uint64_t)4 << 61;
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+// split_pair for a pair that is held as one operand.
+__device__ __forceinline__ void split_two(Two x, uint32_t* piece) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    float a, b;
+    x.get(a, b);
+    const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+    piece[k] = *reinterpret_cast<const uint32_t*>(&p);
+    if (k < 2) x = fma2(Two(-1.f), Two(__uint_as_float(piece[k] << 16), __uint_as_float(piece[k] & 0xffff0000u)), x);
+  }
+}
 
 template <int N>
-__global__ void __launch_bounds__((kChunkWarps + 1) * 32)
-ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const __nv_bfloat16* __restrict__ proj, int ld, int off_dt,
-                 const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
-                 float* __restrict__ state, const int* __restrict__ seq_starts, const int* __restrict__ state_slots,
-                 float* __restrict__ y, int H, int P, int G) {
+__global__ void __launch_bounds__(kChunkThreads, 1)
+ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_constant__ CUtensorMap map_x, const __nv_bfloat16* __restrict__ xbc,
+                 int channels, const __nv_bfloat16* __restrict__ proj, int ld, int off_dt, const float* __restrict__ dt_bias,
+                 const float* __restrict__ a_log, const float* __restrict__ d_skip, float* __restrict__ state,
+                 const int* __restrict__ seq_starts, const int* __restrict__ state_slots, float* __restrict__ y, int H, int P, int G,
+                 int* __restrict__ status) {
   chain_wait();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  ChunkSmem<N>& sm = *reinterpret_cast<ChunkSmem<N>*>(smem_raw);
   const int h = blockIdx.x, seq = blockIdx.y, p0 = blockIdx.z * kChunkCols;
   const int start = seq_starts[seq], n_tok = seq_starts[seq + 1] - start;
   if (n_tok <= 1) return;                                      // (a single token: the scan kernel's)
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (base - raw);
+  ChunkSmem& sm = *reinterpret_cast<ChunkSmem*>(smem);
   const int g = h / (H / G), inner = H * P;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qr = lane >> 2, qc = lane & 3;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_chunks = (n_tok + kChunk - 1) / kChunk;
-  const __nv_bfloat16* rows = xbc + (size_t)start * channels;
+  // G there; the weights' pieces of the chunk's first and last 64 tokens; the weighted x's; dS there; Y there; the state's pieces; a stage's rows (two)
+  constexpr int kBarG = 0, kBarP1 = 1, kBarP2 = 2, kBarW = 3, kBarD = 4, kBarY = 5, kBarS = 6, kBarL = 7;
+  auto bar = [&](int which) { return smem_u32(&sm.bars[which]); };
+  volatile int* abort_flag = &sm.abort;
+  if (threadIdx.x == 0) {
+    for (int i : {kBarG, kBarD, kBarY, kBarL, kBarL + 1}) mbar_init(bar(i), 1);
+    for (int i : {kBarP1, kBarP2, kBarW, kBarS}) mbar_init(bar(i), kChunkWarps);
+    sm.abort = 0;
+    mbar_init_fence();
+  }
+  if (warp == kIssueWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = sm.tmem;
+  // columns of TMEM.  G's first sum: 0; the weights' pieces, 3 x 64, and before them G's second sum: 128; Y0 by the state's first piece | by
+  // the others; dS by three pieces; Y1
+  constexpr uint32_t kColM = 128, kColY0 = 320, kColD = 384, kColY1 = 480;
+  constexpr int kTopThreads = 32 * (kChunkWarps + kStepWarps);
+  float probe = 0.f;                                           // no number once a result was not finite
 
-  auto load_stage = [&](int c) {                               // the threads of the products
-    const int buf = c & 1, c0 = c * kChunk;
-    for (int idx = threadIdx.x; idx < kChunk * (N / 8); idx += kChunkWarps * 32) {
-      const int r = idx / (N / 8), e = 8 * (idx % (N / 8));
-      const bool real = c0 + r < n_tok;
-      const __nv_bfloat16* src = rows + (size_t)(real ? c0 + r : 0) * channels + inner + g * N + e;
-      copy16_or_zero(&sm.b[buf][r][e], src, real);
-      copy16_or_zero(&sm.c[buf][r][e], src + G * N, real);
-    }
-    if (threadIdx.x < kChunk * (kChunkCols / 8)) {
-      const int r = threadIdx.x / (kChunkCols / 8), e = 8 * (threadIdx.x % (kChunkCols / 8));
-      const bool real = c0 + r < n_tok;
-      copy16_or_zero(&sm.x[buf][r][e], rows + (size_t)(real ? c0 + r : 0) * channels + h * P + p0 + e, real);
-    }
-    copy_commit();
-  };
-  const float a = -expf(a_log[h]), bias = dt_bias[h];
-  auto make_steps = [&](int c) {                               // the last warp: tokens 2 lane and 2 lane + 1 of chunk c
-    const int buf = c & 1, t0 = c * kChunk + 2 * lane;
-    float dt[2];
-    double la[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      dt[i] = t0 + i < n_tok ? softplus_f(__bfloat162float(proj[(size_t)(start + t0 + i) * ld + off_dt + h]) + bias) : 0.f;
-      la[i] = (double)a * (double)dt[i];
-    }
-    double sum = la[0] + la[1];                                // inclusive scan over the lanes
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double v = __shfl_up_sync(0xffffffffu, sum, o);
-      if (lane >= o) sum += v;
-    }
-    const double all = __shfl_sync(0xffffffffu, sum, 31);
-    const double cum[2] = {sum - la[1], sum};
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = 2 * lane + i;
-      const double l2 = cum[i] * 1.4426950408889634;
-      const float hi = (float)l2;
-      sm.dt[buf][r] = dt[i];
-      sm.hi[buf][r] = hi;
-      sm.lo[buf][r] = (float)(l2 - (double)hi);
-      sm.grown[buf][r] = (float)exp(cum[i]);
-      sm.weight[buf][r] = (float)((double)dt[i] * exp(all - cum[i]));
-    }
-    if (lane == 0) sm.total[buf] = (float)exp(all);
-  };
+  // the state: thread (row n, quarter qt) holds columns 8 qt .. 8 qt + 7 of row n
+  const int quad = warp & 3, qt = (warp >> 2) & 3, row = 32 * quad + lane;
+  float S[8];
+  float* s_glob = state + (((size_t)state_slots[seq] * H + h) * N + row) * P + p0 + 8 * qt;
+  const bool holds = warp < kChunkWarps && row < N;
 
-  // the state: warp w holds rows 16 (w mod N/16) .. + 15, columns 8 NTW (w div N/16) .. + 8 NTW - 1
-  constexpr int kRowTiles = N / 16, kColGroups = kChunkWarps / kRowTiles < 4 ? kChunkWarps / kRowTiles : 4, NTW = 4 / kColGroups;
-  const bool holds_state = warp < kRowTiles * kColGroups;
-  const int s_row = 16 * (warp % kRowTiles), s_col = 8 * NTW * (warp / kRowTiles);
-  float S[NTW][4];
-  float* s_glob = state + ((size_t)state_slots[seq] * H + h) * N * P + p0;
-  auto publish = [&]() {                                       // the state's pieces to shared memory
+  if (warp < kChunkWarps) {
+    const uint32_t t_lane = tmem + ((uint32_t)(32 * quad) << 16);
+    auto publish = [&]() {                                     // the state's pieces
+      uint32_t piece[4][3];
 #pragma unroll
-    for (int nt = 0; nt < NTW; ++nt)
+      for (int i = 0; i < 4; ++i) split_two(Two(S[2 * i], S[2 * i + 1]), piece[i]);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        uint32_t piece[3];
-        split_pair(S[nt][2 * j], S[nt][2 * j + 1], piece);
+      for (int k = 0; k < 3; ++k)
+        *reinterpret_cast<uint4*>(sm.s[k] + swz64(row, qt)) = make_uint4(piece[0][k], piece[1][k], piece[2][k], piece[3][k]);
+    };
+    auto arrive = [&](int which) {                             // this warp's part is in place for the products
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(which));
+    };
+    auto wait = [&](int which, uint32_t parity) {
+      mbar_wait_or_abort(bar(which), parity, abort_flag);
+      __syncwarp();
+    };
+    auto no_weights = [&](int u, int pieces) {                 // zeros in the unit of 16 columns: it lies above the diagonal
+      const uint32_t zero[8] = {};
+      for (int k = 0; k < pieces; ++k) tmem_st8(t_lane + kColM + 64 * k + 8 * u, zero);
+    };
+#pragma unroll
+    for (int i = 0; i < 8; ++i) S[i] = 0.f;
+    if (holds) {
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {                         // (states are 8-byte aligned)
+        const float2 v = *reinterpret_cast<const float2*>(s_glob + i);
+        S[i] = v.x; S[i + 1] = v.y;
+      }
+    }
+    publish();
+    for (int u = qt; u < 8; u += 4)
+      if (u >= 2 * (quad + 1)) no_weights(u, 3);
+    tmem_st_wait();
+    fence_before_sync();
+    fence_async_proxy();
+    arrive(kBarS);
+    const float dskip = d_skip[h];
+    for (int c = 0; c < n_chunks; ++c) {
+      const int st = c & 1;
+      const uint32_t par = c & 1;
+      named_barrier(1, kTopThreads);                           // this chunk's steps are there, everybody is done with the chunk before
+      wait(kBarL + st, (c >> 1) & 1);
+      {                                                        // weighted x: tokens 32 (warp / 4) .. + 31, columns 8 (warp % 4) .. + 7
+        const int t = 32 * qt + lane;
+        const float f = sm.weight[st][t];
+        const uint4 in = *reinterpret_cast<const uint4*>(sm.x[st] + swz64(t, quad));
+        const uint32_t q[4] = {in.x, in.y, in.z, in.w};
+        uint32_t piece[4][3];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) split_two(Two(f) * Two(__uint_as_float(q[i] << 16), __uint_as_float(q[i] & 0xffff0000u)), piece[i]);
 #pragma unroll
         for (int k = 0; k < 3; ++k)
-          *reinterpret_cast<uint32_t*>(&sm.s[k][s_row + qr + 8 * j][s_col + 8 * nt + 2 * qc]) = piece[k];
+          *reinterpret_cast<uint4*>(sm.w[k] + swz64(t, quad)) = make_uint4(piece[0][k], piece[1][k], piece[2][k], piece[3][k]);
+        fence_async_proxy();
+        arrive(kBarW);
       }
-  };
-  if (warp < kChunkWarps) load_stage(0);
-  else make_steps(0);
-  if (holds_state) {
-#pragma unroll
-    for (int nt = 0; nt < NTW; ++nt)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const float2 v = *reinterpret_cast<const float2*>(s_glob + (size_t)(s_row + qr + 8 * j) * P + s_col + 8 * nt + 2 * qc);
-        S[nt][2 * j] = v.x;
-        S[nt][2 * j + 1] = v.y;
-      }
-    publish();
-  }
-  const int y_row = 16 * (warp >> 2), y_col = 8 * (warp & 3);
-  // the tile of the weights that a warp makes: warps 0 .. 9 take the tiles (row, column) on and below the diagonal
-  const int m_tr = warp < 1 ? 0 : warp < 3 ? 1 : warp < 6 ? 2 : 3;
-  const int m_row = 16 * m_tr, m_col = 16 * (warp - m_tr * (m_tr + 1) / 2);
-  const float dskip = d_skip[h];
-  float probe = 0.f;                                           // no number once a result was not finite
-  for (int c = 0; c < n_chunks; ++c) {
-    const int buf = c & 1;
-    if (warp < kChunkWarps) copy_wait<0>();
-    __syncthreads();                                           // chunk c's rows, steps and state pieces are there; stage c - 1 is free
-    if (warp == kChunkWarps) {
-      if (c + 1 < n_chunks) make_steps(c + 1);
-      __syncthreads();
-      continue;
-    }
-    if (c + 1 < n_chunks) load_stage(c + 1);
-    // the part of y that comes from the state
-    float inter[3][4] = {};
-#pragma unroll
-    for (int k = 0; k < N / 16; k += 2) {
-      uint32_t cf[2][4], b[3][4];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) ldmatrix4(cf[i], &sm.c[buf][y_row + (lane & 15)][16 * (k + i) + 8 * (lane >> 4)]);
-#pragma unroll
-      for (int piece = 0; piece < 3; ++piece) ldmatrix4t(b[piece], &sm.s[piece][16 * k + lane][y_col]);
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int piece = 0; piece < 3; ++piece) mma16816(inter[piece], cf[i], b[piece][2 * i], b[piece][2 * i + 1]);
-    }
-    if (warp < 10) {                                           // a tile of the weights
-      float gram[2][2][4] = {};                                // (two chains: a product does not wait for the one before it)
-#pragma unroll
-      for (int k = 0; k < N / 16; ++k) {
-        uint32_t cf[4], b[4];
-        ldmatrix4(cf, &sm.c[buf][m_row + (lane & 15)][16 * k + 8 * (lane >> 4)]);
-        ldmatrix4(b, &sm.b[buf][m_col + (lane & 7) + 8 * (lane >> 4)][16 * k + 8 * ((lane >> 3) & 1)]);
-        mma16816(gram[k & 1][0], cf, b[0], b[1]);
-        mma16816(gram[k & 1][1], cf, b[2], b[3]);
-      }
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        const int s = m_col + 8 * nt + 2 * qc;
-        const float2 hs = *reinterpret_cast<const float2*>(&sm.hi[buf][s]), ls = *reinterpret_cast<const float2*>(&sm.lo[buf][s]);
-        const float2 ds = *reinterpret_cast<const float2*>(&sm.dt[buf][s]);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int r = m_row + qr + 8 * j;
-          const float hi = sm.hi[buf][r], lo = sm.lo[buf][r];
-          const float v0 = s <= r ? (gram[0][nt][2 * j] + gram[1][nt][2 * j]) * ds.x * exp2f((hi - hs.x) + (lo - ls.x)) : 0.f;
-          const float v1 = s + 1 <= r ? (gram[0][nt][2 * j + 1] + gram[1][nt][2 * j + 1]) * ds.y * exp2f((hi - hs.y) + (lo - ls.y)) : 0.f;
-          uint32_t piece[3];
-          split_pair(v0, v1, piece);
-#pragma unroll
-          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&sm.m[k][r][s]) = piece[k];
-        }
-      }
-    } else {                                                   // weighted x in pieces: 4 columns of one token at a time
-      for (int idx = threadIdx.x - 320; idx < kChunk * (kChunkCols / 4); idx += 192) {
-        const int r = idx >> 3, e = 4 * (idx & 7);
-        float v[4];
-        Pack4<__nv_bfloat16>::load(&sm.x[buf][r][e], v);
-        const float f = sm.weight[buf][r];
-        uint32_t p01[3], p23[3];
-        split_pair(f * v[0], f * v[1], p01);
-        split_pair(f * v[2], f * v[3], p23);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(&sm.w[k][r][e]) = make_uint2(p01[k], p23[k]);
-      }
-    }
-    __syncthreads();                                           // weights and weighted x are complete; nobody reads the state's pieces any more
-    float add[3][NTW][4] = {};
-    if (holds_state) {
-#pragma unroll
-      for (int k = 0; k < kChunk / 16; ++k) {
-        uint32_t bt[4], b[3][4];                               // B^T: 16 state rows x 16 tokens
-        ldmatrix4t(bt, &sm.b[buf][16 * k + (lane & 7) + 8 * (lane >> 4)][s_row + 8 * ((lane >> 3) & 1)]);
-#pragma unroll
-        for (int piece = 0; piece < 3; ++piece) {
-          if (NTW == 2) ldmatrix4t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col + 8 * (lane >> 4)]);
-          else ldmatrix2t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col]);
-        }
-#pragma unroll
-        for (int piece = 0; piece < 3; ++piece)
-#pragma unroll
-          for (int nt = 0; nt < NTW; ++nt) mma16816(add[piece][nt], bt, b[piece][2 * nt], b[piece][2 * nt + 1]);
-      }
-    }
-    float intra[3][4] = {};                                    // the part of y from the chunk's own tokens
-    for (int k = 0; k <= (warp >> 2); k += 2) {
-      uint32_t xb[4], mf[3][4];
-      ldmatrix4t(xb, &sm.x[buf][16 * k + lane][y_col]);        // (rows 16 k .. + 31: the second half may lie behind the diagonal)
+      wait(kBarG, par);
+      fence_after_sync();
+      float gram[2][16];                                       // units qt and qt + 4 of these 32 tokens: 16 columns each
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        if (k + i > (warp >> 2)) break;
+        const int u = qt + 4 * i;
+        if (u < 2 * (quad + 1)) {                              // (the same for the warp)
+          float more[16];
+          tmem_ld16(t_lane + 16 * u, gram[i]);
+          tmem_ld16(t_lane + kColM + 16 * u, more);
+          tmem_ld_wait();
 #pragma unroll
-        for (int piece = 0; piece < 3; ++piece) ldmatrix4(mf[piece], &sm.m[piece][y_row + (lane & 15)][16 * (k + i) + 8 * (lane >> 4)]);
-#pragma unroll
-        for (int piece = 0; piece < 3; ++piece) mma16816(intra[piece], mf[piece], xb[2 * i], xb[2 * i + 1]);
-      }
-    }
-    if (holds_state) {
-      const float total = sm.total[buf];
-#pragma unroll
-      for (int nt = 0; nt < NTW; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) S[nt][i] = fmaf(total, S[nt][i], (add[2][nt][i] + add[1][nt][i]) + add[0][nt][i]);
-      publish();
-    }
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int r = y_row + qr + 8 * j, col = y_col + 2 * qc;
-      if (c * kChunk + r < n_tok) {
-        const float grown = sm.grown[buf][r];
-        const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&sm.x[buf][r][col]));
-        float v[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int q = 2 * j + i;
-          const float before = (inter[2][q] + inter[1][q]) + inter[0][q], own = (intra[2][q] + intra[1][q]) + intra[0][q];
-          v[i] = fmaf(grown, before, own) + dskip * (i ? xv.y : xv.x);
-          probe = fmaf(v[i], 0.f, probe);
+          for (int j = 0; j < 16; ++j) gram[i][j] += more[j];
         }
-        *reinterpret_cast<float2*>(y + (size_t)(start + c * kChunk + r) * inner + h * P + p0 + col) = make_float2(v[0], v[1]);
+      }
+      fence_before_sync();
+      named_barrier(4 + quad, 128);                            // the weights take the place of the second sum: all four warps have read it
+      const Two hi_t(sm.hi[st][row]), lo_t(sm.lo[st][row]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int u = qt + 4 * i;
+        if (u < 2 * (quad + 1)) {
+          uint32_t piece[8][3];
+          const bool diagonal = 16 * u + 15 > 32 * quad;       // (the same for the warp)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int s0 = 16 * u + 4 * j;
+            const float4 hs = *reinterpret_cast<const float4*>(&sm.hi[st][s0]), ls = *reinterpret_cast<const float4*>(&sm.lo[st][s0]);
+            const float4 ds = *reinterpret_cast<const float4*>(&sm.dt[st][s0]);
+            const Two h2[2] = {Two(hs.x, hs.y), Two(hs.z, hs.w)}, l2[2] = {Two(ls.x, ls.y), Two(ls.z, ls.w)}, d2[2] = {Two(ds.x, ds.y), Two(ds.z, ds.w)};
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const Two gap = fma2(Two(-1.f), h2[k], hi_t) + fma2(Two(-1.f), l2[k], lo_t);
+              float e0, e1;
+              gap.get(e0, e1);
+              Two w = Two(gram[i][4 * j + 2 * k], gram[i][4 * j + 2 * k + 1]) * d2[k] * Two(fast_exp2(e0), fast_exp2(e1));
+              if (diagonal) {
+                float w0, w1;
+                w.get(w0, w1);
+                w = Two(s0 + 2 * k <= row ? w0 : 0.f, s0 + 2 * k + 1 <= row ? w1 : 0.f);
+              }
+              split_two(w, piece[2 * j + k]);
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            uint32_t out[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) out[j] = piece[j][k];
+            tmem_st8(t_lane + kColM + 64 * k + 8 * u, out);
+          }
+        } else {
+          no_weights(u, 2);                                    // (the second sum lay over two of the pieces)
+        }
+        tmem_st_wait();
+        fence_before_sync();
+        arrive(i == 0 ? kBarP1 : kBarP2);
+      }
+      // the state
+      wait(kBarD, par);
+      fence_after_sync();
+      float v[8], v1[8], v2[8];
+      tmem_ld8(t_lane + kColD + 8 * qt, v);
+      tmem_ld8(t_lane + kColD + 32 + 8 * qt, v1);
+      tmem_ld8(t_lane + kColD + 64 + 8 * qt, v2);
+      tmem_ld_wait();
+      if (holds) {
+        const float total = sm.total[st];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) S[i] = fmaf(total, S[i], (v2[i] + v1[i]) + v[i]);
+      }
+      publish();
+      fence_before_sync();
+      fence_async_proxy();
+      arrive(kBarS);
+      // the outputs of token `row`
+      wait(kBarY, par);
+      fence_after_sync();
+      float own[8];
+      tmem_ld8(t_lane + kColY0 + 8 * qt, v);
+      tmem_ld8(t_lane + kColY0 + 32 + 8 * qt, v1);
+      tmem_ld8(t_lane + kColY1 + 8 * qt, own);
+      tmem_ld_wait();
+      fence_before_sync();
+      {
+        const float grown = sm.grown[st][row];
+        const uint4 in = *reinterpret_cast<const uint4*>(sm.x[st] + swz64(row, qt));
+        const uint32_t q[4] = {in.x, in.y, in.z, in.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[2 * i] = fmaf(grown, v1[2 * i] + v[2 * i], own[2 * i]) + dskip * __uint_as_float(q[i] << 16);
+          v[2 * i + 1] = fmaf(grown, v1[2 * i + 1] + v[2 * i + 1], own[2 * i + 1]) + dskip * __uint_as_float(q[i] & 0xffff0000u);
+        }
+        if (c * kChunk + row < n_tok)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) probe = fmaf(v[i], 0.f, probe);
+        *reinterpret_cast<float4*>(&sm.out[row][8 * qt]) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(&sm.out[row][8 * qt + 4]) = make_float4(v[4], v[5], v[6], v[7]);
+      }
+      named_barrier(4 + quad, 128);                            // the four warps of these 32 tokens; then eight lanes a token
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int r = 32 * quad + 8 * qt + 4 * i + (lane >> 3), e = 4 * (lane & 7);
+        if (c * kChunk + r < n_tok)
+          *reinterpret_cast<float4*>(y + (size_t)(start + c * kChunk + r) * inner + h * P + p0 + e) = *reinterpret_cast<const float4*>(&sm.out[r][e]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) probe = fmaf(S[i], 0.f, probe);
+  } else if (warp == kIssueWarp) {
+    if (lane == 0) {
+      constexpr uint32_t kIdescG = mma_idesc(128, kChunk, false), kIdesc1 = mma_idesc(128, kChunkCols, true),
+                         kIdesc2 = mma_idesc(128, 2 * kChunkCols, true), kIdescT = mma_idesc(128, 3 * kChunkCols, true) | (1u << 15);
+      constexpr uint64_t kBlock = (kChunk * 128) >> 4;         // from a tile's first 64 state rows to its others, in 16-byte pieces
+      constexpr uint64_t kPiece = (kChunk * 64) >> 4;
+      const uint64_t ds = desc_rows64(smem_u32(sm.s[0])), dw = desc_rows64(smem_u32(sm.w[0]));
+      bool ok = true;
+      auto wait = [&](int which, uint32_t parity) {
+        if (ok) ok = mbar_wait_or_abort(bar(which), parity, abort_flag);
+        fence_after_sync();
+        return ok;
+      };
+      auto issue_g = [&](int c, int half) {                    // a sum of G over half of the state's rows
+        const uint64_t dc = make_desc(smem_u32(sm.c[c & 1][0])), db = make_desc(smem_u32(sm.b[c & 1][0]));
+#pragma unroll
+        for (int i = 0; i < N / 32; ++i) {
+          const int k = half * (N / 32) + i;
+          mma_bf16(tmem + half * kColM, dc + (k >> 2) * kBlock + 2 * (k & 3), db + (k >> 2) * kBlock + 2 * (k & 3), kIdescG, i > 0);
+        }
+      };
+      auto issue_y1 = [&](uint64_t dx, int half) {             // the part of Y1 from half of the chunk's tokens, the smallest pieces first
+#pragma unroll
+        for (int p = 2; p >= 0; --p)
+#pragma unroll
+          for (int i = 0; i < kChunk / 32; ++i) {
+            const int k = half * (kChunk / 32) + i;
+            mma_bf16_a_tmem(tmem + kColY1, tmem + kColM + 64 * p + 8 * k, dx + 64 * k, kIdesc1, half || p < 2 || i > 0);
+          }
+      };
+      if (wait(kBarS, 0) && wait(kBarL, 0)) {
+        issue_g(0, 0);
+        issue_g(0, 1);
+        mma_commit(bar(kBarG));
+      }
+      for (int c = 0; c < n_chunks && ok; ++c) {
+        const int st = c & 1;
+        if (c > 0 && !wait(kBarS, c & 1)) break;
+        if (!wait(kBarW, c & 1)) break;
+        const uint64_t dc = make_desc(smem_u32(sm.c[st][0]));
+#pragma unroll
+        for (int k = 0; k < N / 16; ++k)                       // Y0 = C S
+          mma_bf16(tmem + kColY0, dc + (k >> 2) * kBlock + 2 * (k & 3), ds + 64 * k, kIdesc2, k > 0);
+#pragma unroll
+        for (int k = 0; k < N / 16; ++k)
+          mma_bf16(tmem + kColY0 + 32, dc + (k >> 2) * kBlock + 2 * (k & 3), ds + 2 * kPiece + 64 * k, kIdesc1, 1);
+        // dS = B^T (weighted x): B's rows are its tokens, 64 state rows to a block
+        const uint64_t db = (make_desc(smem_u32(sm.b[st][0])) & ~((uint64_t)0x3fff << 16)) | (kBlock << 16);
+#pragma unroll
+        for (int k = 0; k < kChunk / 16; ++k) mma_bf16(tmem + kColD, db + 128 * k, dw + 64 * k, kIdescT, k > 0);
+        mma_commit(bar(kBarD));
+        const uint64_t dx = desc_rows64(smem_u32(sm.x[st]));
+        if (!wait(kBarP1, c & 1)) break;
+        issue_y1(dx, 0);
+        if (c + 1 < n_chunks) {
+          if (!wait(kBarL + (st ^ 1), ((c + 1) >> 1) & 1)) break;
+          issue_g(c + 1, 0);
+        }
+        if (!wait(kBarP2, c & 1)) break;
+        issue_y1(dx, 1);
+        mma_commit(bar(kBarY));
+        if (c + 1 < n_chunks) {
+          if (!wait(kBarY, c & 1)) break;                      // (the weights have been read: G's second sum goes over them)
+          issue_g(c + 1, 1);
+          mma_commit(bar(kBarG));
+        }
+      }
+    }
+    __syncwarp();
+  } else {                                                     // steps and decays: token 32 w + lane of a chunk
+    const int w = warp - kStepWarp, r = 32 * w + lane;
+    const float a = -expf(a_log[h]), bias = dt_bias[h];
+    auto load_stage = [&](int c) {                             // (rows behind the request's are looked at by nothing that is kept)
+      const int st = c & 1, at = start + c * kChunk;
+      const uint32_t full = bar(kBarL + st);
+      mbar_expect(full, (N > 64 ? 4 : 2) * kChunk * 128 + kChunk * 64);
+      for (int j = 0; j < (N > 64 ? 2 : 1); ++j) {
+        tma_load_box(smem_u32(sm.c[st][j]), &map_bc, inner + (G + g) * N + 64 * j, at, full);
+        tma_load_box(smem_u32(sm.b[st][j]), &map_bc, inner + g * N + 64 * j, at, full);
+      }
+      tma_load_box(smem_u32(sm.x[st]), &map_x, h * P + p0, at, full);
+    };
+    auto make_steps = [&](int c) {
+      const int st = c & 1, t = c * kChunk + r;
+      const float dt = t < n_tok ? softplus_f(__bfloat162float(proj[(size_t)(start + t) * ld + off_dt + h]) + bias) : 0.f;
+      double cum = (double)a * (double)dt;                     // inclusive sums over the lanes, then the warps before
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double v = __shfl_up_sync(0xffffffffu, cum, o);
+        if (lane >= o) cum += v;
+      }
+      if (lane == 31) sm.sums[w] = cum;
+      named_barrier(2, 32 * kStepWarps);
+      double all = 0.0;
+#pragma unroll
+      for (int i = 0; i < kStepWarps; ++i) {
+        if (i == w) cum += all;
+        all += sm.sums[i];
+      }
+      named_barrier(2, 32 * kStepWarps);                       // (all have read the sums)
+      const double l2 = cum * 1.4426950408889634;
+      const float hi = (float)l2;
+      sm.dt[st][r] = dt;
+      sm.hi[st][r] = hi;
+      sm.lo[st][r] = (float)(l2 - (double)hi);
+      sm.grown[st][r] = (float)exp(cum);
+      sm.weight[st][r] = (float)((double)dt * exp(all - cum));
+      if (r == kChunk - 1) sm.total[st] = (float)exp(all);
+    };
+    const bool copies = w == 0 && lane == 0;
+    if (copies) load_stage(0);
+    make_steps(0);
+    for (int c = 0; c < n_chunks; ++c) {
+      named_barrier(1, kTopThreads);
+      if (c + 1 < n_chunks) {
+        if (copies) load_stage(c + 1);
+        __syncwarp();
+        make_steps(c + 1);
       }
     }
   }
-  if (holds_state) {
-#pragma unroll
-    for (int nt = 0; nt < NTW; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) probe = fmaf(S[nt][i], 0.f, probe);
+  const bool odd = __syncthreads_or(!(probe == 0.f));
+  const bool gave_up = *abort_flag != 0;
+  if (gave_up && threadIdx.x == 0) {
+    for (int c = max(0, n_chunks - 2); c < n_chunks; ++c) mbar_wait(bar(kBarL + (c & 1)), (c >> 1) & 1);
+    if (status) atomicCAS(status, 0, 7000000);
   }
-  if (__syncthreads_or(!(probe == 0.f))) {
-    static_assert(scan_smem(N, kChunkCols, N / 8) <= sizeof(ChunkSmem<N>) && N / 8 * kChunkCols <= kChunkWarps * 32, "the walk has room");
-    scan_tokens<__nv_bfloat16, 8, true>(reinterpret_cast<float*>(smem_raw), xbc, channels, proj, ld, off_dt, dt_bias, a_log, d_skip, state,
+  __syncthreads();
+  if (warp == kIssueWarp) {
+    fence_after_sync();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+  if (gave_up) return;
+  if (odd) {
+    static_assert(scan_smem(N, kChunkCols, N / 8) <= sizeof(ChunkSmem) && N / 8 * kChunkCols <= kChunkWarps * 32, "the walk has room");
+    scan_tokens<__nv_bfloat16, 8, true>(reinterpret_cast<float*>(smem), xbc, channels, proj, ld, off_dt, dt_bias, a_log, d_skip, state,
                                         seq_starts, state_slots, y, H, P, N, G, kChunkCols, h, seq, p0);
     return;
   }
-  if (holds_state) {
+  if (holds) {
 #pragma unroll
-    for (int nt = 0; nt < NTW; ++nt)
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        *reinterpret_cast<float2*>(s_glob + (size_t)(s_row + qr + 8 * j) * P + s_col + 8 * nt + 2 * qc) =
-            make_float2(S[nt][2 * j], S[nt][2 * j + 1]);
+    for (int i = 0; i < 8; i += 2) *reinterpret_cast<float2*>(s_glob + i) = make_float2(S[i], S[i + 1]);
   }
 }
 #endif  // ERB_ELEM == 1
@@ -754,17 +910,18 @@ gated_group_norm_vec_kernel(const void* __restrict__ x_, int x_ld, const T* __re
 
 #if ERB_ELEM == 1
 // Whether the chunk kernel is the faster one: the two costs in microseconds, fitted to both kernels' times over 1 to 64
-// requests of 2 to 500 tokens (8 to 64 heads of 64 x 64 and 64 x 128; within 20 % of them).  The walk costs 0.28 us a token
-// of the longest portion or, when the GPU is full, its blocks' tokens and states; a chunk costs 3.7 us for the longest
-// portion or, when it is full, a share of an SM for every chunk, be it full or not.  One request: from 17 (64 x 128) to 24
-// tokens on; 32 requests of equal length: from 32 (64 x 128) to 48.
+// requests of 2 to 2,048 tokens (64 heads of 64 x 128 and 32 of 64 x 64; of 196 pairs measured none is decided wrongly by more than 3 %).
+// The walk costs 0.27 us a token of the longest portion or, when the GPU is full, its blocks' tokens and states; a chunk of 128 tokens
+// costs 3.7 us for the longest portion, or as many rounds of blocks as the SMs need, a block an SM.  One request: from 26 tokens on
+// (64 x 128; 24 tokens 9.8 us walked, 10.5 in a chunk; 32 12.1 | 10.3; 64 20.5 | 10.4); 32 requests of equal length: from 42.
 inline bool chunks_pay(int blocks, int N, int n_tokens, int n_seqs, int longest) {
   if (longest <= 1) return false;
   const double size = N / 128.0, extra = (double)n_tokens - n_seqs - (longest - 1);      // tokens beyond one of the other requests
-  const double others = extra < n_seqs - 1 ? extra : n_seqs - 1;
-  const double chunks = (longest + 63) / 64 + (others > 0.0 ? others + extra / 64.0 : 0.0);
-  const double walk = fmax(3.0 + 0.28 * longest, blocks * size * (0.0015 * n_tokens + 0.008 * n_seqs));
-  const double chunked = fmax(3.5 + 3.7 * ((longest + 63) / 64), 0.036 * blocks * chunks);
+  const double others = fmax(0.0, extra < n_seqs - 1 ? extra : n_seqs - 1);
+  const double longest_chunks = (longest + kChunk - 1) / kChunk, chunks = longest_chunks + (others > 0.0 ? others + extra / kChunk : 0.0);
+  const double walk = fmax(3.0 + 0.27 * longest, blocks * size * (0.00165 * n_tokens + 0.008 * n_seqs));
+  const double rounds = ceil(blocks * (1.0 + others) / sm_count());
+  const double chunked = fmax(6.6 + 3.68 * longest_chunks, rounds * (3.0 + 2.4 * size + 3.65 * chunks / (1.0 + others)));
   return chunked < walk;
 }
 #endif
@@ -808,21 +965,27 @@ ERB_EXPORT int erb_conv_state_update(const void* proj, int n_seqs, int ld, int o
 
 ERB_EXPORT int erb_ssm_scan(const void* xbc, int channels, const void* proj, int ld, int off_dt, const float* dt_bias,
                             const float* a_log, const float* d_skip, float* state, const int* seq_starts,
-                            const int* state_slots, float* y, int n_seqs, int n_tokens, int longest, int H, int P, int N, int G, void* stream) {
+                            const int* state_slots, float* y, int n_seqs, int n_tokens, int longest, int H, int P, int N, int G, int* status,
+                            void* stream) {
   if (n_seqs <= 0) return ERB_OK;
   if (H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G || P > 512) return fail(ERB_ERR_ARG, "ssm_scan: bad sizes (columns of at most 512)");
   int most_tokens = INT_MAX;            // what the scan takes: every portion, or single tokens beside the chunk kernel's portions
 #if ERB_ELEM == 1
   if ((N == 32 || N == 64 || N == 128) && P % kChunkCols == 0 && chunks_pay(H * (P / kChunkCols), N, n_tokens, n_seqs, longest) && channels % 8 == 0 &&
-      !((uintptr_t)xbc & 15) && !((uintptr_t)state & 7) && !((uintptr_t)y & 7)) {
-    const size_t bytes = N == 32 ? sizeof(ChunkSmem<32>) : N == 64 ? sizeof(ChunkSmem<64>) : sizeof(ChunkSmem<128>);
+      !((uintptr_t)xbc & 15) && !((uintptr_t)state & 7) && !((uintptr_t)y & 15)) {
+    constexpr size_t bytes = sizeof(ChunkSmem) + 1024;
     auto kern = N == 32 ? ssm_chunk_kernel<32> : N == 64 ? ssm_chunk_kernel<64> : ssm_chunk_kernel<128>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "ssm_scan: %s", cudaGetErrorString(e));
-    launch_chained(kern, dim3(H, n_seqs, P / kChunkCols), dim3((kChunkWarps + 1) * 32), bytes, (cudaStream_t)stream,
+    CUtensorMap bc, x;
+    int rc;
+    if ((rc = rows_map(&bc, xbc, n_tokens, channels, channels, kChunk, "ssm_scan")) ||
+        (rc = rows_map(&x, xbc, n_tokens, channels, channels, kChunk, "ssm_scan", kChunkCols)))
+      return rc;
+    launch_chained(kern, dim3(H, n_seqs, P / kChunkCols), dim3(kChunkThreads), bytes, (cudaStream_t)stream, bc, x,
                    (const elem_t*)xbc, channels, (const elem_t*)proj, ld, off_dt, dt_bias, a_log, d_skip, state, seq_starts,
-                   state_slots, y, H, P, G);
-    const int rc = check_launch("ssm_chunk");
+                   state_slots, y, H, P, G, status);
+    rc = check_launch("ssm_chunk");
     if (rc || n_seqs == 1) return rc;
     most_tokens = 1;
     n_tokens = n_seqs;                  // (below: the shape for single tokens)

@@ -282,24 +282,24 @@ inline int pool_map(CUtensorMap* out, const void* pool, unsigned long long rows,
   return ERB_OK;
 }
 
-// A tensor map over `rows` rows of `cols` bfloat16, `ld` elements apart, with boxes of 64 columns x `box_rows` rows and the
-// 128-byte swizzle (columns behind `cols` read as zeros).  Kept like the maps of page pools.
+// A tensor map over `rows` rows of `cols` bfloat16, `ld` elements apart, with boxes of `box_cols` columns (64 with the 128-byte swizzle,
+// 32 with the 64-byte one) x `box_rows` rows (columns behind `cols` read as zeros).  Kept like the maps of page pools.
 inline int rows_map(CUtensorMap* out, const void* base, unsigned long long rows, unsigned cols, unsigned long long ld, unsigned box_rows,
-                    const char* who) {
-  static std::map<std::tuple<const void*, unsigned long long, unsigned, unsigned long long, unsigned>, CUtensorMap> maps;
+                    const char* who, unsigned box_cols = 64) {
+  static std::map<std::tuple<const void*, unsigned long long, unsigned, unsigned long long, unsigned, unsigned>, CUtensorMap> maps;
   static std::mutex mutex;
   std::lock_guard<std::mutex> lock(mutex);
-  const auto key = std::make_tuple(base, rows, cols, ld, box_rows);
+  const auto key = std::make_tuple(base, rows, cols, ld, box_rows, box_cols);
   auto it = maps.find(key);
   if (it == maps.end()) {
     CUtensorMap m;
     const cuuint64_t dims[2] = {cols, rows};
     const cuuint64_t strides[1] = {ld * 2};
-    const cuuint32_t box[2] = {64, box_rows};
+    const cuuint32_t box[2] = {box_cols, box_rows};
     const cuuint32_t elem[2] = {1, 1};
     const CUresult r = cuTensorMapEncodeTiled(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
-                                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                                              CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ERB_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed (%d)", who, (int)r);
     if (maps.size() > 4096) maps.clear();
     it = maps.emplace(key, m).first;

@@ -33,7 +33,7 @@ LIBRARIES: dict[str, tuple[str, tuple[str, ...], bool]] = {
     "attention": ("attention.cu", (), True),
     "latent_attention": ("latent_attention.cu", (), True),
     "diff_attention": ("diff_attention.cu", (), True),
-    "ssm": ("ssm.cu", (), True),
+    "ssm": ("ssm.cu", ("-lcuda",), True),
     "delta": ("delta.cu", (), True),
     "depth": ("depth.cu", (), True),
     "moe": ("moe.cu", (), True),

@@ -1,0 +1,38 @@
+"""The state-space recurrence 128 tokens at a time, at the edges of its chunks and of the next request's rows."""
+
+import pytest
+import torch
+
+from edgerag_b200.ops import kernels
+from test_scan_chunks import _ssm_reference
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N", [32, 64, 128])
+@pytest.mark.parametrize("lens", [[127], [128], [129, 1], [256, 255, 2], [257, 5]])
+@pytest.mark.parametrize("bad", [False, True])
+def test_chunks_of_128_tokens(N, lens, bad):
+    """Against float64, within a few hundred roundings of the largest result (both are float throughout).  ``bad``: the request behind
+    brings numbers that are not finite, which lie in the rows that a chunk's copies reach behind their own request."""
+    H, P, G, n = 4, 64, 2, sum(lens)
+    inner = H * P
+    g = torch.Generator().manual_seed(N + n)
+    xbc = (torch.randn(n + 3, inner + 2 * G * N, generator=g) * 0.5).to(torch.bfloat16)
+    proj, a_log = torch.randn(n + 3, H, generator=g).to(torch.bfloat16), torch.randn(H, generator=g) * 0.3
+    dt_bias, skip, before = torch.randn(H, generator=g) - 1.0, torch.randn(H, generator=g), torch.randn(len(lens) + 1, H, N, P, generator=g)
+    if bad:
+        xbc[n:] = float("inf")
+    starts = torch.tensor([0, *torch.tensor(lens + [3]).cumsum(0).tolist()], dtype=torch.int32).cuda()
+    slots = torch.arange(len(lens) + 1, dtype=torch.int32).cuda()
+    dev = [t.cuda() for t in (xbc, proj, dt_bias, a_log, skip)]
+    state, y = before.clone().cuda(), torch.full((n + 3, inner), float("nan"), device="cuda")
+    kernels.ssm_scan(dev[0], dev[1], 0, dev[2], dev[3], dev[4], state, len(lens) + 1, starts, slots, y, G, longest=1 << 20)
+    at = 0
+    for s, length in enumerate(lens):
+        rows = slice(at, at + length)
+        want_y, want_s = _ssm_reference(dev[0][rows], dev[1][rows], dev[2], dev[3], dev[4], before[s].cuda(), H, P, N, G)
+        assert (y[rows].double() - want_y).abs().max() < 3e-5 * max(1.0, want_y.abs().max()), s
+        assert (state[s].double() - want_s).abs().max() < 3e-5 * max(1.0, want_s.abs().max()), s
+        at += length
+    assert bad or torch.isfinite(y).all()
