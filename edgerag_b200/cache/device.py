@@ -26,6 +26,7 @@ class DevicePools:
         self.poison = poison
         #: per group: (key pool, value pool, the dimension of each that counts pages)
         self._pools: list[tuple[torch.Tensor, torch.Tensor, int]] = []
+        self._layer_pages: dict[int, tuple[torch.Tensor, torch.Tensor]] = {}
         self.kv: list[torch.Tensor] = []         # the allocations themselves (one or two per group)
         fill = float("nan") if poison else 0.0
         for g, n in zip(layout.groups, num_pages):
@@ -48,12 +49,15 @@ class DevicePools:
     def pages_of(self, cache_layer: int) -> tuple[torch.Tensor, torch.Tensor]:
         """Key pages ``[pages, kv heads, page_size, head_dim]`` and value pages (the same shape, or
         ``v_head_dim`` wide where the group says so) of one cache layer."""
-        placed = self.layout.placement[cache_layer]
-        if placed is None:
-            raise KeyError(f"cache layer {cache_layer} holds no pages")
-        group, local = placed
-        keys, values, _ = self._pools[group]
-        return keys[local], values[local]
+        views = self._layer_pages.get(cache_layer)      # (the pools stay where they are)
+        if views is None:
+            placed = self.layout.placement[cache_layer]
+            if placed is None:
+                raise KeyError(f"cache layer {cache_layer} holds no pages")
+            group, local = placed
+            keys, values, _ = self._pools[group]
+            views = self._layer_pages[cache_layer] = (keys[local], values[local])
+        return views
 
     def zero_slots(self, slots: list[int]) -> None:
         if slots and self.states:

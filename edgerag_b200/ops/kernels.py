@@ -160,22 +160,41 @@ def launches() -> int:
     return launch_counts["own"] + launch_counts["library"]
 
 
+_host = None             # the module csrc/launch.cpp, once the first entry point has been asked for (False: it cannot be built)
+_KINDS = {c_void_p: "p", c_int: "i", c_longlong: "i", c_float: "f"}
+
+
+def _bind_host() -> None:
+    """Calls and checks through the host module from here on, where there is one."""
+    global _host, _call, _need
+    _host = native.load_host() or False
+    if _host:
+        _host.bind(launch_counts, KernelError, _need_in_python)
+        _call, _need = _host.call, _host.need
+
+
 def _fn(library: str, elem: str | None, name: str):
     key = (library, elem, name)
     fn = _functions.get(key)
     if fn is None:
+        if _host is None:
+            _bind_host()
         lib = native.load(library, elem)
         fn = getattr(lib, name)
-        fn.argtypes = _SIGNATURES[name]
-        fn.restype = c_int
-        fn._erb_lib = lib
-        fn._erb_own = _LAUNCHES.get(name, 1)
+        own = _LAUNCHES.get(name, 1)
+        if _host:
+            address = lambda f: ctypes.cast(f, c_void_p).value      # noqa: E731
+            fn = _host.launcher(address(fn), address(lib.erb_last_error), "".join(_KINDS[t] for t in _SIGNATURES[name]), own)
+        else:
+            fn.argtypes, fn.restype, fn._erb_lib, fn._erb_own = _SIGNATURES[name], c_int, lib, own
         _functions[key] = fn
     return fn
 
 
 def _call(fn, *args) -> None:
-    rc = fn(*args)
+    if _host:               # (the call for which the module was loaded)
+        return _host.call(fn, *args)
+    rc = fn(*(a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args))
     if fn._erb_own:
         launch_counts["own"] += fn._erb_own
     else:
@@ -201,7 +220,7 @@ def _stream() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def _need(t: torch.Tensor | None, name: str, dtype=None, contiguous: bool = True) -> None:
+def _need_in_python(t: torch.Tensor | None, name: str, dtype=None, contiguous: bool = True) -> None:
     if t is None:
         return
     if not t.is_cuda:
@@ -210,6 +229,9 @@ def _need(t: torch.Tensor | None, name: str, dtype=None, contiguous: bool = True
         raise KernelError(f"{name} has dtype {t.dtype}, expected {dtype}")
     if contiguous and not t.is_contiguous():
         raise KernelError(f"{name} is not contiguous")
+
+
+_need = _need_in_python
 
 
 # --- rows ------------------------------------------------------------------------------------
@@ -226,9 +248,9 @@ def embed_rows(hidden: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, sta
         _need(embeds, "embeds", table.dtype)
         if embeds.shape[1] != h or embed_row is None:
             raise KernelError("embed_rows: embeds need embed_row and the hidden width")
-    _call(_fn("elementwise", _elem(table), "erb_embed_rows"), hidden.data_ptr(), table.data_ptr(),
-          _ptr(embeds), ids.data_ptr(), _ptr(embed_row), n, h, table.shape[0],
-          0 if embeds is None else embeds.shape[0], status.data_ptr(), float(scale), _stream())
+    _call(_fn("elementwise", _elem(table), "erb_embed_rows"), hidden, table,
+          embeds, ids, embed_row, n, h, table.shape[0],
+          0 if embeds is None else embeds.shape[0], status, float(scale), _stream())
 
 
 def embed_sum(hidden: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, status: torch.Tensor, positions: torch.Tensor, *,
@@ -257,10 +279,10 @@ def embed_sum(hidden: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, stat
         buckets, mul_prev, mul_cur = (int(v) for v in pair_hash)
         if pairs.shape[0] != buckets + 1:
             raise KernelError("embed_sum: the table of pairs has a row per bucket and one more")
-    _call(_fn("elementwise", _elem(table), "erb_embed_sum"), hidden.data_ptr(), table.data_ptr(), _ptr(embeds), ids.data_ptr(),
-          _ptr(embed_row), n, h, table.shape[0], 0 if embeds is None else embeds.shape[0], status.data_ptr(), float(scale), _ptr(pairs),
-          buckets, mul_prev, mul_cur, _ptr(seq_of_token), _ptr(seq_starts), _ptr(state_slots), _ptr(last_id), positions.data_ptr(),
-          _ptr(pos_table), 0 if pos_table is None else pos_table.shape[0], _stream())
+    _call(_fn("elementwise", _elem(table), "erb_embed_sum"), hidden, table, embeds, ids,
+          embed_row, n, h, table.shape[0], 0 if embeds is None else embeds.shape[0], status, float(scale), pairs,
+          buckets, mul_prev, mul_cur, seq_of_token, seq_starts, state_slots, last_id, positions,
+          pos_table, 0 if pos_table is None else pos_table.shape[0], _stream())
 
 
 def add_rmsnorm(hidden: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, eps: float,
@@ -286,12 +308,12 @@ def add_rmsnorm(hidden: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, e
     if rows is not None and rows.numel() < n:
         raise KernelError("add_rmsnorm: fewer row indices than output rows")
     if in_parts:
-        _call(_fn("elementwise", _elem(out), "erb_add_rmsnorm_parts"), hidden.data_ptr(), delta.data_ptr(), delta.shape[0],
-              delta.stride(0), weight.data_ptr(), out.data_ptr(), _ptr(rows), n, h, float(eps),
+        _call(_fn("elementwise", _elem(out), "erb_add_rmsnorm_parts"), hidden, delta, delta.shape[0],
+              delta.stride(0), weight, out, rows, n, h, float(eps),
               int(write_back and rows is None), int(bool(settled)) | (2 if exact else 0), float(delta_scale), _stream())
         return
-    _call(_fn("elementwise", _elem(out), "erb_add_rmsnorm"), hidden.data_ptr(), _ptr(delta), weight.data_ptr(),
-          out.data_ptr(), _ptr(rows), n, h, float(eps), int(write_back and rows is None),
+    _call(_fn("elementwise", _elem(out), "erb_add_rmsnorm"), hidden, delta, weight,
+          out, rows, n, h, float(eps), int(write_back and rows is None),
           int(bool(settled)) | (2 if exact else 0), float(delta_scale), _stream())
 
 
@@ -303,12 +325,12 @@ def residual_add(hidden: torch.Tensor, delta: torch.Tensor, dtype: torch.dtype |
         _need(delta, "delta", torch.float32)
         if delta.shape[1:] != hidden.shape or dtype is None:
             raise KernelError("residual_add: partial sums need [parts, rows, width] and the element type to round to")
-        _call(_fn("elementwise", _ELEM[dtype], "erb_residual_add_parts"), hidden.data_ptr(), delta.data_ptr(), delta.shape[0],
+        _call(_fn("elementwise", _ELEM[dtype], "erb_residual_add_parts"), hidden, delta, delta.shape[0],
               delta.stride(0), hidden.numel(), float(scale), _stream())
         return
     if hidden.shape != delta.shape:
         raise KernelError("residual_add: shapes disagree")
-    _call(_fn("elementwise", _elem(delta), "erb_residual_add"), hidden.data_ptr(), delta.data_ptr(),
+    _call(_fn("elementwise", _elem(delta), "erb_residual_add"), hidden, delta,
           hidden.numel(), float(scale), _stream())
 
 
@@ -352,9 +374,9 @@ def add_layernorm(hidden: torch.Tensor, weight: torch.Tensor | None, bias: torch
         n, out_ld = hidden.shape[0], h
         if rows is not None:
             raise KernelError("add_layernorm: a selection of rows needs an output")
-    _call(_fn("elementwise", _ELEM[elem], "erb_add_layernorm"), hidden.data_ptr(), _ptr(delta), delta.shape[0] if in_parts else 0,
-          delta.stride(0) if in_parts else 0, _ptr(pw), _ptr(pb), float(peps), _ptr(weight), _ptr(bias), float(eps), _ptr(out),
-          int(out_ld), _ptr(rows), n, h, int(write_back and rows is None), _stream())
+    _call(_fn("elementwise", _ELEM[elem], "erb_add_layernorm"), hidden, delta, delta.shape[0] if in_parts else 0,
+          delta.stride(0) if in_parts else 0, pw, pb, float(peps), weight, bias, float(eps), out,
+          int(out_ld), rows, n, h, int(write_back and rows is None), _stream())
 
 
 def rms_between(hidden: torch.Tensor, out: torch.Tensor | None, *, weight: torch.Tensor | None = None, eps: float = 0.0,
@@ -400,10 +422,10 @@ def rms_between(hidden: torch.Tensor, out: torch.Tensor | None, *, weight: torch
         n, out_ld = hidden.shape[0], h
         if rows is not None:
             raise KernelError("rms_between: a selection of rows needs an output")
-    _call(_fn("elementwise", _ELEM[elem], "erb_rms_between"), hidden.data_ptr(), _ptr(delta), delta.shape[0] if in_parts else 0,
-          delta.stride(0) if in_parts else 0, _ptr(bias), _ptr(own[0]) if own else None, float(own[1]) if own else 0.0,
-          _ptr(post[0]) if post else None, float(post[1]) if post else 0.0, _ptr(weight), float(eps), _ptr(out), int(out_ld),
-          _ptr(rows), n, h, int(write_back and rows is None), _stream())
+    _call(_fn("elementwise", _ELEM[elem], "erb_rms_between"), hidden, delta, delta.shape[0] if in_parts else 0,
+          delta.stride(0) if in_parts else 0, bias, _ptr(own[0]) if own else None, float(own[1]) if own else 0.0,
+          _ptr(post[0]) if post else None, float(post[1]) if post else 0.0, weight, float(eps), out, int(out_ld),
+          rows, n, h, int(write_back and rows is None), _stream())
 
 
 def qkv_whole_norm(qkv: torch.Tensor, positions: torch.Tensor, n_q_heads: int, n_kv_heads: int, head_dim: int, *,
@@ -442,10 +464,10 @@ def qkv_whole_norm(qkv: torch.Tensor, positions: torch.Tensor, n_q_heads: int, n
     if k_pages is not None and (tuple(k_pages.shape[1:]) != (n_kv_heads, page_size, head_dim) or v_pages is None
                                 or v_pages.shape != k_pages.shape or slots is None or slots.numel() < n):
         raise KernelError("qkv_whole_norm: pages or slots disagree with the heads")
-    _call(_fn("elementwise", _elem(qkv), "erb_qkv_whole_norm"), qkv.data_ptr(), qkv.stride(0) if n > 1 else qkv.shape[1],
-          _ptr(q_bias), _ptr(k_bias), _ptr(v_bias), _ptr(q_norm), _ptr(k_norm), int(q_count), int(k_count), float(eps),
-          positions.data_ptr(), _ptr(inv_freq), int(rot_dim), _ptr(slots), _ptr(k_pages), _ptr(v_pages), n, n_q_heads,
-          n_kv_heads, head_dim, int(page_size), int(bool(has_kv)), _ptr(first_values), _ptr(blend), int(blend is None), v_dim, _stream())
+    _call(_fn("elementwise", _elem(qkv), "erb_qkv_whole_norm"), qkv, qkv.stride(0) if n > 1 else qkv.shape[1],
+          q_bias, k_bias, v_bias, q_norm, k_norm, int(q_count), int(k_count), float(eps),
+          positions, inv_freq, int(rot_dim), slots, k_pages, v_pages, n, n_q_heads,
+          n_kv_heads, head_dim, int(page_size), int(bool(has_kv)), first_values, blend, int(blend is None), v_dim, _stream())
 
 
 def cast_rows(src: torch.Tensor, dst: torch.Tensor) -> None:
@@ -454,7 +476,7 @@ def cast_rows(src: torch.Tensor, dst: torch.Tensor) -> None:
     n, width = src.shape
     if dst.shape != (n, width) or dst.stride(1) != 1:
         raise KernelError("cast_rows: shapes disagree")
-    _call(_fn("elementwise", _elem(dst), "erb_cast_rows"), src.data_ptr(), dst.data_ptr(), n, width,
+    _call(_fn("elementwise", _elem(dst), "erb_cast_rows"), src, dst, n, width,
           dst.stride(0) if n > 1 else max(width, dst.stride(0)), _stream())
 
 
@@ -463,7 +485,7 @@ def stream_set(hidden: torch.Tensor, y: torch.Tensor, vec: torch.Tensor | None =
     _need(hidden, "hidden", torch.float32); _need(y, "y"); _need(vec, "vec", torch.float32)
     if y.shape != hidden.shape or (vec is not None and vec.numel() != hidden.shape[1]):
         raise KernelError("stream_set: shapes disagree")
-    _call(_fn("elementwise", _elem(y), "erb_stream_set"), hidden.data_ptr(), y.data_ptr(), _ptr(vec), hidden.shape[0],
+    _call(_fn("elementwise", _elem(y), "erb_stream_set"), hidden, y, vec, hidden.shape[0],
           hidden.shape[1], _stream())
 
 
@@ -495,9 +517,9 @@ def qk_prepare(qkv: torch.Tensor, positions: torch.Tensor, n_q_heads: int, n_kv_
             raise KernelError("qk_prepare: a cache write needs k_pages, v_pages, slots and the page size")
         if tuple(k_pages.shape[1:]) != (n_kv_heads, page_size, head_dim) or k_pages.shape != v_pages.shape:
             raise KernelError("qk_prepare: page layout is not [pages, kv heads, page_size, head_dim]")
-    _call(_fn("elementwise", _elem(qkv), "erb_qk_prepare"), qkv.data_ptr(), qkv.stride(0) if n > 1 else qkv.shape[1], _ptr(q_bias),
-          _ptr(k_bias), _ptr(q_norm), _ptr(k_norm), float(eps), positions.data_ptr(), _ptr(inv_freq), int(rot_dim), int(pairs),
-          _ptr(slots), _ptr(k_pages), _ptr(v_pages), n, n_q_heads, n_kv_heads, head_dim, max(1, int(page_size)),
+    _call(_fn("elementwise", _elem(qkv), "erb_qk_prepare"), qkv, qkv.stride(0) if n > 1 else qkv.shape[1], q_bias,
+          k_bias, q_norm, k_norm, float(eps), positions, inv_freq, int(rot_dim), int(pairs),
+          slots, k_pages, v_pages, n, n_q_heads, n_kv_heads, head_dim, max(1, int(page_size)),
           int(values_are_keys), _stream())
 
 
@@ -506,13 +528,13 @@ def resolve_ids(ids: torch.Tensor, fed: torch.Tensor, dtype: torch.dtype = torch
     before that are still on the device.  ``dtype`` only picks the library that holds the kernel
     (the engine's element type, so that nothing else has to be built)."""
     _need(ids, "ids", torch.int32); _need(fed, "fed", torch.int32)
-    _call(_fn("elementwise", _ELEM[dtype], "erb_resolve_ids"), ids.data_ptr(), ids.numel(),
-          fed.data_ptr(), fed.numel(), _stream())
+    _call(_fn("elementwise", _ELEM[dtype], "erb_resolve_ids"), ids, ids.numel(),
+          fed, fed.numel(), _stream())
 
 
 def gather_cast(src: torch.Tensor, dst: torch.Tensor, rows: torch.Tensor | None) -> None:
     _need(src, "src", torch.float32); _need(dst, "dst"); _need(rows, "rows", torch.int32)
-    _call(_fn("elementwise", _elem(dst), "erb_gather_cast"), src.data_ptr(), dst.data_ptr(), _ptr(rows),
+    _call(_fn("elementwise", _elem(dst), "erb_gather_cast"), src, dst, rows,
           dst.shape[0], dst.shape[1], _stream())
 
 
@@ -538,8 +560,8 @@ def rope_cache_write(qkv: torch.Tensor, positions: torch.Tensor, inv_freq: torch
             raise KernelError("rope_cache_write: page layout is not [pages, kv heads, page_size, head_dim]")
     if rot_dim and (inv_freq is None or inv_freq.numel() != rot_dim // 2):
         raise KernelError("rope_cache_write: inv_freq must hold rot_dim / 2 values")
-    _call(_fn("elementwise", _elem(qkv), "erb_rope_cache_write"), qkv.data_ptr(), positions.data_ptr(),
-          _ptr(inv_freq), _ptr(slots), _ptr(k_pages), _ptr(v_pages), n, n_q_heads, n_kv_heads, head_dim,
+    _call(_fn("elementwise", _elem(qkv), "erb_rope_cache_write"), qkv, positions,
+          inv_freq, slots, k_pages, v_pages, n, n_q_heads, n_kv_heads, head_dim,
           rot_dim, page_size, int(write), _stream())
 
 
@@ -549,7 +571,7 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor) -> None:
     n, inter = out.shape
     if gate_up.shape != (n, 2 * inter):
         raise KernelError("swiglu: gate_up must be [tokens, 2 * intermediate]")
-    _call(_fn("elementwise", _elem(out), "erb_swiglu"), gate_up.data_ptr(), out.data_ptr(), n, inter, _stream())
+    _call(_fn("elementwise", _elem(out), "erb_swiglu"), gate_up, out, n, inter, _stream())
 
 
 GLU_ACTS = {"sigmoid": 0, "gelu_tanh": 1}
@@ -568,8 +590,8 @@ def glu_bounded(gate_up: torch.Tensor, out: torch.Tensor, limit: float = 0.0, al
     n, inter = out.shape
     if gate_up.shape != (n, 2 * inter):
         raise KernelError("glu_bounded: gate_up must be [tokens, 2 * intermediate]")
-    _call(_fn("elementwise", _elem(out), "erb_glu_bounded"), gate_up.data_ptr(), out.data_ptr(), n, inter, float(limit),
-          float(alpha), float(shift), GLU_ACTS[act], _ptr(row_scale), _stream())
+    _call(_fn("elementwise", _elem(out), "erb_glu_bounded"), gate_up, out, n, inter, float(limit),
+          float(alpha), float(shift), GLU_ACTS[act], row_scale, _stream())
 
 
 def softcap(logits: torch.Tensor, cap: float, dtype: torch.dtype) -> None:
@@ -579,7 +601,7 @@ def softcap(logits: torch.Tensor, cap: float, dtype: torch.dtype) -> None:
     if logits.dim() != 2 or logits.stride(1) != 1:
         raise KernelError("softcap: logits must be rows with unit inner stride")
     n, width = logits.shape
-    _call(_fn("elementwise", _ELEM[dtype], "erb_softcap"), logits.data_ptr(), n, width, logits.stride(0) if n > 1 else width,
+    _call(_fn("elementwise", _ELEM[dtype], "erb_softcap"), logits, n, width, logits.stride(0) if n > 1 else width,
           float(cap), _stream())
 
 
@@ -596,7 +618,7 @@ def act_rows(x: torch.Tensor, out: torch.Tensor, act: str, gate_col: int = -1) -
         raise KernelError("act_rows: shapes disagree")
     if act not in ACTS:
         raise KernelError(f"act_rows: unknown activation {act!r}; known: {sorted(ACTS)}")
-    _call(_fn("elementwise", _elem(x), "erb_act_rows"), x.data_ptr(), x.stride(0) if n > 1 else x.shape[1], out.data_ptr(), n, width,
+    _call(_fn("elementwise", _elem(x), "erb_act_rows"), x, x.stride(0) if n > 1 else x.shape[1], out, n, width,
           ACTS[act], int(gate_col), _stream())
 
 
@@ -606,7 +628,7 @@ def scale_rows(x: torch.Tensor, scale: float, dtype: torch.dtype) -> None:
     if x.dim() != 2 or x.stride(1) != 1:
         raise KernelError("scale_rows: rows with unit inner stride")
     n, width = x.shape
-    _call(_fn("elementwise", _ELEM[dtype], "erb_scale_rows"), x.data_ptr(), n, width, x.stride(0) if n > 1 else width, float(scale),
+    _call(_fn("elementwise", _ELEM[dtype], "erb_scale_rows"), x, n, width, x.stride(0) if n > 1 else width, float(scale),
           _stream())
 
 
@@ -616,7 +638,7 @@ def sigmoid_gate(x: torch.Tensor, gate: torch.Tensor) -> None:
     n, width = x.shape
     if gate.shape != x.shape or x.stride(1) != 1 or gate.stride(1) != 1:
         raise KernelError("sigmoid_gate: shapes or strides disagree")
-    _call(_fn("elementwise", _elem(x), "erb_sigmoid_gate"), x.data_ptr(), x.stride(0) if n > 1 else width, gate.data_ptr(),
+    _call(_fn("elementwise", _elem(x), "erb_sigmoid_gate"), x, x.stride(0) if n > 1 else width, gate,
           gate.stride(0) if n > 1 else width, n, width, _stream())
 
 
@@ -642,7 +664,7 @@ def sum_updates(hidden: torch.Tensor, a: torch.Tensor, b: torch.Tensor | None, d
         raise KernelError("sum_updates: out and hidden disagree")
     pa, na, sa = _update(a, hidden, dtype, "sum_updates")
     pb, nb, sb = _update(b, hidden, dtype, "sum_updates")
-    _call(_fn("depth", _ELEM[dtype], "erb_sum_updates"), hidden.data_ptr(), pa, na, sa, pb, nb, sb, _ptr(out), hidden.numel(), _stream())
+    _call(_fn("depth", _ELEM[dtype], "erb_sum_updates"), hidden, pa, na, sa, pb, nb, sb, out, hidden.numel(), _stream())
 
 
 def side_gate(g: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, offset: int, dim: int, out: torch.Tensor) -> None:
@@ -652,8 +674,8 @@ def side_gate(g: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, offset: i
     n, ld_out = out.shape
     if g.shape[0] != n or g.shape[1] < dim or dim > ld_out or g.stride(1) != 1 or ids.numel() < n or not 0 <= offset <= table.shape[1] - dim:
         raise KernelError("side_gate: shapes disagree")
-    _call(_fn("depth", _elem(g), "erb_side_gate"), g.data_ptr(), g.stride(0) if n > 1 else g.shape[1], table.data_ptr(), table.shape[1],
-          table.shape[0], ids.data_ptr(), int(offset), int(dim), out.data_ptr(), ld_out, n, _stream())
+    _call(_fn("depth", _elem(g), "erb_side_gate"), g, g.stride(0) if n > 1 else g.shape[1], table, table.shape[1],
+          table.shape[0], ids, int(offset), int(dim), out, ld_out, n, _stream())
 
 
 DEPTH_OUT = {"cast": 0, "layernorm": 1, "rmsnorm": 2}
@@ -684,10 +706,10 @@ def depth_mix(hidden: torch.Tensor, history: torch.Tensor, layer: int, mix: torc
         raise KernelError("depth_mix: a selection of rows needs an output")
     n_rows = n if out is None else out.shape[0]
     pd, nd, sd = _update(delta, hidden, dtype, "depth_mix")
-    _call(_fn("depth", _ELEM[dtype], "erb_depth_mix"), hidden.data_ptr(), pd, nd, sd, _ptr(post[0]) if post else None,
-          float(post[1]) if post else 0.0, history.data_ptr(), history.stride(0), layer + 1, mix.data_ptr(), DEPTH_OUT[out_kind],
-          _ptr(weight), _ptr(bias), float(eps), _ptr(out), h if out is None else (out.stride(0) if n_rows > 1 else max(h, out.stride(0))),
-          _ptr(rows), n_rows, h, int(write_back and rows is None), _stream())
+    _call(_fn("depth", _ELEM[dtype], "erb_depth_mix"), hidden, pd, nd, sd, _ptr(post[0]) if post else None,
+          float(post[1]) if post else 0.0, history, history.stride(0), layer + 1, mix, DEPTH_OUT[out_kind],
+          weight, bias, float(eps), out, h if out is None else (out.stride(0) if n_rows > 1 else max(h, out.stride(0))),
+          rows, n_rows, h, int(write_back and rows is None), _stream())
 
 
 # --- matrix products -------------------------------------------------------------------------
@@ -727,7 +749,7 @@ def _fn_tc(name: str):
     told = None if _status_word is None else _status_word.data_ptr()
     if told != _status_word_told:
         if _set_status_word is None:
-            _set_status_word = fn._erb_lib.erb_linear_tc_set_status_word
+            _set_status_word = native.load("linear_tc", None).erb_linear_tc_set_status_word
             _set_status_word.argtypes = [c_void_p]
             _set_status_word.restype = c_int
         _set_status_word(told)
@@ -754,7 +776,7 @@ def linear_few_rows(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) ->
         raise KernelError("linear_few_rows: shapes or strides disagree")
     if out.dtype not in (torch.bfloat16, torch.float32) or not linear_few_rows_supported(a, weight, lda):
         raise KernelError("linear_few_rows: operands not supported")
-    _call(_fn("gemm", "bfloat16", "erb_linear_skinny"), a.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k,
+    _call(_fn("gemm", "bfloat16", "erb_linear_skinny"), a, weight, out, m, n, k,
           lda, k, ldo, int(out.dtype == torch.float32), _stream())
 
 
@@ -770,7 +792,7 @@ def linear_tc(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
         raise KernelError("linear_tc: shapes or strides disagree")
     if out.dtype not in (torch.bfloat16, torch.float32) or not linear_few_rows_supported(a, weight, lda):
         raise KernelError("linear_tc: operands not supported")
-    _call(_fn_tc("erb_linear_tc"), a.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k, lda, k, ldo,
+    _call(_fn_tc("erb_linear_tc"), a, weight, out, m, n, k, lda, k, ldo,
           int(out.dtype == torch.float32), _stream())
 
 
@@ -817,7 +839,7 @@ def linear_parts(a: torch.Tensor, weight: torch.Tensor, parts: torch.Tensor) -> 
     if (weight.shape[1] != k or a.stride(1) != 1 or m > TC_MAX_ROWS or n % 4 or not linear_few_rows_supported(a, weight, a.stride(0))
             or tuple(parts.shape) != (linear_parts_slices(weight), m, n)):
         raise KernelError("linear_parts: shapes disagree or the operands are not supported")
-    _call(_fn_tc("erb_linear_tc_parts"), a.data_ptr(), weight.data_ptr(), parts.data_ptr(), m, n, k, a.stride(0), k, n,
+    _call(_fn_tc("erb_linear_tc_parts"), a, weight, parts, m, n, k, a.stride(0), k, n,
           _stream())
 
 
@@ -831,7 +853,7 @@ def linear_tc_glu(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> N
         raise KernelError("linear_tc_glu: shapes, strides or operands not supported")
     lda = a.stride(0) if m > 1 else max(k, a.stride(0))
     ldo = out.stride(0) if m > 1 else max(n, out.stride(0))
-    _call(_fn_tc("erb_linear_tc_glu"), a.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k, lda, k, ldo,
+    _call(_fn_tc("erb_linear_tc_glu"), a, weight, out, m, n, k, lda, k, ldo,
           _stream())
 
 
@@ -852,9 +874,9 @@ def linear_tc_rope_store(a: torch.Tensor, weight: torch.Tensor, qkv: torch.Tenso
         raise KernelError("linear_tc_rope_store: shapes, strides or operands not supported")
     lda = a.stride(0) if m > 1 else max(k, a.stride(0))
     ldo = qkv.stride(0) if m > 1 else max(width, qkv.stride(0))
-    _call(_fn_tc("erb_linear_tc_rope"), a.data_ptr(), weight.data_ptr(), qkv.data_ptr(), m, k, lda, k, ldo,
-          n_q_heads, n_kv_heads, head_dim, positions.data_ptr(), inv_freq.data_ptr(), slots.data_ptr(),
-          k_pages.data_ptr(), v_pages.data_ptr(), page_size, _stream())
+    _call(_fn_tc("erb_linear_tc_rope"), a, weight, qkv, m, k, lda, k, ldo,
+          n_q_heads, n_kv_heads, head_dim, positions, inv_freq, slots,
+          k_pages, v_pages, page_size, _stream())
 
 
 def linear_glu_supported(a: torch.Tensor, weight: torch.Tensor, max_rows: int = SKINNY_MAX_ROWS) -> bool:
@@ -884,10 +906,10 @@ def linear_glu(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, bounded
     if bounded is not None:
         limit, alpha, shift = bounded[:3]
         act = bounded[3] if len(bounded) > 3 else "sigmoid"
-        _call(_fn("gemm", "bfloat16", "erb_linear_skinny_glu_bounded"), a.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k,
-              lda, k, ldo, float(limit), float(alpha), float(shift), GLU_ACTS[act], _ptr(row_scale), _stream())
+        _call(_fn("gemm", "bfloat16", "erb_linear_skinny_glu_bounded"), a, weight, out, m, n, k,
+              lda, k, ldo, float(limit), float(alpha), float(shift), GLU_ACTS[act], row_scale, _stream())
         return
-    _call(_fn("gemm", "bfloat16", "erb_linear_skinny_glu"), a.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k,
+    _call(_fn("gemm", "bfloat16", "erb_linear_skinny_glu"), a, weight, out, m, n, k,
           lda, k, ldo, _stream())
 
 
@@ -919,9 +941,9 @@ def linear_rope_store(a: torch.Tensor, weight: torch.Tensor, qkv: torch.Tensor, 
         raise KernelError("linear_rope_store: shapes, strides or operands not supported")
     lda = a.stride(0) if m > 1 else max(k, a.stride(0))
     ldo = qkv.stride(0) if m > 1 else max(width, qkv.stride(0))
-    _call(_fn("gemm", "bfloat16", "erb_linear_skinny_rope"), a.data_ptr(), weight.data_ptr(), qkv.data_ptr(), m, k,
-          lda, k, ldo, n_q_heads, n_kv_heads, head_dim, positions.data_ptr(), inv_freq.data_ptr(), slots.data_ptr(),
-          k_pages.data_ptr(), v_pages.data_ptr(), page_size, _stream())
+    _call(_fn("gemm", "bfloat16", "erb_linear_skinny_rope"), a, weight, qkv, m, k,
+          lda, k, ldo, n_q_heads, n_kv_heads, head_dim, positions, inv_freq, slots,
+          k_pages, v_pages, page_size, _stream())
 
 
 LINEAR_TUNE_FROM_ROWS = 1024     # rows from which the library's proposals for a shape are timed (as in csrc/gemm.cu)
@@ -967,16 +989,16 @@ def linear(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, accumulate:
     if m <= TC_MAX_ROWS and not accumulate and not library and linear_few_rows_supported(a, weight, lda):
         if m <= SKINNY_MAX_ROWS:
             # a handful of rows: this package's weight-streaming kernel instead of the library product
-            _call(_fn("gemm", "bfloat16", "erb_linear_skinny"), a.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k,
+            _call(_fn("gemm", "bfloat16", "erb_linear_skinny"), a, weight, out, m, n, k,
                   lda, k, ldo, int(out.dtype == torch.float32), _stream())
             return
         if n >= 128 * 2 * _sms(a.device):
-            _call(_fn_tc("erb_linear_tc"), a.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k,
+            _call(_fn_tc("erb_linear_tc"), a, weight, out, m, n, k,
                   lda, k, ldo, int(out.dtype == torch.float32), _stream())
             return
     ws = _workspace(a.device)
-    _call(_fn("gemm", _elem(a), "erb_linear"), a.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k,
-          lda, k, ldo, int(out.dtype == torch.float32), int(accumulate), ws.data_ptr(), ws.numel(), _stream())
+    _call(_fn("gemm", _elem(a), "erb_linear"), a, weight, out, m, n, k,
+          lda, k, ldo, int(out.dtype == torch.float32), int(accumulate), ws, ws.numel(), _stream())
 
 
 def linear_batched(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
@@ -996,8 +1018,8 @@ def linear_batched(a: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> 
     lda = a.stride(0) if m > 1 else max(k, a.stride(0))
     ldo = out.stride(0) if m > 1 else max(n, out.stride(0))
     ws = _workspace(a.device)
-    _call(_fn("gemm", _elem(a), "erb_linear_batched"), a.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k, lda, k, ldo,
-          int(out.dtype == torch.float32), b, a.stride(1), n * k, out.stride(1), ws.data_ptr(), ws.numel(), _stream())
+    _call(_fn("gemm", _elem(a), "erb_linear_batched"), a, weight, out, m, n, k, lda, k, ldo,
+          int(out.dtype == torch.float32), b, a.stride(1), n * k, out.stride(1), ws, ws.numel(), _stream())
 
 
 # --- attention through a latent ----------------------------------------------------------------
@@ -1027,9 +1049,9 @@ def latent_store(proj: torch.Tensor, positions: torch.Tensor, eps: float, *, off
     if q_rank and (q_weight is None or q_latent is None or q_weight.numel() != q_rank or off_q + q_rank > proj.shape[1]
                    or q_latent.shape != (n, q_rank)):
         raise KernelError("latent_store: the query latent lies outside the row or its target has another shape")
-    _call(_fn("latent_attention", _elem(proj), "erb_latent_store"), proj.data_ptr(), n, proj.stride(0) if n > 1 else proj.shape[1],
-          int(off_kv), int(rank), int(rot_dim), _ptr(kv_weight), float(eps), positions.data_ptr(), _ptr(inv_freq), int(rot_dims),
-          float(rot_mult), _ptr(slots), _ptr(pages), int(off_q), int(q_rank), _ptr(q_weight), _ptr(q_latent), _stream())
+    _call(_fn("latent_attention", _elem(proj), "erb_latent_store"), proj, n, proj.stride(0) if n > 1 else proj.shape[1],
+          int(off_kv), int(rank), int(rot_dim), kv_weight, float(eps), positions, inv_freq, int(rot_dims),
+          float(rot_mult), slots, pages, int(off_q), int(q_rank), q_weight, q_latent, _stream())
 
 
 def latent_q_rotate(q: torch.Tensor, positions: torch.Tensor, inv_freq: torch.Tensor | None, n_heads: int, dim: int,
@@ -1042,9 +1064,9 @@ def latent_q_rotate(q: torch.Tensor, positions: torch.Tensor, inv_freq: torch.Te
     n = q.shape[0]
     if q.stride(1) != 1 or q.shape[1] < n_heads * (dim + rot_dim) or q_lat.shape != (n, n_heads, rank + rot_dim):
         raise KernelError("latent_q_rotate: shapes disagree")
-    _call(_fn("latent_attention", _elem(q), "erb_latent_q_rotate"), q.data_ptr(), n, q.stride(0) if n > 1 else q.shape[1],
-          n_heads, dim, rot_dim, rank, positions.data_ptr(), _ptr(inv_freq), int(rot_dims),
-          float(rot_mult), q_lat.data_ptr(), _stream())
+    _call(_fn("latent_attention", _elem(q), "erb_latent_q_rotate"), q, n, q.stride(0) if n > 1 else q.shape[1],
+          n_heads, dim, rot_dim, rank, positions, inv_freq, int(rot_dims),
+          float(rot_mult), q_lat, _stream())
 
 
 def latent_scratch_floats(n_tokens: int, n_heads: int, rank: int, n_splits: int) -> int:
@@ -1080,9 +1102,9 @@ def latent_attention(q_lat: torch.Tensor, pages: torch.Tensor, block_tables: tor
         raise KernelError("latent_attention: the scratch for the splits is too small")
     fn = _fn("latent_attention", _elem(pages), "erb_latent_attention")
     fn._erb_own = 2 if n_splits > 1 else 1
-    _call(fn, q_lat.data_ptr(), pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1], seq_of_token.data_ptr(),
-          positions.data_ptr(), _ptr(gate), 0 if gate is None else (gate.stride(0) if n > 1 else heads), _ptr(sink),
-          out.data_ptr(), _ptr(part), int(first_token), int(n_tokens), heads, rank, dk - rank, page_size, int(split_keys),
+    _call(fn, q_lat, pages, block_tables, block_tables.shape[1], seq_of_token,
+          positions, gate, 0 if gate is None else (gate.stride(0) if n > 1 else heads), sink,
+          out, part, int(first_token), int(n_tokens), heads, rank, dk - rank, page_size, int(split_keys),
           int(n_splits), float(scale), int(window), _stream())
 
 
@@ -1135,13 +1157,13 @@ def latent_attention_mma(q_lat: torch.Tensor, pages: torch.Tensor, block_tables:
                          part.numel() < latent_scratch_floats(n_tokens, heads, rank, n_splits)):
         raise KernelError("latent_attention_mma: splits need scratch and a split size that is a multiple of the key tile")
     gate_ld = 0 if gate is None else (gate.stride(0) if n > 1 else heads)
-    _call(_fn("latent_attention", "bfloat16", "erb_latent_attention_mma"), q_lat.data_ptr(), pages.data_ptr(),
-          block_tables.data_ptr(), block_tables.shape[1], seq_starts.data_ptr(), positions.data_ptr(), _ptr(gate), gate_ld,
-          _ptr(sink), out.data_ptr(), _ptr(part), int(first_token), int(first_seq), int(n_seqs), int(n_tiles), int(row_tiles),
+    _call(_fn("latent_attention", "bfloat16", "erb_latent_attention_mma"), q_lat, pages,
+          block_tables, block_tables.shape[1], seq_starts, positions, gate, gate_ld,
+          sink, out, part, int(first_token), int(first_seq), int(n_seqs), int(n_tiles), int(row_tiles),
           heads, rank, dk - rank, pages.shape[2], int(split_keys), int(n_splits), float(scale), int(window), _stream())
     if n_splits > 1:
-        _call(_fn("latent_attention", "bfloat16", "erb_latent_combine"), part.data_ptr(), _ptr(gate), gate_ld, _ptr(sink),
-              out.data_ptr(), int(first_token), int(n_tokens), heads, rank, int(n_splits), _stream())
+        _call(_fn("latent_attention", "bfloat16", "erb_latent_combine"), part, gate, gate_ld, sink,
+              out, int(first_token), int(n_tokens), heads, rank, int(n_splits), _stream())
 
 
 LATENT_WIDE_ROWS = 256     # tokens of one head that a block of the kernel over up-projected rows takes
@@ -1167,8 +1189,8 @@ def latent_gather(pages: torch.Tensor, block_tables: torch.Tensor, seq_starts: t
     n_seqs, width = seq_starts.numel() - 1, pages.shape[3]
     if pages.shape[1] != 1 or n_seqs < 1 or block_tables.shape[0] < n_seqs or out.shape != (n_seqs * kv_rows, width):
         raise KernelError("latent_gather: pages, tables and out disagree")
-    _call(_fn("attention_wide", None, "erb_latent_gather"), pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
-          seq_starts.data_ptr(), positions.data_ptr(), n_seqs, int(kv_rows), width, pages.shape[2], int(window), out.data_ptr(), _stream())
+    _call(_fn("attention_wide", None, "erb_latent_gather"), pages, block_tables, block_tables.shape[1],
+          seq_starts, positions, n_seqs, int(kv_rows), width, pages.shape[2], int(window), out, _stream())
 
 
 def latent_q_rows(q: torch.Tensor, positions: torch.Tensor, inv_freq: torch.Tensor | None, n_heads: int, dim: int, rot_dim: int,
@@ -1180,8 +1202,8 @@ def latent_q_rows(q: torch.Tensor, positions: torch.Tensor, inv_freq: torch.Tens
     n = q.shape[0]
     if q.shape[1] != n_heads * (dim + rot_dim) or q.stride(1) != 1 or out.shape != (n, n_heads, 64) or positions.numel() < n:
         raise KernelError("latent_q_rows: shapes disagree")
-    _call(_fn("attention_wide", None, "erb_latent_q_rows"), q.data_ptr(), n, q.stride(0) if n > 1 else q.shape[1], int(n_heads), int(dim),
-          int(rot_dim), positions.data_ptr(), _ptr(inv_freq), int(rot_dims), float(rot_mult), out.data_ptr(), _stream())
+    _call(_fn("attention_wide", None, "erb_latent_q_rows"), q, n, q.stride(0) if n > 1 else q.shape[1], int(n_heads), int(dim),
+          int(rot_dim), positions, inv_freq, int(rot_dims), float(rot_mult), out, _stream())
 
 
 def latent_attention_wide(q: torch.Tensor, q_rot: torch.Tensor, kv: torch.Tensor, latents: torch.Tensor, seq_starts: torch.Tensor,
@@ -1205,10 +1227,10 @@ def latent_attention_wide(q: torch.Tensor, q_rot: torch.Tensor, kv: torch.Tensor
         raise KernelError("latent_attention_wide: q, kv, latents and out disagree, or the sizes are not supported")
     if (gate is not None and (gate.shape != (n, heads) or gate.stride(1) != 1)) or (sink is not None and sink.numel() != heads):
         raise KernelError("latent_attention_wide: gate must be [tokens, heads] with unit inner stride, one sink per head")
-    _call(_fn("attention_wide", None, "erb_attention_wide_rows"), q.data_ptr(), q.stride(0) if n > 1 else q.shape[1], q_rot.data_ptr(),
-          kv.data_ptr(), latents.data_ptr(), seq_starts.data_ptr(), positions.data_ptr(), out.data_ptr(), n_seqs, int(kv_rows), int(n_blocks),
-          heads, int(dim), int(rot_dim), v_dim, rank, int(window), float(scale), _ptr(sink), _ptr(gate),
-          0 if gate is None else (gate.stride(0) if n > 1 else heads), status.data_ptr(), _stream())
+    _call(_fn("attention_wide", None, "erb_attention_wide_rows"), q, q.stride(0) if n > 1 else q.shape[1], q_rot,
+          kv, latents, seq_starts, positions, out, n_seqs, int(kv_rows), int(n_blocks),
+          heads, int(dim), int(rot_dim), v_dim, rank, int(window), float(scale), sink, gate,
+          0 if gate is None else (gate.stride(0) if n > 1 else heads), status, _stream())
 
 
 # --- differential attention ----------------------------------------------------------------------
@@ -1255,10 +1277,10 @@ def diff_prepare(proj: torch.Tensor, q_out: torch.Tensor, positions: torch.Tenso
         if k_pages is None or v_pages is None or tuple(k_pages.shape[1:]) != (n_kv_heads, page_size, 2 * dim) or \
                 tuple(v_pages.shape[1:]) != (n_kv_heads, page_size, v_dim) or slots.numel() < n:
             raise KernelError("diff_prepare: pages must be [pages, kv heads, page_size, 2 dim] and [..., v_dim]")
-    _call(_fn("diff_attention", _elem(proj), "erb_diff_prepare"), proj.data_ptr(), n, proj.stride(0) if n > 1 else proj.shape[1],
-          _ptr(conv_w), int(taps), _ptr(conv_state), _ptr(seq_of_token), _ptr(seq_starts), _ptr(state_slots), positions.data_ptr(),
-          _ptr(inv_freq), int(rot_dims), int(n_heads), int(n_kv_heads), int(dim), int(v_dim), q_out.data_ptr(), _ptr(slots),
-          _ptr(k_pages), _ptr(v_pages), int(page_size), _stream())
+    _call(_fn("diff_attention", _elem(proj), "erb_diff_prepare"), proj, n, proj.stride(0) if n > 1 else proj.shape[1],
+          conv_w, int(taps), conv_state, seq_of_token, seq_starts, state_slots, positions,
+          inv_freq, int(rot_dims), int(n_heads), int(n_kv_heads), int(dim), int(v_dim), q_out, slots,
+          k_pages, v_pages, int(page_size), _stream())
 
 
 def diff_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, block_tables: torch.Tensor,
@@ -1287,8 +1309,8 @@ def diff_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor
         raise KernelError("diff_attention: the scratch for the splits is too small")
     fn = _fn("diff_attention", _elem(q), "erb_diff_attention")
     fn._erb_own = 2 if n_splits > 1 else 1
-    _call(fn, q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
-          seq_of_token.data_ptr(), positions.data_ptr(), out.data_ptr(), _ptr(part), int(first_token), int(n_tokens), int(n_heads),
+    _call(fn, q, k_pages, v_pages, block_tables, block_tables.shape[1],
+          seq_of_token, positions, out, part, int(first_token), int(n_tokens), int(n_heads),
           int(n_kv), two_dim // 2, v_dim, page_size, int(window), int(split_keys), int(n_splits), float(scale), float(softcap),
           float(lam), float(eps), float(out_scale), _stream())
 
@@ -1339,8 +1361,8 @@ def diff_attention_mma(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Te
         raise KernelError("diff_attention_mma: the scratch for the splits is too small")
     fn = _fn("diff_attention", "bfloat16", "erb_diff_attention_mma")
     fn._erb_own = 2 if n_splits > 1 else 1
-    _call(fn, q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
-          seq_starts.data_ptr(), positions.data_ptr(), out.data_ptr(), _ptr(part), int(first_token), int(n_tokens), int(first_seq),
+    _call(fn, q, k_pages, v_pages, block_tables, block_tables.shape[1],
+          seq_starts, positions, out, part, int(first_token), int(n_tokens), int(first_seq),
           int(n_seqs), int(n_tiles), int(tile_rows), int(n_heads), int(n_kv), two_dim // 2, v_dim, page_size, int(window),
           int(split_keys), int(n_splits), float(scale), float(softcap), float(lam), float(eps), float(out_scale), _stream())
 
@@ -1369,10 +1391,10 @@ def diff_attention_wide(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.T
             out.shape != (n, n_heads * v_pages.shape[3]) or n_heads % n_kv or tuple(v_pages.shape[:3]) != (n_pages, n_kv, page_size) or \
             seq_starts.numel() < 2 or block_tables.shape[0] < seq_starts.numel() - 1 or positions.numel() < n:
         raise KernelError("diff_attention_wide: q, pages and out disagree, or the sizes are not supported")
-    _call(_fn("attention_wide", None, "erb_attention_wide_diff"), q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), n_pages,
-          block_tables.data_ptr(), block_tables.shape[1], seq_starts.data_ptr(), positions.data_ptr(), out.data_ptr(),
+    _call(_fn("attention_wide", None, "erb_attention_wide_diff"), q, k_pages, v_pages, n_pages,
+          block_tables, block_tables.shape[1], seq_starts, positions, out,
           seq_starts.numel() - 1, int(n_blocks), int(n_heads), int(n_kv), page_size, int(window), float(scale), float(softcap), float(lam),
-          float(eps), float(out_scale), status.data_ptr(), _stream())
+          float(eps), float(out_scale), status, _stream())
 
 
 # --- state-space mixer -------------------------------------------------------------------------
@@ -1391,9 +1413,9 @@ def conv_silu(proj: torch.Tensor, off: int, weight: torch.Tensor, bias: torch.Te
     if proj.stride(1) != 1 or off + channels > proj.shape[1] or out.shape != (n, channels) or \
             tuple(conv_state.shape[1:]) != (taps - 1, channels):
         raise KernelError("conv_silu: shapes disagree")
-    _call(_fn("ssm", _elem(proj), "erb_conv_silu"), proj.data_ptr(), n, proj.stride(0) if n > 1 else proj.shape[1], int(off),
-          channels, taps, weight.data_ptr(), _ptr(bias), conv_state.data_ptr(), seq_of_token.data_ptr(), seq_starts.data_ptr(),
-          state_slots.data_ptr(), out.data_ptr(), _stream())
+    _call(_fn("ssm", _elem(proj), "erb_conv_silu"), proj, n, proj.stride(0) if n > 1 else proj.shape[1], int(off),
+          channels, taps, weight, bias, conv_state, seq_of_token, seq_starts,
+          state_slots, out, _stream())
 
 
 def qkv_conv(proj: torch.Tensor, q_out: torch.Tensor, n_q_heads: int, n_kv_heads: int, head_dim: int, *, taps: int,
@@ -1422,9 +1444,9 @@ def qkv_conv(proj: torch.Tensor, q_out: torch.Tensor, n_q_heads: int, n_kv_heads
         raise KernelError("qkv_conv: pages or slots disagree with the heads")
     fn = _fn("ssm", _elem(proj), "erb_qkv_conv")
     fn._erb_own = 2 if taps > 1 and n_seqs > first_portion else 1
-    _call(fn, proj.data_ptr(), proj.stride(0) if n > 1 else proj.shape[1], _ptr(bias), _ptr(weight), int(taps),
-          _ptr(conv_state) if taps > 1 else None, seq_of_token.data_ptr(), seq_starts.data_ptr(), state_slots.data_ptr(), _ptr(slots),
-          q_out.data_ptr(), _ptr(k_pages), _ptr(v_pages), n, int(n_seqs), int(first_portion), n_q_heads, n_kv_heads, head_dim,
+    _call(fn, proj, proj.stride(0) if n > 1 else proj.shape[1], bias, weight, int(taps),
+          conv_state if taps > 1 else None, seq_of_token, seq_starts, state_slots, slots,
+          q_out, k_pages, v_pages, n, int(n_seqs), int(first_portion), n_q_heads, n_kv_heads, head_dim,
           int(page_size), _stream())
 
 
@@ -1437,8 +1459,8 @@ def conv_state_update(proj: torch.Tensor, off: int, conv_state: torch.Tensor, n_
     _, keep, channels = conv_state.shape
     if off + channels > proj.shape[1] or seq_starts.numel() < n_seqs + 1 or state_slots.numel() < n_seqs:
         raise KernelError("conv_state_update: shapes disagree")
-    _call(_fn("ssm", _elem(proj), "erb_conv_state_update"), proj.data_ptr(), int(n_seqs), proj.stride(0) if n > 1 else proj.shape[1],
-          int(off), channels, keep + 1, conv_state.data_ptr(), seq_starts.data_ptr(), state_slots.data_ptr(), _stream())
+    _call(_fn("ssm", _elem(proj), "erb_conv_state_update"), proj, int(n_seqs), proj.stride(0) if n > 1 else proj.shape[1],
+          int(off), channels, keep + 1, conv_state, seq_starts, state_slots, _stream())
 
 
 def ssm_scan(xbc: torch.Tensor, proj: torch.Tensor, off_dt: int, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
@@ -1459,11 +1481,11 @@ def ssm_scan(xbc: torch.Tensor, proj: torch.Tensor, off_dt: int, dt_bias: torch.
     if xbc.shape[1] != heads * p + 2 * n_groups * n_state or y.shape != (n, heads * p) or off_dt + heads > proj.shape[1] or \
             dt_bias.numel() != heads or a_log.numel() != heads or d_skip.numel() != heads or proj.shape[0] != n:
         raise KernelError("ssm_scan: shapes disagree")
-    _call(_fn("ssm", _elem(xbc), "erb_ssm_scan"), xbc.data_ptr(), xbc.shape[1], proj.data_ptr(),
-          proj.stride(0) if n > 1 else proj.shape[1], int(off_dt), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(),
-          state.data_ptr(), seq_starts.data_ptr(), state_slots.data_ptr(), y.data_ptr(), int(n_seqs), n,
+    _call(_fn("ssm", _elem(xbc), "erb_ssm_scan"), xbc, xbc.shape[1], proj,
+          proj.stride(0) if n > 1 else proj.shape[1], int(off_dt), dt_bias, a_log, d_skip,
+          state, seq_starts, state_slots, y, int(n_seqs), n,
           n - int(n_seqs) + 1 if longest is None else int(longest), heads, p, n_state,
-          int(n_groups), _ptr(_status_word), _stream())
+          int(n_groups), _status_word, _stream())
 
 
 def gated_group_norm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, eps: float, parts: int = 1,
@@ -1477,7 +1499,7 @@ def gated_group_norm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, e
             x.stride(1) != 1 or out.stride(1) != 1 or (gate is not None and (gate.shape != (n, width) or gate.stride(1) != 1)):
         raise KernelError("gated_group_norm: shapes or types disagree")
     ld = lambda t: t.stride(0) if n > 1 else width   # noqa: E731
-    _call(_fn("ssm", _elem(out), "erb_gated_group_norm"), x.data_ptr(), int(x.dtype == torch.float32), ld(x), _ptr(gate), 0 if gate is None else ld(gate), weight.data_ptr(), out.data_ptr(), ld(out), n, width, int(parts),
+    _call(_fn("ssm", _elem(out), "erb_gated_group_norm"), x, int(x.dtype == torch.float32), ld(x), gate, 0 if gate is None else ld(gate), weight, out, ld(out), n, width, int(parts),
           float(eps), _stream())
 
 
@@ -1531,9 +1553,9 @@ def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt
     _need(scratch, "scratch", torch.float32)
     if scratch.numel() < need:
         raise KernelError("delta_scan: the scratch is too small")
-    _call(_fn("delta", _elem(qkv), "erb_delta_scan"), qkv.data_ptr(), qkv.shape[1], proj.data_ptr(),
-          proj.stride(0) if n > 1 else proj.shape[1], int(off_b), int(off_a), dt_bias.data_ptr(), a_log.data_ptr(),
-          state.data_ptr(), seq_starts.data_ptr(), state_slots.data_ptr(), out.data_ptr(), scratch.data_ptr(), scratch.numel(), int(n_seqs), n,
+    _call(_fn("delta", _elem(qkv), "erb_delta_scan"), qkv, qkv.shape[1], proj,
+          proj.stride(0) if n > 1 else proj.shape[1], int(off_b), int(off_a), dt_bias, a_log,
+          state, seq_starts, state_slots, out, scratch, scratch.numel(), int(n_seqs), n,
           n - int(n_seqs) + 1 if longest is None else int(longest), heads, int(n_key_heads), d, vdim, _stream())
 
 
@@ -1547,8 +1569,8 @@ def head_norm_gate(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, ou
     if width % n_heads or weight.numel() != width // n_heads or out.shape != (n, width) or gate.shape != (n, width) or \
             gate.stride(1) != 1:
         raise KernelError("head_norm_gate: shapes disagree")
-    _call(_fn("delta", _elem(out), "erb_head_norm_gate"), o.data_ptr(), gate.data_ptr(), gate.stride(0) if n > 1 else width,
-          weight.data_ptr(), out.data_ptr(), n, int(n_heads), width // n_heads, float(eps), _stream())
+    _call(_fn("delta", _elem(out), "erb_head_norm_gate"), o, gate, gate.stride(0) if n > 1 else width,
+          weight, out, n, int(n_heads), width // n_heads, float(eps), _stream())
 
 
 # --- routed experts ------------------------------------------------------------------------------
@@ -1619,11 +1641,11 @@ def moe_route(x: torch.Tensor, w_router: torch.Tensor, top: int, lists: torch.Te
     if w_router.shape[1] != width or x.stride(1) != 1 or score.numel() < n * top:
         raise KernelError("moe_route: shapes disagree")
     choice, order, counts, offsets, tiles = _moe_lists(lists, n, n_experts, top)
-    _call(_fn("moe", _elem(x), "erb_moe_route"), x.data_ptr(), x.stride(0) if n > 1 else width, w_router.data_ptr(), n, width,
-          n_experts, int(top), choice.data_ptr(), score.data_ptr(), counts.data_ptr(), offsets.data_ptr(), tiles.data_ptr(),
-          order.data_ptr(), int(tile_rows), MOE_SCORES[scores], int(n_groups), int(keep), _ptr(correction),
-          MOE_GROUP_SCORES[group_score], int(bool(normalise)), float(weight), _ptr(side_gate),
-          _ptr(logits), _stream())
+    _call(_fn("moe", _elem(x), "erb_moe_route"), x, x.stride(0) if n > 1 else width, w_router, n, width,
+          n_experts, int(top), choice, score, counts, offsets, tiles,
+          order, int(tile_rows), MOE_SCORES[scores], int(n_groups), int(keep), correction,
+          MOE_GROUP_SCORES[group_score], int(bool(normalise)), float(weight), side_gate,
+          logits, _stream())
 
 
 def moe_tc_supported(dtype: torch.dtype, width: int, ff: int) -> bool:
@@ -1653,8 +1675,8 @@ def moe_tc_gather(x: torch.Tensor, lists: torch.Tensor, score: torch.Tensor | No
     if xs.shape != (n * top, width) or x.stride(1) != 1:
         raise KernelError("moe_tc_gather: shapes disagree")
     _, order, _, _, _ = _moe_lists(lists, n, n_experts, top)
-    _call(_fn("moe_tc", None, "erb_moe_tc_gather"), x.data_ptr(), x.stride(0) if n > 1 else width, order.data_ptr(), _ptr(score),
-          int(top), n, width, xs.data_ptr(), _stream())
+    _call(_fn("moe_tc", None, "erb_moe_tc_gather"), x, x.stride(0) if n > 1 else width, order, score,
+          int(top), n, width, xs, _stream())
 
 
 def moe_tc_gate_up(xs: torch.Tensor, w_gate_up: torch.Tensor, lists: torch.Tensor, top: int, tile_rows: int, act: torch.Tensor) -> None:
@@ -1666,8 +1688,8 @@ def moe_tc_gate_up(xs: torch.Tensor, w_gate_up: torch.Tensor, lists: torch.Tenso
     if k != width or two_ff % 2 or pairs % top or act.shape != (pairs, two_ff // 2):
         raise KernelError("moe_tc_gate_up: shapes disagree")
     _, order, _, offsets, tiles = _moe_lists(lists, pairs // top, n_experts, top)
-    _call(_fn("moe_tc", None, "erb_moe_tc_gate_up"), xs.data_ptr(), w_gate_up.data_ptr(), offsets.data_ptr(), tiles.data_ptr(),
-          order.data_ptr(), n_experts, int(top), pairs // top, two_ff // 2, width, int(tile_rows), act.data_ptr(), _ptr(_status_word),
+    _call(_fn("moe_tc", None, "erb_moe_tc_gate_up"), xs, w_gate_up, offsets, tiles,
+          order, n_experts, int(top), pairs // top, two_ff // 2, width, int(tile_rows), act, _status_word,
           _stream())
 
 
@@ -1679,8 +1701,8 @@ def moe_tc_up_act(xs: torch.Tensor, w_up: torch.Tensor, lists: torch.Tensor, top
     if k != width or pairs % top or act.shape != (pairs, ff):
         raise KernelError("moe_tc_up_act: shapes disagree")
     _, order, _, offsets, tiles = _moe_lists(lists, pairs // top, n_experts, top)
-    _call(_fn("moe_tc", None, "erb_moe_tc_up_act"), xs.data_ptr(), w_up.data_ptr(), offsets.data_ptr(), tiles.data_ptr(),
-          order.data_ptr(), n_experts, int(top), pairs // top, ff, width, int(tile_rows), act.data_ptr(), _ptr(_status_word),
+    _call(_fn("moe_tc", None, "erb_moe_tc_up_act"), xs, w_up, offsets, tiles,
+          order, n_experts, int(top), pairs // top, ff, width, int(tile_rows), act, _status_word,
           _stream())
 
 
@@ -1694,8 +1716,8 @@ def moe_tc_down(act: torch.Tensor, w_down: torch.Tensor, lists: torch.Tensor, to
     if act.shape != (n * top, ff) or parts.dim() != 3 or parts.shape[0] < top or parts.shape[1:] != (n, width):
         raise KernelError("moe_tc_down: shapes disagree")
     _, order, _, offsets, tiles = _moe_lists(lists, n, n_experts, top)
-    _call(_fn("moe_tc", None, "erb_moe_tc_down"), act.data_ptr(), w_down.data_ptr(), offsets.data_ptr(), tiles.data_ptr(),
-          order.data_ptr(), n_experts, int(top), n, width, ff, int(tile_rows), parts.data_ptr(), _ptr(out_score), _ptr(_status_word),
+    _call(_fn("moe_tc", None, "erb_moe_tc_down"), act, w_down, offsets, tiles,
+          order, n_experts, int(top), n, width, ff, int(tile_rows), parts, out_score, _status_word,
           _stream())
 
 
@@ -1709,9 +1731,9 @@ def moe_gate_up(x: torch.Tensor, w_gate_up: torch.Tensor, lists: torch.Tensor, s
     if k != width or two_ff % 2 or act.shape != (n * top, two_ff // 2) or x.stride(1) != 1:
         raise KernelError("moe_gate_up: shapes disagree")
     _, order, _, offsets, tiles = _moe_lists(lists, n, n_experts, top)
-    _call(_fn("moe", _elem(x), "erb_moe_product"), x.data_ptr(), x.stride(0) if n > 1 else width, w_gate_up.data_ptr(),
-          offsets.data_ptr(), tiles.data_ptr(), order.data_ptr(), _ptr(score), n_experts, int(top), n, two_ff // 2, width,
-          1, act.data_ptr(), None, _stream())
+    _call(_fn("moe", _elem(x), "erb_moe_product"), x, x.stride(0) if n > 1 else width, w_gate_up,
+          offsets, tiles, order, score, n_experts, int(top), n, two_ff // 2, width,
+          1, act, None, _stream())
 
 
 def moe_up_act(x: torch.Tensor, w_up: torch.Tensor, lists: torch.Tensor, top: int, act: torch.Tensor) -> None:
@@ -1723,9 +1745,9 @@ def moe_up_act(x: torch.Tensor, w_up: torch.Tensor, lists: torch.Tensor, top: in
     if k != width or act.shape != (n * top, ff) or x.stride(1) != 1:
         raise KernelError("moe_up_act: shapes disagree")
     _, order, _, offsets, tiles = _moe_lists(lists, n, n_experts, top)
-    _call(_fn("moe", _elem(x), "erb_moe_product"), x.data_ptr(), x.stride(0) if n > 1 else width, w_up.data_ptr(),
-          offsets.data_ptr(), tiles.data_ptr(), order.data_ptr(), None, n_experts, int(top), n, ff, width,
-          2, act.data_ptr(), None, _stream())
+    _call(_fn("moe", _elem(x), "erb_moe_product"), x, x.stride(0) if n > 1 else width, w_up,
+          offsets, tiles, order, None, n_experts, int(top), n, ff, width,
+          2, act, None, _stream())
 
 
 def moe_down(act: torch.Tensor, w_down: torch.Tensor, lists: torch.Tensor, top: int, parts: torch.Tensor,
@@ -1739,8 +1761,8 @@ def moe_down(act: torch.Tensor, w_down: torch.Tensor, lists: torch.Tensor, top: 
     if act.shape != (n * top, ff) or parts.dim() != 3 or parts.shape[0] < top or parts.shape[1:] != (n, width):
         raise KernelError("moe_down: shapes disagree")
     _, order, _, offsets, tiles = _moe_lists(lists, n, n_experts, top)
-    _call(_fn("moe", _elem(act), "erb_moe_product"), act.data_ptr(), ff, w_down.data_ptr(), offsets.data_ptr(),
-          tiles.data_ptr(), order.data_ptr(), _ptr(out_score), n_experts, int(top), n, width, ff, 0, None, parts.data_ptr(), _stream())
+    _call(_fn("moe", _elem(act), "erb_moe_product"), act, ff, w_down, offsets,
+          tiles, order, out_score, n_experts, int(top), n, width, ff, 0, None, parts, _stream())
 
 
 # --- attention -------------------------------------------------------------------------------
@@ -1800,9 +1822,9 @@ def attention_rows(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor
     _, nkv, page_size, d = k_pages.shape
     if q.stride(1) != 1 or out.stride(1) != 1 or q.shape[1] < n_q_heads * d or out.shape[1] < n_q_heads * d:
         raise KernelError("attention_rows: q/out layout disagrees with the head counts")
-    _call(_fn("attention", _elem(q), "erb_attention_rows"), q.data_ptr(), q.stride(0), k_pages.data_ptr(),
-          v_pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1], seq_of_token.data_ptr(),
-          positions.data_ptr(), out.data_ptr(), out.stride(0), n, n_q_heads, nkv, d, page_size, mask_reach(window, chunk),
+    _call(_fn("attention", _elem(q), "erb_attention_rows"), q, q.stride(0), k_pages,
+          v_pages, block_tables, block_tables.shape[1], seq_of_token,
+          positions, out, out.stride(0), n, n_q_heads, nkv, d, page_size, mask_reach(window, chunk),
           int(keep_first), float(scale), _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d),
           int(tiled), _stream())
 
@@ -1990,9 +2012,9 @@ def attention_decode(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
         raise KernelError("attention_decode: scratch too small")
     if q.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("attention_decode: q/out inner stride must be 1")
-    _call(_fn("attention", _elem(q), "erb_attention_decode"), q.data_ptr(), q.stride(0), k_pages.data_ptr(),
-          v_pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1], token_of_seq.data_ptr(),
-          positions.data_ptr(), out.data_ptr(), out.stride(0), part_acc.data_ptr(), part_ml.data_ptr(),
+    _call(_fn("attention", _elem(q), "erb_attention_decode"), q, q.stride(0), k_pages,
+          v_pages, block_tables, block_tables.shape[1], token_of_seq,
+          positions, out, out.stride(0), part_acc, part_ml,
           max_splits, n_seqs, n_q_heads, nkv, d, page_size, mask_reach(window, chunk), int(keep_first), int(split_keys),
           float(scale), _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d), _stream())
 
@@ -2053,11 +2075,11 @@ def attention_decode_bulk(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch
         raise KernelError("attention_decode_bulk: scratch too small")
     if q.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("attention_decode_bulk: q/out inner stride must be 1")
-    _call(_fn("attention_tc", None, "erb_attention_decode_bulk"), q.data_ptr(), q.stride(0), k_pages.data_ptr(),
-          v_pages.data_ptr(), n_pages, block_tables.data_ptr(), block_tables.shape[1], token_of_seq.data_ptr(),
-          positions.data_ptr(), out.data_ptr(), out.stride(0), part_acc.data_ptr(), part_ml.data_ptr(), max_splits,
-          n_seqs, n_q_heads, nkv, d, page_size, int(split_keys), float(scale), status.data_ptr(),
-          split_counters(q.device, n_seqs * nkv).data_ptr(), int(head_group), mask_reach(window, chunk), int(keep_first),
+    _call(_fn("attention_tc", None, "erb_attention_decode_bulk"), q, q.stride(0), k_pages,
+          v_pages, n_pages, block_tables, block_tables.shape[1], token_of_seq,
+          positions, out, out.stride(0), part_acc, part_ml, max_splits,
+          n_seqs, n_q_heads, nkv, d, page_size, int(split_keys), float(scale), status,
+          split_counters(q.device, n_seqs * nkv), int(head_group), mask_reach(window, chunk), int(keep_first),
           _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d), int(bool(even)), _stream())
 
 
@@ -2093,11 +2115,11 @@ def attention_decode_gqa(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.
         raise KernelError("attention_decode_gqa: scratch too small or pools disagree")
     if q.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("attention_decode_gqa: q/out inner stride must be 1")
-    _call(_fn("attention_tc", None, "erb_attention_decode_gqa"), q.data_ptr(), q.stride(0), k_pages.data_ptr(),
-          v_pages.data_ptr(), n_pages, block_tables.data_ptr(), block_tables.shape[1], token_of_seq.data_ptr(),
-          positions.data_ptr(), out.data_ptr(), out.stride(0), part_acc.data_ptr(), part_ml.data_ptr(), max_splits,
-          n_seqs, n_q_heads, nkv, d, page_size, int(split_keys), float(scale), status.data_ptr(),
-          split_counters(q.device, n_seqs * nkv).data_ptr(), mask_reach(window, chunk), int(keep_first),
+    _call(_fn("attention_tc", None, "erb_attention_decode_gqa"), q, q.stride(0), k_pages,
+          v_pages, n_pages, block_tables, block_tables.shape[1], token_of_seq,
+          positions, out, out.stride(0), part_acc, part_ml, max_splits,
+          n_seqs, n_q_heads, nkv, d, page_size, int(split_keys), float(scale), status,
+          split_counters(q.device, n_seqs * nkv), mask_reach(window, chunk), int(keep_first),
           _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d), int(bool(even)), _stream())
 
 
@@ -2166,10 +2188,10 @@ def attention_prefill_tc(qkv: torch.Tensor, k_pages: torch.Tensor, v_pages: torc
         need_o, need_ml = prefill_tc_scratch_floats(qkv.shape[0], n_q_heads, key_splits)
         if part_o is None or part_ml is None or part_o.numel() < need_o or part_ml.numel() < need_ml or not 0 <= first_row < qkv.shape[0]:
             raise KernelError("attention_prefill_tc: scratch for the key ranges is missing or too small")
-    _call(_fn("attention_prefill", None, "erb_attention_prefill_tc"), qkv.data_ptr(), qkv.stride(0), k_pages.data_ptr(),
-          v_pages.data_ptr(), n_pages, block_tables.data_ptr(), block_tables.shape[1], seq_starts.data_ptr(),
-          positions.data_ptr(), out.data_ptr(), out.stride(0), n_seqs, int(n_blocks), n_q_heads, nkv, d, page_size,
-          float(scale), status.data_ptr(), int(key_splits), int(first_row), qkv.shape[0] - int(first_row), _ptr(part_o), _ptr(part_ml),
+    _call(_fn("attention_prefill", None, "erb_attention_prefill_tc"), qkv, qkv.stride(0), k_pages,
+          v_pages, n_pages, block_tables, block_tables.shape[1], seq_starts,
+          positions, out, out.stride(0), n_seqs, int(n_blocks), n_q_heads, nkv, d, page_size,
+          float(scale), status, int(key_splits), int(first_row), qkv.shape[0] - int(first_row), part_o, part_ml,
           mask_reach(window, chunk), int(keep_first), _penalty(penalty, n_q_heads), float(softcap),
           *_gate(gate, out, n_q_heads * d), _stream())
     if key_splits > 1:
@@ -2185,8 +2207,8 @@ def sample_rows(logits: torch.Tensor, tokens: torch.Tensor, temperature: torch.T
     _need(temperature, "temperature", torch.float32); _need(rng_state, "rng_state", torch.int64)
     if logits.stride(1) != 1 or tokens.numel() < logits.shape[0]:
         raise KernelError("sample_rows: layout disagrees")
-    _call(_fn("sampling", None, "erb_sample_rows"), logits.data_ptr(), logits.stride(0) if logits.shape[0] > 1 else max(logits.stride(0), logits.shape[1]),
-          logits.shape[0], logits.shape[1], _ptr(temperature), _ptr(rng_state), tokens.data_ptr(), _stream())
+    _call(_fn("sampling", None, "erb_sample_rows"), logits, logits.stride(0) if logits.shape[0] > 1 else max(logits.stride(0), logits.shape[1]),
+          logits.shape[0], logits.shape[1], temperature, rng_state, tokens, _stream())
 
 
 def uniform_from_state(state: int) -> float:

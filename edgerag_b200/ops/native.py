@@ -53,6 +53,9 @@ NVCC_FLAGS = (
 
 ELEM_CODES = {"float32": 0, "bfloat16": 1}
 
+#: the module through which Python calls the libraries' entry points (``csrc/launch.cpp``), compiled for the host
+HOST_SOURCE = CSRC / "launch.cpp"
+
 
 class NativeBuildError(RuntimeError):
     """A CUDA library of the engine is missing and could not be built."""
@@ -185,8 +188,69 @@ def load(library: str, elem: str | None = None) -> ctypes.CDLL:
     return lib
 
 
+def _host_command(out: Path) -> list[str]:
+    import sysconfig
+
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cxx = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
+    if not cxx or not (Path(sysconfig.get_paths()["include"]) / "Python.h").is_file():
+        raise NativeBuildError("no C++ compiler or no Python.h for the host module")
+    return [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            f"-I{root / 'include'}", f"-I{root / 'include/torch/csrc/api/include'}", f"-I{sysconfig.get_paths()['include']}", "-o", str(out),
+            str(HOST_SOURCE), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10"]
+
+
+def build_host(verbose: bool = True) -> Path:
+    """Compile the host module if its source, the Python or the torch it is built against changed; return its path."""
+    import sysconfig
+
+    import torch
+
+    name = "launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
+    h = hashlib.sha256(HOST_SOURCE.read_bytes())
+    h.update(f"{torch.__version__} {sys.version}".encode())
+    stamp = h.hexdigest()
+    ready = _find_prebuilt(name, stamp)
+    if ready is not None:
+        return ready
+    folder = _ext_dir()
+    lib = folder / name
+    with open(folder / (name + ".lock"), "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        try:
+            if _find_prebuilt(name, stamp) is None:
+                tmp = folder / f".{name}.{os.getpid()}.tmp.so"
+                if verbose:
+                    _say(f"compiling {name} for the host (first use) ...")
+                proc = subprocess.run(_host_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+                if proc.returncode != 0:
+                    tmp.unlink(missing_ok=True)
+                    raise NativeBuildError(f"the compiler failed for {name}:\n{proc.stdout}")
+                os.replace(tmp, lib)
+                (folder / (name + ".stamp")).write_text(stamp)
+            return lib
+        finally:
+            fcntl.flock(lock, fcntl.LOCK_UN)
+
+
+def load_host():
+    """The host module, or None (said once on stderr) where it cannot be built: calls then go through ctypes, slower."""
+    import importlib.util
+
+    try:
+        spec = importlib.util.spec_from_file_location("launch", build_host())
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module
+    except (NativeBuildError, ImportError, OSError) as exc:
+        _say(f"calls of kernels go through ctypes: {exc}")
+        return None
+
+
 def build_all(verbose: bool = True, jobs: int | None = None) -> list[Path]:
-    """Compile every library for both element types (the "does it build" check)."""
+    """Compile every library for both element types, and the host module (the "does it build" check)."""
     from concurrent.futures import ThreadPoolExecutor
 
     work = []
@@ -196,4 +260,5 @@ def build_all(verbose: bool = True, jobs: int | None = None) -> list[Path]:
         for elem in (ELEM_CODES if per_elem else (None,)):
             work.append((library, elem))
     with ThreadPoolExecutor(max_workers=jobs or min(8, os.cpu_count() or 2)) as pool:
-        return list(pool.map(lambda w: build(w[0], w[1], verbose), work))
+        host = pool.submit(build_host, verbose)
+        return [*pool.map(lambda w: build(w[0], w[1], verbose), work), host.result()]

@@ -309,19 +309,22 @@ class Attention(Mixer):
             need_acc, need_ml = kernels.decode_scratch_floats(nd, self.n_q, d, max_splits)
             part_acc = ctx.buf("attn.part_acc", (need_acc,), torch.float32)
             part_ml = ctx.buf("attn.part_ml", (need_ml,), torch.float32)
+            q_rows, out_rows, tokens = (qkv, out, ctx.token_of_seq) if nd == n else (qkv[:nd], out[:nd], ctx.token_of_seq)
+            if tokens.shape[0] != nd:
+                tokens = tokens[:nd]
             if may_group and kernels.decode_gqa_supported(self.dtype, d, self.window, self.n_q, self.n_kv, ctx.page_size, split, max_splits):
-                kernels.attention_decode_gqa(qkv[:nd], k_pages, v_pages, tables, ctx.token_of_seq[:nd], ctx.positions,
-                                             out[:nd], self.n_q, self.scale, part_acc, part_ml, max_splits, ctx.status,
+                kernels.attention_decode_gqa(q_rows, k_pages, v_pages, tables, tokens, ctx.positions,
+                                             out_rows, self.n_q, self.scale, part_acc, part_ml, max_splits, ctx.status,
                                              split_keys=split, window=self.window, keep_first=self.keep_first, chunk=self.chunk, gate=head_gate,
                                              even=even is not None, **score)
             elif kernels.decode_bulk_supported(self.dtype, d, self.window, self.n_q, self.n_kv, max_splits):
-                kernels.attention_decode_bulk(qkv[:nd], k_pages, v_pages, tables, ctx.token_of_seq[:nd], ctx.positions,
-                                              out[:nd], self.n_q, self.scale, part_acc, part_ml, max_splits, ctx.status,
+                kernels.attention_decode_bulk(q_rows, k_pages, v_pages, tables, tokens, ctx.positions,
+                                              out_rows, self.n_q, self.scale, part_acc, part_ml, max_splits, ctx.status,
                                               split_keys=split, head_group=heads_per_block, window=self.window,
                                               keep_first=self.keep_first, chunk=self.chunk, gate=head_gate, even=even is not None, **score)
             else:
-                kernels.attention_decode(qkv[:nd], k_pages, v_pages, tables, ctx.token_of_seq[:nd], ctx.positions,
-                                         out[:nd], self.n_q, self.scale, part_acc, part_ml, max_splits,
+                kernels.attention_decode(q_rows, k_pages, v_pages, tables, tokens, ctx.positions,
+                                         out_rows, self.n_q, self.scale, part_acc, part_ml, max_splits,
                                          window=self.window, split_keys=split, keep_first=self.keep_first, chunk=self.chunk,
                                          gate=head_gate, **score)
         if n > nd and kernels.prefill_tc_supported(self.dtype, d, self.window, ctx.page_size):

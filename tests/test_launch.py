@@ -1,0 +1,76 @@
+"""The module through which Python calls the kernels' entry points: what an entry point receives, what is refused, what is counted."""
+
+from __future__ import annotations
+
+import ctypes
+import itertools
+
+import pytest
+import torch
+
+from edgerag_b200.ops import kernels, native
+
+KINDS = {ctypes.c_void_p: "p", ctypes.c_int: "i", ctypes.c_longlong: "i", ctypes.c_float: "f"}
+
+
+@pytest.fixture()
+def host():
+    module = native.load_host()
+    assert module is not None
+    counts = {"own": 0, "library": 0}
+    module.bind(counts, kernels.KernelError, kernels._need_in_python)
+    yield module, counts
+    if kernels._host:
+        module = kernels._host
+    module.bind(kernels.launch_counts, kernels.KernelError, kernels._need_in_python)
+
+
+def _entry(host, types, result=0, own=1):
+    got = []
+    fn = ctypes.CFUNCTYPE(ctypes.c_int, *types)(lambda *a: got.append(a) or result)
+    error = ctypes.CFUNCTYPE(ctypes.c_char_p)(lambda: b"what went wrong")
+    address = lambda f: ctypes.cast(f, ctypes.c_void_p).value      # noqa: E731
+    return host.launcher(address(fn), address(error), "".join(KINDS[t] for t in types), own), got, (fn, error)
+
+
+@pytest.mark.parametrize("name", sorted(kernels._SIGNATURES))
+def test_every_signature_arrives_in_order(host, name):
+    types = kernels._SIGNATURES[name]
+    fn, got, _keep = _entry(host[0], types)
+    t = torch.arange(7.0)[3:]
+    numbers = itertools.count(3)
+    args = [t if k is ctypes.c_void_p and i % 3 == 0 else None if k is ctypes.c_void_p and i % 3 == 1 else
+            next(numbers) / 4 if k is ctypes.c_float else -next(numbers) if k is ctypes.c_int else (1 << 40) + next(numbers)
+            for i, k in enumerate(types)]
+    host[0].call(fn, *args)
+    assert got == [tuple(t.data_ptr() if a is t else a for a in args)]
+    assert host[1] == {"own": 1, "library": 0}
+
+
+def test_results_counts_and_refusals(host):
+    module, counts = host
+    fn, got, _a = _entry(module, [ctypes.c_int], result=5, own=0)
+    assert fn(3) == 5 and counts == {"own": 0, "library": 0}
+    with pytest.raises(kernels.KernelError, match="what went wrong"):
+        module.call(fn, True)
+    assert counts == {"own": 0, "library": 1} and got == [(3,), (1,)]
+    fn._erb_own = 2
+    with pytest.raises(kernels.KernelError):
+        module.call(fn, -1)
+    assert counts == {"own": 2, "library": 1}
+    for bad in ((), (1, 2), (1.5,), (None,), ("1",)):
+        with pytest.raises(TypeError):
+            module.call(fn, *bad)
+    assert len(got) == 3
+
+
+def test_checks_are_those_of_python(host):
+    t = torch.zeros(4, 4)
+    for args, kw in (((None, "x"), {}), ((t, "x"), {}), ((t, "x", torch.float32), {"contiguous": False}), ((t.t(), "x", torch.int32), {})):
+        outcomes = []
+        for check in (host[0].need, kernels._need_in_python):
+            try:
+                outcomes.append(check(*args, **kw))
+            except kernels.KernelError as e:
+                outcomes.append(str(e))
+        assert outcomes[0] == outcomes[1]
