@@ -52,30 +52,32 @@ conv_silu_kernel(const T* __restrict__ proj, int ld, int off, int channels, int 
                              : old[(size_t)(taps - 1 + r) * channels + ch];
       acc = fmaf(Elem<T>::load(weight + (size_t)ch * taps + j), v, acc);
     }
+#if ERB_ELEM == 1
+    float s0, s1;
+    silu_two(Two(acc)).get(s0, s1);                            // (as conv_silu_vec_kernel: the same bits)
+    Elem<T>::store(out + (size_t)t * channels + ch, s0);
+#else
     Elem<T>::store(out + (size_t)t * channels + ch, silu_f(acc));
+#endif
   }
 }
 
 #if ERB_ELEM == 1
-// The same for TAPS taps and rows whose channels come in aligned runs of eight (bfloat16 build): a thread owns eight channels
-// of TT neighbouring tokens, keeps its weights in registers and reads every input once with 16-byte loads instead of TAPS
-// times with 2-byte ones.  Same arithmetic in the same order: the same bits.  2,048 tokens of 6,144 channels:
-// 70 us before, 26 us; 64 single tokens 16 us before, 3.6 us.  What is left is the arithmetic of silu.  (Built for four taps, what the
-// benchmarked sizes have; the eight channels' weights are then 16-byte pieces.  Others take the kernel above.)
-template <int TAPS, int TT>
+// The same for four taps and rows whose channels come in aligned runs of eight (bfloat16 build): a thread owns eight channels
+// of TT neighbouring tokens, keeps its weights in registers and reads every input once with 16-byte loads instead of four
+// times with 2-byte ones.  The sums are made in the same order: their bits are those of the kernel above, and silu is as near (silu_two).
+// 2,048 tokens of 6,144 channels: 70 us by the kernel above, 25.6 us with its arithmetic, 17.5 us with two channels an
+// instruction, tokens of one request without looking each one's request up, and this silu, four tokens a thread (two 21.8, eight 19.6 us);
+// 64 single tokens 16 us and 3.6 us.
+template <int TT>
 __global__ void __launch_bounds__(128)
 conv_silu_vec_kernel(const __nv_bfloat16* __restrict__ proj, int ld, int off, int channels, const __nv_bfloat16* __restrict__ weight,
                      const __nv_bfloat16* __restrict__ bias, const float* __restrict__ conv_state, const int* __restrict__ seq_of_token,
                      const int* __restrict__ seq_starts, const int* __restrict__ state_slots, __nv_bfloat16* __restrict__ out, int n_tokens) {
+  constexpr int TAPS = 4;
   chain_wait();
   const int ch = 8 * (blockIdx.y * blockDim.x + threadIdx.x), t0 = blockIdx.x * TT;
   if (ch >= channels) return;
-  float w[8 * TAPS], b[8];
-#pragma unroll
-  for (int i = 0; i < TAPS; ++i) load8(weight + (size_t)ch * TAPS + 8 * i, w + 8 * i);     // [channel][tap]
-#pragma unroll
-  for (int i = 0; i < 8; ++i) b[i] = 0.f;
-  if (bias) load8(bias + ch, b);
   uint4 raw[TT + TAPS - 1];                                   // inputs t0 - (TAPS - 1) .. t0 + TT - 1
 #pragma unroll
   for (int k = 0; k < TT + TAPS - 1; ++k) {
@@ -83,37 +85,59 @@ conv_silu_vec_kernel(const __nv_bfloat16* __restrict__ proj, int ld, int off, in
     raw[k] = make_uint4(0, 0, 0, 0);
     if (t >= 0 && t < n_tokens) raw[k] = *reinterpret_cast<const uint4*>(proj + (size_t)t * ld + off + ch);
   }
+  Two w[TAPS][4], b[4];                                       // pairs of channels
+  {
+    float v[8 * TAPS], u[8] = {};
+#pragma unroll
+    for (int i = 0; i < TAPS; ++i) load8(weight + (size_t)ch * TAPS + 8 * i, v + 8 * i);     // [channel][tap]
+    if (bias) load8(bias + ch, u);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      b[e] = Two(u[2 * e], u[2 * e + 1]);
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) w[j][e] = Two(v[2 * e * TAPS + j], v[(2 * e + 1) * TAPS + j]);
+    }
+  }
+  // tokens of one request that have their earlier inputs in this portion need no look at the request
+  const int first = seq_of_token[t0];
+  const bool plain = t0 - seq_starts[first] >= TAPS - 1 && seq_of_token[min(t0 + TT, n_tokens) - 1] == first;
 #pragma unroll
   for (int k = 0; k < TT; ++k) {
     const int t = t0 + k;
     if (t >= n_tokens) break;
-    const int seq = seq_of_token[t], i = t - seq_starts[seq];
-    float acc[8];
+    Two acc[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = b[e];
+    for (int e = 0; e < 4; ++e) acc[e] = b[e];
+    int i = TAPS, seq = first;
+    if (!plain) {
+      seq = seq_of_token[t];
+      i = t - seq_starts[seq];
+    }
 #pragma unroll
     for (int j = 0; j < TAPS; ++j) {
       const int r = i - (TAPS - 1 - j);                        // portion index of the input under tap j
-      float v[8];
+      Two v[4];
       if (r >= 0) {
         const uint32_t u[4] = {raw[k + j].x, raw[k + j].y, raw[k + j].z, raw[k + j].w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          v[2 * e] = __uint_as_float(u[e] << 16);
-          v[2 * e + 1] = __uint_as_float(u[e] & 0xffff0000u);
-        }
+        for (int e = 0; e < 4; ++e) v[e] = Two(__uint_as_float(u[e] << 16), __uint_as_float(u[e] & 0xffff0000u));
       } else {
         const float* old = conv_state + ((size_t)state_slots[seq] * (TAPS - 1) + TAPS - 1 + r) * channels + ch;
-        load4(old, v);
-        load4(old + 4, v + 4);
+        float x[8];
+        load4(old, x);
+        load4(old + 4, x + 4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = Two(x[2 * e], x[2 * e + 1]);
       }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] = fmaf(w[e * TAPS + j], v[e], acc[e]);
+      for (int e = 0; e < 4; ++e) acc[e] = fma2(w[j][e], v[e], acc[e]);
     }
     uint32_t o[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const __nv_bfloat162 p = __floats2bfloat162_rn(silu_f(acc[2 * e]), silu_f(acc[2 * e + 1]));
+      float s0, s1;
+      silu_two(acc[e]).get(s0, s1);
+      const __nv_bfloat162 p = __floats2bfloat162_rn(s0, s1);
       o[e] = *reinterpret_cast<const uint32_t*>(&p);
     }
     *reinterpret_cast<uint4*>(out + (size_t)t * channels + ch) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -936,13 +960,13 @@ ERB_EXPORT int erb_conv_silu(const void* proj, int n_tokens, int ld, int off, in
 #if ERB_ELEM == 1
   // Few channels of few tokens: the kernel above, whose threads have less to do one after the other (8 tokens of 6,144 channels 1.9 us
   // there, 2.5 here; 256 of 72 1.8 | 2.5); from 64 tokens on it gives a token's channels to one block (64 of 1,024 3.1 | 2.5, of
-  // 6,144 12.6 | 2.9).  Eight tokens a thread read the weights seldom, but take 7 us whatever they do: from about 2,048 tokens of
-  // 2,048 channels on (256 of 1,024 2.6 us with one token a thread, 7.4 with eight; 768 of 6,144 11.9 | 10.1).
+  // 6,144 12.6 | 2.9).  Four tokens a thread read the weights and the inputs seldom: from about 700 tokens of 6,144 channels on (8.7 us, and
+  // 10.2 with one token a thread and the earlier arithmetic; 256 tokens 5.6 us with four, 5.2 with one).
   const long long sums = (long long)n_tokens * channels;
   if ((sums >= 100000 || (n_tokens >= 64 && channels >= 1024)) && taps == 4 && channels % 8 == 0 && ld % 8 == 0 && off % 8 == 0 &&
       !(((uintptr_t)proj | (uintptr_t)weight | (uintptr_t)bias | (uintptr_t)conv_state | (uintptr_t)out) & 15)) {
-    const int per = sums >= 4000000 ? 8 : 1;
-    launch_chained(per == 8 ? conv_silu_vec_kernel<4, 8> : conv_silu_vec_kernel<4, 1>,
+    const int per = sums >= 4000000 ? 4 : 1;
+    launch_chained(per == 4 ? conv_silu_vec_kernel<4> : conv_silu_vec_kernel<1>,
                    dim3((n_tokens + per - 1) / per, (channels / 8 + 127) / 128), dim3(128), 0, (cudaStream_t)stream, (const elem_t*)proj,
                    ld, off, channels, (const elem_t*)weight, (const elem_t*)bias, conv_state, seq_of_token, seq_starts, state_slots,
                    (elem_t*)out, n_tokens);

@@ -232,30 +232,6 @@ __device__ __forceinline__ float capped_score(float x, float c2) { return fmaf(-
 constexpr float kTanh0 = 0.99999941f, kTanh1 = -0.33329042f, kTanh2 = 0.13281434f, kTanh3 = -0.051605674f, kTanh4 = 0.016743115f,
                 kTanh5 = -0.0030670603f;
 
-// Two floats that one instruction multiplies and adds (both rounded as fmaf rounds one).
-struct Two {
-  unsigned long long v;
-  __device__ __forceinline__ Two() {}
-  __device__ __forceinline__ Two(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
-  __device__ __forceinline__ explicit Two(float a) : Two(a, a) {}
-  __device__ __forceinline__ void get(float& a, float& b) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-};
-__device__ __forceinline__ Two operator*(Two a, Two b) {
-  Two d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-  return d;
-}
-__device__ __forceinline__ Two operator+(Two a, Two b) {
-  Two d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-  return d;
-}
-__device__ __forceinline__ Two fma2(Two a, Two b, Two c) {
-  Two d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return d;
-}
-
 // Tensor maps over a page pool seen as [rows = pages * kv heads * page_size][64 bfloat16] with boxes
 // of `box_rows` rows and the 128-byte swizzle.  Encoding is a host-side computation; the maps are
 // kept per (pool, rows, box) in the library that includes this header.
