@@ -185,15 +185,20 @@ attention_rows_kernel(const T* __restrict__ q, int q_row_stride, const T* __rest
 // time and then onto the accumulator, so that its rounding is no worse than that of the row kernel's 32 partial sums.
 // Tiles start at absolute multiples of 64 positions, and a tile that a row does not see changes nothing of it: a row's
 // result does not depend on the other tokens.  Tokens of several sequences in a block are taken one sequence after the other.
-// Bound by the reads of shared memory and the multiplications, about alike, and for few blocks by a tile's chain (5 us).  9 heads of 64 over
-// 3 kv heads, row kernel | this one: 333 tokens 93 | 34 us, 333 behind 7,000 2,896 | 612, 2,048 tokens 2,354 | 358; 8 heads of 128, 333 behind
-// 100 246 | 69.
+// A block has two groups of 256 threads, each with buffers of its own: one walks the even tiles, one the odd ones (counted from
+// position 0), and the groups' maxima, sums and accumulators are put together at the end in the groups' order.  So a row's result still depends on
+// nothing but its own keys.
+// Bound by the reads of shared memory and the multiplications, about alike, and for few blocks by a tile's chain (5 us), which is why
+// there are groups.  9 heads of 64 over 3 kv heads, row kernel | one group | two: 333 tokens 93 | 34 | 26.7 us, 96 tokens 16.1 | 14.8 | 12.2,
+// 333 behind 7,000 2,896 | 613 | 459, 2,048 tokens 2,354 | 357 | 329; 8 heads of 128, 333 behind 100 246 | 69 | 56.  (Four groups of 128 threads
+// with four rows each: 2,048 tokens 276, but 16 portions of 32 tokens 12.8 instead of 9.3.)
 // ---------------------------------------------------------------------------------------------
-constexpr int kTileRows = 32, kTileKeys = 64, kTileThreads = 256;
-template <int D> constexpr size_t tile_smem() { return sizeof(float) * ((kTileRows + 2 * kTileKeys) * (D + 4) + kTileRows * (kTileKeys + 4)); }
+constexpr int kTileRows = 32, kTileKeys = 64, kTileThreads = 256, kTileGroups = 2;       // (threads of a group)
+template <int D> __host__ __device__ constexpr int tile_group_floats() { return 2 * kTileKeys * (D + 4) + kTileRows * (kTileKeys + 4); }
+template <int D> constexpr size_t tile_smem() { return sizeof(float) * (kTileRows * (D + 4) + kTileGroups * tile_group_floats<D>()); }
 
 template <int D>
-__global__ void __launch_bounds__(kTileThreads, 2)
+__global__ void __launch_bounds__(kTileGroups * kTileThreads, 1)
 attention_tile_kernel(const float* __restrict__ q, int q_row_stride, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
                       const int* __restrict__ block_tables, int max_pages, const int* __restrict__ seq_of_token,
                       const int* __restrict__ positions, float* __restrict__ out, int out_row_stride, int n_tokens, int nq, int nkv,
@@ -203,13 +208,14 @@ attention_tile_kernel(const float* __restrict__ q, int q_row_stride, const float
   constexpr int LD = D + 4, LP = kTileKeys + 4, kGroups = D / 64;
   extern __shared__ __align__(16) float smem[];
   float* q_s = smem;                             // [kTileRows][LD]
-  float* k_s = q_s + kTileRows * LD;             // [kTileKeys][LD]
+  const int group = threadIdx.x / kTileThreads;
+  float* k_s = q_s + kTileRows * LD + group * tile_group_floats<D>();       // [kTileKeys][LD]
   float* v_s = k_s + kTileKeys * LD;
   float* p_s = v_s + kTileKeys * LD;             // [kTileRows][LP]
   const int t0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kTileRows, n_here = min(kTileRows, n_tokens - t0);   // (the longest walks first)
   const int h = blockIdx.y, kvh = h / (nq / nkv);
-  const int tid = threadIdx.x, lane = tid & 31, tx = tid & 15, r0 = 2 * (tid >> 4);
-  for (int i = tid; i < kTileRows * D; i += kTileThreads) {
+  const int tid = threadIdx.x % kTileThreads, lane = tid & 31, tx = tid & 15, r0 = 2 * (tid >> 4);
+  for (int i = threadIdx.x; i < kTileRows * D; i += kTileGroups * kTileThreads) {
     const int r = i / D, d = i % D;
     q_s[r * LD + d] = r < n_here ? q[(size_t)(t0 + r) * q_row_stride + (size_t)h * D + d] : 0.f;
   }
@@ -219,6 +225,9 @@ attention_tile_kernel(const float* __restrict__ q, int q_row_stride, const float
   const int pos0 = __shfl_sync(0xffffffffu, pos_l, r0), pos1 = __shfl_sync(0xffffffffu, pos_l, r0 + 1);
   const int lo0 = __shfl_sync(0xffffffffu, lo_l, r0), lo1 = __shfl_sync(0xffffffffu, lo_l, r0 + 1);
   const Penalty pen(penalty, h, nq);
+  const int page_shift = (page_size & (page_size - 1)) == 0 ? __ffs(page_size) - 1 : -1;
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(kTileThreads) : "memory"); };
+  __syncthreads();                               // (q is there)
 
   for (int begin = 0, end; begin < n_here; begin = end) {          // runs of one sequence
     const int seq = __shfl_sync(0xffffffffu, seq_l, begin);
@@ -233,20 +242,38 @@ attention_tile_kernel(const float* __restrict__ q, int q_row_stride, const float
     for (int i = 0; i < 4 * kGroups; ++i) acc[0][i] = acc[1][i] = 0.f;
     for (int j = 0; j * kTileKeys <= hi; ++j) {
       if (j * kTileKeys >= keep_first) j = max(j, lo / kTileKeys);         // past the kept first keys: on to the first that a row sees
+      if (j % kTileGroups != group) continue;
       const int k0 = j * kTileKeys;
-      __syncthreads();                                                      // (q is there; the tile before is done with)
-      for (int i = tid; i < kTileKeys * (D / 4); i += kTileThreads) {
-        const int r = i / (D / 4), c = 4 * (i % (D / 4)), k = k0 + r;
-        float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-        if (k <= hi) {
-          const size_t row = (((size_t)bt[k / page_size] * nkv + kvh) * page_size + (k % page_size)) * D + c;
-          kv = *reinterpret_cast<const float4*>(k_pages + row);
-          vv = *reinterpret_cast<const float4*>(v_pages + row);
+      group_sync();                                                         // (the tile before is done with)
+      constexpr int kRowsAtOnce = 4 * kTileThreads / D, kBatch = 4;       // rows that the group's threads copy at a time
+      const int r_own = tid / (D / 4), c = 4 * (tid % (D / 4));
+#pragma unroll
+      for (int first = 0; first < kTileKeys; first += kRowsAtOnce * kBatch) {
+        int page[kBatch];                        // (the loads of several rows under way at once: their pages, then keys and values)
+        float4 kv[kBatch], vv[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+          const int k = k0 + first + i * kRowsAtOnce + r_own;
+          page[i] = k <= hi ? bt[page_shift >= 0 ? k >> page_shift : k / page_size] : -1;
         }
-        *reinterpret_cast<float4*>(k_s + r * LD + c) = kv;
-        *reinterpret_cast<float4*>(v_s + r * LD + c) = vv;
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+          const int k = k0 + first + i * kRowsAtOnce + r_own;
+          kv[i] = vv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (page[i] >= 0) {
+            const size_t row = (((size_t)page[i] * nkv + kvh) * page_size + (page_shift >= 0 ? k & (page_size - 1) : k % page_size)) * D + c;
+            kv[i] = *reinterpret_cast<const float4*>(k_pages + row);
+            vv[i] = *reinterpret_cast<const float4*>(v_pages + row);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+          const int r = first + i * kRowsAtOnce + r_own;
+          *reinterpret_cast<float4*>(k_s + r * LD + c) = kv[i];
+          *reinterpret_cast<float4*>(v_s + r * LD + c) = vv[i];
+        }
       }
-      __syncthreads();
+      group_sync();
       const bool whole = k0 + kTileKeys - 1 <= pos_min && (k0 >= lo_max || k0 + kTileKeys <= keep_first);    // every row sees every key
       float s[2][4];
 #pragma unroll
@@ -325,9 +352,50 @@ attention_tile_kernel(const float* __restrict__ q, int q_row_stride, const float
       if (whole) products(std::false_type{}); else products(std::true_type{});
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int o = 8; o; o >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], o);
+    {                                            // the groups' parts of these rows, put together by the first one
+      constexpr int kPart = 2 * (2 + 4 * kGroups);
+      __syncthreads();                           // (the tiles are done with: their room holds the parts)
+      float* part = q_s + kTileRows * LD + tid * (kPart + 1);
+      if (group > 0) {
+        float* mine = part + group * tile_group_floats<D>();
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          mine[i] = m[i];
+          mine[2 + i] = l[i];
+#pragma unroll
+          for (int c = 0; c < 4 * kGroups; ++c) mine[4 + 4 * kGroups * i + c] = acc[i][c];
+        }
+      }
+      __syncthreads();
+      if (group == 0) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          float top = m[i];
+          for (int g = 1; g < kTileGroups; ++g) top = fmaxf(top, part[g * tile_group_floats<D>() + i]);
+          const float ref = top == -INFINITY ? 0.f : top;
+          // (a maximum of +inf is its own: its part's sum holds such keys with weight 1)
+          const float f0 = m[i] == top ? 1.f : expf(m[i] - ref);
+          l[i] *= f0;
+#pragma unroll
+          for (int c = 0; c < 4 * kGroups; ++c) acc[i][c] *= f0;
+          for (int g = 1; g < kTileGroups; ++g) {
+            const float* from = part + g * tile_group_floats<D>();
+            if (from[i] == -INFINITY && from[2 + i] == 0.f) continue;      // (saw no key of this row)
+            const float f = from[i] == top ? 1.f : expf(from[i] - ref);
+            l[i] = fmaf(from[2 + i], f, l[i]);
+#pragma unroll
+            for (int c = 0; c < 4 * kGroups; ++c) acc[i][c] = fmaf(from[4 + 4 * kGroups * i + c], f, acc[i][c]);
+          }
+        }
+      }
+      __syncthreads();
+    }
+    if (group > 0) continue;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
       const int r = r0 + i, t = t0 + r;
       if (r < begin || r >= end) continue;
       const float inv = 1.f / l[i];
@@ -348,10 +416,12 @@ int launch_tiles(const void* q, int q_row_stride, const void* k_pages, const voi
                  const int* seq_of_token, const int* positions, void* out, int out_row_stride, int n_tokens, int nq, int nkv, int page_size,
                  int window, int keep_first, float scale, const float* penalty, float softcap, const void* gate, int gate_stride,
                  cudaStream_t s) {
+  const dim3 grid((n_tokens + kTileRows - 1) / kTileRows, nq);
   auto kern = attention_tile_kernel<D>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem<D>());
+  constexpr size_t smem = tile_smem<D>();
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "attention_rows: %s", cudaGetErrorString(e));
-  launch_chained(kern, dim3((n_tokens + kTileRows - 1) / kTileRows, nq), dim3(kTileThreads), tile_smem<D>(), s, (const float*)q, q_row_stride,
+  launch_chained(kern, grid, dim3(kTileGroups * kTileThreads), smem, s, (const float*)q, q_row_stride,
                  (const float*)k_pages, (const float*)v_pages, block_tables, max_pages, seq_of_token, positions, (float*)out, out_row_stride,
                  n_tokens, nq, nkv, page_size, window, keep_first, scale, penalty, softcap, (const float*)gate, gate_stride);
   return check_launch("attention_tile");

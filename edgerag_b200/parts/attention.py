@@ -350,7 +350,7 @@ class Attention(Mixer):
 
     def _tiled(self, ctx) -> bool:
         """Whether the step's portions are long enough that the 32-bit kernel for 32 tokens at a time takes them: 9 heads of 64, a
-        portion without a past, by rows | by tiles: 64 tokens 9.1 | 10.3 us, 96 tokens 16.1 | 14.8, 333 tokens 93 | 34; behind 7,000
+        portion without a past, by rows | by tiles: 64 tokens 9.1 | 10.3 us, 96 tokens 16.1 | 12.2, 333 tokens 93 | 26.7; behind 7,000
         tokens from the first; several portions share a block one after the other (512 tokens in portions of 17 15.6 | 19.6, of 32
         20.8 | 9.6)."""
         lens = ctx.host_q_len[ctx.n_decode:]
