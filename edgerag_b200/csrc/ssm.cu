@@ -437,18 +437,23 @@ ssm_scan16_kernel(const T* __restrict__ xbc, int channels, const T* __restrict__
 // nothing is rounded to 16 bits.  c is summed in double and kept as two floats, since its differences, not its values, matter.
 //
 // Block: one (head, request, 32 columns).  Sixteen warps do what is between the products, an issuing warp asks for the products, four warps
-// make the next chunk's steps and decays, one of their lanes brings the next chunk's rows by TMA tensor copies.  Per chunk c:
+// make the steps and decays a chunk ahead and store the outputs of the chunk before, one of their lanes brings the next chunk's rows by TMA
+// tensor copies.  Per chunk c:
 //   G = C B^T                       as two sums over half of the state's rows each (the unit cuts its sums; one sum of 128 was a third
 //                                   further from float64), issued while the chunk before is finished
-//   the weighted x's pieces in shared memory; the weights' pieces from G, as the left operand in TMEM
-//   Y0 = C S, dS = B^T (weighted x) while the weights are made; Y1 = (weights) x, its first half of the tokens as soon as those weights are there
-//   the state in registers, S <- exp(c_128) S + dS, and its pieces; y = exp(c_t) Y0 + Y1 + D x
+//   Y0 = C S while the weights' pieces are made from G, as the left operand in TMEM; then dS = B^T (weighted x), and Y1 = (weights) x,
+//   its first half of the tokens as soon as those weights are there
+//   the state in registers, S <- exp(c_128) S + dS, and its pieces; the next chunk's weighted x; y = exp(c_t) Y0 + Y1 + D x
 // The pieces of the state and of the weighted x are neighbouring columns of one product: a product of 32 columns costs as much as one
-// of 96 (54 clocks, the left operand's reads).  Only the state's own line waits for the chunk before.
+// of 96 (54 clocks, the left operand's reads).  Only the state's own line waits for the chunk before.  A weight's decay is one
+// exponential where t and s lie in the same 32 tokens; elsewhere it is the product of two factors, from s to the end of its 32 and on to the
+// last token before t's 32, and from there to t, which are made once a token, in double, and rounded once.
 //
-// What bounds it: a chunk's line, 6,500 clocks: the weighted x 900, G 500, the weights 3,200 (those of the last 32 tokens are all made by one
-// scheduler's warps, which alone reach their lanes of TMEM), the second half of Y1 700, outputs 850.  The products take 2,900 beside it.  2,048 tokens of 64 heads of 64 x 128: 64.5 us; 132 us
-// in chunks of 64 by mma.sync, 566 us walked.  Error against float64 1.2e-7 for y, 7.4e-8 for the state, as those.
+// What bounds it: a chunk's line, about 5,200 clocks: G read 700, the weights 2,500 (shared memory serves the products' operands meanwhile),
+// dS awaited and the state published 1,000, weighted x 700, outputs 400.  2,048 tokens of 64 heads of 64 x 128: 52.3 us; 64.5 us with an
+// exponential a weight, a lone lane issuing (110 clocks a product; an elected lane of a whole warp has what they take in uniform
+// registers) and steps, stores and weighted x in the line; 132 us in chunks of 64 by mma.sync, 566 us walked.  (The weighted x made by the step warps:
+// 55 us; there they are the longer line.)  Error against float64 1.2e-7 for y, 7.4e-8 for the state, as those.
 //
 // The products are causal for finite numbers only: above the diagonal the weights are zeros, and 0 * inf is no number; nor are the
 // pieces of an infinity, or the differences of c where a decay is exactly zero; and a chunk's last rows may be another request's.
@@ -469,16 +474,16 @@ struct ChunkSmem {
   uint8_t s[3][kChunk * 64];                 // the state before the chunk: a row per state row
   float dt[2][kChunk], hi[2][kChunk], lo[2][kChunk];           // step, c_t / ln 2 in two floats
   float grown[2][kChunk], weight[2][kChunk];                   // exp(c_t), dt_t exp(c_128 - c_t)
+  float fall[2][kChunk], rise[2][3][kChunk];                   // exp(c_t - c_r), r the last token before t's 32; dt_s exp(c_r - c_s) for the later 32s' r
   alignas(16) float out[kChunk][kChunkCols + 4];               // a chunk's y on its way to whole lines
-  double sums[kStepWarps];                                     // the sums of 32 logarithms each
-  uint64_t bars[9];
-  float total[2];                                              // exp(c_128)
+  double decay[kStepWarps];                                    // of 32 tokens each
+  uint64_t bars[11];
   int abort;
   uint32_t tmem;
 };
 static_assert(offsetof(ChunkSmem, dt) % 16 == 0 && offsetof(ChunkSmem, hi) % 16 == 0 && offsetof(ChunkSmem, lo) % 16 == 0 &&
-                  offsetof(ChunkSmem, out) % 16 == 0 && (kChunkCols + 4) % 4 == 0 && offsetof(ChunkSmem, bars) % 8 == 0 &&
-                  offsetof(ChunkSmem, sums) % 8 == 0 && offsetof(ChunkSmem, b) % 1024 == 0 && offsetof(ChunkSmem, x) % 1024 == 0 &&
+                  offsetof(ChunkSmem, out) % 16 == 0 && offsetof(ChunkSmem, rise) % 16 == 0 && (kChunkCols + 4) % 4 == 0 && offsetof(ChunkSmem, bars) % 8 == 0 &&
+                  offsetof(ChunkSmem, decay) % 8 == 0 && offsetof(ChunkSmem, b) % 1024 == 0 && offsetof(ChunkSmem, x) % 1024 == 0 &&
                   offsetof(ChunkSmem, w) % 1024 == 0 && offsetof(ChunkSmem, s) % 1024 == 0, "read 16 bytes at a time; tiles start where their swizzle does");
 // byte offset of 16-byte piece c of row r in a tile of 64-byte rows with the 64-byte swizzle
 __device__ __forceinline__ uint32_t swz64(int r, int c) { return (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); }
@@ -522,12 +527,14 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
   const int g = h / (H / G), inner = H * P;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_chunks = (n_tok + kChunk - 1) / kChunk;
-  // G there; the weights' pieces of the chunk's first and last 64 tokens; the weighted x's; dS there; Y there; the state's pieces; a stage's rows (two)
-  constexpr int kBarG = 0, kBarP1 = 1, kBarP2 = 2, kBarW = 3, kBarD = 4, kBarY = 5, kBarS = 6, kBarL = 7;
+  // G there; the weights' pieces of the chunk's first and last 64 tokens; the weighted x's; dS there; Y there; the state's pieces; a stage's rows
+  // (two); the outputs of the chunk before read; those stored and the next chunk's steps there
+  constexpr int kBarG = 0, kBarP1 = 1, kBarP2 = 2, kBarW = 3, kBarD = 4, kBarY = 5, kBarS = 6, kBarL = 7, kBarR = 9, kBarT = 10;
   auto bar = [&](int which) { return smem_u32(&sm.bars[which]); };
   volatile int* abort_flag = &sm.abort;
   if (threadIdx.x == 0) {
-    for (int i : {kBarG, kBarD, kBarY, kBarL, kBarL + 1}) mbar_init(bar(i), 1);
+    for (int i : {kBarG, kBarD, kBarY, kBarL, kBarL + 1, kBarR}) mbar_init(bar(i), 1);
+    mbar_init(bar(kBarT), kStepWarps);
     for (int i : {kBarP1, kBarP2, kBarW, kBarS}) mbar_init(bar(i), kChunkWarps);
     sm.abort = 0;
     mbar_init_fence();
@@ -540,9 +547,10 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = sm.tmem;
-  // columns of TMEM.  G's first sum: 0; the weights' pieces, 3 x 64, and before them G's second sum: 128; Y0 by the state's first piece | by
-  // the others; dS by three pieces; Y1
-  constexpr uint32_t kColM = 128, kColY0 = 320, kColD = 384, kColY1 = 480;
+  // columns of TMEM.  G's first sum, then dS by three pieces: 0; Y0 by the state's three pieces; Y1; the weights' pieces for the chunk's last 64
+  // tokens, 3 x 32, then for its first 64; G's second sum lies over two of those and the 64 columns behind them
+  constexpr uint32_t kColD = 0, kColY0 = 128, kColY1 = 224, kColM = 352, kColG = 384;
+  auto col_m = [](int unit, int piece) { return kColM - (unit >> 2) * 96 + 32 * piece + 8 * (unit & 3); };
   constexpr int kTopThreads = 32 * (kChunkWarps + kStepWarps);
   float probe = 0.f;                                           // no number once a result was not finite
 
@@ -570,9 +578,9 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
       mbar_wait_or_abort(bar(which), parity, abort_flag);
       __syncwarp();
     };
-    auto no_weights = [&](int u, int pieces) {                 // zeros in the unit of 16 columns: it lies above the diagonal
+    auto no_weights = [&](int u, int piece) {                  // zeros in the unit of 16 columns from a piece on: it lies above the diagonal
       const uint32_t zero[8] = {};
-      for (int k = 0; k < pieces; ++k) tmem_st8(t_lane + kColM + 64 * k + 8 * u, zero);
+      for (; piece < 3; ++piece) tmem_st8(t_lane + col_m(u, piece), zero);
     };
 #pragma unroll
     for (int i = 0; i < 8; ++i) S[i] = 0.f;
@@ -585,31 +593,35 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
     }
     publish();
     for (int u = qt; u < 8; u += 4)
-      if (u >= 2 * (quad + 1)) no_weights(u, 3);
+      if (u >= 2 * (quad + 1)) no_weights(u, 0);
     tmem_st_wait();
     fence_before_sync();
     fence_async_proxy();
     arrive(kBarS);
+    auto weigh = [&](int c) {                                  // weighted x: tokens 32 (warp / 4) .. + 31, columns 8 (warp % 4) .. + 7
+      const int st = c & 1, t = 32 * qt + lane;
+      wait(kBarL + st, (c >> 1) & 1);
+      const float f = sm.weight[st][t];
+      const uint4 in = *reinterpret_cast<const uint4*>(sm.x[st] + swz64(t, quad));
+      const uint32_t q[4] = {in.x, in.y, in.z, in.w};
+      uint32_t piece[4][3];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) split_two(Two(f) * Two(__uint_as_float(q[i] << 16), __uint_as_float(q[i] & 0xffff0000u)), piece[i]);
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        *reinterpret_cast<uint4*>(sm.w[k] + swz64(t, quad)) = make_uint4(piece[0][k], piece[1][k], piece[2][k], piece[3][k]);
+      fence_async_proxy();
+      arrive(kBarW);
+    };
+    wait(kBarT, 0);
+    weigh(0);
     const float dskip = d_skip[h];
     for (int c = 0; c < n_chunks; ++c) {
       const int st = c & 1;
       const uint32_t par = c & 1;
       named_barrier(1, kTopThreads);                           // this chunk's steps are there, everybody is done with the chunk before
-      wait(kBarL + st, (c >> 1) & 1);
-      {                                                        // weighted x: tokens 32 (warp / 4) .. + 31, columns 8 (warp % 4) .. + 7
-        const int t = 32 * qt + lane;
-        const float f = sm.weight[st][t];
-        const uint4 in = *reinterpret_cast<const uint4*>(sm.x[st] + swz64(t, quad));
-        const uint32_t q[4] = {in.x, in.y, in.z, in.w};
-        uint32_t piece[4][3];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) split_two(Two(f) * Two(__uint_as_float(q[i] << 16), __uint_as_float(q[i] & 0xffff0000u)), piece[i]);
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-          *reinterpret_cast<uint4*>(sm.w[k] + swz64(t, quad)) = make_uint4(piece[0][k], piece[1][k], piece[2][k], piece[3][k]);
-        fence_async_proxy();
-        arrive(kBarW);
-      }
+      if (threadIdx.x == 0) mbar_arrive(bar(kBarR));
+      __syncwarp();
       wait(kBarG, par);
       fence_after_sync();
       float gram[2][16];                                       // units qt and qt + 4 of these 32 tokens: 16 columns each
@@ -619,7 +631,7 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
         if (u < 2 * (quad + 1)) {                              // (the same for the warp)
           float more[16];
           tmem_ld16(t_lane + 16 * u, gram[i]);
-          tmem_ld16(t_lane + kColM + 16 * u, more);
+          tmem_ld16(t_lane + kColG + 16 * u, more);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 16; ++j) gram[i][j] += more[j];
@@ -633,25 +645,29 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
         const int u = qt + 4 * i;
         if (u < 2 * (quad + 1)) {
           uint32_t piece[8][3];
-          const bool diagonal = 16 * u + 15 > 32 * quad;       // (the same for the warp)
+          if (u < 2 * quad) {                                  // (the same for the warp) before these tokens' group: two factors
+            const Two fall(sm.fall[st][row]);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int s0 = 16 * u + 4 * j;
-            const float4 hs = *reinterpret_cast<const float4*>(&sm.hi[st][s0]), ls = *reinterpret_cast<const float4*>(&sm.lo[st][s0]);
-            const float4 ds = *reinterpret_cast<const float4*>(&sm.dt[st][s0]);
-            const Two h2[2] = {Two(hs.x, hs.y), Two(hs.z, hs.w)}, l2[2] = {Two(ls.x, ls.y), Two(ls.z, ls.w)}, d2[2] = {Two(ds.x, ds.y), Two(ds.z, ds.w)};
+            for (int j = 0; j < 4; ++j) {
+              const float4 f = *reinterpret_cast<const float4*>(&sm.rise[st][quad - 1][16 * u + 4 * j]);
+              split_two(Two(gram[i][4 * j], gram[i][4 * j + 1]) * Two(f.x, f.y) * fall, piece[2 * j]);
+              split_two(Two(gram[i][4 * j + 2], gram[i][4 * j + 3]) * Two(f.z, f.w) * fall, piece[2 * j + 1]);
+            }
+          } else {
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              const Two gap = fma2(Two(-1.f), h2[k], hi_t) + fma2(Two(-1.f), l2[k], lo_t);
-              float e0, e1;
-              gap.get(e0, e1);
-              Two w = Two(gram[i][4 * j + 2 * k], gram[i][4 * j + 2 * k + 1]) * d2[k] * Two(fast_exp2(e0), fast_exp2(e1));
-              if (diagonal) {
-                float w0, w1;
-                w.get(w0, w1);
-                w = Two(s0 + 2 * k <= row ? w0 : 0.f, s0 + 2 * k + 1 <= row ? w1 : 0.f);
+            for (int j = 0; j < 4; ++j) {
+              const int s0 = 16 * u + 4 * j;
+              const float4 hs = *reinterpret_cast<const float4*>(&sm.hi[st][s0]), ls = *reinterpret_cast<const float4*>(&sm.lo[st][s0]);
+              const float4 ds = *reinterpret_cast<const float4*>(&sm.dt[st][s0]);
+              const Two h2[2] = {Two(hs.x, hs.y), Two(hs.z, hs.w)}, l2[2] = {Two(ls.x, ls.y), Two(ls.z, ls.w)}, d2[2] = {Two(ds.x, ds.y), Two(ds.z, ds.w)};
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                const Two gap = fma2(Two(-1.f), h2[k], hi_t) + fma2(Two(-1.f), l2[k], lo_t);
+                float e0, e1, w0, w1;
+                gap.get(e0, e1);
+                (Two(gram[i][4 * j + 2 * k], gram[i][4 * j + 2 * k + 1]) * d2[k] * Two(fast_exp2(e0), fast_exp2(e1))).get(w0, w1);
+                split_two(Two(s0 + 2 * k <= row ? w0 : 0.f, s0 + 2 * k + 1 <= row ? w1 : 0.f), piece[2 * j + k]);
               }
-              split_two(w, piece[2 * j + k]);
             }
           }
 #pragma unroll
@@ -659,10 +675,10 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
             uint32_t out[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) out[j] = piece[j][k];
-            tmem_st8(t_lane + kColM + 64 * k + 8 * u, out);
+            tmem_st8(t_lane + col_m(u, k), out);
           }
-        } else {
-          no_weights(u, 2);                                    // (the second sum lay over two of the pieces)
+        } else if (u < 4) {
+          no_weights(u, 1);                                    // (the second sum lay over two of the pieces)
         }
         tmem_st_wait();
         fence_before_sync();
@@ -677,7 +693,7 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
       tmem_ld8(t_lane + kColD + 64 + 8 * qt, v2);
       tmem_ld_wait();
       if (holds) {
-        const float total = sm.total[st];
+        const float total = sm.grown[st][kChunk - 1];
 #pragma unroll
         for (int i = 0; i < 8; ++i) S[i] = fmaf(total, S[i], (v2[i] + v1[i]) + v[i]);
       }
@@ -685,12 +701,15 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
       fence_before_sync();
       fence_async_proxy();
       arrive(kBarS);
+      wait(kBarT, par ^ 1);
+      if (c + 1 < n_chunks) weigh(c + 1);
       // the outputs of token `row`
       wait(kBarY, par);
       fence_after_sync();
       float own[8];
       tmem_ld8(t_lane + kColY0 + 8 * qt, v);
       tmem_ld8(t_lane + kColY0 + 32 + 8 * qt, v1);
+      tmem_ld8(t_lane + kColY0 + 64 + 8 * qt, v2);
       tmem_ld8(t_lane + kColY1 + 8 * qt, own);
       tmem_ld_wait();
       fence_before_sync();
@@ -700,8 +719,8 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
         const uint32_t q[4] = {in.x, in.y, in.z, in.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          v[2 * i] = fmaf(grown, v1[2 * i] + v[2 * i], own[2 * i]) + dskip * __uint_as_float(q[i] << 16);
-          v[2 * i + 1] = fmaf(grown, v1[2 * i + 1] + v[2 * i + 1], own[2 * i + 1]) + dskip * __uint_as_float(q[i] & 0xffff0000u);
+          v[2 * i] = fmaf(grown, (v2[2 * i] + v1[2 * i]) + v[2 * i], own[2 * i]) + dskip * __uint_as_float(q[i] << 16);
+          v[2 * i + 1] = fmaf(grown, (v2[2 * i + 1] + v1[2 * i + 1]) + v[2 * i + 1], own[2 * i + 1]) + dskip * __uint_as_float(q[i] & 0xffff0000u);
         }
         if (c * kChunk + row < n_tok)
 #pragma unroll
@@ -709,82 +728,95 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
         *reinterpret_cast<float4*>(&sm.out[row][8 * qt]) = make_float4(v[0], v[1], v[2], v[3]);
         *reinterpret_cast<float4*>(&sm.out[row][8 * qt + 4]) = make_float4(v[4], v[5], v[6], v[7]);
       }
-      named_barrier(4 + quad, 128);                            // the four warps of these 32 tokens; then eight lanes a token
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int r = 32 * quad + 8 * qt + 4 * i + (lane >> 3), e = 4 * (lane & 7);
-        if (c * kChunk + r < n_tok)
-          *reinterpret_cast<float4*>(y + (size_t)(start + c * kChunk + r) * inner + h * P + p0 + e) = *reinterpret_cast<const float4*>(&sm.out[r][e]);
-      }
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) probe = fmaf(S[i], 0.f, probe);
+    named_barrier(1, kTopThreads);
   } else if (warp == kIssueWarp) {
-    if (lane == 0) {
-      constexpr uint32_t kIdescG = mma_idesc(128, kChunk, false), kIdesc1 = mma_idesc(128, kChunkCols, true),
-                         kIdesc2 = mma_idesc(128, 2 * kChunkCols, true), kIdescT = mma_idesc(128, 3 * kChunkCols, true) | (1u << 15);
-      constexpr uint64_t kBlock = (kChunk * 128) >> 4;         // from a tile's first 64 state rows to its others, in 16-byte pieces
-      constexpr uint64_t kPiece = (kChunk * 64) >> 4;
-      const uint64_t ds = desc_rows64(smem_u32(sm.s[0])), dw = desc_rows64(smem_u32(sm.w[0]));
-      bool ok = true;
-      auto wait = [&](int which, uint32_t parity) {
-        if (ok) ok = mbar_wait_or_abort(bar(which), parity, abort_flag);
-        fence_after_sync();
-        return ok;
-      };
-      auto issue_g = [&](int c, int half) {                    // a sum of G over half of the state's rows
-        const uint64_t dc = make_desc(smem_u32(sm.c[c & 1][0])), db = make_desc(smem_u32(sm.b[c & 1][0]));
+    // The whole warp walks the chunks and one elected lane issues: what a product takes then lies in uniform registers (a lone lane
+    // took 110 clocks a product, 56 products a chunk).
+    constexpr uint32_t kIdescG = mma_idesc(128, kChunk, false), kIdesc1 = mma_idesc(128, kChunkCols, true),
+                       kIdesc3 = mma_idesc(128, 3 * kChunkCols, true), kIdescT = kIdesc3 | (1u << 15);
+    constexpr uint64_t kBlock = (kChunk * 128) >> 4;           // from a tile's first 64 state rows to its others, in 16-byte pieces
+    constexpr uint64_t kPiece = (kChunk * 64) >> 4;
+    const bool elected = elect_one();
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const int chunks = __shfl_sync(0xffffffffu, n_chunks, 0);
+    const uint64_t ds = desc_rows64(smem_u32(sm.s[0])), dw = desc_rows64(smem_u32(sm.w[0])), dx0 = desc_rows64(smem_u32(sm.x[0]));
+    const uint64_t dc0 = make_desc(smem_u32(sm.c[0][0])), db0 = make_desc(smem_u32(sm.b[0][0]));
+    bool ok = true;
+    auto wait = [&](int which, uint32_t parity) {
+      if (ok) ok = mbar_wait_or_abort(bar(which), parity, abort_flag);
+      return ok = __all_sync(0xffffffffu, ok) != 0;
+    };
+    auto issue_g = [&](int c, int half) {                      // a sum of G over half of the state's rows
+      const uint64_t dc = dc0 + (c & 1) * 2 * kBlock, db = db0 + (c & 1) * 2 * kBlock;
 #pragma unroll
-        for (int i = 0; i < N / 32; ++i) {
-          const int k = half * (N / 32) + i;
-          mma_bf16(tmem + half * kColM, dc + (k >> 2) * kBlock + 2 * (k & 3), db + (k >> 2) * kBlock + 2 * (k & 3), kIdescG, i > 0);
+      for (int i = 0; i < N / 32; ++i) {
+        const int k = half * (N / 32) + i;
+        mma_bf16(tm + half * kColG, dc + (k >> 2) * kBlock + 2 * (k & 3), db + (k >> 2) * kBlock + 2 * (k & 3), kIdescG, i > 0);
+      }
+    };
+    auto issue_y1 = [&](uint64_t dx, int half) {               // the part of Y1 from half of the chunk's tokens, the smallest pieces first
+#pragma unroll
+      for (int p = 2; p >= 0; --p)
+#pragma unroll
+        for (int i = 0; i < kChunk / 32; ++i) {
+          const int k = half * (kChunk / 32) + i;
+          mma_bf16_a_tmem(tm + kColY1, tm + col_m(k, p), dx + 64 * k, kIdesc1, half || p < 2 || i > 0);
         }
-      };
-      auto issue_y1 = [&](uint64_t dx, int half) {             // the part of Y1 from half of the chunk's tokens, the smallest pieces first
-#pragma unroll
-        for (int p = 2; p >= 0; --p)
-#pragma unroll
-          for (int i = 0; i < kChunk / 32; ++i) {
-            const int k = half * (kChunk / 32) + i;
-            mma_bf16_a_tmem(tmem + kColY1, tmem + kColM + 64 * p + 8 * k, dx + 64 * k, kIdesc1, half || p < 2 || i > 0);
-          }
-      };
-      if (wait(kBarS, 0) && wait(kBarL, 0)) {
+    };
+    if (wait(kBarS, 0) && wait(kBarL, 0)) {
+      fence_after_sync();
+      if (elected) {
         issue_g(0, 0);
         issue_g(0, 1);
         mma_commit(bar(kBarG));
       }
-      for (int c = 0; c < n_chunks && ok; ++c) {
-        const int st = c & 1;
-        if (c > 0 && !wait(kBarS, c & 1)) break;
-        if (!wait(kBarW, c & 1)) break;
-        const uint64_t dc = make_desc(smem_u32(sm.c[st][0]));
+      __syncwarp();
+    }
+    for (int c = 0; c < chunks && ok; ++c) {
+      const int st = c & 1;
+      const bool more = c + 1 < chunks;
+      // dS = B^T (weighted x): B's rows are its tokens, 64 state rows to a block
+      const uint64_t dc = dc0 + st * 2 * kBlock, dx = dx0 + st * kPiece, db = ((db0 + st * 2 * kBlock) & ~((uint64_t)0x3fff << 16)) | (kBlock << 16);
+      if (!wait(kBarR, c & 1)) break;
+      fence_after_sync();
+      if (elected) {
 #pragma unroll
         for (int k = 0; k < N / 16; ++k)                       // Y0 = C S
-          mma_bf16(tmem + kColY0, dc + (k >> 2) * kBlock + 2 * (k & 3), ds + 64 * k, kIdesc2, k > 0);
+          mma_bf16(tm + kColY0, dc + (k >> 2) * kBlock + 2 * (k & 3), ds + 64 * k, kIdesc3, k > 0);
+      }
+      __syncwarp();
+      if (!wait(kBarW, c & 1) || !wait(kBarP1, c & 1)) break;  // (all of G has been read)
+      fence_after_sync();
+      if (elected) {
 #pragma unroll
-        for (int k = 0; k < N / 16; ++k)
-          mma_bf16(tmem + kColY0 + 32, dc + (k >> 2) * kBlock + 2 * (k & 3), ds + 2 * kPiece + 64 * k, kIdesc1, 1);
-        // dS = B^T (weighted x): B's rows are its tokens, 64 state rows to a block
-        const uint64_t db = (make_desc(smem_u32(sm.b[st][0])) & ~((uint64_t)0x3fff << 16)) | (kBlock << 16);
-#pragma unroll
-        for (int k = 0; k < kChunk / 16; ++k) mma_bf16(tmem + kColD, db + 128 * k, dw + 64 * k, kIdescT, k > 0);
-        mma_commit(bar(kBarD));
-        const uint64_t dx = desc_rows64(smem_u32(sm.x[st]));
-        if (!wait(kBarP1, c & 1)) break;
+        for (int k = 0; k < kChunk / 16; ++k) mma_bf16(tm + kColD, db + 128 * k, dw + 64 * k, kIdescT, k > 0);
+        mma_commit(bar(kBarD));                                // (the state's pieces have been read, too)
         issue_y1(dx, 0);
-        if (c + 1 < n_chunks) {
-          if (!wait(kBarL + (st ^ 1), ((c + 1) >> 1) & 1)) break;
-          issue_g(c + 1, 0);
-        }
-        if (!wait(kBarP2, c & 1)) break;
+      }
+      __syncwarp();
+      if (more) {
+        if (!wait(kBarL + (st ^ 1), ((c + 1) >> 1) & 1)) break;
+        if (elected) issue_g(c + 1, 1);                        // (behind the products that read the weights it lies over)
+        __syncwarp();
+      }
+      if (!wait(kBarP2, c & 1)) break;
+      fence_after_sync();
+      if (elected) {
         issue_y1(dx, 1);
         mma_commit(bar(kBarY));
-        if (c + 1 < n_chunks) {
-          if (!wait(kBarY, c & 1)) break;                      // (the weights have been read: G's second sum goes over them)
-          issue_g(c + 1, 1);
+      }
+      __syncwarp();
+      if (more) {
+        if (!wait(kBarS, (c + 1) & 1)) break;                  // (dS has been read)
+        fence_after_sync();
+        if (elected) {
+          issue_g(c + 1, 0);
           mma_commit(bar(kBarG));
         }
+        __syncwarp();
       }
     }
     __syncwarp();
@@ -801,44 +833,79 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
       }
       tma_load_box(smem_u32(sm.x[st]), &map_x, h * P + p0, at, full);
     };
-    auto make_steps = [&](int c) {
-      const int st = c & 1, t = c * kChunk + r;
-      const float dt = t < n_tok ? softplus_f(__bfloat162float(proj[(size_t)(start + t) * ld + off_dt + h]) + bias) : 0.f;
-      double cum = (double)a * (double)dt;                     // inclusive sums over the lanes, then the warps before
+    float dt, hi, lo, fall, rise[kStepWarps - 1], grown, weight;   // of a chunk's token, on their way
+    auto raw_step = [&](int c) { return c * kChunk + r < n_tok ? __bfloat162float(proj[(size_t)(start + c * kChunk + r) * ld + off_dt + h]) : 0.f; };
+    auto make_steps = [&](int c, float raw_dt) {
+      dt = c * kChunk + r < n_tok ? softplus_f(raw_dt + bias) : 0.f;
+      double cum = (double)a * (double)dt;                     // inclusive sums over the group's lanes
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const double v = __shfl_up_sync(0xffffffffu, cum, o);
         if (lane >= o) cum += v;
       }
-      if (lane == 31) sm.sums[w] = cum;
+      const double sum = __shfl_sync(0xffffffffu, cum, 31), l2 = cum * 1.4426950408889634;
+      hi = (float)l2;
+      lo = (float)(l2 - (double)hi);
+      double from = exp(cum), to = (double)dt * exp(sum - cum);     // from the group's start, to its end
+      fall = (float)from;
+      named_barrier(2, 32 * kStepWarps);                       // (all have read the decays of the chunk before)
+      if (lane == 31) sm.decay[w] = from;
       named_barrier(2, 32 * kStepWarps);
-      double all = 0.0;
 #pragma unroll
       for (int i = 0; i < kStepWarps; ++i) {
-        if (i == w) cum += all;
-        all += sm.sums[i];
+        if (i < w) from *= sm.decay[i];
+        if (i > w) {
+          rise[i > 0 ? i - 1 : 0] = (float)to;
+          to *= sm.decay[i];
+        }
       }
-      named_barrier(2, 32 * kStepWarps);                       // (all have read the sums)
-      const double l2 = cum * 1.4426950408889634;
-      const float hi = (float)l2;
+      grown = (float)from;
+      weight = (float)to;
+    };
+    auto place_steps = [&](int c) {
+      const int st = c & 1;
       sm.dt[st][r] = dt;
       sm.hi[st][r] = hi;
-      sm.lo[st][r] = (float)(l2 - (double)hi);
-      sm.grown[st][r] = (float)exp(cum);
-      sm.weight[st][r] = (float)((double)dt * exp(all - cum));
-      if (r == kChunk - 1) sm.total[st] = (float)exp(all);
+      sm.lo[st][r] = lo;
+      sm.fall[st][r] = fall;
+      sm.grown[st][r] = grown;
+#pragma unroll
+      for (int i = 1; i < kStepWarps; ++i)
+        if (i > w) sm.rise[st][i - 1][r] = rise[i - 1];
+      sm.weight[st][r] = weight;
+    };
+    auto store = [&](int c) {                                  // the outputs of chunk c: eight lanes a token, whole lines
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int t = 32 * w + 4 * i + (lane >> 3), e = 4 * (lane & 7);
+        if (c * kChunk + t < n_tok)
+          *reinterpret_cast<float4*>(y + (size_t)(start + c * kChunk + t) * inner + h * P + p0 + e) = *reinterpret_cast<const float4*>(&sm.out[t][e]);
+      }
     };
     const bool copies = w == 0 && lane == 0;
     if (copies) load_stage(0);
-    make_steps(0);
+    __syncwarp();
+    float raw_dt = raw_step(1);                                // asked for before it is used
+    make_steps(0, raw_step(0));
+    place_steps(0);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(kBarT));
+    if (n_chunks > 1) make_steps(1, raw_dt);
+    raw_dt = raw_step(2);
     for (int c = 0; c < n_chunks; ++c) {
+      const bool more = c + 1 < n_chunks;
       named_barrier(1, kTopThreads);
-      if (c + 1 < n_chunks) {
-        if (copies) load_stage(c + 1);
-        __syncwarp();
-        make_steps(c + 1);
-      }
+      if (copies && more) load_stage(c + 1);
+      __syncwarp();
+      if (more) place_steps(c + 1);
+      if (c > 0) store(c - 1);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(kBarT));
+      if (c + 2 < n_chunks) make_steps(c + 2, raw_dt);
+      raw_dt = raw_step(c + 3);
     }
+    named_barrier(1, kTopThreads);
+    store(n_chunks - 1);
   }
   const bool odd = __syncthreads_or(!(probe == 0.f));
   const bool gave_up = *abort_flag != 0;
@@ -934,10 +1001,10 @@ gated_group_norm_vec_kernel(const void* __restrict__ x_, int x_ld, const T* __re
 
 #if ERB_ELEM == 1
 // Whether the chunk kernel is the faster one: the two costs in microseconds, fitted to both kernels' times over 1 to 64
-// requests of 2 to 2,048 tokens (64 heads of 64 x 128 and 32 of 64 x 64; of 196 pairs measured none is decided wrongly by more than 3 %).
+// requests of 2 to 2,048 tokens (64 heads of 64 x 128 and 32 of 64 x 64; of 196 pairs measured one is decided wrongly, 33.4 us against 30.3).
 // The walk costs 0.27 us a token of the longest portion or, when the GPU is full, its blocks' tokens and states; a chunk of 128 tokens
-// costs 3.7 us for the longest portion, or as many rounds of blocks as the SMs need, a block an SM.  One request: from 26 tokens on
-// (64 x 128; 24 tokens 9.8 us walked, 10.5 in a chunk; 32 12.1 | 10.3; 64 20.5 | 10.4); 32 requests of equal length: from 42.
+// costs 2.8 us for the longest portion, or as many rounds of blocks as the SMs need, a block an SM.  One request: from 25 tokens on
+// (64 x 128; 24 tokens 9.9 us walked, 10.3 in a chunk; 32 11.7 | 10.2; 64 20.6 | 10.2); 32 requests of equal length: from about 40.
 inline bool chunks_pay(int blocks, int N, int n_tokens, int n_seqs, int longest) {
   if (longest <= 1) return false;
   const double size = N / 128.0, extra = (double)n_tokens - n_seqs - (longest - 1);      // tokens beyond one of the other requests
@@ -945,7 +1012,7 @@ inline bool chunks_pay(int blocks, int N, int n_tokens, int n_seqs, int longest)
   const double longest_chunks = (longest + kChunk - 1) / kChunk, chunks = longest_chunks + (others > 0.0 ? others + extra / kChunk : 0.0);
   const double walk = fmax(3.0 + 0.27 * longest, blocks * size * (0.00165 * n_tokens + 0.008 * n_seqs));
   const double rounds = ceil(blocks * (1.0 + others) / sm_count());
-  const double chunked = fmax(6.6 + 3.68 * longest_chunks, rounds * (3.0 + 2.4 * size + 3.65 * chunks / (1.0 + others)));
+  const double chunked = fmax(7.0 + 2.7 * longest_chunks, rounds * (2.6 + 2.8 * size + 2.9 * chunks / (1.0 + others)));
   return chunked < walk;
 }
 #endif
