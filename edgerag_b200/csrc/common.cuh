@@ -156,6 +156,11 @@ __device__ __forceinline__ float glu_gate(float g, float u, int act, float limit
 #endif
 }
 
+// A barrier among `count` threads of a block (a multiple of 32).
+__device__ __forceinline__ void named_barrier(int id, int count) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
 // Two floats that one instruction multiplies and adds (both rounded as fmaf rounds one).
 struct Two {
   unsigned long long v;

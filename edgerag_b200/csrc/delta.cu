@@ -340,14 +340,15 @@ head_norm_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ gat
 // are (their lengths are factors of rows and columns); every other operand goes in as three bfloat16 pieces (mma_split.cuh), so
 // that nothing is rounded to 16 bits.  c is summed in double and kept as two floats.
 //
-// What bounds it: the three dependent phases of a chunk, and the 64 KB of operands a block reads of it.  The walk takes 0.46 us
-// a token (2,048 tokens of 16 heads of 128 x 128: 971 us with its preparing); the chunks 3.5 us for 64 tokens (144 us for both
-// kernels).  Error against float64: 1.7e-7, as the walk's.
-constexpr int kChunk = 64, kChunkCols = 16, kChunkWarps = 16, kChunkPrepWarps = 8;
+// What bounds it: the three dependent phases of a chunk, and the 64 KB of operands a block reads of it, which four warps bring that do
+// nothing else.  The walk takes 0.46 us a token (2,048 tokens of 16 heads of 128 x 128: 971 us with its preparing); both kernels of the chunks
+// 115.6 us (143.6 us while the warps that make the products also asked for the copies, 2,300 of a chunk's 6,200 clocks, and the first kernel
+// made its roots one after the other).  Error against float64: 1.7e-7, as the walk's.
+constexpr int kChunk = 64, kChunkCols = 16, kChunkWarps = 16, kCopyWarps = 4, kChunkPrepWarps = 8;
 constexpr int kPieceElems = kChunk * kChunk;
 
-// What the first kernel leaves of one (chunk, head): the weights of the second line and T, each as three pieces [64][64] (tiles
-// of 16 x 16 above the diagonal are not written), per token (beta, exp(c) / |k|, exp(c) / |q|, exp(c_64 - c) / |k|), exp(c_64).
+// What the first kernel leaves of one (chunk, head): the weights of the second line and T, each as three pieces [64][64] (laid
+// out as shared memory has them; tiles of 16 x 16 above the diagonal are not written), per token (beta, exp(c) / |k|, exp(c) / |q|, exp(c_64 - c) / |k|), exp(c_64).
 struct ChunkRecord {
   __nv_bfloat16 p[3][kPieceElems];
   __nv_bfloat16 t[3][kPieceElems];
@@ -355,6 +356,9 @@ struct ChunkRecord {
   float4 total;
 };
 static_assert(sizeof(ChunkRecord) == 4 * 12548, "copied 16 bytes at a time; the size that callers give the scratch by");
+
+// where entry (r, c) of such a piece lies: rows of 128 bytes, 16-byte pieces exchanged by the row's number
+__device__ __forceinline__ int entry(int r, int c) { return r * kChunk + ((c & ~7) ^ ((r & 7) << 3)) + (c & 7); }
 
 // Chunks before request `seq` (requests of one token have none).
 __device__ __forceinline__ int chunks_before(const int* seq_starts, int seq) {
@@ -374,6 +378,7 @@ struct DeltaPrepSmem {
   float a[kChunk][kChunk + 4];                                 // A, then T in its place
   float x[3][16][17];
   float beta[kChunk], ik[kChunk], iq[kChunk], hi[kChunk], lo[kChunk], grown[kChunk], left[kChunk];
+  double sums[2];
 };
 
 template <int D>
@@ -408,58 +413,58 @@ delta_chunk_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, 
     copy16_or_zero(&ks[r][e], src + G * D, real);
   }
   copy_commit();
-  if (warp == 0) {                                             // write strengths and decays: tokens 2 lane and 2 lane + 1
-    double lg[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = 2 * lane + i;
-      double beta = 0.0;
-      lg[i] = 0.0;
-      if (c0 + r < n_tok) {
-        const __nv_bfloat16* raw = proj + (size_t)(start + c0 + r) * ld;
-        beta = 1.0 / (1.0 + exp(-(double)__bfloat162float(raw[off_b + h])));
-        const double z = (double)(__bfloat162float(raw[off_a + h]) + dt_bias[h]);
-        lg[i] = -exp((double)a_log[h]) * (z > 30.0 ? z : log1p(exp(z)));
-      }
-      beta_s[r] = (float)beta;
-    }
-    double sum = lg[0] + lg[1];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double v = __shfl_up_sync(0xffffffffu, sum, o);
-      if (lane >= o) sum += v;
-    }
-    const double all = __shfl_sync(0xffffffffu, sum, 31);
-    const double cum[2] = {sum - lg[1], sum};
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = 2 * lane + i;
-      const double l2 = cum[i] * 1.4426950408889634;
-      hi_s[r] = (float)l2;
-      lo_s[r] = (float)(l2 - (double)(float)l2);
-      grown_s[r] = (float)exp(cum[i]);
-      left_s[r] = (float)exp(all - cum[i]);
-    }
-    if (lane == 0) rec.total = make_float4((float)exp(all), 0.f, 0.f, 0.f);
-  }
+  // Per token, in double and rounded once: warps 0 and 1 the decays, 2 and 3 the write strengths, the others the roots of the lengths, whose
+  // sums they make a row at a time and keep in a lane each.  (One warp for decays and strengths and a root after every row: 13,000 clocks of a
+  // block's 32,000.)
+  float raw = 0.f;
+  const int tok = 32 * (warp & 1) + lane;
+  if (warp < 4 && c0 + tok < n_tok) raw = __bfloat162float(proj[(size_t)(start + c0 + tok) * ld + (warp < 2 ? off_a : off_b) + h]);
   copy_wait<0>();
   __syncthreads();
-#pragma unroll
-  for (int i = 0; i < kChunk / kChunkPrepWarps; ++i) {         // lengths, a row at a time (the roots in double, as the walk's)
-    const int r = warp + kChunkPrepWarps * i;
-    float sk = 0.f, sq = 0.f;
-#pragma unroll
-    for (int e = 0; e < D / 64; ++e) {
-      const float2 kv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ks[r][2 * lane + 64 * e]));
-      const float2 qv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qs[r][2 * lane + 64 * e]));
-      sk = fmaf(kv.x, kv.x, sk); sk = fmaf(kv.y, kv.y, sk);
-      sq = fmaf(qv.x, qv.x, sq); sq = fmaf(qv.y, qv.y, sq);
+  if (warp < 2) {
+    double cum = 0.0;
+    if (c0 + tok < n_tok) {
+      const double z = (double)(raw + dt_bias[h]);
+      cum = -exp((double)a_log[h]) * (z > 30.0 ? z : log1p(exp(z)));
     }
-    sk = warp_sum(sk);
-    sq = warp_sum(sq);
-    if (lane == 0) {
-      ik_s[r] = (float)(1.0 / sqrt((double)sk + 1e-6));
-      iq_s[r] = (float)((double)q_scale / sqrt((double)sq + 1e-6));
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, cum, o);
+      if (lane >= o) cum += v;
+    }
+    if (lane == 31) sm.sums[warp] = cum;
+    named_barrier(1, 64);
+    const double all = sm.sums[0] + sm.sums[1];
+    if (warp == 1) cum += sm.sums[0];
+    const double l2 = cum * 1.4426950408889634;
+    hi_s[tok] = (float)l2;
+    lo_s[tok] = (float)(l2 - (double)(float)l2);
+    grown_s[tok] = (float)exp(cum);
+    left_s[tok] = (float)exp(all - cum);
+    if (tok == kChunk - 1) rec.total = make_float4(grown_s[tok], 0.f, 0.f, 0.f);
+  } else if (warp < 4) {
+    beta_s[tok] = c0 + tok < n_tok ? (float)(1.0 / (1.0 + exp(-(double)raw))) : 0.f;
+  } else {
+    constexpr int kRows = kChunk / (kChunkPrepWarps - 4);
+    float sum_k = 0.f, sum_q = 0.f;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int r = kRows * (warp - 4) + i;
+      float sk = 0.f, sq = 0.f;
+#pragma unroll
+      for (int e = 0; e < D / 64; ++e) {
+        const float2 kv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ks[r][2 * lane + 64 * e]));
+        const float2 qv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qs[r][2 * lane + 64 * e]));
+        sk = fmaf(kv.x, kv.x, sk); sk = fmaf(kv.y, kv.y, sk);
+        sq = fmaf(qv.x, qv.x, sq); sq = fmaf(qv.y, qv.y, sq);
+      }
+      sk = warp_sum(sk);
+      sq = warp_sum(sq);
+      if (lane == i) { sum_k = sk; sum_q = sq; }
+    }
+    if (lane < kRows) {
+      ik_s[kRows * (warp - 4) + lane] = (float)(1.0 / sqrt((double)sum_k + 1e-6));
+      iq_s[kRows * (warp - 4) + lane] = (float)((double)q_scale / sqrt((double)sum_q + 1e-6));
     }
   }
   __syncthreads();
@@ -497,7 +502,7 @@ delta_chunk_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, 
           uint32_t piece[3];
           split_pair(v[0], v[1], piece);
 #pragma unroll
-          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&rec.p[k][r * kChunk + s]) = piece[k];
+          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&rec.p[k][entry(r, s)]) = piece[k];
         } else {
           a_s[r][s] = v[0];
           a_s[r][s + 1] = v[1];
@@ -574,7 +579,7 @@ delta_chunk_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, 
     split_pair(v.x, v.y, p01);
     split_pair(v.z, v.w, p23);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(&rec.t[k][r * kChunk + e]) = make_uint2(p01[k], p23[k]);
+    for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(&rec.t[k][entry(r, e)]) = make_uint2(p01[k], p23[k]);
   }
 }
 
@@ -582,7 +587,7 @@ delta_chunk_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, 
 //   1  warps 0-7: R = beta (v - exp(c) S^T k), a 16 x 8 tile each;  warps 8-15: S^T q, kept in registers
 //   2  warps 0-7: U = T R, and U as the state will take it;  warps 8-15 wait
 //   3  warps 0-7: the state, in accumulators (D / 16 tiles of 16 keys);  warps 8-15: o
-// The next chunk's operands are copied meanwhile.
+// Four more warps copy the next chunk's operands meanwhile.
 //
 // The products are causal for finite numbers only: above the diagonal T and the weights are zeros, and 0 * inf is no number; nor are
 // the pieces of an infinity, or the differences of c where a decay is exactly zero.  Whatever is not finite makes an o of its own
@@ -595,11 +600,8 @@ struct DeltaChunkSmem {
   struct Stage {
     __nv_bfloat16 k[kChunk][LdD];
     __nv_bfloat16 q[kChunk][LdD];
-    __nv_bfloat16 p[3][kPieceElems];                           // rows of 128 bytes, 16-byte pieces exchanged by the row's number
-    __nv_bfloat16 t[3][kPieceElems];
     __nv_bfloat16 v[kChunk][LdC];
-    float4 sc[kChunk];
-    float4 total;
+    ChunkRecord rec;
   } stage[2];
   __nv_bfloat16 s[3][D][LdC];                                  // the state before the chunk, in pieces
   __nv_bfloat16 r[3][kChunk][LdC];
@@ -608,7 +610,7 @@ struct DeltaChunkSmem {
 };
 
 template <int D>
-__global__ void __launch_bounds__(kChunkWarps * 32)
+__global__ void __launch_bounds__((kChunkWarps + kCopyWarps) * 32)
 delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const ChunkRecord* __restrict__ records, float* __restrict__ state,
                    const int* __restrict__ seq_starts, const int* __restrict__ state_slots, float* __restrict__ out, int H, int G, int dv,
                    const __nv_bfloat16* __restrict__ proj, int ld, int off_b, int off_a, const float* __restrict__ dt_bias,
@@ -625,36 +627,48 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
   const ChunkRecord* rec0 = records + (size_t)chunks_before(seq_starts, seq) * H + h;
   const __nv_bfloat16* rows = qkv + (size_t)start * channels;
 
-  auto load_stage = [&](int c) {
-    typename Smem::Stage& st = sm.stage[c & 1];
-    const int c0 = c * kChunk;
-    const ChunkRecord* rec = rec0 + (size_t)c * H;
-    for (int idx = threadIdx.x; idx < kChunk * (D / 8); idx += kChunkWarps * 32) {
-      const int r = idx / (D / 8), e = 8 * (idx % (D / 8));
-      const bool real = c0 + r < n_tok;
-      const __nv_bfloat16* src = rows + (size_t)(real ? c0 + r : 0) * channels + kh * D + e;
-      copy16_or_zero(&st.q[r][e], src, real);
-      copy16_or_zero(&st.k[r][e], src + G * D, real);
+  if (warp >= kChunkWarps) {                                   // the copies: a chunk's operands while the one before is worked on
+    const int t = threadIdx.x - kChunkWarps * 32;
+    constexpr int kThreads = kCopyWarps * 32, kRow = D / 8, kRows = kThreads / kRow;      // 16-byte pieces of a row; rows a round of the threads
+    const int r0 = t / kRow, e0 = 8 * (t % kRow);
+    int at[3];                                                 // where this thread's pieces of P and T lie: those not above the diagonal's tiles
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      int n = t + kThreads * i, tile = 0;
+      while (n >= 32 * (tile + 1)) n -= 32 * ++tile;           // (16 rows of 2 (tile + 1) pieces)
+      at[i] = t + kThreads * i < 320 ? entry(16 * tile + n / (2 * (tile + 1)), 8 * (n % (2 * (tile + 1)))) : -1;
     }
-    for (int idx = threadIdx.x; idx < 3 * kChunk * (kChunk / 8); idx += kChunkWarps * 32) {
-      const int row = idx >> 3, r = row & (kChunk - 1), piece = row / kChunk, e = idx & 7;
-      if (e >= 2 * (r / 16 + 1)) continue;                     // (above the diagonal)
-      const int dst = r * kChunk + 8 * (e ^ (r & 7));
-      copy16_or_zero(&st.p[piece][dst], &rec->p[piece][r * kChunk + 8 * e], true);
-      copy16_or_zero(&st.t[piece][dst], &rec->t[piece][r * kChunk + 8 * e], true);
+    for (int c = 0; c < n_chunks; ++c) {
+      typename Smem::Stage& st = sm.stage[c & 1];
+      const int left = n_tok - c * kChunk;                     // tokens from this chunk on (rows behind the request's are zeros)
+      const ChunkRecord* rec = rec0 + (size_t)c * H;
+      const __nv_bfloat16* src = rows + (size_t)(c * kChunk) * channels;
+#pragma unroll
+      for (int i = 0; i < kChunk / kRows; ++i) {
+        const int r = r0 + kRows * i;
+        const __nv_bfloat16* row = src + (size_t)(r < left ? r : 0) * channels + kh * D + e0;
+        copy16_or_zero(&st.q[r][e0], row, r < left);
+        copy16_or_zero(&st.k[r][e0], row + G * D, r < left);
+      }
+      {
+        const int r = t >> 1, e = 8 * (t & 1);
+        copy16_or_zero(&st.v[r][e], src + (size_t)(r < left ? r : 0) * channels + 2 * G * D + h * dv + p0 + e, r < left);
+      }
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        if (at[i] >= 0)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            copy16_or_zero(&st.rec.p[k][at[i]], &rec->p[k][at[i]], true);
+            copy16_or_zero(&st.rec.t[k][at[i]], &rec->t[k][at[i]], true);
+          }
+      if (t < kChunk) copy16_or_zero(&st.rec.sc[t], &rec->sc[t], true);
+      else if (t == kChunk) copy16_or_zero(&st.rec.total, &rec->total, true);
+      copy_commit();
+      copy_wait<0>();
+      __syncthreads();                                         // (a chunk's first barrier)
     }
-    if (threadIdx.x < 2 * kChunk) {
-      const int r = threadIdx.x >> 1, e = 8 * (threadIdx.x & 1);
-      const bool real = c0 + r < n_tok;
-      copy16_or_zero(&st.v[r][e], rows + (size_t)(real ? c0 + r : 0) * channels + 2 * G * D + h * dv + p0 + e, real);
-    } else if (threadIdx.x < 3 * kChunk) {
-      copy16_or_zero(&st.sc[threadIdx.x - 2 * kChunk], &rec->sc[threadIdx.x - 2 * kChunk], true);
-    } else if (threadIdx.x == 3 * kChunk) {
-      copy16_or_zero(&st.total, &rec->total, true);
-    }
-    copy_commit();
-  };
-
+  }
   // the state (stored [values][keys]): warp w < 8 holds keys 16 (w mod D/16) .. + 15, values 8 NTW (w div D/16) .. + 8 NTW - 1
   constexpr int kRowTiles = D / 16, NTW = kRowTiles / 4;
   const int s_row = 16 * (warp % kRowTiles), s_col = 8 * NTW * (warp / kRowTiles);
@@ -672,7 +686,6 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
           *reinterpret_cast<uint32_t*>(&sm.s[k][s_row + qr + 8 * j][s_col + 8 * nt + 2 * qc]) = piece[k];
       }
   };
-  load_stage(0);
   if (warp < 8) {
 #pragma unroll
     for (int nt = 0; nt < NTW; ++nt)
@@ -689,7 +702,7 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
       const int r = row + (lane & 15), e = (k >> 3) + (lane >> 4);
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        ldmatrix4(a[i], &m[i][r * kChunk + 8 * (e ^ (r & 7))]);
+        ldmatrix4(a[i], &m[i][entry(r, 8 * e)]);
         ldmatrix2t(b[i], &x[i][k + (lane & 15)][col]);
       }
       mma16816(acc[0], a[0], b[0][0], b[0][1]);
@@ -703,11 +716,9 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
     for (int i = 0; i < 4; ++i) result[i] = (acc[2][i] + acc[1][i]) + acc[0][i];
   };
   float probe = 0.f;                                           // no number once a result was not finite
-  for (int c = 0; c < n_chunks; ++c) {
+  for (int c = 0; c < n_chunks && warp < kChunkWarps; ++c) {
     typename Smem::Stage& st = sm.stage[c & 1];
-    copy_wait<0>();
     __syncthreads();                                           // chunk c's operands and the state's pieces are there
-    if (c + 1 < n_chunks) load_stage(c + 1);
     float from_state[4];                                       // 16 x 8 of k S (warps 0-7) or q S, rows as they came
     {
       float acc[3][4] = {};
@@ -731,7 +742,7 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int r = row + qr + 8 * j;
-        const float4 sc = st.sc[r];
+        const float4 sc = st.rec.sc[r];
         const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.v[r][col + 2 * qc]));
         uint32_t piece[3];
         split_pair(sc.x * fmaf(-sc.y, from_state[2 * j], v.x), sc.x * fmaf(-sc.y, from_state[2 * j + 1], v.y), piece);
@@ -739,14 +750,14 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
         for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&sm.r[k][r][col + 2 * qc]) = piece[k];
       }
     }
-    __syncthreads();                                           // R is there; the state's pieces have been read
+    named_barrier(1, kChunkWarps * 32);                        // R is there; the state's pieces have been read
     if (warp < 8) {
       float u[4];
-      triangular(st.t, sm.r, u);
+      triangular(st.rec.t, sm.r, u);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int r = row + qr + 8 * j;
-        const float left = st.sc[r].w;
+        const float left = st.rec.sc[r].w;
         uint32_t piece[3], weighted[3];
         split_pair(u[2 * j], u[2 * j + 1], piece);
         split_pair(left * u[2 * j], left * u[2 * j + 1], weighted);
@@ -757,7 +768,7 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
         }
       }
     }
-    __syncthreads();                                           // U is there
+    named_barrier(1, kChunkWarps * 32);                        // U is there
     if (warp < 8) {
       float add[3][NTW][4] = {};
 #pragma unroll
@@ -774,7 +785,7 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
 #pragma unroll
           for (int nt = 0; nt < NTW; ++nt) mma16816(add[piece][nt], kt, b[piece][2 * nt], b[piece][2 * nt + 1]);
       }
-      const float total = st.total.x;
+      const float total = st.rec.total.x;
 #pragma unroll
       for (int nt = 0; nt < NTW; ++nt)
 #pragma unroll
@@ -782,12 +793,12 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
       publish();
     } else {
       float own[4];
-      triangular(st.p, sm.u, own);
+      triangular(st.rec.p, sm.u, own);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int r = row + qr + 8 * j;
         if (c * kChunk + r < n_tok) {
-          const float grown = st.sc[r].z;
+          const float grown = st.rec.sc[r].z;
           const float2 o = make_float2(fmaf(grown, from_state[2 * j], own[2 * j]), fmaf(grown, from_state[2 * j + 1], own[2 * j + 1]));
           probe = fmaf(o.x, 0.f, fmaf(o.y, 0.f, probe));
           *reinterpret_cast<float2*>(out + ((size_t)(start + c * kChunk + r) * H + h) * dv + p0 + col + 2 * qc) = o;
@@ -877,7 +888,7 @@ ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, i
     auto kern = d == 64 ? delta_chunk_kernel<64> : delta_chunk_kernel<128>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "delta_scan: %s", cudaGetErrorString(e));
-    launch_chained(kern, dim3(H, n_seqs, dv / kChunkCols), dim3(kChunkWarps * 32), bytes, (cudaStream_t)stream, (const elem_t*)qkv,
+    launch_chained(kern, dim3(H, n_seqs, dv / kChunkCols), dim3((kChunkWarps + kCopyWarps) * 32), bytes, (cudaStream_t)stream, (const elem_t*)qkv,
                    channels, records, state, seq_starts, state_slots, out, H, G, dv, (const elem_t*)proj, ld, off_b, off_a, dt_bias, a_log,
                    1.f / sqrtf((float)d));
     if ((rc = check_launch("delta_chunk")) || n_seqs == 1) return rc;

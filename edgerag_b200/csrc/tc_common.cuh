@@ -191,9 +191,6 @@ __device__ __forceinline__ bool named_barrier_any(int id, int count, bool pred) 
       : "memory");
   return any != 0;
 }
-__device__ __forceinline__ void named_barrier(int id, int count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
 
 // A TMA tensor copy of `box rows` whole rows (64 bfloat16 each) starting at `row` of a page pool.
 __device__ __forceinline__ void tma_load_rows(uint32_t dst, const CUtensorMap* map, int row, uint32_t bar) {
