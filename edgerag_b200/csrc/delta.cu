@@ -30,6 +30,7 @@
 #include "common.cuh"
 #if ERB_ELEM == 1
 #include "mma_split.cuh"
+#include "tc_common.cuh"
 #endif
 
 using namespace erb;
@@ -335,22 +336,28 @@ head_norm_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ gat
 //     o_t = exp(c_t) S^T q_t + sum_{s <= t} exp(c_t - c_s) (q_t . k_s) u_s
 //     S  <- exp(c_64) S + sum_s exp(c_64 - c_s) k_s u_s^T
 // The first line is a triangular system (I + A) U = R whose matrix does not depend on the state: a first kernel, parallel over
-// (chunk, head), makes T = (I + A)^-1 in float and the weights of the second line; the second kernel, parallel over (request,
-// head, 16 columns of values), walks the chunks with products of matrices alone.  The raw queries and keys are bfloat16 as they
-// are (their lengths are factors of rows and columns); every other operand goes in as three bfloat16 pieces (mma_split.cuh), so
-// that nothing is rounded to 16 bits.  c is summed in double and kept as two floats.
+// (chunk, head), makes T = (I + A)^-1 in float and P T, with P the weights of the second line, so that U = T R and P U = (P T) R come from R side by
+// side; the second kernel, parallel over (request, head, 16 columns of values), walks the chunks with products of matrices alone.  The raw
+// queries and keys are bfloat16 as they are (their lengths are factors of rows and columns); every other operand goes in as three bfloat16
+// pieces (mma_split.cuh), so that nothing is rounded to 16 bits.  c is summed in double and kept as two floats.
 //
-// What bounds it: the three dependent phases of a chunk, and the 64 KB of operands a block reads of it, which four warps bring that do
+// The product of a chunk's 128 rows of keys and queries with the state is tcgen05's, its sums in TMEM (two, over half of a row's entries each: the unit
+// cuts its sums); the triangular ones and the state's are mma.sync.  What bounds it: the three dependent phases of a chunk, 4,500 clocks
+// (700 the first product, 1,100 R, 900 U, 1,700 the state), and the 64 KB of operands a block reads of it, which four warps bring that do
 // nothing else.  The walk takes 0.46 us a token (2,048 tokens of 16 heads of 128 x 128: 971 us with its preparing); both kernels of the chunks
-// 115.6 us (143.6 us while the warps that make the products also asked for the copies, 2,300 of a chunk's 6,200 clocks, and the first kernel
-// made its roots one after the other).  Error against float64: 1.7e-7, as the walk's.
-constexpr int kChunk = 64, kChunkCols = 16, kChunkWarps = 16, kCopyWarps = 4, kChunkPrepWarps = 8;
+// 105.7 us (27 of it the first); 115.6 us with all products by mma.sync and o from U, 143.6 us while the warps that make the products also asked
+// for the copies, 2,300 of a chunk's 6,200 clocks, and the first kernel made its roots one after the other.  (All products by tcgen05: 104.7 us, and the
+// state a twentieth further from float64.)  Error against float64: o 1.6e-7, the state 1.0e-7, not above the walk's.
+//
+// Every wait for a product is bounded; a thread that gives up raises a block-wide flag, all warps still come to the barriers of the remaining
+// chunks, the block records 8000000 in *status, frees its TMEM and returns.
+constexpr int kChunk = 64, kChunkCols = 16, kChunkWarps = 16, kCopyWarps = 4, kIssueWarp = 15, kChunkPrepWarps = 8;
 constexpr int kPieceElems = kChunk * kChunk;
 
-// What the first kernel leaves of one (chunk, head): the weights of the second line and T, each as three pieces [64][64] (laid
+// What the first kernel leaves of one (chunk, head): P T and T, each as three pieces [64][64] (laid
 // out as shared memory has them; tiles of 16 x 16 above the diagonal are not written), per token (beta, exp(c) / |k|, exp(c) / |q|, exp(c_64 - c) / |k|), exp(c_64).
 struct ChunkRecord {
-  __nv_bfloat16 p[3][kPieceElems];
+  __nv_bfloat16 pt[3][kPieceElems];
   __nv_bfloat16 t[3][kPieceElems];
   float4 sc[kChunk];
   float4 total;
@@ -372,6 +379,16 @@ __device__ __forceinline__ int chunks_before(const int* seq_starts, int seq) {
   return n;
 }
 
+// The products of two operands in three pieces each that matter, sums by their size.
+__device__ __forceinline__ void six_products(float (&acc)[3][4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
+  mma16816(acc[0], a[0], b[0][0], b[0][1]);
+  mma16816(acc[1], a[0], b[1][0], b[1][1]);
+  mma16816(acc[2], a[0], b[2][0], b[2][1]);
+  mma16816(acc[1], a[1], b[0][0], b[0][1]);
+  mma16816(acc[2], a[1], b[1][0], b[1][1]);
+  mma16816(acc[2], a[2], b[0][0], b[0][1]);
+}
+
 template <int D>
 struct DeltaPrepSmem {
   __nv_bfloat16 k[kChunk][D + 8], q[kChunk][D + 8];
@@ -379,6 +396,8 @@ struct DeltaPrepSmem {
   float x[3][16][17];
   float beta[kChunk], ik[kChunk], iq[kChunk], hi[kChunk], lo[kChunk], grown[kChunk], left[kChunk];
   double sums[2];
+  alignas(16) __nv_bfloat16 p[3][kChunk][kChunk + 8];          // P in pieces
+  alignas(16) __nv_bfloat16 t[D < 128 ? 3 : 1][kChunk][kChunk + 8];      // T in pieces (keys of 128: in the place of k and q)
 };
 
 template <int D>
@@ -502,7 +521,7 @@ delta_chunk_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, 
           uint32_t piece[3];
           split_pair(v[0], v[1], piece);
 #pragma unroll
-          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&rec.p[k][entry(r, s)]) = piece[k];
+          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&sm.p[k][r][s]) = piece[k];
         } else {
           a_s[r][s] = v[0];
           a_s[r][s + 1] = v[1];
@@ -571,6 +590,8 @@ delta_chunk_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, 
     }
   }
   __syncthreads();
+  static_assert(sizeof(sm.p) <= sizeof(sm.k) + sizeof(sm.q) || D < 128, "T's pieces take the keys' and queries' place");
+  __nv_bfloat16 (*t_s)[kChunk][kChunk + 8] = D < 128 ? sm.t : reinterpret_cast<__nv_bfloat16 (*)[kChunk][kChunk + 8]>(&ks[0][0]);
   for (int idx = threadIdx.x; idx < kPieceElems / 4; idx += blockDim.x) {
     const int r = idx / (kChunk / 4), e = 4 * (idx % (kChunk / 4));
     if (e >= 16 * (r / 16 + 1)) continue;
@@ -579,44 +600,81 @@ delta_chunk_prepare_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, 
     split_pair(v.x, v.y, p01);
     split_pair(v.z, v.w, p23);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(&rec.t[k][entry(r, e)]) = make_uint2(p01[k], p23[k]);
+    for (int k = 0; k < 3; ++k) {
+      *reinterpret_cast<uint2*>(&rec.t[k][entry(r, e)]) = make_uint2(p01[k], p23[k]);
+      *reinterpret_cast<uint2*>(&t_s[k][r][e]) = make_uint2(p01[k], p23[k]);
+    }
+  }
+  __syncthreads();
+  // P T, 16 x 8 at a time on and below the diagonal's tiles, the six products of pieces that matter
+  for (int item = warp; item < 20; item += kChunkPrepWarps) {
+    const int tile = item >> 1, tr = tile < 1 ? 0 : tile < 3 ? 1 : tile < 6 ? 2 : 3;
+    const int row = 16 * tr, first = 16 * (tile - tr * (tr + 1) / 2), col = first + 8 * (item & 1);
+    float acc[3][4] = {};
+    for (int k = first; k <= row; k += 16) {
+      uint32_t a[3][4], b[3][2];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        ldmatrix4(a[i], &sm.p[i][row + (lane & 15)][k + 8 * (lane >> 4)]);
+        ldmatrix2t(b[i], &t_s[i][k + (lane & 15)][col]);
+      }
+      six_products(acc, a, b);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      uint32_t piece[3];
+      split_pair((acc[2][2 * j] + acc[1][2 * j]) + acc[0][2 * j], (acc[2][2 * j + 1] + acc[1][2 * j + 1]) + acc[0][2 * j + 1], piece);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&rec.pt[k][entry(row + qr + 8 * j, col + 2 * qc)]) = piece[k];
+    }
   }
 }
 
 // grid (H, requests, columns / 16).  Phases of a chunk, a barrier after each:
-//   1  warps 0-7: R = beta (v - exp(c) S^T k), a 16 x 8 tile each;  warps 8-15: S^T q, kept in registers
-//   2  warps 0-7: U = T R, and U as the state will take it;  warps 8-15 wait
-//   3  warps 0-7: the state, in accumulators (D / 16 tiles of 16 keys);  warps 8-15: o
+//   1  S^T k and S^T q, one product of 128 rows; R = beta (v - exp(c) S^T k), exp(c) S^T q
+//   2  warps 0-7: U = T R, as the state will take it;  warps 8-15: o = (P T) R + exp(c) S^T q
+//   3  the state, in accumulators (a tile of 16 keys x 8 values a warp)
 // Four more warps copy the next chunk's operands meanwhile.
 //
 // The products are causal for finite numbers only: above the diagonal T and the weights are zeros, and 0 * inf is no number; nor are
 // the pieces of an infinity, or the differences of c where a decay is exactly zero.  Whatever is not finite makes an o of its own
 // token or the last state not finite, so both are looked at (one multiplication an output), and a block that finds one walks its
 // portion once more from the state as it was, with the bits of delta_scan_kernel.  (2,048 tokens of 16 heads of 128 x 128, both
-// kernels: 142.5 us without the look, 143.7 us with it.)
+// kernels: 142.5 us without the look, 143.7 us with it, before the steps above.)
 template <int D>
 struct DeltaChunkSmem {
-  static constexpr int LdD = D + 8, LdC = kChunkCols + 8;      // rows 16 bytes longer than a power of two: no bank conflicts
-  struct Stage {
-    __nv_bfloat16 k[kChunk][LdD];
-    __nv_bfloat16 q[kChunk][LdD];
+  static constexpr int LdC = kChunkCols + 8;                   // rows 16 bytes longer than a power of two: no bank conflicts
+  struct alignas(1024) Stage {
+    __nv_bfloat16 kq[D / 64][2 * kChunk][64];                  // the keys' rows, then the queries', 64 entries at a time; 128-byte swizzle
     __nv_bfloat16 v[kChunk][LdC];
     ChunkRecord rec;
   } stage[2];
-  __nv_bfloat16 s[3][D][LdC];                                  // the state before the chunk, in pieces
+  // the state before the chunk, a row per key: of 4 columns the three pieces and 4 entries of nothing, then the next 4; 128-byte swizzle
+  __nv_bfloat16 s[D][64];
   __nv_bfloat16 r[3][kChunk][LdC];
-  __nv_bfloat16 u[3][kChunk][LdC];
   __nv_bfloat16 w[3][kChunk][LdC];                             // exp(c_64 - c) / |k| u
+  alignas(16) float qs[kChunk][kChunkCols + 4];                // exp(c) / |q| S^T q
+  uint64_t bar;                                                // the products with the state are there
+  int abort;
+  uint32_t tmem;
 };
+static_assert(sizeof(DeltaChunkSmem<128>::Stage) % 1024 == 0 && offsetof(DeltaChunkSmem<128>, s) % 1024 == 0 && offsetof(DeltaChunkSmem<64>, s) % 1024 == 0 &&
+                  offsetof(DeltaChunkSmem<128>, r) % 16 == 0 && offsetof(DeltaChunkSmem<128>, qs) % 16 == 0 && offsetof(DeltaChunkSmem<64>, qs) % 16 == 0 &&
+                  offsetof(DeltaChunkSmem<128>, bar) % 8 == 0 && offsetof(DeltaChunkSmem<64>, bar) % 8 == 0 &&
+                  offsetof(DeltaChunkSmem<128>::Stage, v) % 16 == 0 && offsetof(DeltaChunkSmem<128>::Stage, rec) % 16 == 0 &&
+                  offsetof(DeltaChunkSmem<64>::Stage, rec) % 16 == 0 && sizeof(DeltaChunkSmem<128>) + 1024 <= 232448, "tiles start where their swizzle does");
+// entry `col` (under 64) of row `row` in a tile of 128-byte rows with the 128-byte swizzle
+__device__ __forceinline__ int swizzled(int row, int col) { return (((col >> 3) ^ (row & 7)) << 3) + (col & 7); }
 
 template <int D>
 __global__ void __launch_bounds__((kChunkWarps + kCopyWarps) * 32)
 delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const ChunkRecord* __restrict__ records, float* __restrict__ state,
                    const int* __restrict__ seq_starts, const int* __restrict__ state_slots, float* __restrict__ out, int H, int G, int dv,
                    const __nv_bfloat16* __restrict__ proj, int ld, int off_b, int off_a, const float* __restrict__ dt_bias,
-                   const float* __restrict__ a_log, float q_scale) {
+                   const float* __restrict__ a_log, float q_scale, int* __restrict__ status) {
   chain_wait();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_all[];
+  unsigned char* smem_raw = smem_all + ((1024u - (smem_u32(smem_all) & 1023u)) & 1023u);
   typedef DeltaChunkSmem<D> Smem;
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int h = blockIdx.x, seq = blockIdx.y, p0 = blockIdx.z * kChunkCols, kh = h / (H / G);
@@ -626,6 +684,21 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
   const int n_chunks = (n_tok + kChunk - 1) / kChunk;
   const ChunkRecord* rec0 = records + (size_t)chunks_before(seq_starts, seq) * H + h;
   const __nv_bfloat16* rows = qkv + (size_t)start * channels;
+  volatile int* abort_flag = &sm.abort;
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&sm.bar), 1);
+    sm.abort = 0;
+    mbar_init_fence();
+  }
+  if (warp == kIssueWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)), "r"(128) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem, 0);
+  constexpr int kColHalf = 64;                                 // columns of TMEM: three pieces' sums over the first half of the keys; over the others
 
   if (warp >= kChunkWarps) {                                   // the copies: a chunk's operands while the one before is worked on
     const int t = threadIdx.x - kChunkWarps * 32;
@@ -647,8 +720,8 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
       for (int i = 0; i < kChunk / kRows; ++i) {
         const int r = r0 + kRows * i;
         const __nv_bfloat16* row = src + (size_t)(r < left ? r : 0) * channels + kh * D + e0;
-        copy16_or_zero(&st.q[r][e0], row, r < left);
-        copy16_or_zero(&st.k[r][e0], row + G * D, r < left);
+        copy16_or_zero(&st.kq[e0 >> 6][kChunk + r][swizzled(r, e0 & 63)], row, r < left);
+        copy16_or_zero(&st.kq[e0 >> 6][r][swizzled(r, e0 & 63)], row + G * D, r < left);
       }
       {
         const int r = t >> 1, e = 8 * (t & 1);
@@ -659,38 +732,35 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
         if (at[i] >= 0)
 #pragma unroll
           for (int k = 0; k < 3; ++k) {
-            copy16_or_zero(&st.rec.p[k][at[i]], &rec->p[k][at[i]], true);
+            copy16_or_zero(&st.rec.pt[k][at[i]], &rec->pt[k][at[i]], true);
             copy16_or_zero(&st.rec.t[k][at[i]], &rec->t[k][at[i]], true);
           }
       if (t < kChunk) copy16_or_zero(&st.rec.sc[t], &rec->sc[t], true);
       else if (t == kChunk) copy16_or_zero(&st.rec.total, &rec->total, true);
       copy_commit();
       copy_wait<0>();
+      fence_async_proxy();
       __syncthreads();                                         // (a chunk's first barrier)
     }
   }
-  // the state (stored [values][keys]): warp w < 8 holds keys 16 (w mod D/16) .. + 15, values 8 NTW (w div D/16) .. + 8 NTW - 1
-  constexpr int kRowTiles = D / 16, NTW = kRowTiles / 4;
-  const int s_row = 16 * (warp % kRowTiles), s_col = 8 * NTW * (warp / kRowTiles);
-  float S[NTW][4];
+  // the state (stored [values][keys]): warp w holds keys 16 (w mod D/16) .. + 15, values 8 (w div D/16) .. + 7
+  constexpr int kStateWarps = D / 8;
+  const int s_row = 16 * (warp % (D / 16)), s_col = 8 * (warp / (D / 16));
+  float S[4];
   float* s_glob = state + (((size_t)state_slots[seq] * H + h) * dv + p0) * D;
   auto publish = [&]() {
 #pragma unroll
-    for (int nt = 0; nt < NTW; ++nt)
+    for (int j = 0; j < 2; ++j) {
+      uint32_t piece[3];
+      split_pair(S[2 * j], S[2 * j + 1], piece);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        uint32_t piece[3];
-        split_pair(S[nt][2 * j], S[nt][2 * j + 1], piece);
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-          *reinterpret_cast<uint32_t*>(&sm.s[k][s_row + qr + 8 * j][s_col + 8 * nt + 2 * qc]) = piece[k];
-      }
+      for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&sm.s[s_row + qr + 8 * j][swizzled(qr, 4 * ((s_col + 2 * qc) & ~3) + 4 * k + (2 * qc & 3))]) = piece[k];
+    }
+    fence_async_proxy();
   };
-  if (warp < 8) {
+  if (warp < kStateWarps) {
 #pragma unroll
-    for (int nt = 0; nt < NTW; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) S[nt][i] = s_glob[(size_t)(s_col + 8 * nt + 2 * qc + (i & 1)) * D + s_row + qr + 8 * (i >> 1)];
+    for (int i = 0; i < 4; ++i) S[i] = s_glob[(size_t)(s_col + 2 * qc + (i & 1)) * D + s_row + qr + 8 * (i >> 1)];
     publish();
   }
   const int row = 16 * ((warp & 7) >> 1), col = 8 * (warp & 1);       // a warp's tile of R, U and o
@@ -705,12 +775,7 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
         ldmatrix4(a[i], &m[i][entry(r, 8 * e)]);
         ldmatrix2t(b[i], &x[i][k + (lane & 15)][col]);
       }
-      mma16816(acc[0], a[0], b[0][0], b[0][1]);
-      mma16816(acc[1], a[0], b[1][0], b[1][1]);
-      mma16816(acc[2], a[0], b[2][0], b[2][1]);
-      mma16816(acc[1], a[1], b[0][0], b[0][1]);
-      mma16816(acc[2], a[1], b[1][0], b[1][1]);
-      mma16816(acc[2], a[2], b[0][0], b[0][1]);
+      six_products(acc, a, b);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) result[i] = (acc[2][i] + acc[1][i]) + acc[0][i];
@@ -719,38 +784,44 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
   for (int c = 0; c < n_chunks && warp < kChunkWarps; ++c) {
     typename Smem::Stage& st = sm.stage[c & 1];
     __syncthreads();                                           // chunk c's operands and the state's pieces are there
-    float from_state[4];                                       // 16 x 8 of k S (warps 0-7) or q S, rows as they came
+    if (warp == kIssueWarp) {                                  // S^T of keys and queries, rows as they came: the whole warp, one elected lane issues
+      constexpr uint32_t kIdesc = mma_idesc(2 * kChunk, 64, true);
+      const uint64_t da = make_desc(smem_u32(&st.kq[0][0][0])), db = make_desc(smem_u32(&sm.s[0][0]));
+      fence_after_sync();
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k)
+          mma_bf16(tmem + (k / (D / 32)) * kColHalf, da + (k >> 2) * (2 * kChunk * 128 >> 4) + 2 * (k & 3), db + k * (16 * 128 >> 4), kIdesc, k % (D / 32) > 0);
+        mma_commit(smem_u32(&sm.bar));
+      }
+      __syncwarp();
+    }
+    mbar_wait_or_abort(smem_u32(&sm.bar), c & 1, abort_flag);
+    __syncwarp();
+    fence_after_sync();
     {
-      float acc[3][4] = {};
-      const __nv_bfloat16 (*m)[Smem::LdD] = warp < 8 ? st.k : st.q;
+      // a thread: row 32 (warp mod 4) + lane, keys' rows first; columns 4 (warp div 4) .. + 3
+      const int quad = warp & 3, t = 32 * (quad & 1) + lane, first = 4 * (warp >> 2);
+      float sum[4], low[16], high[16];
+      tmem_ld16(tmem + ((uint32_t)(32 * quad) << 16) + 4 * first, low);
+      tmem_ld16(tmem + ((uint32_t)(32 * quad) << 16) + kColHalf + 4 * first, high);
+      tmem_ld_wait();
+      fence_before_sync();
 #pragma unroll
-      for (int k = 0; k < D / 16; k += 2) {
-        uint32_t a[2][4], b[3][4];
+      for (int i = 0; i < 4; ++i) sum[i] = ((low[8 + i] + high[8 + i]) + (low[4 + i] + high[4 + i])) + (low[i] + high[i]);
+      const float4 sc = st.rec.sc[t];
+      if (quad < 2) {
+        const uint2 in = *reinterpret_cast<const uint2*>(&st.v[t][first]);
+        uint32_t p01[3], p23[3];
+        split_pair(sc.x * fmaf(-sc.y, sum[0], __uint_as_float(in.x << 16)), sc.x * fmaf(-sc.y, sum[1], __uint_as_float(in.x & 0xffff0000u)), p01);
+        split_pair(sc.x * fmaf(-sc.y, sum[2], __uint_as_float(in.y << 16)), sc.x * fmaf(-sc.y, sum[3], __uint_as_float(in.y & 0xffff0000u)), p23);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) ldmatrix4(a[i], &m[row + (lane & 15)][16 * (k + i) + 8 * (lane >> 4)]);
-#pragma unroll
-        for (int piece = 0; piece < 3; ++piece) ldmatrix4t(b[piece], &sm.s[piece][16 * k + lane][col]);
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int piece = 0; piece < 3; ++piece) mma16816(acc[piece], a[i], b[piece][2 * i], b[piece][2 * i + 1]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) from_state[i] = (acc[2][i] + acc[1][i]) + acc[0][i];
-    }
-    if (warp < 8) {
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int r = row + qr + 8 * j;
-        const float4 sc = st.rec.sc[r];
-        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.v[r][col + 2 * qc]));
-        uint32_t piece[3];
-        split_pair(sc.x * fmaf(-sc.y, from_state[2 * j], v.x), sc.x * fmaf(-sc.y, from_state[2 * j + 1], v.y), piece);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&sm.r[k][r][col + 2 * qc]) = piece[k];
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(&sm.r[k][t][first]) = make_uint2(p01[k], p23[k]);
+      } else {
+        *reinterpret_cast<float4*>(&sm.qs[t][first]) = make_float4(sc.z * sum[0], sc.z * sum[1], sc.z * sum[2], sc.z * sum[3]);
       }
     }
-    named_barrier(1, kChunkWarps * 32);                        // R is there; the state's pieces have been read
+    named_barrier(1, kChunkWarps * 32);                        // R is there
     if (warp < 8) {
       float u[4];
       triangular(st.rec.t, sm.r, u);
@@ -758,61 +829,58 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
       for (int j = 0; j < 2; ++j) {
         const int r = row + qr + 8 * j;
         const float left = st.rec.sc[r].w;
-        uint32_t piece[3], weighted[3];
-        split_pair(u[2 * j], u[2 * j + 1], piece);
+        uint32_t weighted[3];
         split_pair(left * u[2 * j], left * u[2 * j + 1], weighted);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          *reinterpret_cast<uint32_t*>(&sm.u[k][r][col + 2 * qc]) = piece[k];
-          *reinterpret_cast<uint32_t*>(&sm.w[k][r][col + 2 * qc]) = weighted[k];
-        }
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&sm.w[k][r][col + 2 * qc]) = weighted[k];
       }
-    }
-    named_barrier(1, kChunkWarps * 32);                        // U is there
-    if (warp < 8) {
-      float add[3][NTW][4] = {};
-#pragma unroll
-      for (int k = 0; k < kChunk / 16; ++k) {
-        uint32_t kt[4], b[3][4];                               // K^T: 16 keys x 16 tokens
-        ldmatrix4t(kt, &st.k[16 * k + (lane & 7) + 8 * (lane >> 4)][s_row + 8 * ((lane >> 3) & 1)]);
-#pragma unroll
-        for (int piece = 0; piece < 3; ++piece) {
-          if (NTW == 2) ldmatrix4t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col + 8 * (lane >> 4)]);
-          else ldmatrix2t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col]);
-        }
-#pragma unroll
-        for (int piece = 0; piece < 3; ++piece)
-#pragma unroll
-          for (int nt = 0; nt < NTW; ++nt) mma16816(add[piece][nt], kt, b[piece][2 * nt], b[piece][2 * nt + 1]);
-      }
-      const float total = st.rec.total.x;
-#pragma unroll
-      for (int nt = 0; nt < NTW; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) S[nt][i] = fmaf(total, S[nt][i], (add[2][nt][i] + add[1][nt][i]) + add[0][nt][i]);
-      publish();
     } else {
       float own[4];
-      triangular(st.rec.p, sm.u, own);
+      triangular(st.rec.pt, sm.r, own);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int r = row + qr + 8 * j;
         if (c * kChunk + r < n_tok) {
-          const float grown = st.rec.sc[r].z;
-          const float2 o = make_float2(fmaf(grown, from_state[2 * j], own[2 * j]), fmaf(grown, from_state[2 * j + 1], own[2 * j + 1]));
+          const float2 q = *reinterpret_cast<const float2*>(&sm.qs[r][col + 2 * qc]);
+          const float2 o = make_float2(q.x + own[2 * j], q.y + own[2 * j + 1]);
           probe = fmaf(o.x, 0.f, fmaf(o.y, 0.f, probe));
           *reinterpret_cast<float2*>(out + ((size_t)(start + c * kChunk + r) * H + h) * dv + p0 + col + 2 * qc) = o;
         }
       }
     }
-  }
-  if (warp < 8) {
+    named_barrier(1, kChunkWarps * 32);                        // U is there
+    if (warp < kStateWarps) {
+      float add[3][4] = {};
 #pragma unroll
-    for (int nt = 0; nt < NTW; ++nt)
+      for (int k = 0; k < kChunk / 16; ++k) {
+        uint32_t kt[4], b[3][2];                               // K^T: 16 keys x 16 tokens
+        const int e = s_row + 8 * ((lane >> 3) & 1);
+        ldmatrix4t(kt, &st.kq[e >> 6][16 * k + (lane & 7) + 8 * (lane >> 4)][swizzled(lane, e & 63)]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) probe = fmaf(S[nt][i], 0.f, probe);
+        for (int piece = 0; piece < 3; ++piece) {
+          ldmatrix2t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col]);
+          mma16816(add[piece], kt, b[piece][0], b[piece][1]);
+        }
+      }
+      const float total = st.rec.total.x;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) S[i] = fmaf(total, S[i], (add[2][i] + add[1][i]) + add[0][i]);
+      publish();
+    }
   }
-  if (__syncthreads_or(!(probe == 0.f))) {
+  if (warp < kStateWarps) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) probe = fmaf(S[i], 0.f, probe);
+  }
+  const bool odd = __syncthreads_or(!(probe == 0.f)), gave_up = *abort_flag != 0;
+  if (gave_up && threadIdx.x == 0 && status) atomicCAS(status, 0, 8000000);
+  __syncthreads();
+  if (warp == kIssueWarp) {
+    fence_after_sync();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128) : "memory");
+  }
+  if (gave_up) return;
+  if (odd) {
     static_assert(2 * kDeltaChunk * (2 * D + kChunkCols + 4) * sizeof(float) <= sizeof(Smem) && D / 16 * kChunkCols <= kChunkWarps * 32, "the walk has room");
     auto prepared = [&](int c0, int nc, float* qk_s, float* v_s, float* sc_s) {      // what `prepare` makes of a token, a warp each
       for (int t = warp; t < nc; t += kChunkWarps) {
@@ -826,11 +894,9 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
     walk_tokens<D / 16, true>(reinterpret_cast<float*>(smem_raw), prepared, state, seq_starts, state_slots, out, H, D, dv, kChunkCols, h, seq, p0);
     return;
   }
-  if (warp < 8) {
+  if (warp < kStateWarps) {
 #pragma unroll
-    for (int nt = 0; nt < NTW; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) s_glob[(size_t)(s_col + 8 * nt + 2 * qc + (i & 1)) * D + s_row + qr + 8 * (i >> 1)] = S[nt][i];
+    for (int i = 0; i < 4; ++i) s_glob[(size_t)(s_col + 2 * qc + (i & 1)) * D + s_row + qr + 8 * (i >> 1)] = S[i];
   }
 }
 
@@ -842,19 +908,20 @@ inline long long chunk_scratch_floats(int n_tokens, int n_seqs, int H, int G, in
   return chunk_records(n_tokens, n_seqs, H) * (long long)(sizeof(ChunkRecord) / 4) + (long long)delta_scratch_floats(n_seqs, H, G, d, dv);
 }
 
-// Whether the chunks are the faster form: both costs in microseconds, fitted to the times of 1 to 64 requests of 2 to 500 tokens
+// Whether the chunks are the faster form: both costs in microseconds, fitted to the times of 1 to 64 requests of 16 to 2,048 tokens
 // (4 to 16 heads of 64 x 48 and 128 x 128).  The walk is taken for 0.49 us a token of the longest portion (0.46 now) or, when the GPU is full,
-// its blocks' tokens and states; the chunks cost two more launches, 3.7 us a chunk of the longest portion or, when the GPU is
-// full, a share of an SM for every chunk, be it full or not, and requests of one token are then walked by themselves.  One
-// request: from 34 tokens on (8 heads of 128 x 128: 28 tokens 16.3 us walked, 20.0 in a chunk; 32 17.3 | 20.0; 36 18.8 | 20.1;
-// 44 21.3 | 20.1); 32 requests of equal length: from about 50.
+// its blocks' tokens and states; the chunks cost two more launches, 2.8 us a chunk of the longest portion or as many rounds of blocks as
+// the SMs need, a block an SM, and requests of one token are then walked by themselves.  Of 297 layouts three of 36 and 44 tokens get chunks
+// where the walk is faster, by 3.2 us at most.  One request: from 34 tokens on (16 heads of 128 x 128: 28 tokens 18.7 us walked, 17.4 in a chunk;
+// 36 21.5 | 17.2; 4 of 64 x 48: 36 14.5 | 15.5); 32 requests of equal length: from about 65.
 inline bool chunks_pay(int blocks, int n_tokens, int n_seqs, int longest) {
   if (longest < 34) return false;
   const double extra = (double)n_tokens - n_seqs - (longest - 1);      // tokens beyond one of the other requests
   const double others = fmax(0.0, fmin(extra, n_seqs - 1.0)), singles = n_seqs - 1.0 - others;
   const double own = (longest + 63) / 64, chunks = own + (others > 0.0 ? others + extra / 64.0 : 0.0);
   const double walk = fmax(6.0 + 0.49 * longest, blocks * (0.00086 * n_tokens + 0.0024 * n_seqs));
-  return 15.0 + fmax(3.7 * own, 0.0384 * blocks * chunks) + 0.003 * blocks * singles < walk;
+  const double rounds = ceil(blocks * (1.0 + others) / sm_count());
+  return fmax(14.5 + 2.8 * own, 4.0 + rounds * (4.0 + 2.2 * chunks / (1.0 + others))) + 0.003 * blocks * singles < walk;
 }
 #endif  // ERB_ELEM == 1
 
@@ -863,7 +930,7 @@ inline bool chunks_pay(int blocks, int n_tokens, int n_seqs, int longest) {
 ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, int ld, int off_b, int off_a,
                               const float* dt_bias, const float* a_log, float* state, const int* seq_starts,
                               const int* state_slots, float* out, float* scratch, long long scratch_floats, int n_seqs, int n_tokens,
-                              int longest, int H, int G, int d, int dv, void* stream) {
+                              int longest, int H, int G, int d, int dv, int* status, void* stream) {
   if (n_seqs <= 0 || n_tokens <= 0) return ERB_OK;
   if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 || d > 32 * kDeltaRows)
     return fail(ERB_ERR_ARG, "delta_scan: bad sizes (%d heads over %d, keys of %d up to %d)", H, G, d, 32 * kDeltaRows);
@@ -884,13 +951,13 @@ ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, i
                    channels, (const elem_t*)proj, ld, off_b, off_a, dt_bias, a_log, seq_starts, n_seqs, records, H, G, 1.f / sqrtf((float)d));
     int rc = check_launch("delta_chunk_prepare");
     if (rc) return rc;
-    const size_t bytes = d == 64 ? sizeof(DeltaChunkSmem<64>) : sizeof(DeltaChunkSmem<128>);
+    const size_t bytes = 1024 + (d == 64 ? sizeof(DeltaChunkSmem<64>) : sizeof(DeltaChunkSmem<128>));
     auto kern = d == 64 ? delta_chunk_kernel<64> : delta_chunk_kernel<128>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "delta_scan: %s", cudaGetErrorString(e));
     launch_chained(kern, dim3(H, n_seqs, dv / kChunkCols), dim3((kChunkWarps + kCopyWarps) * 32), bytes, (cudaStream_t)stream, (const elem_t*)qkv,
                    channels, records, state, seq_starts, state_slots, out, H, G, dv, (const elem_t*)proj, ld, off_b, off_a, dt_bias, a_log,
-                   1.f / sqrtf((float)d));
+                   1.f / sqrtf((float)d), status);
     if ((rc = check_launch("delta_chunk")) || n_seqs == 1) return rc;
     singles = true;
     walk_tokens = n_seqs;

@@ -429,7 +429,7 @@ class ModelRunner:
             if code >= 1000000:
                 raise StepError(f"an attention kernel gave up (code {code}: 1xxxxxx prefill wait, 2xxxxxx decode wait, 3000000 shared-memory "
                                 "alignment, 4xxxxxx a wait of a product for few rows, 5xxxxxx of the experts' products, 7000000 of the "
-                                "state-space chunks); the step's results are not valid")
+                                "state-space chunks, 8000000 of the delta rule's); the step's results are not valid")
             raise StepError(f"a kernel flagged token {code - 1} of the batch (id or row out of range)")
 
     def drop_graphs(self) -> None:

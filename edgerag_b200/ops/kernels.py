@@ -130,7 +130,7 @@ _SIGNATURES = {
                            c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                            c_void_p, c_void_p, c_int, c_int, c_void_p],
     "erb_delta_scan": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                       c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                       c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "erb_head_norm_gate": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
     "erb_moe_route": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p],
@@ -1556,7 +1556,8 @@ def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt
     _call(_fn("delta", _elem(qkv), "erb_delta_scan"), qkv, qkv.shape[1], proj,
           proj.stride(0) if n > 1 else proj.shape[1], int(off_b), int(off_a), dt_bias, a_log,
           state, seq_starts, state_slots, out, scratch, scratch.numel(), int(n_seqs), n,
-          n - int(n_seqs) + 1 if longest is None else int(longest), heads, int(n_key_heads), d, vdim, _stream())
+          n - int(n_seqs) + 1 if longest is None else int(longest), heads, int(n_key_heads), d, vdim,
+          _status_word, _stream())
 
 
 def head_norm_gate(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, n_heads: int, eps: float) -> None:
