@@ -477,7 +477,7 @@ struct ChunkSmem {
   float fall[2][kChunk], rise[2][3][kChunk];                   // exp(c_t - c_r), r the last token before t's 32; dt_s exp(c_r - c_s) for the later 32s' r
   alignas(16) float out[kChunk][kChunkCols + 4];               // a chunk's y on its way to whole lines
   double decay[kStepWarps];                                    // of 32 tokens each
-  uint64_t bars[11];
+  uint64_t bars[12];
   int abort;
   uint32_t tmem;
 };
@@ -528,12 +528,12 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_chunks = (n_tok + kChunk - 1) / kChunk;
   // G there; the weights' pieces of the chunk's first and last 64 tokens; the weighted x's; dS there; Y there; the state's pieces; a stage's rows
-  // (two); the outputs of the chunk before read; those stored and the next chunk's steps there
-  constexpr int kBarG = 0, kBarP1 = 1, kBarP2 = 2, kBarW = 3, kBarD = 4, kBarY = 5, kBarS = 6, kBarL = 7, kBarR = 9, kBarT = 10;
+  // (two); the outputs of the chunk before read; those stored and the next chunk's steps there; the first half of Y1 there
+  constexpr int kBarG = 0, kBarP1 = 1, kBarP2 = 2, kBarW = 3, kBarD = 4, kBarY = 5, kBarS = 6, kBarL = 7, kBarR = 9, kBarT = 10, kBarH = 11;
   auto bar = [&](int which) { return smem_u32(&sm.bars[which]); };
   volatile int* abort_flag = &sm.abort;
   if (threadIdx.x == 0) {
-    for (int i : {kBarG, kBarD, kBarY, kBarL, kBarL + 1, kBarR}) mbar_init(bar(i), 1);
+    for (int i : {kBarG, kBarD, kBarY, kBarL, kBarL + 1, kBarR, kBarH}) mbar_init(bar(i), 1);
     mbar_init(bar(kBarT), kStepWarps);
     for (int i : {kBarP1, kBarP2, kBarW, kBarS}) mbar_init(bar(i), kChunkWarps);
     sm.abort = 0;
@@ -795,13 +795,9 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
         for (int k = 0; k < kChunk / 16; ++k) mma_bf16(tm + kColD, db + 128 * k, dw + 64 * k, kIdescT, k > 0);
         mma_commit(bar(kBarD));                                // (the state's pieces have been read, too)
         issue_y1(dx, 0);
+        mma_commit(bar(kBarH));
       }
       __syncwarp();
-      if (more) {
-        if (!wait(kBarL + (st ^ 1), ((c + 1) >> 1) & 1)) break;
-        if (elected) issue_g(c + 1, 1);                        // (behind the products that read the weights it lies over)
-        __syncwarp();
-      }
       if (!wait(kBarP2, c & 1)) break;
       fence_after_sync();
       if (elected) {
@@ -809,7 +805,14 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
         mma_commit(bar(kBarY));
       }
       __syncwarp();
+      if (!wait(kBarH, c & 1)) break;
       if (more) {
+        // G's second sum lies over weights that the first half of Y1 read (products of other shapes and sums: nothing says that they are
+        // finished in the order of issue); the second half is still under way meanwhile
+        if (!wait(kBarL + (st ^ 1), ((c + 1) >> 1) & 1)) break;
+        fence_after_sync();
+        if (elected) issue_g(c + 1, 1);
+        __syncwarp();
         if (!wait(kBarS, (c + 1) & 1)) break;                  // (dS has been read)
         fence_after_sync();
         if (elected) {
