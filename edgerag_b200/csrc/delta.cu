@@ -350,7 +350,8 @@ head_norm_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ gat
 // state a twentieth further from float64.)  Error against float64: o 1.6e-7, the state 1.0e-7, not above the walk's.
 //
 // Every wait for a product is bounded; a thread that gives up raises a block-wide flag, all warps still come to the barriers of the remaining
-// chunks, the block records 8000000 in *status, frees its TMEM and returns.
+// chunks, and the block frees its TMEM.  It then records 8000000 in *status and returns, or, where the caller named no status word, walks its
+// portion like the block that finds a number that is not finite.
 constexpr int kChunk = 64, kChunkCols = 16, kChunkWarps = 16, kCopyWarps = 4, kIssueWarp = 15, kChunkPrepWarps = 8;
 constexpr int kPieceElems = kChunk * kChunk;
 
@@ -879,9 +880,9 @@ delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const Ch
     fence_after_sync();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128) : "memory");
   }
-  if (gave_up) return;
-  if (odd) {
-    static_assert(2 * kDeltaChunk * (2 * D + kChunkCols + 4) * sizeof(float) <= sizeof(Smem) && D / 16 * kChunkCols <= kChunkWarps * 32, "the walk has room");
+  if (gave_up && status) return;
+  if (odd || gave_up) {
+    static_assert(2 * kDeltaChunk * (2 * D + kChunkCols + 4) * sizeof(float) <= offsetof(Smem, bar) && D / 16 * kChunkCols <= kChunkWarps * 32, "the walk has room");
     auto prepared = [&](int c0, int nc, float* qk_s, float* v_s, float* sc_s) {      // what `prepare` makes of a token, a warp each
       for (int t = warp; t < nc; t += kChunkWarps) {
         const __nv_bfloat16* at = rows + (size_t)(c0 + t) * channels;

@@ -462,7 +462,8 @@ ssm_scan16_kernel(const T* __restrict__ xbc, int channels, const T* __restrict__
 // its bits.
 //
 // Every wait for a product, a copy or warps is bounded; a thread that gives up raises a block-wide flag, all warps still come to the
-// barriers of the remaining chunks, the block records 7000000 in *status, lets its copies land, frees its TMEM and returns.
+// barriers of the remaining chunks, the block lets its copies land and frees its TMEM.  It then records 7000000 in *status and returns, or, where
+// the caller named no status word, walks its portion like the block that finds a number that is not finite.
 constexpr int kChunk = 128, kChunkCols = 32, kChunkWarps = 16, kIssueWarp = 16, kStepWarp = 17, kStepWarps = 4,
               kChunkThreads = 32 * (kStepWarp + kStepWarps);
 
@@ -921,10 +922,11 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
     fence_after_sync();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
-  if (gave_up) return;
-  if (odd) {
-    static_assert(scan_smem(N, kChunkCols, N / 8) <= sizeof(ChunkSmem) && N / 8 * kChunkCols <= kChunkWarps * 32, "the walk has room");
-    scan_tokens<__nv_bfloat16, 8, true>(reinterpret_cast<float*>(smem), xbc, channels, proj, ld, off_dt, dt_bias, a_log, d_skip, state,
+  if (gave_up && status) return;
+  if (odd || gave_up) {                                        // (in room that no copy and no barrier uses)
+    static_assert(offsetof(ChunkSmem, w) + scan_smem(N, kChunkCols, N / 8) <= offsetof(ChunkSmem, bars) && N / 8 * kChunkCols <= kChunkWarps * 32,
+                  "the walk has room");
+    scan_tokens<__nv_bfloat16, 8, true>(reinterpret_cast<float*>(sm.w), xbc, channels, proj, ld, off_dt, dt_bias, a_log, d_skip, state,
                                         seq_starts, state_slots, y, H, P, N, G, kChunkCols, h, seq, p0);
     return;
   }

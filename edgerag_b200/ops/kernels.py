@@ -728,14 +728,14 @@ def _workspace(device: torch.device) -> torch.Tensor:
 
 
 _set_status_word = None
-_status_word: torch.Tensor | None = None     # where the tensor-core weight-streaming kernel reports
+_status_word: torch.Tensor | None = None     # where the tensor-core weight-streaming kernel and the experts' products report
 _status_word_told: int | None = None         # ... and what the library was last told
 
 
 def linear_status_word(status: torch.Tensor | None) -> None:
-    """Name the device word (int32) to which the TMA + tcgen05 weight-streaming kernel reports a wait
-    that ran out (code 4000000 + block).  Kept until named again.  The library itself is told when it
-    is next used (a model that never brings 17 to 64 rows to a large product never builds it)."""
+    """Name the device word (int32) to which the TMA + tcgen05 weight-streaming kernel (code 4000000 + block) and the
+    routed experts' products (5000000 + block) report a wait that ran out.  Kept until named again.  The weight-streaming
+    library itself is told when it is next used (a model that never brings 17 to 64 rows to a large product never builds it)."""
     global _status_word
     if status is not None:
         _need(status, "status", torch.int32)
@@ -1465,17 +1465,18 @@ def conv_state_update(proj: torch.Tensor, off: int, conv_state: torch.Tensor, n_
 
 def ssm_scan(xbc: torch.Tensor, proj: torch.Tensor, off_dt: int, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, n_seqs: int, seq_starts: torch.Tensor, state_slots: torch.Tensor, y: torch.Tensor,
-             n_groups: int, longest: int | None = None) -> None:
+             n_groups: int, longest: int | None = None, status: torch.Tensor | None = None) -> None:
     """The recurrence of the state-space mixer over every request's rows, from and to its record in ``state``
     (float ``[slots, heads, N, P]``): ``xbc`` rows ``[x (heads * P) | B (groups * N) | C (groups * N)]``, raw
     step sizes in columns ``off_dt .. off_dt + heads`` of ``proj``; ``y`` float ``[tokens, heads * P]``.  ``longest``: the
     largest number of tokens of a request, by which the kernel is chosen (None: what the totals allow); the results do not
-    depend on it beyond rounding."""
+    depend on it beyond rounding.  ``status``: the word (int32) to which a block that waited for a product in vain reports (code
+    7000000, its results are not valid); without one such a block walks its portion token after token."""
     _need(xbc, "xbc"); _need(proj, "proj", xbc.dtype, contiguous=False); _need(state, "state", torch.float32)
     _need(y, "y", torch.float32)
     for name, t in (("dt_bias", dt_bias), ("a_log", a_log), ("d_skip", d_skip)):
         _need(t, name, torch.float32)
-    _need(seq_starts, "seq_starts", torch.int32); _need(state_slots, "state_slots", torch.int32)
+    _need(seq_starts, "seq_starts", torch.int32); _need(state_slots, "state_slots", torch.int32); _need(status, "status", torch.int32)
     n = xbc.shape[0]
     _, heads, n_state, p = state.shape
     if xbc.shape[1] != heads * p + 2 * n_groups * n_state or y.shape != (n, heads * p) or off_dt + heads > proj.shape[1] or \
@@ -1485,7 +1486,7 @@ def ssm_scan(xbc: torch.Tensor, proj: torch.Tensor, off_dt: int, dt_bias: torch.
           proj.stride(0) if n > 1 else proj.shape[1], int(off_dt), dt_bias, a_log, d_skip,
           state, seq_starts, state_slots, y, int(n_seqs), n,
           n - int(n_seqs) + 1 if longest is None else int(longest), heads, p, n_state,
-          int(n_groups), _status_word, _stream())
+          int(n_groups), status, _stream())
 
 
 def gated_group_norm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, eps: float, parts: int = 1,
@@ -1526,7 +1527,8 @@ def delta_scratch_floats(n_tokens: int, n_heads: int, n_key_heads: int, key_dim:
 
 def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
                state: torch.Tensor, n_seqs: int, seq_starts: torch.Tensor, state_slots: torch.Tensor, out: torch.Tensor,
-               n_key_heads: int, key_dim: int, scratch: torch.Tensor | None = None, longest: int | None = None) -> None:
+               n_key_heads: int, key_dim: int, scratch: torch.Tensor | None = None, longest: int | None = None,
+               status: torch.Tensor | None = None) -> None:
     """The gated delta rule over every request's rows, from and to its record in ``state`` (float ``[slots, heads,
     vdim, key_dim]``, the matrix of a head stored with the value index first).  ``qkv``: convolved and activated rows
     ``[q (key heads * key_dim) | k (the same) | v (heads * vdim)]``; the raw write strengths and decay inputs are
@@ -1536,10 +1538,12 @@ def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt
     ``scratch``: float, ``delta_scratch_floats`` entries (None: allocated here), where a first kernel leaves every token's
     unit vectors, scalars and values for the walk along the tokens.  Where it has room (``n_seqs`` given to that function) and
     the sizes allow it, long portions are taken in chunks of 64 tokens; ``longest``: the largest number of tokens of a request,
-    by which that is chosen (None: what the totals allow).  The results do not depend on it beyond rounding."""
+    by which that is chosen (None: what the totals allow).  The results do not depend on it beyond rounding.  ``status``: the word
+    (int32) to which a block that waited for a product in vain reports (code 8000000, its results are not valid); without one
+    such a block walks its portion token after token."""
     _need(qkv, "qkv"); _need(proj, "proj", qkv.dtype, contiguous=False); _need(state, "state", torch.float32)
     _need(out, "out", torch.float32); _need(dt_bias, "dt_bias", torch.float32); _need(a_log, "a_log", torch.float32)
-    _need(seq_starts, "seq_starts", torch.int32); _need(state_slots, "state_slots", torch.int32)
+    _need(seq_starts, "seq_starts", torch.int32); _need(state_slots, "state_slots", torch.int32); _need(status, "status", torch.int32)
     n = qkv.shape[0]
     _, heads, vdim, d = state.shape
     if d != key_dim or qkv.shape[1] != 2 * n_key_heads * d + heads * vdim or out.shape != (n, heads * vdim) or \
@@ -1557,7 +1561,7 @@ def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt
           proj.stride(0) if n > 1 else proj.shape[1], int(off_b), int(off_a), dt_bias, a_log,
           state, seq_starts, state_slots, out, scratch, scratch.numel(), int(n_seqs), n,
           n - int(n_seqs) + 1 if longest is None else int(longest), heads, int(n_key_heads), d, vdim,
-          _status_word, _stream())
+          status, _stream())
 
 
 def head_norm_gate(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, n_heads: int, eps: float) -> None:
