@@ -878,12 +878,20 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
         if (i > w) sm.rise[st][i - 1][r] = rise[i - 1];
       sm.weight[st][r] = weight;
     };
+    const bool on_16 = ((uintptr_t)y & 15) == 0;               // (8 at least)
     auto store = [&](int c) {                                  // the outputs of chunk c: eight lanes a token, whole lines
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int t = 32 * w + 4 * i + (lane >> 3), e = 4 * (lane & 7);
-        if (c * kChunk + t < n_tok)
-          *reinterpret_cast<float4*>(y + (size_t)(start + c * kChunk + t) * inner + h * P + p0 + e) = *reinterpret_cast<const float4*>(&sm.out[t][e]);
+        if (c * kChunk + t >= n_tok) continue;
+        const float4 v = *reinterpret_cast<const float4*>(&sm.out[t][e]);
+        float* to = y + (size_t)(start + c * kChunk + t) * inner + h * P + p0 + e;
+        if (on_16) {
+          *reinterpret_cast<float4*>(to) = v;
+        } else {
+          *reinterpret_cast<float2*>(to) = make_float2(v.x, v.y);
+          *reinterpret_cast<float2*>(to + 2) = make_float2(v.z, v.w);
+        }
       }
     };
     const bool copies = w == 0 && lane == 0;
@@ -1068,7 +1076,7 @@ ERB_EXPORT int erb_ssm_scan(const void* xbc, int channels, const void* proj, int
   int most_tokens = INT_MAX;            // what the scan takes: every portion, or single tokens beside the chunk kernel's portions
 #if ERB_ELEM == 1
   if ((N == 32 || N == 64 || N == 128) && P % kChunkCols == 0 && chunks_pay(H * (P / kChunkCols), N, n_tokens, n_seqs, longest) && channels % 8 == 0 &&
-      !((uintptr_t)xbc & 15) && !((uintptr_t)state & 7) && !((uintptr_t)y & 15)) {
+      !((uintptr_t)xbc & 15) && !((uintptr_t)state & 7) && !((uintptr_t)y & 7)) {
     constexpr size_t bytes = sizeof(ChunkSmem) + 1024;
     auto kern = N == 32 ? ssm_chunk_kernel<32> : N == 64 ? ssm_chunk_kernel<64> : ssm_chunk_kernel<128>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

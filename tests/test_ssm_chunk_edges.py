@@ -36,3 +36,24 @@ def test_chunks_of_128_tokens(N, lens, bad):
         assert (state[s].double() - want_s).abs().max() < 3e-5 * max(1.0, want_s.abs().max()), s
         at += length
     assert bad or torch.isfinite(y).all()
+
+
+@pytest.mark.parametrize("offset", [2, 4])
+def test_outputs_on_8_bytes_come_from_the_chunks_too(offset):
+    """The outputs' alignment does not change who makes them: the bits of the chunks, which the walk's are not."""
+    H, P, N, G, n = 4, 64, 64, 2, 300
+    inner = H * P
+    g = torch.Generator().manual_seed(1)
+    xbc = (torch.randn(n, inner + 2 * G * N, generator=g) * 0.5).to(torch.bfloat16).cuda()
+    proj, vec = torch.randn(n, H, generator=g).to(torch.bfloat16).cuda(), [torch.randn(H, generator=g).cuda() - 1.0 for _ in range(3)]
+    starts, slots = torch.tensor([0, n], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda()
+
+    def scan(y, longest):
+        state = torch.zeros(1, H, N, P, device="cuda")
+        kernels.ssm_scan(xbc, proj, 0, *vec, state, 1, starts, slots, y, G, longest=longest)
+        return y, state
+
+    y, state = scan(torch.empty(n, inner, device="cuda"), n)
+    off_y, off_state = scan(torch.empty(n * inner + offset, device="cuda")[offset:].view(n, inner), n)
+    assert torch.equal(y, off_y) and torch.equal(state, off_state)
+    assert not torch.equal(y, scan(torch.empty_like(y), 1)[0])
