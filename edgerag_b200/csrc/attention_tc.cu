@@ -778,12 +778,13 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     const int key_abs0 = tile_begin(tile);
     if (ok && serves && key0 < n_here) {
       const uint32_t k_st = sK + (uint32_t)s * kGqaStageBytes, v_st = sV + (uint32_t)s * kGqaStageBytes;
-      // Rows past the last key may hold anything (unwritten slots, an earlier tile): their scores are
-      // masked below, and their values are zeroed here, since 0 * NaN would spoil the product.
-      if (key0 + 16 > n_here) {
-        for (int k = max(n_here, key0) * 8 + lane; k < (key0 + 16) * 8; k += 32) {
+      // Rows past the last key may hold anything (unwritten slots, an earlier tile), rows before the window numbers that are not
+      // finite: their scores are masked below, and their values are zeroed here, since 0 * NaN would spoil the product.
+      if (key0 + 16 > n_here || key_abs0 + key0 < k_lo) {
+        for (int k = key0 * 8 + lane; k < (key0 + 16) * 8; k += 32) {
           const int key = k >> 3, chunk = k & 7;
-          *reinterpret_cast<uint4*>(smem + (v_st - base) + row_of(key) * 128 + chunk * 16) = make_uint4(0, 0, 0, 0);
+          if (key >= n_here || (key_abs0 + key < k_lo && key_abs0 + key >= keep_first))
+            *reinterpret_cast<uint4*>(smem + (v_st - base) + row_of(key) * 128 + chunk * 16) = make_uint4(0, 0, 0, 0);
         }
         __syncwarp();
       }
