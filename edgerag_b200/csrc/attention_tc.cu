@@ -905,14 +905,18 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
       continue;
     }
     const size_t slot = ((size_t)seq * nq + kvh0 * R + row) * max_splits + split;
-    *reinterpret_cast<float2*>(part_acc + slot * D + 2 * lane) = sum;
-    if (lane == 0) *reinterpret_cast<float2*>(part_ml + slot * 2) = make_float2(m, l);
+    part_acc[slot * D + 2 * lane] = sum.x;
+    part_acc[slot * D + 2 * lane + 1] = sum.y;
+    if (lane == 0) { part_ml[slot * 2] = m; part_ml[slot * 2 + 1] = l; }      // (part_ml may start at any float)
   }
   if (max_splits > 1 && counters)
     merge_splits_if_last<D>(counters + (size_t)seq * gridDim.y + blockIdx.y, part_acc, part_ml,
                             (size_t)seq * nq + (size_t)kvh0 * R, hg_here * R, min(pos / split_keys - first_split + 1, max_splits), max_splits,
                             out + (size_t)t * out_row_stride + (size_t)kvh0 * R * D, gate_row ? gate_row + kvh0 * R * D : nullptr);
 }
+
+// Whether the last block of a sequence can merge its splits: a lane reads D / 32 floats of a partial result at a time.
+bool merge_reads(const float* part_acc, int head_dim) { return !((uintptr_t)part_acc & (head_dim / 8 - 1)); }
 
 // Whether the kernel above takes these sizes with hg kv heads per block.
 bool decode_mma_fits(int nkv, int page_size, int split_keys, int hg) {
@@ -983,6 +987,8 @@ ERB_EXPORT int erb_attention_decode_gqa(const void* q, int q_row_stride, const v
   if (q_row_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)k_pages & 127) || ((uintptr_t)v_pages & 127))
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: q rows must be 16-byte aligned, pools 128-byte aligned");
   if (n_seqs > 65535 || nkv > 65535) return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: grid too large");
+  if (counters && max_splits > 1 && !merge_reads(part_acc, head_dim))
+    return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: part_acc must be aligned to %d bytes", head_dim / 8);
   if (max_splits > kCombineMaxSplits)
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: %d splits (at most %d)", max_splits, kCombineMaxSplits);
   if ((unsigned long long)n_pool_pages * nkv * page_size > 0x7fffffffull)
@@ -1040,6 +1046,8 @@ ERB_EXPORT int erb_attention_decode_bulk(const void* q, int q_row_stride, const 
   if (q_row_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)k_pages & 15) || ((uintptr_t)v_pages & 15))
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_bulk: rows must be 16-byte aligned");
   if (n_seqs > 65535 || nkv > 65535) return fail(ERB_ERR_UNSUPPORTED, "attention_decode_bulk: grid too large");
+  if (counters && max_splits > 1 && !merge_reads(part_acc, head_dim))
+    return fail(ERB_ERR_UNSUPPORTED, "attention_decode_bulk: part_acc must be aligned to %d bytes", head_dim / 8);
   if (max_splits > kCombineMaxSplits)
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_bulk: %d splits (at most %d)", max_splits, kCombineMaxSplits);
   const float scale_log2 = scale * 1.4426950408889634f;

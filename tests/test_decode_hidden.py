@@ -45,3 +45,16 @@ def test_a_value_before_the_window_is_not_seen(nq, nkv, heads, mask, bad):
             hidden += 1
     assert hidden > 8 and torch.isfinite(clean.float()).all()
     assert torch.equal(_run(case, nq, nkv, 2, 64, heads=heads, **mask), clean)
+
+
+@pytest.mark.parametrize("nq,nkv", [(4, 4), (6, 2)])
+def test_scratch_that_starts_at_an_odd_float(nq, nkv):
+    """The maxima and sums of the splits may lie at any float; partial results that the merge cannot read are refused."""
+    case = paged_case(torch.bfloat16, 6, nq, nkv, 64, 16, [60, 200], [1, 1])
+    assert torch.equal(_run(case, nq, nkv, 4, 64, offset=1), _run(case, nq, nkv, 4, 64))
+    q, pages, i32 = case["q"].cuda(), case["kp"].cuda(), lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
+    scratch = torch.zeros(4096, device="cuda")
+    call = K.attention_decode_bulk if nq == nkv else K.attention_decode_gqa
+    with pytest.raises(K.KernelError, match="aligned"):
+        call(q, pages, pages, case["tables"].cuda(), i32(0, 1), case["pos"].cuda(), torch.empty_like(q), nq, 0.125, scratch[1:], scratch, 4, i32(0),
+             split_keys=64)
