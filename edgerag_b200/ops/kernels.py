@@ -1942,6 +1942,9 @@ def _choose_decode_plan(device: int, n_seqs: int, n_kv_heads: int, max_keys: int
     return split, 0
 
 
+EVEN_SPLIT_PAGES = 1024      # pages of an equal split at most
+
+
 def choose_even_plan(n_seqs: int, n_q_heads: int, n_kv_heads: int, max_keys: int, page_size: int, head_dim: int) -> tuple[int, int, int] | None:
     """(bound on the keys per split, kv heads per block, splits) for a decode step in which every sequence's keys are cut into as many
     equal splits, or None where the tensor-core decode kernel does not run or such splits leave the GPU half empty
@@ -1964,7 +1967,8 @@ def _choose_even_plan(device: int, n_seqs: int, n_q_heads: int, n_kv_heads: int,
     keys in one split, which nobody has to merge (8 sequences, a step: 200 keys 1,075 -> 1,017 us, 520 keys 1,162 -> 1,139; attention of
     64 x 1,000 87 -> 82).  Fewer blocks and short contexts keep the other plan (4 x 520: 1,056 us, equal splits 1,063 to 1,080).
 
-    A wave is filled to 0.9: with 288 of 296 places some blocks waited for the kernel before."""
+    A wave is filled to 0.9: with 288 of 296 places some blocks waited for the kernel before.  A split's page numbers lie in shared
+    memory: splits of more than ``EVEN_SPLIT_PAGES`` would leave room for one block an SM, and of some 25,000 for none."""
     if head_dim != 64 or n_q_heads % n_kv_heads:
         return None
     lib = native.load("attention_tc", None)
@@ -1985,6 +1989,8 @@ def _choose_even_plan(device: int, n_seqs: int, n_q_heads: int, n_kv_heads: int,
         if splits < by_keys and blocks * splits < 0.6 * slots:
             continue
         split = -(-max_keys // (splits * page_size)) * page_size
+        if split > EVEN_SPLIT_PAGES * page_size:
+            continue
         return split, heads, -(-max_keys // split)
     return None
 
