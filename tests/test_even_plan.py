@@ -7,8 +7,8 @@ import pytest
 from edgerag_b200.ops import kernels
 
 
-@pytest.mark.parametrize("n_seqs,nq,nkv,bound,page", [(140, 15, 5, 1 << 20, 16), (140, 15, 5, 1 << 18, 8), (200, 4, 1, 400_000, 16), (30, 8, 8, 1 << 21, 16),
-                                                      (1, 15, 5, 1 << 24, 8), (140, 15, 5, 8192, 16)])
+@pytest.mark.parametrize("n_seqs,nq,nkv,bound,page", [(200, 15, 5, 1 << 20, 16), (200, 15, 5, 1 << 18, 8), (200, 4, 1, 400_000, 16), (30, 8, 8, 1 << 21, 16),
+                                                      (1, 15, 5, 1 << 24, 8), (200, 15, 5, 8192, 16)])
 def test_a_split_has_room_for_its_pages(monkeypatch, n_seqs, nq, nkv, bound, page):
     """One wave of blocks cuts few splits of many sequences: they keep to what shared memory holds, or the other plan stands."""
     monkeypatch.setitem(kernels._sm_counts, 0, 148)
