@@ -195,11 +195,9 @@ PyMethodDef methods[] = {
     {nullptr, nullptr, 0, nullptr},
 };
 
-PyModuleDef module = {PyModuleDef_HEAD_INIT, "launch", nullptr, -1, methods};
-
-}  // namespace
-
-PyMODINIT_FUNC PyInit_launch() {
+// The module is made in two phases: it then belongs to whoever loads it, and takes no name in sys.modules.
+int start(PyObject*) {
+  if (g_own) return 0;              // (loaded before)
   launcher_type.tp_name = "edgerag_b200.launcher";
   launcher_type.tp_basicsize = sizeof(Launcher);
   launcher_type.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL;
@@ -207,8 +205,16 @@ PyMODINIT_FUNC PyInit_launch() {
   launcher_type.tp_call = PyVectorcall_Call;
   launcher_type.tp_members = launcher_members;
   launcher_type.tp_dealloc = [](PyObject* self) { PyObject_Free(self); };
-  if (PyType_Ready(&launcher_type) < 0) return nullptr;
-  g_own = PyUnicode_InternFromString("own");
+  if (PyType_Ready(&launcher_type) < 0) return -1;
   g_library = PyUnicode_InternFromString("library");
-  return PyModule_Create(&module);
+  if (!g_library || !(g_own = PyUnicode_InternFromString("own"))) return -1;
+  return 0;
 }
+
+PyModuleDef_Slot slots[] = {{Py_mod_exec, reinterpret_cast<void*>(start)}, {0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "edgerag_b200._launch", nullptr, 0, methods, slots, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__launch() { return PyModuleDef_Init(&module); }

@@ -208,7 +208,7 @@ def build_host(verbose: bool = True) -> Path:
 
     import torch
 
-    name = "launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
+    name = "_launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
     h = hashlib.sha256(HOST_SOURCE.read_bytes())
     h.update(f"{torch.__version__} {sys.version}".encode())
     stamp = h.hexdigest()
@@ -240,7 +240,7 @@ def load_host():
     import importlib.util
 
     try:
-        spec = importlib.util.spec_from_file_location("launch", build_host())
+        spec = importlib.util.spec_from_file_location("edgerag_b200._launch", build_host())
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         return module

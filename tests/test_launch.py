@@ -74,3 +74,15 @@ def test_checks_are_those_of_python(host):
             except kernels.KernelError as e:
                 outcomes.append(str(e))
         assert outcomes[0] == outcomes[1]
+
+
+def test_a_program_keeps_its_own_module_of_any_name(monkeypatch):
+    """Loading the host module takes no name among the modules of the program."""
+    import sys
+
+    own = object()
+    monkeypatch.setitem(sys.modules, "launch", own)
+    before = {name: id(module) for name, module in sys.modules.items()}
+    module = native.load_host()
+    assert module is not None and {name: id(m) for name, m in sys.modules.items()} == before
+    assert callable(module.need) and module.__name__.startswith("edgerag_b200.")
