@@ -11,6 +11,7 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstddef>
@@ -69,6 +70,9 @@ bool run(Launcher* self, PyObject* const* args, Py_ssize_t n, int* rc) {
     } else if (self->kinds[i] == 'p' && THPVariable_Check(a)) {
       try {
         w[ni++] = (Word)(uintptr_t)THPVariable_Unpack(a).data_ptr();
+      } catch (python_error& e) {                              // (a tensor class of Python's own)
+        e.restore();
+        return false;
       } catch (const std::exception& e) {
         PyErr_SetString(PyExc_RuntimeError, e.what());
         return false;
@@ -168,9 +172,12 @@ PyObject* need(PyObject*, PyObject* const* args, Py_ssize_t n, PyObject* kwnames
   if (known && args[0] == Py_None) Py_RETURN_NONE;
   if (known && THPVariable_Check(args[0]) && (contiguous == Py_True || contiguous == Py_False) && (dtype == Py_None || THPDtype_Check(dtype))) {
     const at::Tensor& t = THPVariable_Unpack(args[0]);
-    if (t.is_cuda() && (dtype == Py_None || t.scalar_type() == reinterpret_cast<THPDtype*>(dtype)->scalar_type) &&
-        (contiguous == Py_False || t.is_contiguous()))
-      Py_RETURN_NONE;
+    try {
+      if (t.is_cuda() && (dtype == Py_None || t.scalar_type() == reinterpret_cast<THPDtype*>(dtype)->scalar_type) &&
+          (contiguous == Py_False || t.is_contiguous()))
+        Py_RETURN_NONE;
+    } catch (const std::exception&) {                          // (layouts and tensor classes that do not say: asked there, they raise)
+    }
   }
   return PyObject_Vectorcall(g_need, args, (size_t)n, kwnames);
 }

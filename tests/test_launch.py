@@ -86,3 +86,37 @@ def test_a_program_keeps_its_own_module_of_any_name(monkeypatch):
     module = native.load_host()
     assert module is not None and {name: id(m) for name, m in sys.modules.items()} == before
     assert callable(module.need) and module.__name__.startswith("edgerag_b200.")
+
+
+class _Silent(torch.Tensor):
+    """A tensor class on a device that answers no question about its layout or memory."""
+
+    @staticmethod
+    def __new__(cls):
+        return torch.Tensor._make_wrapper_subclass(cls, (4, 4), device="cuda", dtype=torch.float32, dispatch_sizes_strides_policy="strides")
+
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        raise RuntimeError(f"no answer to {func}")
+
+
+def test_a_tensor_that_raises_does_not_end_the_process():
+    """What torch throws behind the check or the pointer is an exception in Python (in a child: it used to abort)."""
+    import multiprocessing
+
+    child = multiprocessing.get_context("spawn").Process(target=_ask_a_silent_tensor)
+    child.start()
+    child.join(120)
+    assert child.exitcode == 0
+
+
+def _ask_a_silent_tensor():
+    module = native.load_host()
+    module.bind(dict.fromkeys(("own", "library"), 0), kernels.KernelError, kernels._need_in_python)
+    fn, got, _keep = _entry(module, [ctypes.c_void_p])
+    for ask in (lambda: kernels._need_in_python(_Silent(), "x"), lambda: module.need(_Silent(), "x"), lambda: module.call(fn, _Silent())):
+        try:
+            ask()
+        except RuntimeError:
+            continue
+        assert got and got[0][0] is None, got            # (memory that is not there is a null pointer)
