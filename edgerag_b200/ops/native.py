@@ -188,6 +188,18 @@ def load(library: str, elem: str | None = None) -> ctypes.CDLL:
     return lib
 
 
+HOST_FLAGS = ("-O2", "-std=c++17", "-fPIC", "-shared")
+HOST_LINK = ("-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10")
+
+
+def _host_fingerprint() -> str:
+    import torch
+
+    h = hashlib.sha256(HOST_SOURCE.read_bytes())
+    h.update(" ".join((torch.__version__, str(torch._C._GLIBCXX_USE_CXX11_ABI), sys.version, *HOST_FLAGS, *HOST_LINK, os.environ.get("CXX", ""))).encode())
+    return h.hexdigest()
+
+
 def _host_command(out: Path) -> list[str]:
     import sysconfig
 
@@ -197,21 +209,18 @@ def _host_command(out: Path) -> list[str]:
     cxx = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
     if not cxx or not (Path(sysconfig.get_paths()["include"]) / "Python.h").is_file():
         raise NativeBuildError("no C++ compiler or no Python.h for the host module")
-    return [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    return [cxx, *HOST_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
             f"-I{root / 'include'}", f"-I{root / 'include/torch/csrc/api/include'}", f"-I{sysconfig.get_paths()['include']}", "-o", str(out),
-            str(HOST_SOURCE), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10"]
+            str(HOST_SOURCE), f"-L{root / 'lib'}", *HOST_LINK]
 
 
 def build_host(verbose: bool = True) -> Path:
-    """Compile the host module if its source, the Python or the torch it is built against changed; return its path."""
+    """Compile the host module if its source, its flags, the compiler named by $CXX, the Python or the torch it is built against
+    changed; return its path."""
     import sysconfig
 
-    import torch
-
     name = "_launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
-    h = hashlib.sha256(HOST_SOURCE.read_bytes())
-    h.update(f"{torch.__version__} {sys.version}".encode())
-    stamp = h.hexdigest()
+    stamp = _host_fingerprint()
     ready = _find_prebuilt(name, stamp)
     if ready is not None:
         return ready

@@ -20,3 +20,31 @@ def test_libraries_are_built_without_the_host_module(monkeypatch, capfd, error):
     built = native.build_all(verbose=False)
     assert len(built) > 10 and all(p.name.startswith("lib") for p in built)
     assert "ctypes" in capfd.readouterr().err
+
+
+@pytest.fixture()
+def folder(monkeypatch, tmp_path):
+    """An empty folder for what is built, and a compiler that counts its runs and writes what it is asked for, or fails."""
+    runs = []
+
+    def command(out):
+        runs.append(out)
+        return ["sh", "-c", "exit 3" if (tmp_path / "broken").exists() else f"echo built > {out}"]
+
+    monkeypatch.setattr(native, "PACKAGE_EXT", tmp_path)
+    monkeypatch.setattr(native.tempfile, "gettempdir", lambda: str(tmp_path / "other"))
+    monkeypatch.delenv("EDGERAG_B200_EXT_DIR", raising=False)
+    monkeypatch.setattr(native, "_host_command", command)
+    return tmp_path, runs
+
+
+def test_other_flags_or_another_compiler_build_anew(folder, monkeypatch):
+    _, runs = folder
+    native.build_host(False), native.build_host(False)
+    assert len(runs) == 1
+    monkeypatch.setattr(native, "HOST_FLAGS", (*native.HOST_FLAGS, "-g"))
+    native.build_host(False), native.build_host(False)
+    assert len(runs) == 2
+    monkeypatch.setenv("CXX", "another-c++")
+    native.build_host(False), native.build_host(False)
+    assert len(runs) == 3
