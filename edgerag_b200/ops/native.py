@@ -214,9 +214,9 @@ def _host_command(out: Path) -> list[str]:
             str(HOST_SOURCE), f"-L{root / 'lib'}", *HOST_LINK]
 
 
-def build_host(verbose: bool = True) -> Path:
+def build_host(verbose: bool = True, retry: bool = True) -> Path:
     """Compile the host module if its source, its flags, the compiler named by $CXX, the Python or the torch it is built against
-    changed; return its path."""
+    changed; return its path.  ``retry`` False: a compiler that failed on the same before is not asked again."""
     import sysconfig
 
     name = "_launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
@@ -225,7 +225,9 @@ def build_host(verbose: bool = True) -> Path:
     if ready is not None:
         return ready
     folder = _ext_dir()
-    lib = folder / name
+    lib, failed = folder / name, folder / (name + ".failed")
+    if not retry and failed.is_file() and failed.read_text().startswith(stamp):
+        raise NativeBuildError(f"the compiler failed for {name} before (its words: {failed})")
     with open(folder / (name + ".lock"), "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
         try:
@@ -236,9 +238,11 @@ def build_host(verbose: bool = True) -> Path:
                 proc = subprocess.run(_host_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
                 if proc.returncode != 0:
                     tmp.unlink(missing_ok=True)
+                    failed.write_text(f"{stamp}\n{proc.stdout}")
                     raise NativeBuildError(f"the compiler failed for {name}:\n{proc.stdout}")
                 os.replace(tmp, lib)
                 (folder / (name + ".stamp")).write_text(stamp)
+                failed.unlink(missing_ok=True)
             return lib
         finally:
             fcntl.flock(lock, fcntl.LOCK_UN)
@@ -249,7 +253,7 @@ def load_host():
     import importlib.util
 
     try:
-        spec = importlib.util.spec_from_file_location("edgerag_b200._launch", build_host())
+        spec = importlib.util.spec_from_file_location("edgerag_b200._launch", build_host(retry=False))
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         return module

@@ -48,3 +48,18 @@ def test_other_flags_or_another_compiler_build_anew(folder, monkeypatch):
     monkeypatch.setenv("CXX", "another-c++")
     native.build_host(False), native.build_host(False)
     assert len(runs) == 3
+
+
+def test_a_failed_compilation_is_remembered(folder):
+    """A program's start does not ask a compiler again that failed on the same; the build of everything does."""
+    at, runs = folder
+    (at / "broken").touch()
+    for _ in range(2):
+        assert native.load_host() is None
+    assert len(runs) == 1
+    with pytest.raises(native.NativeBuildError):
+        native.build_host(False)
+    assert len(runs) == 2
+    (at / "broken").unlink()
+    assert native.load_host() is None and len(runs) == 2
+    assert native.build_host(False).is_file() and native.build_host(False, retry=False).is_file() and len(runs) == 3
