@@ -126,15 +126,18 @@ def decode_attention(a) -> dict:
     out = torch.empty_like(q)
     pos = torch.full((a.batch,), a.context - 1, dtype=torch.int32, device="cuda")
     tok = torch.arange(a.batch, dtype=torch.int32, device="cuda")
+    even = None             # (bound on the keys per split, kv heads per block, splits) of equal splits
     if a.split <= 0:        # as the engine chooses it: from the batch and a power-of-two bound on the context
         bound, granule = kernels.context_bound(-(-a.context // a.page))
         if window > 0 or chunk > 0:
             bound = min(bound, -(-(window + keep + chunk) // a.page))
             granule = bound
-        a.split, heads = kernels.choose_decode_plan(a.batch, a.kv_heads, bound * a.page, a.page, a.head_dim, a.kernel != "bulk",
-                                                    granule * a.page)
+        elif a.kernel != "general" and dtype == torch.bfloat16 and not a.head_group:
+            even = kernels.choose_even_plan(a.batch, a.heads, a.kv_heads, bound * a.page, a.page, a.head_dim)
+        a.split, heads = even[:2] if even else kernels.choose_decode_plan(a.batch, a.kv_heads, bound * a.page, a.page, a.head_dim,
+                                                                          a.kernel != "bulk", granule * a.page)
         a.head_group = a.head_group or heads
-    splits = (a.context - 1) // a.split + 1
+    splits = even[2] if even else (a.context - 1) // a.split + 1
     if window > 0 or chunk > 0:
         splits = min(splits, (window + chunk) // a.split + 2)
     acc_n, ml_n = kernels.decode_scratch_floats(a.batch, a.heads, a.head_dim, splits)
@@ -143,17 +146,18 @@ def decode_attention(a) -> dict:
     scale = a.head_dim ** -0.5
     if a.kernel == "gqa":
         fn = lambda: kernels.attention_decode_gqa(q, *cache(), tok, pos, out, a.heads, scale, acc, ml, splits,  # noqa: E731
-                                                  status, split_keys=a.split, window=window, keep_first=keep, chunk=chunk, **score)
+                                                  status, split_keys=a.split, window=window, keep_first=keep, chunk=chunk,
+                                                  even=even is not None, **score)
     elif a.kernel == "bulk":
         fn = lambda: kernels.attention_decode_bulk(q, *cache(), tok, pos, out, a.heads, scale, acc, ml, splits,  # noqa: E731
                                                    status, split_keys=a.split, head_group=a.head_group, window=window, keep_first=keep,
-                                                   chunk=chunk, **score)
+                                                   chunk=chunk, even=even is not None, **score)
     else:
         fn = lambda: kernels.attention_decode(q, *cache(), tok, pos, out, a.heads, scale, acc, ml, splits,  # noqa: E731
                                               split_keys=a.split, window=window, keep_first=keep, chunk=chunk, **score)
     us = _time(fn, max(a.iters, 2 * reps), a.warmup)
-    return {"case": "decode-attention", "kernel": a.kernel, "split": a.split, "head_group": a.head_group, "us": round(us, 2),
-            "bytes": nbytes, "gbs": round(nbytes / us / 1e3, 1), "frac_hbm": round(nbytes / us / 1e3 / HBM_GBS, 4),
+    return {"case": "decode-attention", "kernel": a.kernel, "split": a.split, "splits": splits, "even": even is not None,
+            "head_group": a.head_group, "us": round(us, 2), "bytes": nbytes, "gbs": round(nbytes / us / 1e3, 1), "frac_hbm": round(nbytes / us / 1e3 / HBM_GBS, 4),
             "status": int(status), "from_dram": bool(a.cold) or nbytes > 126e6, "window": window, "keep_first": keep, "chunk": chunk,
             **_score_record(a)}
 
@@ -773,7 +777,8 @@ def main(argv=None) -> int:
     d.add_argument("--batch", type=int, default=8)
     d.add_argument("--context", type=int, default=8192)
     d.add_argument("--split", type=int, default=0, help="keys per split; 0: the engine's choice for this batch")
-    d.add_argument("--kernel", choices=["bulk", "gqa", "general"], default="bulk")
+    d.add_argument("--kernel", choices=["bulk", "gqa", "general"], default="bulk",
+                   help="the entry point; for heads of 64 with one query head per kv head the bulk one runs the tensor-core kernel of gqa")
     d.add_argument("--head-group", type=int, default=0, help="kv heads per block of the bulk kernel; 0: its own choice")
     d.add_argument("--cold", action="store_true", help="rotate over several caches so that none is found in L2")
     p = sub.add_parser("prefill-attention", parents=[common, att])

@@ -67,3 +67,17 @@ def test_the_plan_of_equal_splits(nq, nkv):
                 groups = -(-nkv // (heads or 8))
                 assert split % 16 == 0 and split * splits >= bound and splits <= 64 and n * groups * splits <= slots
     assert K.choose_even_plan(8, nq, nkv, 1024, 16, 128) is None and K.choose_even_plan(8, nq, nkv, 1024, 12, 64) is None
+
+
+@pytest.mark.parametrize("batch,nq,nkv,context,kernel", [(64, 15, 5, 700, "gqa"), (8, 32, 32, 1000, "bulk")])
+def test_the_timed_launch_is_the_engines(batch, nq, nkv, context, kernel):
+    """The program that times one kernel takes the splits that a step of these sequences takes."""
+    from argparse import Namespace
+
+    from edgerag_b200.ops import microbench
+
+    a = Namespace(batch=batch, context=context, heads=nq, kv_heads=nkv, head_dim=64, page=16, split=0, kernel=kernel, head_group=0, dtype="bfloat16",
+                  cold=False, iters=2, warmup=1, sequential_pages=False)
+    out = microbench.decode_attention(a)
+    split, heads, splits = K.choose_even_plan(batch, nq, nkv, K.context_bound(-(-context // 16))[0] * 16, 16, 64)
+    assert (out["split"], out["head_group"], out["splits"], out["even"], out["status"]) == (split, heads, splits, True, 0)
