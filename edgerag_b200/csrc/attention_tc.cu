@@ -582,9 +582,12 @@ int dispatch_group(int r, const void* q, int q_row_stride, const void* k_pages, 
 // over the page pools with the 128-byte swizzle, so that the ldmatrix reads of 8 rows x 16 bytes
 // touch all banks.  bfloat16, head size 64, pages of a multiple of 8 tokens.
 //
-// Measured with equal splits (one layer with its projections and norm): 8 sequences of 8,192 tokens of 32 heads 103 us by the kernel
-// above in splits at multiples of 2,048, 93.7 us here (a decode step at 520 tokens 1,162 | 1,139 us); 64 of 7,531 tokens of 15 heads
-// over 5 132 | 122 us here with splits at multiples of 2,048 | equal splits.
+// With one query head per kv head it is the faster one where a block walks far and where equal splits count, which the kernel above does
+// not have (32 heads, caches from DRAM, above at multiples of the same bound | here in equal splits: 8 x 6,200 keys in two splits 82.5 | 64.7 us,
+// 8 x 5,000 62.9 | 53.4, 1 x 5,000 in 16 13.7 | 11.4, 16 x 8,192 in one 159 | 155, 64 x 8,192 648 | 615); short walks and small
+// copies cost it more (1 x 200 keys in splits of 64 5.1 | 6.1, 16 x 200 in one split 7.5 | 8.5, a window of 512 of 1 x 4,000 6.1 | 7.0): callers choose.
+// Several query heads per kv head: 64 x 7,531 tokens of 15 heads over 5, a layer with its projections and norm, 132 us with splits at multiples of
+// 2,048, 122.5 us with equal ones.
 // =============================================================================================
 namespace {
 
@@ -1030,13 +1033,15 @@ ERB_EXPORT int erb_attention_decode_bulk_head_group(int nkv, int head_dim, int p
 // with head_dim 32 / 64 / 128, at most 8 query heads per kv head, and page rows that are 16-byte multiples.
 // window > 0: the token sees its last `window` keys (its own included) and the first `keep_first` ones;
 // window < 0: the keys of its own run of -window positions (runs counted from position 0) up to itself.
+// mma: heads of 64 with one query head per kv head by the tensor-core kernel, wherever whole pages make its stages (1: equal splits of split_keys
+// at most, without a window; 2: splits at multiples of split_keys); 0, and everything else: the kernel on CUDA cores, at multiples.
 ERB_EXPORT int erb_attention_decode_bulk(const void* q, int q_row_stride, const void* k_pages, const void* v_pages,
                                          int n_pool_pages, const int* block_tables, int max_pages, const int* token_of_seq,
                                          const int* positions, void* out, int out_row_stride, float* part_acc,
                                          float* part_ml, int max_splits, int n_seqs, int nq, int nkv, int head_dim,
                                          int page_size, int split_keys, float scale, int* status, int* counters,
                                          int head_group, int window, int keep_first, const float* penalty, float softcap,
-                                         const void* gate, int gate_stride, int even_splits, void* stream) {
+                                         const void* gate, int gate_stride, int mma, void* stream) {
   if (n_seqs <= 0) return ERB_OK;
   if (penalty && softcap > 0.f) return fail(ERB_ERR_UNSUPPORTED, "attention_decode_bulk: a penalty and a cap of the scores exclude each other");
   if (nq <= 0 || nkv <= 0 || nq % nkv) return fail(ERB_ERR_ARG, "attention_decode_bulk: bad head counts");
@@ -1053,13 +1058,12 @@ ERB_EXPORT int erb_attention_decode_bulk(const void* q, int q_row_stride, const 
   const float scale_log2 = scale * 1.4426950408889634f;
   cudaStream_t s = (cudaStream_t)stream;
   const int r = nq / nkv;
-  // Heads of 64 with one query head per kv head: the tensor-core kernel, wherever whole pages make its stages.
-  const int hg = r == 1 && head_dim == 64 ? decode_head_group(nkv, 64, page_size, split_keys, head_group) : 0;
-  const bool mma = hg > 0 && decode_mma_fits(nkv, page_size, split_keys, hg) && n_pool_pages > 0 && !((uintptr_t)k_pages & 127) &&
+  const int hg = mma && r == 1 && head_dim == 64 ? decode_head_group(nkv, 64, page_size, split_keys, head_group) : 0;
+  const bool on_mma = hg > 0 && decode_mma_fits(nkv, page_size, split_keys, hg) && n_pool_pages > 0 && !((uintptr_t)k_pages & 127) &&
                    !((uintptr_t)v_pages & 127) && (unsigned long long)n_pool_pages * nkv * page_size <= 0x7fffffffull;
   int rc;
-  if (mma) rc = launch_decode_mma(q, q_row_stride, k_pages, v_pages, n_pool_pages, block_tables, max_pages, token_of_seq, positions, out,
-                                  out_row_stride, part_acc, part_ml, max_splits, n_seqs, nq, nkv, page_size, split_keys, even_splits, scale_log2, hg,
+  if (on_mma) rc = launch_decode_mma(q, q_row_stride, k_pages, v_pages, n_pool_pages, block_tables, max_pages, token_of_seq, positions, out,
+                                  out_row_stride, part_acc, part_ml, max_splits, n_seqs, nq, nkv, page_size, split_keys, mma == 1, scale_log2, hg,
                                   status, counters, window, keep_first, penalty, softcap, gate, gate_stride, s);
   else switch (head_dim) {
     case 32: rc = dispatch_group<32>(r, q, q_row_stride, k_pages, v_pages, block_tables, max_pages, token_of_seq,

@@ -1952,6 +1952,21 @@ def choose_even_plan(n_seqs: int, n_q_heads: int, n_kv_heads: int, max_keys: int
     return _choose_even_plan(torch._C._cuda_getDevice(), n_seqs, n_q_heads, n_kv_heads, max_keys, page_size, head_dim)
 
 
+def single_heads_on_tensor_cores(plan: tuple[int, int, int], n_seqs: int, n_kv_heads: int, max_keys: int, shaped: bool, sms: int) -> bool:
+    """Whether a step of one query head per kv head takes ``plan`` (of ``choose_even_plan``) on the tensor cores, in equal splits; else the
+    kernel on CUDA cores takes it, at multiples of the plan's bound.  ``shaped``: penalty, cap or gate.
+
+    32 heads, caches from DRAM, CUDA cores | tensor cores.  Above 2,048 keys equal splits count, and so does a block's long walk: 8 x 6,200 82.5 |
+    64.7 us, 1 x 5,000 13.7 | 11.4, 4 x 3,100 23.7 | 21.5, in one split 16 x 5,000 98.5 | 97.4; splits of fewer than 384 keys do not pay (8 heads, 1 x
+    5,000 7.8 | 9.7, 2 x 6,200 9.3 | 12.0).  Up to there 16 x 200 7.5 | 8.5, 16 x 1,000 22.5 | 23.4, 64 x 640 51.1 | 51.7, 8 x 1,000 14.8 | 15.7, but
+    with a block an SM at most and one split 8 x 640 12.1 | 12.0 and 8 x 760 14.3 | 13.8 (a captured step at 640 1,400 | 1,378), 8 x 200 5.0 | 5.7;
+    with a penalty 8 x 200 5.6 | 7.1."""
+    split, heads, splits = plan
+    if max_keys > 2048:
+        return splits == 1 or split >= 384
+    return splits == 1 and max_keys > 512 and not shaped and n_seqs * -(-n_kv_heads // heads) <= sms
+
+
 @functools.lru_cache(maxsize=4096)
 def _choose_even_plan(device: int, n_seqs: int, n_q_heads: int, n_kv_heads: int, max_keys: int, page_size: int,
                       head_dim: int) -> tuple[int, int, int] | None:
@@ -1963,9 +1978,11 @@ def _choose_even_plan(device: int, n_seqs: int, n_q_heads: int, n_kv_heads: int,
     other plan; then splits of 48 to 96 keys as far as a wave reaches (15 over 5, steps with splits of 128 | these: 200 keys 8 sequences
     829 | 720 us, 400 keys 847 | 785; attention of 64 x 7,531 116 | 109, of 8 x 7,531 26.1 | 22.7).
 
-    One query head per kv head: the fewest kv heads per block whose blocks fit into one wave, and where they fill a third of it up to 768
-    keys in one split, which nobody has to merge (8 sequences, a step: 200 keys 1,075 -> 1,017 us, 520 keys 1,162 -> 1,139; attention of
-    64 x 1,000 87 -> 82).  Fewer blocks and short contexts keep the other plan (4 x 520: 1,056 us, equal splits 1,063 to 1,080).
+    One query head per kv head (``single_heads_on_tensor_cores`` says by which kernel): the fewest kv heads per block whose blocks fit into
+    one wave, and where they fill a third of it up to 768 keys in one split, which nobody has to merge (32 heads, the other plan | this one, on
+    CUDA cores: 8 x 200 6.9 | 5.0 us, 8 x 520 12.9 | 10.8, 64 x 200 22.4 | 19.6, 64 x 1,000 82.6 | 78.7).  Pages of 64 tokens and more make
+    long copies of single heads, which the other plan takes (8 x 640, pages of 64: 8.9 | 11.5).  Fewer blocks and short contexts keep the
+    other plan, too.
 
     A wave is filled to 0.9: with 288 of 296 places some blocks waited for the kernel before.  A split's page numbers lie in shared
     memory: splits of more than ``EVEN_SPLIT_PAGES`` would leave room for one block an SM, and of some 25,000 for none."""
@@ -1981,6 +1998,8 @@ def _choose_even_plan(device: int, n_seqs: int, n_q_heads: int, n_kv_heads: int,
         blocks = n_seqs * groups
         if blocks > slots or not lib.erb_attention_decode_even_supported(n_q_heads, n_kv_heads, head_dim, page_size, page_size, heads):
             continue
+        if not grouped and max_keys <= 768 and page_size >= 64:
+            return None
         if not grouped and max_keys <= 768:
             return (-(-max_keys // page_size) * page_size, heads, 1) if blocks >= 0.3 * slots else None
         fewest_keys = 128 if not grouped else 48 if max_keys <= 256 else 96 if 512 < max_keys <= 768 else 64
@@ -2066,8 +2085,10 @@ def attention_decode_bulk(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch
                           scale: float, part_acc: torch.Tensor, part_ml: torch.Tensor, max_splits: int,
                           status: torch.Tensor, split_keys: int = DECODE_SPLIT_KEYS, head_group: int = 0, window: int = 0,
                           keep_first: int = 0, chunk: int = 0, penalty: torch.Tensor | None = None, softcap: float = 0.0,
-                          gate: torch.Tensor | None = None, even: bool = False) -> None:
+                          gate: torch.Tensor | None = None, even: bool = False, tensor_cores: bool | None = None) -> None:
     """``attention_decode`` for bfloat16 with keys and values streamed by bulk asynchronous copies.
+    ``tensor_cores`` (None: as ``even``): heads of 64 with one query head per kv head by the tensor-core kernel; ``even``: there, every
+    sequence in ``max_splits`` equal splits of ``split_keys`` at most.
     ``chunk`` > 0 (instead of a window): the mask of chunks of ``attention_rows``.
     ``window`` > 0: the last ``window`` keys and the first ``keep_first``; the splits are counted from the one
     that holds the window's first key, and the first of them also walks the kept keys.
@@ -2091,7 +2112,8 @@ def attention_decode_bulk(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch
           positions, out, out.stride(0), part_acc, part_ml, max_splits,
           n_seqs, n_q_heads, nkv, d, page_size, int(split_keys), float(scale), status,
           split_counters(q.device, n_seqs * nkv), int(head_group), mask_reach(window, chunk), int(keep_first),
-          _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d), int(bool(even)), _stream())
+          _penalty(penalty, n_q_heads), float(softcap), *_gate(gate, out, n_q_heads * d),
+          (1 if even else 2) if (even if tensor_cores is None else tensor_cores) else 0, _stream())
 
 
 @functools.lru_cache(maxsize=4096)

@@ -122,7 +122,6 @@ def decode_attention(a) -> dict:
         return caches[state["i"]]
 
     q = (torch.randn((a.batch, a.heads * a.head_dim), device="cuda") * float(getattr(a, "q_scale", 1.0) or 1.0)).to(dtype)
-    score = _score_of(a, a.batch, dtype)
     out = torch.empty_like(q)
     pos = torch.full((a.batch,), a.context - 1, dtype=torch.int32, device="cuda")
     tok = torch.arange(a.batch, dtype=torch.int32, device="cuda")
@@ -138,6 +137,10 @@ def decode_attention(a) -> dict:
                                                                           a.kernel != "bulk", granule * a.page)
         a.head_group = a.head_group or heads
     splits = even[2] if even else (a.context - 1) // a.split + 1
+    score = _score_of(a, a.batch, dtype)
+    equal = even is not None and (a.kernel != "bulk" or a.heads != a.kv_heads or kernels.single_heads_on_tensor_cores(
+        even, a.batch, a.kv_heads, bound * a.page, bool(score["penalty"] is not None or score["softcap"] or score["gate"] is not None),
+        kernels._sms(torch.device("cuda"))))
     if window > 0 or chunk > 0:
         splits = min(splits, (window + chunk) // a.split + 2)
     acc_n, ml_n = kernels.decode_scratch_floats(a.batch, a.heads, a.head_dim, splits)
@@ -147,16 +150,16 @@ def decode_attention(a) -> dict:
     if a.kernel == "gqa":
         fn = lambda: kernels.attention_decode_gqa(q, *cache(), tok, pos, out, a.heads, scale, acc, ml, splits,  # noqa: E731
                                                   status, split_keys=a.split, window=window, keep_first=keep, chunk=chunk,
-                                                  even=even is not None, **score)
+                                                  even=equal, **score)
     elif a.kernel == "bulk":
         fn = lambda: kernels.attention_decode_bulk(q, *cache(), tok, pos, out, a.heads, scale, acc, ml, splits,  # noqa: E731
                                                    status, split_keys=a.split, head_group=a.head_group, window=window, keep_first=keep,
-                                                   chunk=chunk, even=even is not None, **score)
+                                                   chunk=chunk, even=equal, **score)
     else:
         fn = lambda: kernels.attention_decode(q, *cache(), tok, pos, out, a.heads, scale, acc, ml, splits,  # noqa: E731
                                               split_keys=a.split, window=window, keep_first=keep, chunk=chunk, **score)
     us = _time(fn, max(a.iters, 2 * reps), a.warmup)
-    return {"case": "decode-attention", "kernel": a.kernel, "split": a.split, "splits": splits, "even": even is not None,
+    return {"case": "decode-attention", "kernel": a.kernel, "split": a.split, "splits": splits, "even": equal,
             "head_group": a.head_group, "us": round(us, 2), "bytes": nbytes, "gbs": round(nbytes / us / 1e3, 1), "frac_hbm": round(nbytes / us / 1e3 / HBM_GBS, 4),
             "status": int(status), "from_dram": bool(a.cold) or nbytes > 126e6, "window": window, "keep_first": keep, "chunk": chunk,
             **_score_record(a)}
@@ -778,7 +781,7 @@ def main(argv=None) -> int:
     d.add_argument("--context", type=int, default=8192)
     d.add_argument("--split", type=int, default=0, help="keys per split; 0: the engine's choice for this batch")
     d.add_argument("--kernel", choices=["bulk", "gqa", "general"], default="bulk",
-                   help="the entry point; for heads of 64 with one query head per kv head the bulk one runs the tensor-core kernel of gqa")
+                   help="the entry point; heads of 64 with one query head per kv head take the tensor-core kernel of gqa through the bulk one where the engine does")
     d.add_argument("--head-group", type=int, default=0, help="kv heads per block of the bulk kernel; 0: its own choice")
     d.add_argument("--cold", action="store_true", help="rotate over several caches so that none is found in L2")
     p = sub.add_parser("prefill-attention", parents=[common, att])

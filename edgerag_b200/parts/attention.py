@@ -293,9 +293,15 @@ class Attention(Mixer):
             even = None                 # every sequence in equal splits
             if not ctx.batch_invariant and reach_mask <= 0 and self.dtype == torch.bfloat16:
                 even = kernels.choose_even_plan(nd, self.n_q, self.n_kv, ctx.max_keys_bound(), ctx.page_size, d)
+            on_tensor_cores = even is not None      # (of one query head per kv head; grouped heads always are)
             if even is not None:
                 split, heads_per_block, max_splits = even
-            elif ctx.batch_invariant:   # one plan for every batch: a sequence's sums are then added in one order
+                if self.n_q == self.n_kv:
+                    on_tensor_cores = kernels.single_heads_on_tensor_cores(
+                        even, nd, self.n_kv, ctx.max_keys_bound(), bool(self.penalty is not None or self.softcap or gate is not None), kernels._sms(x.device))
+            elif ctx.batch_invariant:   # one plan and one kernel for every batch: a sequence's sums are then added in one order
+                # (32 heads, one query head each, CUDA cores | tensor cores: 1 x 640 18.1 | 16.0 us, 1 x 2,000 18.5 | 16.4, 8 x 640 18.9 | 17.7,
+                # 8 x 4,000 48.4 | 50.3, 64 x 200 22.0 | 24.3)
                 split, heads_per_block = kernels.DECODE_SPLIT_KEYS, 0
             elif reach_mask > 0:        # a token reads its window (or chunk) and the kept keys, however long its context is
                 reach = min(ctx.max_keys_bound(), -(-(reach_mask + self.keep_first) // ctx.page_size) * ctx.page_size)
@@ -321,7 +327,8 @@ class Attention(Mixer):
                 kernels.attention_decode_bulk(q_rows, k_pages, v_pages, tables, tokens, ctx.positions,
                                               out_rows, self.n_q, self.scale, part_acc, part_ml, max_splits, ctx.status,
                                               split_keys=split, head_group=heads_per_block, window=self.window,
-                                              keep_first=self.keep_first, chunk=self.chunk, gate=head_gate, even=even is not None, **score)
+                                              keep_first=self.keep_first, chunk=self.chunk, gate=head_gate, even=even is not None and on_tensor_cores,
+                                              tensor_cores=on_tensor_cores or (ctx.batch_invariant and reach_mask <= 0), **score)
             else:
                 kernels.attention_decode(q_rows, k_pages, v_pages, tables, tokens, ctx.positions,
                                          out_rows, self.n_q, self.scale, part_acc, part_ml, max_splits,

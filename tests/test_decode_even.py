@@ -69,8 +69,8 @@ def test_the_plan_of_equal_splits(nq, nkv):
     assert K.choose_even_plan(8, nq, nkv, 1024, 16, 128) is None and K.choose_even_plan(8, nq, nkv, 1024, 12, 64) is None
 
 
-@pytest.mark.parametrize("batch,nq,nkv,context,kernel", [(64, 15, 5, 700, "gqa"), (8, 32, 32, 1000, "bulk")])
-def test_the_timed_launch_is_the_engines(batch, nq, nkv, context, kernel):
+@pytest.mark.parametrize("batch,nq,nkv,context,kernel,equal", [(64, 15, 5, 700, "gqa", True), (8, 32, 32, 1000, "bulk", False), (8, 32, 32, 2500, "bulk", True)])
+def test_the_timed_launch_is_the_engines(batch, nq, nkv, context, kernel, equal):
     """The program that times one kernel takes the splits that a step of these sequences takes."""
     from argparse import Namespace
 
@@ -80,4 +80,4 @@ def test_the_timed_launch_is_the_engines(batch, nq, nkv, context, kernel):
                   cold=False, iters=2, warmup=1, sequential_pages=False)
     out = microbench.decode_attention(a)
     split, heads, splits = K.choose_even_plan(batch, nq, nkv, K.context_bound(-(-context // 16))[0] * 16, 16, 64)
-    assert (out["split"], out["head_group"], out["splits"], out["even"], out["status"]) == (split, heads, splits, True, 0)
+    assert (out["split"], out["head_group"], out["splits"], out["even"], out["status"]) == (split, heads, splits, equal, 0)
