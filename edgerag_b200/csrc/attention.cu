@@ -189,9 +189,9 @@ attention_rows_kernel(const T* __restrict__ q, int q_row_stride, const T* __rest
 // position 0), and the groups' maxima, sums and accumulators are put together at the end in the groups' order.  So a row's result still depends on
 // nothing but its own keys.
 // Bound by the reads of shared memory and the multiplications, about alike, and for few blocks by a tile's chain (5 us), which is why
-// there are groups.  9 heads of 64 over 3 kv heads, row kernel | one group | two: 333 tokens 93 | 34 | 26.7 us, 96 tokens 16.1 | 14.8 | 12.2,
+// there are groups.  9 heads of 64 over 3 kv heads, row kernel | one group | two: 333 tokens 94 | 34 | 26 us, 96 tokens 15 | 14.8 | 11.1,
 // 333 behind 7,000 2,896 | 613 | 459, 2,048 tokens 2,354 | 357 | 329; 8 heads of 128, 333 behind 100 246 | 69 | 56.  (Four groups of 128 threads
-// with four rows each: 2,048 tokens 276, but 16 portions of 32 tokens 12.8 instead of 9.3.)
+// with four rows each: 2,048 tokens 276, but 16 portions of 32 tokens 12.8 instead of 8.5.)
 // ---------------------------------------------------------------------------------------------
 constexpr int kTileRows = 32, kTileKeys = 64, kTileThreads = 256, kTileGroups = 2;       // (threads of a group)
 template <int D> __host__ __device__ constexpr int tile_group_floats() { return 2 * kTileKeys * (D + 4) + kTileRows * (kTileKeys + 4); }

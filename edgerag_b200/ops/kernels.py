@@ -1976,7 +1976,9 @@ def _choose_even_plan(device: int, n_seqs: int, n_q_heads: int, n_kv_heads: int,
 
     Several query heads per kv head: up to 128 keys one split (9 over 3, 90 keys: a step of 452 us in one split, 519 in two), so the
     other plan; then splits of 48 to 96 keys as far as a wave reaches (15 over 5, steps with splits of 128 | these: 200 keys 8 sequences
-    829 | 720 us, 400 keys 847 | 785; attention of 64 x 7,531 116 | 109, of 8 x 7,531 26.1 | 22.7).
+    829 | 720 us, 400 keys 847 | 785; attention of 64 x 7,531 116 | 109, of 8 x 7,531 26.1 | 22.7).  The merge takes eight splits at a time,
+    so the bounds up to 1,024 get 8 or 16 of them: 64 keys for 512 and 1,024, 96 for the one between (attention of 8 x 640 in splits of 48 |
+    64 | 96 | 128: 15 over 5 12.4 | 10.4 | 9.1 | 10.4 us, 9 over 3 8.6 | 7.3 | 6.7 | 7.3; of 8 x 1,000 12.8 | 10.1 | 12.2 | 11.3).
 
     One query head per kv head (``single_heads_on_tensor_cores`` says by which kernel): the fewest kv heads per block whose blocks fit into
     one wave, and where they fill a third of it up to 768 keys in one split, which nobody has to merge (32 heads, the other plan | this one, on

@@ -356,10 +356,13 @@ class Attention(Mixer):
         return self._project_out(out, ctx)
 
     def _tiled(self, ctx) -> bool:
-        """Whether the step's portions are long enough that the 32-bit kernel for 32 tokens at a time takes them: 9 heads of 64, a
-        portion without a past, by rows | by tiles: 64 tokens 9.1 | 10.3 us, 96 tokens 16.1 | 12.2, 333 tokens 93 | 26.7; behind 7,000
-        tokens from the first; several portions share a block one after the other (512 tokens in portions of 17 15.6 | 19.6, of 32
-        20.8 | 9.6)."""
+        """Whether the step's portions are long enough that the 32-bit kernel for 32 tokens at a time takes them.  A portion without a
+        past, by rows | by tiles: 9 heads of 64 64 tokens 8.0 | 8.4 us, 72 10.8 | 10.1, 96 14.8 | 11.1, 333 94 | 26; 32 heads 32 tokens 8.8 |
+        8.4; 3 heads 72 tokens 9.7 | 10.0, 96 10.8 | 11.1, 128 13.5 | 11.4; so the line lies where the tiles lose nothing to speak of with
+        few heads.  Behind 500 tokens and more the tiles are the faster ones from the first on (17 behind 7,000 609 | 425), which this rule
+        leaves: a prompt's last, short portion.  Several portions share a block one after the other, 9 heads: 17 x 30 tokens 14.4 | 19.0,
+        24 x 20 16.5 | 13.6, 28 x 8 11.6 | 13.7, 32 x 8 13.1 | 8.5, 32 x 16 19.7 | 8.5, and of portions that 32 does not divide 40 x 4 11.0 |
+        13.7, 48 x 2 9.1 | 13.7."""
         lens = ctx.host_q_len[ctx.n_decode:]
         return not ctx.batch_invariant and sum(lens) >= 96 and sum(lens) >= 32 * len(lens)
 
