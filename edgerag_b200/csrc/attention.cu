@@ -185,20 +185,25 @@ attention_rows_kernel(const T* __restrict__ q, int q_row_stride, const T* __rest
 // time and then onto the accumulator, so that its rounding is no worse than that of the row kernel's 32 partial sums.
 // Tiles start at absolute multiples of 64 positions, and a tile that a row does not see changes nothing of it: a row's
 // result does not depend on the other tokens.  Tokens of several sequences in a block are taken one sequence after the other.
-// A block has two groups of 256 threads, each with buffers of its own: one walks the even tiles, one the odd ones (counted from
-// position 0), and the groups' maxima, sums and accumulators are put together at the end in the groups' order.  So a row's result still depends on
-// nothing but its own keys.
+// The even tiles and the odd ones (counted from position 0) are walked apart, and the two maxima, sums and accumulators are put together at
+// the end in that order, so that a row's result depends on nothing but its own keys.  A block has two groups of 256 threads, each with
+// buffers of its own, for the two halves, or one group, which walks one after the other: the same bits.  One group, two blocks an SM, where
+// there are many blocks, or more than SMs with walks so short that one of two groups would often stand idle (the caller counts; 32 heads, one
+// group | two: 16 portions of 32 tokens 21.4 | 31.1 us, 2 of 333 89 | 98, 2,048 tokens 926 | 1,008).
 // Bound by the reads of shared memory and the multiplications, about alike, and for few blocks by a tile's chain (5 us), which is why
-// there are groups.  9 heads of 64 over 3 kv heads, row kernel | one group | two: 333 tokens 94 | 34 | 26 us, 96 tokens 15 | 14.8 | 11.1,
-// 333 behind 7,000 2,896 | 613 | 459, 2,048 tokens 2,354 | 357 | 329; 8 heads of 128, 333 behind 100 246 | 69 | 56.  (Four groups of 128 threads
+// there are two groups.  9 heads of 64 over 3 kv heads, row kernel | one group | two: 333 tokens 94 | 31 | 26 us, 96 tokens 15 | 13.5 | 11.1,
+// 333 behind 7,000 2,896 | 613 | 459, 2,048 tokens 2,354 | 345 | 329; 8 heads of 128, 333 behind 100 246 | 69 | 56.  (Four groups of 128 threads
 // with four rows each: 2,048 tokens 276, but 16 portions of 32 tokens 12.8 instead of 8.5.)
 // ---------------------------------------------------------------------------------------------
-constexpr int kTileRows = 32, kTileKeys = 64, kTileThreads = 256, kTileGroups = 2;       // (threads of a group)
+constexpr int kTileRows = 32, kTileKeys = 64, kTileThreads = 256, kTileParts = 2;       // (threads of a group; even and odd tiles)
 template <int D> __host__ __device__ constexpr int tile_group_floats() { return 2 * kTileKeys * (D + 4) + kTileRows * (kTileKeys + 4); }
-template <int D> constexpr size_t tile_smem() { return sizeof(float) * (kTileRows * (D + 4) + kTileGroups * tile_group_floats<D>()); }
+template <int D> __host__ __device__ constexpr int tile_part_floats() { return 2 * (2 + 4 * (D / 64)) + 1; }      // of a thread, odd: no bank conflicts
+template <int D, int GROUPS> constexpr size_t tile_smem() {
+  return sizeof(float) * (kTileRows * (D + 4) + GROUPS * tile_group_floats<D>() + (GROUPS == 1 ? kTileThreads * tile_part_floats<D>() : 0));
+}
 
-template <int D>
-__global__ void __launch_bounds__(kTileGroups * kTileThreads, 1)
+template <int D, int GROUPS>
+__global__ void __launch_bounds__(GROUPS * kTileThreads, kTileParts / GROUPS)
 attention_tile_kernel(const float* __restrict__ q, int q_row_stride, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
                       const int* __restrict__ block_tables, int max_pages, const int* __restrict__ seq_of_token,
                       const int* __restrict__ positions, float* __restrict__ out, int out_row_stride, int n_tokens, int nq, int nkv,
@@ -215,7 +220,7 @@ attention_tile_kernel(const float* __restrict__ q, int q_row_stride, const float
   const int t0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kTileRows, n_here = min(kTileRows, n_tokens - t0);   // (the longest walks first)
   const int h = blockIdx.y, kvh = h / (nq / nkv);
   const int tid = threadIdx.x % kTileThreads, lane = tid & 31, tx = tid & 15, r0 = 2 * (tid >> 4);
-  for (int i = threadIdx.x; i < kTileRows * D; i += kTileGroups * kTileThreads) {
+  for (int i = threadIdx.x; i < kTileRows * D; i += GROUPS * kTileThreads) {
     const int r = i / D, d = i % D;
     q_s[r * LD + d] = r < n_here ? q[(size_t)(t0 + r) * q_row_stride + (size_t)h * D + d] : 0.f;
   }
@@ -237,162 +242,163 @@ attention_tile_kernel(const float* __restrict__ q, int q_row_stride, const float
     const int hi = __reduce_max_sync(0xffffffffu, in ? pos_l : INT_MIN), pos_min = __reduce_min_sync(0xffffffffu, in ? pos_l : INT_MAX);
     const int lo = __reduce_min_sync(0xffffffffu, in ? lo_l : INT_MAX), lo_max = __reduce_max_sync(0xffffffffu, in ? lo_l : INT_MIN);
     const int* bt = block_tables + (size_t)seq * max_pages;
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, acc[2][4 * kGroups];
-#pragma unroll
-    for (int i = 0; i < 4 * kGroups; ++i) acc[0][i] = acc[1][i] = 0.f;
-    for (int j = 0; j * kTileKeys <= hi; ++j) {
-      if (j * kTileKeys >= keep_first) j = max(j, lo / kTileKeys);         // past the kept first keys: on to the first that a row sees
-      if (j % kTileGroups != group) continue;
-      const int k0 = j * kTileKeys;
-      group_sync();                                                         // (the tile before is done with)
-      constexpr int kRowsAtOnce = 4 * kTileThreads / D, kBatch = 4;       // rows that the group's threads copy at a time
-      const int r_own = tid / (D / 4), c = 4 * (tid % (D / 4));
-#pragma unroll
-      for (int first = 0; first < kTileKeys; first += kRowsAtOnce * kBatch) {
-        int page[kBatch];                        // (the loads of several rows under way at once: their pages, then keys and values)
-        float4 kv[kBatch], vv[kBatch];
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-          const int k = k0 + first + i * kRowsAtOnce + r_own;
-          page[i] = k <= hi ? bt[page_shift >= 0 ? k >> page_shift : k / page_size] : -1;
-        }
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-          const int k = k0 + first + i * kRowsAtOnce + r_own;
-          kv[i] = vv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (page[i] >= 0) {
-            const size_t row = (((size_t)page[i] * nkv + kvh) * page_size + (page_shift >= 0 ? k & (page_size - 1) : k % page_size)) * D + c;
-            kv[i] = *reinterpret_cast<const float4*>(k_pages + row);
-            vv[i] = *reinterpret_cast<const float4*>(v_pages + row);
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-          const int r = first + i * kRowsAtOnce + r_own;
-          *reinterpret_cast<float4*>(k_s + r * LD + c) = kv[i];
-          *reinterpret_cast<float4*>(v_s + r * LD + c) = vv[i];
-        }
-      }
-      group_sync();
-      const bool whole = k0 + kTileKeys - 1 <= pos_min && (k0 >= lo_max || k0 + kTileKeys <= keep_first);    // every row sees every key
-      float s[2][4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) s[0][u] = s[1][u] = 0.f;
-#pragma unroll 4
-      for (int d = 0; d < D; d += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(q_s + r0 * LD + d), b = *reinterpret_cast<const float4*>(q_s + (r0 + 1) * LD + d);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float4 k4 = *reinterpret_cast<const float4*>(k_s + (tx + 16 * u) * LD + d);
-          s[0][u] = fmaf(a.x, k4.x, s[0][u]); s[0][u] = fmaf(a.y, k4.y, s[0][u]); s[0][u] = fmaf(a.z, k4.z, s[0][u]); s[0][u] = fmaf(a.w, k4.w, s[0][u]);
-          s[1][u] = fmaf(b.x, k4.x, s[1][u]); s[1][u] = fmaf(b.y, k4.y, s[1][u]); s[1][u] = fmaf(b.z, k4.z, s[1][u]); s[1][u] = fmaf(b.w, k4.w, s[1][u]);
-        }
-      }
-      float alpha[2];
+    float m[2], l[2], acc[2][4 * kGroups];
+    // where a thread leaves what the odd tiles gave: of two groups the second one's buffers, whose tiles are done with by then
+    float* odd = q_s + kTileRows * LD + tile_group_floats<D>() + tid * tile_part_floats<D>();
+    auto leave = [&]() {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int pos = i ? pos1 : pos0, first = i ? lo1 : lo0;
-        bool seen[4];
-        float top = m[i];
+        odd[i] = m[i];
+        odd[2 + i] = l[i];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int k = k0 + tx + 16 * u;
-          seen[u] = whole || (k <= pos && (k >= first || k < keep_first));
-          float v = fmaf(s[i][u], scale, -pen.at(seen[u] ? pos - k : 0));
-          if (softcap > 0.f) v = softcap * tanhf(v / softcap);
-          s[i][u] = v;
-          if (seen[u]) top = fmaxf(top, v);
-        }
-#pragma unroll
-        for (int o = 8; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        alpha[i] = m[i] == top ? 1.f : expf(m[i] - top);
-        m[i] = top;
-        const float ref = top == -INFINITY ? 0.f : top;
-        float sum = 0.f;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float p = s[i][u] == ref ? 1.f : expf(s[i][u] - ref);
-          if (seen[u]) sum += p;
-          p_s[(r0 + i) * LP + tx + 16 * u] = seen[u] ? p : -1.f;           // (below 0: not seen, whatever its value holds)
-        }
-        l[i] = l[i] * alpha[i] + sum;
+        for (int c = 0; c < 4 * kGroups; ++c) odd[4 + 4 * kGroups * i + c] = acc[i][c];
       }
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < 4 * kGroups; ++i) { acc[0][i] *= alpha[0]; acc[1][i] *= alpha[1]; }
-      auto products = [&](auto masked) {
+    };
 #pragma unroll 1
-        for (int k1 = 0; k1 < kTileKeys; k1 += 32) {
-          float part[2][4 * kGroups];
+    for (int walk = GROUPS == 1 ? kTileParts - 1 : group; walk >= (GROUPS == 1 ? 0 : group); --walk) {
 #pragma unroll
-          for (int i = 0; i < 4 * kGroups; ++i) part[0][i] = part[1][i] = 0.f;
-#pragma unroll 2
-          for (int k = k1; k < k1 + 32; k += 4) {
-            float p[2][4];
-            *reinterpret_cast<float4*>(p[0]) = *reinterpret_cast<const float4*>(p_s + r0 * LP + k);
-            *reinterpret_cast<float4*>(p[1]) = *reinterpret_cast<const float4*>(p_s + (r0 + 1) * LP + k);
+      for (int i = 0; i < 2; ++i) { m[i] = -INFINITY; l[i] = 0.f; }
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+      for (int i = 0; i < 4 * kGroups; ++i) acc[0][i] = acc[1][i] = 0.f;
+      for (int j = 0; j * kTileKeys <= hi; ++j) {
+        if (j * kTileKeys >= keep_first) j = max(j, lo / kTileKeys);         // past the kept first keys: on to the first that a row sees
+        if (j % kTileParts != walk) continue;
+        const int k0 = j * kTileKeys;
+        group_sync();                                                         // (the tile before is done with)
+        constexpr int kRowsAtOnce = 4 * kTileThreads / D, kBatch = 4;       // rows that the group's threads copy at a time
+        const int r_own = tid / (D / 4), c = 4 * (tid % (D / 4));
 #pragma unroll
-              for (int g = 0; g < kGroups; ++g) {
-                float v[4];
-                *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(v_s + (k + u) * LD + 64 * g + 4 * tx);
+        for (int first = 0; first < kTileKeys; first += kRowsAtOnce * kBatch) {
+          int page[kBatch];                        // (the loads of several rows under way at once: their pages, then keys and values)
+          float4 kv[kBatch], vv[kBatch];
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                  if (decltype(masked)::value && p[i][u] < 0.f) continue;
-#pragma unroll
-                  for (int c = 0; c < 4; ++c) part[i][4 * g + c] = fmaf(p[i][u], v[c], part[i][4 * g + c]);
-                }
-              }
+          for (int i = 0; i < kBatch; ++i) {
+            const int k = k0 + first + i * kRowsAtOnce + r_own;
+            page[i] = k <= hi ? bt[page_shift >= 0 ? k >> page_shift : k / page_size] : -1;
           }
 #pragma unroll
-          for (int i = 0; i < 4 * kGroups; ++i) { acc[0][i] += part[0][i]; acc[1][i] += part[1][i]; }
+          for (int i = 0; i < kBatch; ++i) {
+            const int k = k0 + first + i * kRowsAtOnce + r_own;
+            kv[i] = vv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (page[i] >= 0) {
+              const size_t row = (((size_t)page[i] * nkv + kvh) * page_size + (page_shift >= 0 ? k & (page_size - 1) : k % page_size)) * D + c;
+              kv[i] = *reinterpret_cast<const float4*>(k_pages + row);
+              vv[i] = *reinterpret_cast<const float4*>(v_pages + row);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < kBatch; ++i) {
+            const int r = first + i * kRowsAtOnce + r_own;
+            *reinterpret_cast<float4*>(k_s + r * LD + c) = kv[i];
+            *reinterpret_cast<float4*>(v_s + r * LD + c) = vv[i];
+          }
         }
-      };
-      if (whole) products(std::false_type{}); else products(std::true_type{});
-    }
+        group_sync();
+        const bool whole = k0 + kTileKeys - 1 <= pos_min && (k0 >= lo_max || k0 + kTileKeys <= keep_first);    // every row sees every key
+        float s[2][4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+        for (int u = 0; u < 4; ++u) s[0][u] = s[1][u] = 0.f;
+#pragma unroll 4
+        for (int d = 0; d < D; d += 4) {
+          const float4 a = *reinterpret_cast<const float4*>(q_s + r0 * LD + d), b = *reinterpret_cast<const float4*>(q_s + (r0 + 1) * LD + d);
 #pragma unroll
-      for (int o = 8; o; o >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], o);
-    {                                            // the groups' parts of these rows, put together by the first one
-      constexpr int kPart = 2 * (2 + 4 * kGroups);
-      __syncthreads();                           // (the tiles are done with: their room holds the parts)
-      float* part = q_s + kTileRows * LD + tid * (kPart + 1);
-      if (group > 0) {
-        float* mine = part + group * tile_group_floats<D>();
+          for (int u = 0; u < 4; ++u) {
+            const float4 k4 = *reinterpret_cast<const float4*>(k_s + (tx + 16 * u) * LD + d);
+            s[0][u] = fmaf(a.x, k4.x, s[0][u]); s[0][u] = fmaf(a.y, k4.y, s[0][u]); s[0][u] = fmaf(a.z, k4.z, s[0][u]); s[0][u] = fmaf(a.w, k4.w, s[0][u]);
+            s[1][u] = fmaf(b.x, k4.x, s[1][u]); s[1][u] = fmaf(b.y, k4.y, s[1][u]); s[1][u] = fmaf(b.z, k4.z, s[1][u]); s[1][u] = fmaf(b.w, k4.w, s[1][u]);
+          }
+        }
+        float alpha[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          mine[i] = m[i];
-          mine[2 + i] = l[i];
-#pragma unroll
-          for (int c = 0; c < 4 * kGroups; ++c) mine[4 + 4 * kGroups * i + c] = acc[i][c];
-        }
-      }
-      __syncthreads();
-      if (group == 0) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
+          const int pos = i ? pos1 : pos0, first = i ? lo1 : lo0;
+          bool seen[4];
           float top = m[i];
-          for (int g = 1; g < kTileGroups; ++g) top = fmaxf(top, part[g * tile_group_floats<D>() + i]);
-          const float ref = top == -INFINITY ? 0.f : top;
-          // (a maximum of +inf is its own: its part's sum holds such keys with weight 1)
-          const float f0 = m[i] == top ? 1.f : expf(m[i] - ref);
-          l[i] *= f0;
 #pragma unroll
-          for (int c = 0; c < 4 * kGroups; ++c) acc[i][c] *= f0;
-          for (int g = 1; g < kTileGroups; ++g) {
-            const float* from = part + g * tile_group_floats<D>();
-            if (from[i] == -INFINITY && from[2 + i] == 0.f) continue;      // (saw no key of this row)
-            const float f = from[i] == top ? 1.f : expf(from[i] - ref);
-            l[i] = fmaf(from[2 + i], f, l[i]);
-#pragma unroll
-            for (int c = 0; c < 4 * kGroups; ++c) acc[i][c] = fmaf(from[4 + 4 * kGroups * i + c], f, acc[i][c]);
+          for (int u = 0; u < 4; ++u) {
+            const int k = k0 + tx + 16 * u;
+            seen[u] = whole || (k <= pos && (k >= first || k < keep_first));
+            float v = fmaf(s[i][u], scale, -pen.at(seen[u] ? pos - k : 0));
+            if (softcap > 0.f) v = softcap * tanhf(v / softcap);
+            s[i][u] = v;
+            if (seen[u]) top = fmaxf(top, v);
           }
+#pragma unroll
+          for (int o = 8; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+          alpha[i] = m[i] == top ? 1.f : expf(m[i] - top);
+          m[i] = top;
+          const float ref = top == -INFINITY ? 0.f : top;
+          float sum = 0.f;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float p = s[i][u] == ref ? 1.f : expf(s[i][u] - ref);
+            if (seen[u]) sum += p;
+            p_s[(r0 + i) * LP + tx + 16 * u] = seen[u] ? p : -1.f;           // (below 0: not seen, whatever its value holds)
+          }
+          l[i] = l[i] * alpha[i] + sum;
         }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4 * kGroups; ++i) { acc[0][i] *= alpha[0]; acc[1][i] *= alpha[1]; }
+        auto products = [&](auto masked) {
+#pragma unroll 1
+          for (int k1 = 0; k1 < kTileKeys; k1 += 32) {
+            float part[2][4 * kGroups];
+#pragma unroll
+            for (int i = 0; i < 4 * kGroups; ++i) part[0][i] = part[1][i] = 0.f;
+#pragma unroll 2
+            for (int k = k1; k < k1 + 32; k += 4) {
+              float p[2][4];
+              *reinterpret_cast<float4*>(p[0]) = *reinterpret_cast<const float4*>(p_s + r0 * LP + k);
+              *reinterpret_cast<float4*>(p[1]) = *reinterpret_cast<const float4*>(p_s + (r0 + 1) * LP + k);
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int g = 0; g < kGroups; ++g) {
+                  float v[4];
+                  *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(v_s + (k + u) * LD + 64 * g + 4 * tx);
+#pragma unroll
+                  for (int i = 0; i < 2; ++i) {
+                    if (decltype(masked)::value && p[i][u] < 0.f) continue;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) part[i][4 * g + c] = fmaf(p[i][u], v[c], part[i][4 * g + c]);
+                  }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4 * kGroups; ++i) { acc[0][i] += part[0][i]; acc[1][i] += part[1][i]; }
+          }
+        };
+        if (whole) products(std::false_type{}); else products(std::true_type{});
       }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int o = 8; o; o >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], o);
+      if (GROUPS == 1 && walk > 0) leave();
+    }
+    if (GROUPS > 1) {
+      __syncthreads();                           // (the tiles are done with)
+      if (group > 0) leave();
       __syncthreads();
     }
+    if (group == 0) {                            // both parts of these rows
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float top = fmaxf(m[i], odd[i]), ref = top == -INFINITY ? 0.f : top;
+        // (a maximum of +inf is its own: its part's sum holds such keys with weight 1)
+        const float f0 = m[i] == top ? 1.f : expf(m[i] - ref);
+        l[i] *= f0;
+#pragma unroll
+        for (int c = 0; c < 4 * kGroups; ++c) acc[i][c] *= f0;
+        if (odd[i] == -INFINITY && odd[2 + i] == 0.f) continue;            // (saw no key of this row)
+        const float f = odd[i] == top ? 1.f : expf(odd[i] - ref);
+        l[i] = fmaf(odd[2 + i], f, l[i]);
+#pragma unroll
+        for (int c = 0; c < 4 * kGroups; ++c) acc[i][c] = fmaf(odd[4 + 4 * kGroups * i + c], f, acc[i][c]);
+      }
+    }
+    if (GROUPS > 1) __syncthreads();             // (the next run's tiles come into that room)
     if (group > 0) continue;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -411,17 +417,17 @@ attention_tile_kernel(const float* __restrict__ q, int q_row_stride, const float
   }
 }
 
-template <int D>
+template <int D, int GROUPS>
 int launch_tiles(const void* q, int q_row_stride, const void* k_pages, const void* v_pages, const int* block_tables, int max_pages,
                  const int* seq_of_token, const int* positions, void* out, int out_row_stride, int n_tokens, int nq, int nkv, int page_size,
                  int window, int keep_first, float scale, const float* penalty, float softcap, const void* gate, int gate_stride,
                  cudaStream_t s) {
   const dim3 grid((n_tokens + kTileRows - 1) / kTileRows, nq);
-  auto kern = attention_tile_kernel<D>;
-  constexpr size_t smem = tile_smem<D>();
+  auto kern = attention_tile_kernel<D, GROUPS>;
+  constexpr size_t smem = tile_smem<D, GROUPS>();
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "attention_rows: %s", cudaGetErrorString(e));
-  launch_chained(kern, grid, dim3(kTileGroups * kTileThreads), smem, s, (const float*)q, q_row_stride,
+  launch_chained(kern, grid, dim3(GROUPS * kTileThreads), smem, s, (const float*)q, q_row_stride,
                  (const float*)k_pages, (const float*)v_pages, block_tables, max_pages, seq_of_token, positions, (float*)out, out_row_stride,
                  n_tokens, nq, nkv, page_size, window, keep_first, scale, penalty, softcap, (const float*)gate, gate_stride);
   return check_launch("attention_tile");
@@ -620,7 +626,7 @@ int check_common(const char* who, int nq, int nkv, int head_dim, int page_size, 
 
 // q: [n_tokens, ...] with `q_row_stride` elements between rows, head h at column h * head_dim.
 // out: the same shape convention.  block_tables: int32 [n_seqs, max_pages].  tiled: the tokens are portions of prompts, for the kernel
-// that takes 32 neighbouring ones together (32 bits, heads of 64 and 128; else without meaning).
+// that takes 32 neighbouring ones together (32 bits, heads of 64 and 128; else without meaning); 2: heads of 64 by one group of threads a block.
 ERB_EXPORT int erb_attention_rows(const void* q, int q_row_stride, const void* k_pages, const void* v_pages,
                                   const int* block_tables, int max_pages, const int* seq_of_token,
                                   const int* positions, void* out, int out_row_stride, int n_tokens, int nq,
@@ -633,9 +639,9 @@ ERB_EXPORT int erb_attention_rows(const void* q, int q_row_stride, const void* k
   cudaStream_t s = (cudaStream_t)stream;
 #if ERB_ELEM == 0
   if (tiled && (head_dim == 64 || head_dim == 128) && !(((uintptr_t)k_pages | (uintptr_t)v_pages) & 15))
-    return (head_dim == 64 ? launch_tiles<64> : launch_tiles<128>)(q, q_row_stride, k_pages, v_pages, block_tables, max_pages, seq_of_token,
-                                                                   positions, out, out_row_stride, n_tokens, nq, nkv, page_size, window,
-                                                                   window > 0 ? keep_first : 0, scale, penalty, softcap, gate, gate_stride, s);
+    return (head_dim == 128 ? launch_tiles<128, 2> : tiled == 2 ? launch_tiles<64, 1> : launch_tiles<64, 2>)(
+        q, q_row_stride, k_pages, v_pages, block_tables, max_pages, seq_of_token, positions, out, out_row_stride, n_tokens, nq, nkv, page_size,
+        window, window > 0 ? keep_first : 0, scale, penalty, softcap, gate, gate_stride, s);
 #endif
   ERB_DISPATCH_D(launch_rows, q, q_row_stride, k_pages, v_pages, block_tables, max_pages, seq_of_token,
                  positions, out, out_row_stride, n_tokens, nq, nkv, page_size, window, window > 0 ? keep_first : 0, scale, penalty,

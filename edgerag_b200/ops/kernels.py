@@ -1802,13 +1802,37 @@ def _gate(gate: torch.Tensor | None, out: torch.Tensor, width: int) -> tuple[int
     return gate.data_ptr(), gate.stride(0) if gate.shape[0] > 1 else max(width, gate.stride(0))
 
 
+@functools.lru_cache(maxsize=1024)
+def one_group_pays(lens: tuple, lasts: tuple, reach: int, n_q_heads: int, sms: int) -> bool:
+    """Whether 32-bit portions (lengths, last positions; ``reach`` > 0: the keys that a row's mask lets it see) with heads of 64 are better walked by
+    two blocks of one group of threads an SM than by one block of two groups for the even and the odd tiles.  From four and a quarter blocks
+    an SM on they are (one group | two: 32 heads, 1,000 tokens 274 | 291 us, 2,048 926 | 1,008; 16 heads, 2,048 518 | 534; but 9 heads, 2,048
+    345 | 329).  Below that where walks are so short that one of the two groups often stands idle: a pair of tiles takes two groups 7.6 us, a tile
+    of each of two blocks 8.1 us (32 heads, 16 portions of 32 21.4 | 31.1, behind 100 tokens 50.1 | 61.9, 2 of 333 89 | 98; 32 heads, 333 behind
+    500 162 | 146).  Hardly more blocks than SMs: only where every walk is one tile (4 portions of 40 18.9 | 21.1, behind 500 tokens 135 | 116)."""
+    first, rows = [], []        # per run of a block: its first position, its rows
+    filled = 0
+    for n, last in zip(lens, lasts):
+        at = last - n + 1
+        while at <= last:
+            take = min(32 - filled % 32, last - at + 1)
+            first.append(at), rows.append(take)
+            at, filled = at + take, filled + take
+    walks = [(a + n - 1) // 64 - (max(0, a - reach + 1) // 64 if reach > 0 else 0) + 1 for a, n in zip(first, rows)]
+    blocks = -(-filled // 32) * n_q_heads
+    if blocks > 4.25 * sms:
+        return True
+    return blocks > (sms if max(walks) == 1 else 1.5 * sms) and 8.1 / 2 * sum(walks) < 7.6 * sum((w + 1) // 2 for w in walks)
+
+
 def attention_rows(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, block_tables: torch.Tensor,
                    seq_of_token: torch.Tensor, positions: torch.Tensor, out: torch.Tensor, n_q_heads: int,
                    scale: float, window: int = 0, keep_first: int = 0, chunk: int = 0,
                    penalty: torch.Tensor | None = None, softcap: float = 0.0, gate: torch.Tensor | None = None,
-                   tiled: bool = False) -> None:
+                   tiled: int = 0) -> None:
     """Causal attention of every token over its sequence's pages (general kernel, any portion sizes).
-    ``tiled``: the tokens are portions of prompts and may be taken 32 neighbouring ones together (float32, heads of 64 and 128).
+    ``tiled``: the tokens are portions of prompts and may be taken 32 neighbouring ones together (float32, heads of 64 and 128);
+    2: of heads of 64 by one group of threads a block, where ``one_group_pays`` (the same bits).
     ``window`` > 0: a query sees the last ``window`` keys (its own included) and the first ``keep_first`` of the sequence.
     ``chunk`` > 0 (instead of a window): a query sees the earlier keys of its own run of ``chunk`` positions, runs
     counted from position 0 of the sequence.  ``penalty`` float ``[2, n_q_heads]`` (``r1``, then ``r2`` of every query

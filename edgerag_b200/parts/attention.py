@@ -355,7 +355,7 @@ class Attention(Mixer):
                                    gate=gate if gate is None else gate[nd:], tiled=self._tiled(ctx), **score)
         return self._project_out(out, ctx)
 
-    def _tiled(self, ctx) -> bool:
+    def _tiled(self, ctx) -> int:
         """Whether the step's portions are long enough that the 32-bit kernel for 32 tokens at a time takes them.  A portion without a
         past, by rows | by tiles: 9 heads of 64 64 tokens 8.0 | 8.4 us, 72 10.8 | 10.1, 96 14.8 | 11.1, 333 94 | 26; 32 heads 32 tokens 8.8 |
         8.4; 3 heads 72 tokens 9.7 | 10.0, 96 10.8 | 11.1, 128 13.5 | 11.4; so the line lies where the tiles lose nothing to speak of with
@@ -364,7 +364,11 @@ class Attention(Mixer):
         24 x 20 16.5 | 13.6, 28 x 8 11.6 | 13.7, 32 x 8 13.1 | 8.5, 32 x 16 19.7 | 8.5, and of portions that 32 does not divide 40 x 4 11.0 |
         13.7, 48 x 2 9.1 | 13.7."""
         lens = ctx.host_q_len[ctx.n_decode:]
-        return not ctx.batch_invariant and sum(lens) >= 96 and sum(lens) >= 32 * len(lens)
+        if ctx.batch_invariant or sum(lens) < 96 or sum(lens) < 32 * len(lens):
+            return 0
+        one_group = self.head_dim == 64 and self.dtype == torch.float32 and kernels.one_group_pays(
+            tuple(lens), tuple(ctx.host_positions_last[ctx.n_decode:]), self.window or self.chunk, self.n_q, kernels._sms(self.device))
+        return 2 if one_group else 1
 
     def _project_out(self, out: torch.Tensor, ctx) -> torch.Tensor:
         n = out.shape[0]

@@ -81,3 +81,20 @@ def test_tokens_together_as_alone(dim, heads, kv, page, portions, how):
         out = torch.empty(n - 17, heads * dim, device="cuda")
         K.attention_rows(*cut, out, heads, scale, penalty=cuda(penalty), gate=cuda(gate)[17:] if gate is not None else None, tiled=True, **how)
         assert torch.equal(out.cpu(), together[17:])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", [{}, {"window": 70, "keep_first": 5}, {"chunk": 100}, {"softcap": 20.0}])
+@pytest.mark.parametrize("lens,pasts", [([96], [0]), ([32, 32, 33], [0, 100, 31]), ([200, 7, 65], [300, 0, 64])])
+def test_one_group_of_threads_gives_the_bits_of_two(how, lens, pasts):
+    """The even and the odd key tiles one after the other or side by side, blocks of one and of several requests."""
+    from test_kernels import paged_case
+
+    case = paged_case(torch.float32, 9, 6, 2, 64, 16, [n + p for n, p in zip(lens, pasts)], lens)
+    dev = [case[n].cuda() for n in ("q", "kp", "vp", "tables", "seq_of", "pos")]
+    outs = []
+    for tiled in (1, 2):
+        out = torch.full_like(dev[0], float("nan"))
+        K.attention_rows(*dev, out, 6, 0.125, tiled=tiled, **how)
+        outs.append(out)
+    assert torch.isfinite(outs[0]).all() and torch.equal(*outs)
