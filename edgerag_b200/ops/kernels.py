@@ -1984,11 +1984,11 @@ def single_heads_on_tensor_cores(plan: tuple[int, int, int], n_seqs: int, n_kv_h
     64.7 us, 1 x 5,000 13.7 | 11.4, 4 x 3,100 23.7 | 21.5, in one split 16 x 5,000 98.5 | 97.4; splits of fewer than 384 keys do not pay (8 heads, 1 x
     5,000 7.8 | 9.7, 2 x 6,200 9.3 | 12.0).  Up to there 16 x 200 7.5 | 8.5, 16 x 1,000 22.5 | 23.4, 64 x 640 51.1 | 51.7, 8 x 1,000 14.8 | 15.7, but
     with a block an SM at most and one split 8 x 640 12.1 | 12.0 and 8 x 760 14.3 | 13.8 (a captured step at 640 1,400 | 1,378), 8 x 200 5.0 | 5.7;
-    with a penalty 8 x 200 5.6 | 7.1."""
+    with a penalty 8 x 200 5.6 | 7.1; and with eight heads a block 64 x 1,300 101.6 | 101.1 (a step of 64 x 1,000 4,032 | 4,002)."""
     split, heads, splits = plan
     if max_keys > 2048:
         return splits == 1 or split >= 384
-    return splits == 1 and max_keys > 512 and not shaped and n_seqs * -(-n_kv_heads // heads) <= sms
+    return splits == 1 and not shaped and (heads >= 8 and max_keys > 768 or max_keys > 512 and n_seqs * -(-n_kv_heads // heads) <= sms)
 
 
 @functools.lru_cache(maxsize=4096)

@@ -24,7 +24,8 @@ def test_a_launch_says_which_kernel(monkeypatch, how, expected):
 @pytest.mark.parametrize("plan,n_seqs,heads,bound,shaped,wanted", [
     ((4096, 2, 2), 8, 32, 8192, False, True), ((8192, 8, 1), 64, 32, 8192, True, True), ((512, 2, 16), 1, 32, 8192, False, True),
     ((128, 2, 48), 1, 8, 5120, False, False), ((768, 2, 1), 8, 32, 768, False, True), ((768, 2, 1), 8, 32, 768, True, False),
-    ((256, 2, 1), 8, 32, 256, False, False), ((768, 2, 1), 16, 32, 768, False, False), ((1024, 2, 2), 8, 32, 2048, False, False)])
+    ((256, 2, 1), 8, 32, 256, False, False), ((768, 2, 1), 16, 32, 768, False, False), ((1024, 2, 2), 8, 32, 2048, False, False),
+    ((1024, 8, 1), 64, 32, 1024, False, True), ((1024, 4, 1), 32, 32, 1024, False, False), ((768, 8, 1), 64, 32, 768, False, False)])
 def test_where_the_tensor_cores_pay(plan, n_seqs, heads, bound, shaped, wanted):
     assert kernels.single_heads_on_tensor_cores(plan, n_seqs, heads, bound, shaped, 148) is wanted
 
