@@ -210,6 +210,22 @@ __device__ __forceinline__ Two silu_two(Two v) {
   return v * Two(0.25f) * fma2(y, r, y);
 }
 
+// The nth request (from 0) with more than one token, or -1; the whole warp asks.
+__device__ __forceinline__ int nth_portion(const int* __restrict__ seq_starts, int n_seqs, int nth) {
+  const int lane = threadIdx.x & 31;
+  for (int s0 = 0; s0 < n_seqs; s0 += 32) {
+    const int s = s0 + lane;
+    unsigned more = __ballot_sync(0xffffffffu, s < n_seqs && seq_starts[min(s, n_seqs - 1) + 1] - seq_starts[min(s, n_seqs - 1)] > 1);
+    const int here = __popc(more);
+    if (nth < here) {
+      for (; nth > 0; --nth) more &= more - 1;
+      return s0 + __ffs(more) - 1;
+    }
+    nth -= here;
+  }
+  return -1;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -672,13 +672,15 @@ __global__ void __launch_bounds__((kChunkWarps + kCopyWarps) * 32)
 delta_chunk_kernel(const __nv_bfloat16* __restrict__ qkv, int channels, const ChunkRecord* __restrict__ records, float* __restrict__ state,
                    const int* __restrict__ seq_starts, const int* __restrict__ state_slots, float* __restrict__ out, int H, int G, int dv,
                    const __nv_bfloat16* __restrict__ proj, int ld, int off_b, int off_a, const float* __restrict__ dt_bias,
-                   const float* __restrict__ a_log, float q_scale, int* __restrict__ status) {
+                   const float* __restrict__ a_log, float q_scale, int n_seqs, int* __restrict__ status) {
   chain_wait();
   extern __shared__ __align__(16) unsigned char smem_all[];
   unsigned char* smem_raw = smem_all + ((1024u - (smem_u32(smem_all) & 1023u)) & 1023u);
   typedef DeltaChunkSmem<D> Smem;
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
-  const int h = blockIdx.x, seq = blockIdx.y, p0 = blockIdx.z * kChunkCols, kh = h / (H / G);
+  const int h = blockIdx.x, p0 = blockIdx.z * kChunkCols, kh = h / (H / G);
+  const int seq = (int)gridDim.y == n_seqs ? (int)blockIdx.y : nth_portion(seq_starts, n_seqs, blockIdx.y);
+  if (seq < 0) return;
   const int start = seq_starts[seq], n_tok = seq_starts[seq + 1] - start;
   if (n_tok <= 1) return;                                      // (a single token is walked)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qr = lane >> 2, qc = lane & 3;
@@ -931,12 +933,13 @@ inline bool chunks_pay(int blocks, int n_tokens, int n_seqs, int longest) {
 ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, int ld, int off_b, int off_a,
                               const float* dt_bias, const float* a_log, float* state, const int* seq_starts,
                               const int* state_slots, float* out, float* scratch, long long scratch_floats, int n_seqs, int n_tokens,
-                              int longest, int H, int G, int d, int dv, int* status, void* stream) {
+                              int longest, int portions, int H, int G, int d, int dv, int* status, void* stream) {
   if (n_seqs <= 0 || n_tokens <= 0) return ERB_OK;
   if (H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 || d > 32 * kDeltaRows)
     return fail(ERB_ERR_ARG, "delta_scan: bad sizes (%d heads over %d, keys of %d up to %d)", H, G, d, 32 * kDeltaRows);
   if (channels < 2 * G * d + H * dv) return fail(ERB_ERR_ARG, "delta_scan: rows too narrow");
   if (!scratch || ((uintptr_t)scratch & 15)) return fail(ERB_ERR_ARG, "delta_scan: the scratch must be 16-byte aligned");
+  if (portions <= 0 || portions > n_seqs) portions = n_seqs;
   bool singles = false;                  // whether the walk is left with the requests of one token
   int walk_tokens = n_tokens;
 #if ERB_ELEM == 1
@@ -948,7 +951,7 @@ ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, i
     const size_t prep_bytes = d == 64 ? sizeof(DeltaPrepSmem<64>) : sizeof(DeltaPrepSmem<128>);
     cudaError_t e = cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_bytes);
     if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "delta_scan: %s", cudaGetErrorString(e));
-    launch_chained(prep, dim3(H, n_tokens / kChunk + n_seqs), dim3(kChunkPrepWarps * 32), prep_bytes, (cudaStream_t)stream, (const elem_t*)qkv,
+    launch_chained(prep, dim3(H, (n_tokens - (n_seqs - portions)) / kChunk + portions), dim3(kChunkPrepWarps * 32), prep_bytes, (cudaStream_t)stream, (const elem_t*)qkv,
                    channels, (const elem_t*)proj, ld, off_b, off_a, dt_bias, a_log, seq_starts, n_seqs, records, H, G, 1.f / sqrtf((float)d));
     int rc = check_launch("delta_chunk_prepare");
     if (rc) return rc;
@@ -956,9 +959,9 @@ ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, i
     auto kern = d == 64 ? delta_chunk_kernel<64> : delta_chunk_kernel<128>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "delta_scan: %s", cudaGetErrorString(e));
-    launch_chained(kern, dim3(H, n_seqs, dv / kChunkCols), dim3((kChunkWarps + kCopyWarps) * 32), bytes, (cudaStream_t)stream, (const elem_t*)qkv,
+    launch_chained(kern, dim3(H, portions, dv / kChunkCols), dim3((kChunkWarps + kCopyWarps) * 32), bytes, (cudaStream_t)stream, (const elem_t*)qkv,
                    channels, records, state, seq_starts, state_slots, out, H, G, dv, (const elem_t*)proj, ld, off_b, off_a, dt_bias, a_log,
-                   1.f / sqrtf((float)d), status);
+                   1.f / sqrtf((float)d), n_seqs, status);
     if ((rc = check_launch("delta_chunk")) || n_seqs == 1) return rc;
     singles = true;
     walk_tokens = n_seqs;

@@ -12,7 +12,7 @@
 //
 // A request's tokens of one step are neighbours in the batch (rows seq_starts[s] .. seq_starts[s+1]),
 // its slot is state_slots[s].  Every (request, head, block of columns) is scanned by exactly one block: token after token, or
-// (bfloat16, the sizes of ssm_chunk_kernel) 128 tokens at a time as products of matrices.
+// (bfloat16, the sizes of ssm_chunk_kernel) 128 or 64 tokens at a time as products of matrices.
 #include <limits.h>
 #include <math.h>
 #include <stddef.h>
@@ -516,9 +516,12 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
                  int channels, const __nv_bfloat16* __restrict__ proj, int ld, int off_dt, const float* __restrict__ dt_bias,
                  const float* __restrict__ a_log, const float* __restrict__ d_skip, float* __restrict__ state,
                  const int* __restrict__ seq_starts, const int* __restrict__ state_slots, float* __restrict__ y, int H, int P, int G,
-                 int* __restrict__ status) {
+                 int n_seqs, int* __restrict__ status) {
   chain_wait();
-  const int h = blockIdx.x, seq = blockIdx.y, p0 = blockIdx.z * kChunkCols;
+  // (a block of single tokens would hold an SM's shared memory for half a microsecond only to leave: 31 of them beside a portion 14 us)
+  const int h = blockIdx.x, p0 = blockIdx.z * kChunkCols;
+  const int seq = (int)gridDim.y == n_seqs ? (int)blockIdx.y : nth_portion(seq_starts, n_seqs, blockIdx.y);
+  if (seq < 0) return;
   const int start = seq_starts[seq], n_tok = seq_starts[seq + 1] - start;
   if (n_tok <= 1) return;                                      // (a single token: the scan kernel's)
   extern __shared__ uint8_t smem_raw[];
@@ -529,7 +532,8 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_chunks = (n_tok + kChunk - 1) / kChunk;
   // G there; the weights' pieces of the chunk's first and last 64 tokens; the weighted x's; dS there; Y there; the state's pieces; a stage's rows
-  // (two); the outputs of the chunk before read; those stored and the next chunk's steps there; the first half of Y1 there
+  // (two); the outputs of the chunk before read; those stored and the next chunk's steps there; the first half of Y1 from the
+  // two smaller pieces there
   constexpr int kBarG = 0, kBarP1 = 1, kBarP2 = 2, kBarW = 3, kBarD = 4, kBarY = 5, kBarS = 6, kBarL = 7, kBarR = 9, kBarT = 10, kBarH = 11;
   auto bar = [&](int which) { return smem_u32(&sm.bars[which]); };
   volatile int* abort_flag = &sm.abort;
@@ -758,14 +762,12 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
         mma_bf16(tm + half * kColG, dc + (k >> 2) * kBlock + 2 * (k & 3), db + (k >> 2) * kBlock + 2 * (k & 3), kIdescG, i > 0);
       }
     };
-    auto issue_y1 = [&](uint64_t dx, int half) {               // the part of Y1 from half of the chunk's tokens, the smallest pieces first
+    auto issue_y1 = [&](uint64_t dx, int half, int p) {        // the part of Y1 from a piece of the weights for half of the chunk's tokens
 #pragma unroll
-      for (int p = 2; p >= 0; --p)
-#pragma unroll
-        for (int i = 0; i < kChunk / 32; ++i) {
-          const int k = half * (kChunk / 32) + i;
-          mma_bf16_a_tmem(tm + kColY1, tm + col_m(k, p), dx + 64 * k, kIdesc1, half || p < 2 || i > 0);
-        }
+      for (int i = 0; i < kChunk / 32; ++i) {
+        const int k = half * (kChunk / 32) + i;
+        mma_bf16_a_tmem(tm + kColY1, tm + col_m(k, p), dx + 64 * k, kIdesc1, half || p < 2 || i > 0);
+      }
     };
     if (wait(kBarS, 0) && wait(kBarL, 0)) {
       fence_after_sync();
@@ -795,25 +797,30 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
 #pragma unroll
         for (int k = 0; k < kChunk / 16; ++k) mma_bf16(tm + kColD, db + 128 * k, dw + 64 * k, kIdescT, k > 0);
         mma_commit(bar(kBarD));                                // (the state's pieces have been read, too)
-        issue_y1(dx, 0);
+        issue_y1(dx, 0, 2);                                    // (the smallest pieces first)
+        issue_y1(dx, 0, 1);
         mma_commit(bar(kBarH));
+        issue_y1(dx, 0, 0);
       }
       __syncwarp();
-      if (!wait(kBarP2, c & 1)) break;
-      fence_after_sync();
-      if (elected) {
-        issue_y1(dx, 1);
-        mma_commit(bar(kBarY));
-      }
-      __syncwarp();
+      // G's second sum lies over the two smaller pieces of these weights, and nothing says that products of other shapes and sums are finished
+      // in the order of issue: it waits for their commit.  The weights for the second half are still being made meanwhile.
       if (!wait(kBarH, c & 1)) break;
       if (more) {
-        // G's second sum lies over weights that the first half of Y1 read (products of other shapes and sums: nothing says that they are
-        // finished in the order of issue); the second half is still under way meanwhile
         if (!wait(kBarL + (st ^ 1), ((c + 1) >> 1) & 1)) break;
         fence_after_sync();
         if (elected) issue_g(c + 1, 1);
         __syncwarp();
+      }
+      if (!wait(kBarP2, c & 1)) break;
+      fence_after_sync();
+      if (elected) {
+#pragma unroll
+        for (int p = 2; p >= 0; --p) issue_y1(dx, 1, p);
+        mma_commit(bar(kBarY));
+      }
+      __syncwarp();
+      if (more) {
         if (!wait(kBarS, (c + 1) & 1)) break;                  // (dS has been read)
         fence_after_sync();
         if (elected) {
@@ -878,20 +885,12 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
         if (i > w) sm.rise[st][i - 1][r] = rise[i - 1];
       sm.weight[st][r] = weight;
     };
-    const bool on_16 = ((uintptr_t)y & 15) == 0;               // (8 at least)
     auto store = [&](int c) {                                  // the outputs of chunk c: eight lanes a token, whole lines
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int t = 32 * w + 4 * i + (lane >> 3), e = 4 * (lane & 7);
-        if (c * kChunk + t >= n_tok) continue;
-        const float4 v = *reinterpret_cast<const float4*>(&sm.out[t][e]);
-        float* to = y + (size_t)(start + c * kChunk + t) * inner + h * P + p0 + e;
-        if (on_16) {
-          *reinterpret_cast<float4*>(to) = v;
-        } else {
-          *reinterpret_cast<float2*>(to) = make_float2(v.x, v.y);
-          *reinterpret_cast<float2*>(to + 2) = make_float2(v.z, v.w);
-        }
+        if (c * kChunk + t < n_tok)
+          *reinterpret_cast<float4*>(y + (size_t)(start + c * kChunk + t) * inner + h * P + p0 + e) = *reinterpret_cast<const float4*>(&sm.out[t][e]);
       }
     };
     const bool copies = w == 0 && lane == 0;
@@ -941,6 +940,277 @@ ssm_chunk_kernel(const __grid_constant__ CUtensorMap map_bc, const __grid_consta
   if (holds) {
 #pragma unroll
     for (int i = 0; i < 8; i += 2) *reinterpret_cast<float2*>(s_glob + i) = make_float2(S[i], S[i + 1]);
+  }
+}
+
+// The same sums 64 tokens at a time with mma.sync, for portions of at most 64 tokens (longer ones it takes, too, a chunk after the other): without
+// TMEM to fetch and give back, copies through descriptors and a chunk of 128 rows, of which half or more would be zeros, a portion of up to 64
+// tokens takes 7.5 us instead of 10.0 (64 heads of 64 x 128; 8 of 32 x 32 5.1 | 6.9), eight of 40 46.1 | 64.1, one of 64 beside 31 single tokens 41.6 |
+// 56.2; at 65 tokens and more the kernel above is as fast or faster (300 tokens 23 | 14).
+// Block: one (head, request, 32 columns), 16 warps of products and one that makes the next chunk's steps and decays; the state stays in the
+// accumulators' registers.  Between the two barriers of a chunk the work is cut into pieces of about the same length: first 10 of the warps make a
+// tile of the weights (C B^T below the diagonal) each, the others the weighted x, and every warp 16 rows x 8 columns of the part of y that comes from
+// the state; then the same 16 x 8 of the part within the chunk, and 16 rows of the state.  What is not finite is walked, as above.
+constexpr int kShortChunk = 64, kShortWarps = 16;
+
+template <int N>
+struct ShortSmem {
+  static constexpr int LdN = N + 8, LdP = kChunkCols + 8, LdM = kShortChunk + 8;   // rows 16 bytes longer than a power of two: no bank conflicts
+  __nv_bfloat16 c[2][kShortChunk][LdN];
+  __nv_bfloat16 b[2][kShortChunk][LdN];
+  __nv_bfloat16 x[2][kShortChunk][LdP];
+  __nv_bfloat16 s[3][N][LdP];                                  // the state before the chunk, in pieces
+  __nv_bfloat16 w[3][kShortChunk][LdP];                             // the weighted x, in pieces
+  __nv_bfloat16 m[3][kShortChunk][LdM];                             // the weights of the sum within the chunk, in pieces (tiles above the diagonal unused)
+  float dt[2][kShortChunk], hi[2][kShortChunk], lo[2][kShortChunk];           // step, c_t / ln 2 in two floats
+  float grown[2][kShortChunk], weight[2][kShortChunk];                   // exp(c_t), dt_t exp(c_64 - c_t)
+  float total[2];                                              // exp(c_64)
+};
+
+template <int N>
+__global__ void __launch_bounds__((kShortWarps + 1) * 32)
+ssm_short_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const __nv_bfloat16* __restrict__ proj, int ld, int off_dt,
+                 const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
+                 float* __restrict__ state, const int* __restrict__ seq_starts, const int* __restrict__ state_slots,
+                 float* __restrict__ y, int H, int P, int G, int n_seqs) {
+  chain_wait();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ShortSmem<N>& sm = *reinterpret_cast<ShortSmem<N>*>(smem_raw);
+  const int h = blockIdx.x, p0 = blockIdx.z * kChunkCols;
+  const int seq = (int)gridDim.y == n_seqs ? (int)blockIdx.y : nth_portion(seq_starts, n_seqs, blockIdx.y);
+  if (seq < 0) return;
+  const int start = seq_starts[seq], n_tok = seq_starts[seq + 1] - start;
+  if (n_tok <= 1) return;                                      // (a single token: the scan kernel's)
+  const int g = h / (H / G), inner = H * P;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qr = lane >> 2, qc = lane & 3;
+  const int n_chunks = (n_tok + kShortChunk - 1) / kShortChunk;
+  const __nv_bfloat16* rows = xbc + (size_t)start * channels;
+
+  auto load_stage = [&](int c) {                               // the threads of the products
+    const int buf = c & 1, c0 = c * kShortChunk;
+    for (int idx = threadIdx.x; idx < kShortChunk * (N / 8); idx += kShortWarps * 32) {
+      const int r = idx / (N / 8), e = 8 * (idx % (N / 8));
+      const bool real = c0 + r < n_tok;
+      const __nv_bfloat16* src = rows + (size_t)(real ? c0 + r : 0) * channels + inner + g * N + e;
+      copy16_or_zero(&sm.b[buf][r][e], src, real);
+      copy16_or_zero(&sm.c[buf][r][e], src + G * N, real);
+    }
+    if (threadIdx.x < kShortChunk * (kChunkCols / 8)) {
+      const int r = threadIdx.x / (kChunkCols / 8), e = 8 * (threadIdx.x % (kChunkCols / 8));
+      const bool real = c0 + r < n_tok;
+      copy16_or_zero(&sm.x[buf][r][e], rows + (size_t)(real ? c0 + r : 0) * channels + h * P + p0 + e, real);
+    }
+    copy_commit();
+  };
+  const float a = -expf(a_log[h]), bias = dt_bias[h];
+  auto make_steps = [&](int c) {                               // the last warp: tokens 2 lane and 2 lane + 1 of chunk c
+    const int buf = c & 1, t0 = c * kShortChunk + 2 * lane;
+    float dt[2];
+    double la[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      dt[i] = t0 + i < n_tok ? softplus_f(__bfloat162float(proj[(size_t)(start + t0 + i) * ld + off_dt + h]) + bias) : 0.f;
+      la[i] = (double)a * (double)dt[i];
+    }
+    double sum = la[0] + la[1];                                // inclusive scan over the lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
+    }
+    const double all = __shfl_sync(0xffffffffu, sum, 31);
+    const double cum[2] = {sum - la[1], sum};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = 2 * lane + i;
+      const double l2 = cum[i] * 1.4426950408889634;
+      const float hi = (float)l2;
+      sm.dt[buf][r] = dt[i];
+      sm.hi[buf][r] = hi;
+      sm.lo[buf][r] = (float)(l2 - (double)hi);
+      sm.grown[buf][r] = (float)exp(cum[i]);
+      sm.weight[buf][r] = (float)((double)dt[i] * exp(all - cum[i]));
+    }
+    if (lane == 0) sm.total[buf] = (float)exp(all);
+  };
+
+  // the state: warp w holds rows 16 (w mod N/16) .. + 15, columns 8 NTW (w div N/16) .. + 8 NTW - 1
+  constexpr int kRowTiles = N / 16, kColGroups = kShortWarps / kRowTiles < 4 ? kShortWarps / kRowTiles : 4, NTW = 4 / kColGroups;
+  const bool holds_state = warp < kRowTiles * kColGroups;
+  const int s_row = 16 * (warp % kRowTiles), s_col = 8 * NTW * (warp / kRowTiles);
+  float S[NTW][4];
+  float* s_glob = state + ((size_t)state_slots[seq] * H + h) * N * P + p0;
+  auto publish = [&]() {                                       // the state's pieces to shared memory
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        uint32_t piece[3];
+        split_pair(S[nt][2 * j], S[nt][2 * j + 1], piece);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          *reinterpret_cast<uint32_t*>(&sm.s[k][s_row + qr + 8 * j][s_col + 8 * nt + 2 * qc]) = piece[k];
+      }
+  };
+  if (warp < kShortWarps) load_stage(0);
+  else make_steps(0);
+  if (holds_state) {
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float2 v = *reinterpret_cast<const float2*>(s_glob + (size_t)(s_row + qr + 8 * j) * P + s_col + 8 * nt + 2 * qc);
+        S[nt][2 * j] = v.x;
+        S[nt][2 * j + 1] = v.y;
+      }
+    publish();
+  }
+  const int y_row = 16 * (warp >> 2), y_col = 8 * (warp & 3);
+  // the tile of the weights that a warp makes: warps 0 .. 9 take the tiles (row, column) on and below the diagonal
+  const int m_tr = warp < 1 ? 0 : warp < 3 ? 1 : warp < 6 ? 2 : 3;
+  const int m_row = 16 * m_tr, m_col = 16 * (warp - m_tr * (m_tr + 1) / 2);
+  const float dskip = d_skip[h];
+  float probe = 0.f;                                           // no number once a result was not finite
+  for (int c = 0; c < n_chunks; ++c) {
+    const int buf = c & 1;
+    if (warp < kShortWarps) copy_wait<0>();
+    __syncthreads();                                           // chunk c's rows, steps and state pieces are there; stage c - 1 is free
+    if (warp == kShortWarps) {
+      if (c + 1 < n_chunks) make_steps(c + 1);
+      __syncthreads();
+      continue;
+    }
+    if (c + 1 < n_chunks) load_stage(c + 1);
+    // the part of y that comes from the state
+    float inter[3][4] = {};
+#pragma unroll
+    for (int k = 0; k < N / 16; k += 2) {
+      uint32_t cf[2][4], b[3][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) ldmatrix4(cf[i], &sm.c[buf][y_row + (lane & 15)][16 * (k + i) + 8 * (lane >> 4)]);
+#pragma unroll
+      for (int piece = 0; piece < 3; ++piece) ldmatrix4t(b[piece], &sm.s[piece][16 * k + lane][y_col]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) mma16816(inter[piece], cf[i], b[piece][2 * i], b[piece][2 * i + 1]);
+    }
+    if (warp < 10) {                                           // a tile of the weights
+      float gram[2][2][4] = {};                                // (two chains: a product does not wait for the one before it)
+#pragma unroll
+      for (int k = 0; k < N / 16; ++k) {
+        uint32_t cf[4], b[4];
+        ldmatrix4(cf, &sm.c[buf][m_row + (lane & 15)][16 * k + 8 * (lane >> 4)]);
+        ldmatrix4(b, &sm.b[buf][m_col + (lane & 7) + 8 * (lane >> 4)][16 * k + 8 * ((lane >> 3) & 1)]);
+        mma16816(gram[k & 1][0], cf, b[0], b[1]);
+        mma16816(gram[k & 1][1], cf, b[2], b[3]);
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        const int s = m_col + 8 * nt + 2 * qc;
+        const float2 hs = *reinterpret_cast<const float2*>(&sm.hi[buf][s]), ls = *reinterpret_cast<const float2*>(&sm.lo[buf][s]);
+        const float2 ds = *reinterpret_cast<const float2*>(&sm.dt[buf][s]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int r = m_row + qr + 8 * j;
+          const float hi = sm.hi[buf][r], lo = sm.lo[buf][r];
+          const float v0 = s <= r ? (gram[0][nt][2 * j] + gram[1][nt][2 * j]) * ds.x * exp2f((hi - hs.x) + (lo - ls.x)) : 0.f;
+          const float v1 = s + 1 <= r ? (gram[0][nt][2 * j + 1] + gram[1][nt][2 * j + 1]) * ds.y * exp2f((hi - hs.y) + (lo - ls.y)) : 0.f;
+          uint32_t piece[3];
+          split_pair(v0, v1, piece);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&sm.m[k][r][s]) = piece[k];
+        }
+      }
+    } else {                                                   // weighted x in pieces: 4 columns of one token at a time
+      for (int idx = threadIdx.x - 320; idx < kShortChunk * (kChunkCols / 4); idx += 192) {
+        const int r = idx >> 3, e = 4 * (idx & 7);
+        float v[4];
+        Pack4<__nv_bfloat16>::load(&sm.x[buf][r][e], v);
+        const float f = sm.weight[buf][r];
+        uint32_t p01[3], p23[3];
+        split_pair(f * v[0], f * v[1], p01);
+        split_pair(f * v[2], f * v[3], p23);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(&sm.w[k][r][e]) = make_uint2(p01[k], p23[k]);
+      }
+    }
+    __syncthreads();                                           // weights and weighted x are complete; nobody reads the state's pieces any more
+    float add[3][NTW][4] = {};
+    if (holds_state) {
+#pragma unroll
+      for (int k = 0; k < kShortChunk / 16; ++k) {
+        uint32_t bt[4], b[3][4];                               // B^T: 16 state rows x 16 tokens
+        ldmatrix4t(bt, &sm.b[buf][16 * k + (lane & 7) + 8 * (lane >> 4)][s_row + 8 * ((lane >> 3) & 1)]);
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) {
+          if (NTW == 2) ldmatrix4t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col + 8 * (lane >> 4)]);
+          else ldmatrix2t(b[piece], &sm.w[piece][16 * k + (lane & 15)][s_col]);
+        }
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece)
+#pragma unroll
+          for (int nt = 0; nt < NTW; ++nt) mma16816(add[piece][nt], bt, b[piece][2 * nt], b[piece][2 * nt + 1]);
+      }
+    }
+    float intra[3][4] = {};                                    // the part of y from the chunk's own tokens
+    for (int k = 0; k <= (warp >> 2); k += 2) {
+      uint32_t xb[4], mf[3][4];
+      ldmatrix4t(xb, &sm.x[buf][16 * k + lane][y_col]);        // (rows 16 k .. + 31: the second half may lie behind the diagonal)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (k + i > (warp >> 2)) break;
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) ldmatrix4(mf[piece], &sm.m[piece][y_row + (lane & 15)][16 * (k + i) + 8 * (lane >> 4)]);
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) mma16816(intra[piece], mf[piece], xb[2 * i], xb[2 * i + 1]);
+      }
+    }
+    if (holds_state) {
+      const float total = sm.total[buf];
+#pragma unroll
+      for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[nt][i] = fmaf(total, S[nt][i], (add[2][nt][i] + add[1][nt][i]) + add[0][nt][i]);
+      publish();
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int r = y_row + qr + 8 * j, col = y_col + 2 * qc;
+      if (c * kShortChunk + r < n_tok) {
+        const float grown = sm.grown[buf][r];
+        const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&sm.x[buf][r][col]));
+        float v[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int q = 2 * j + i;
+          const float before = (inter[2][q] + inter[1][q]) + inter[0][q], own = (intra[2][q] + intra[1][q]) + intra[0][q];
+          v[i] = fmaf(grown, before, own) + dskip * (i ? xv.y : xv.x);
+          probe = fmaf(v[i], 0.f, probe);
+        }
+        *reinterpret_cast<float2*>(y + (size_t)(start + c * kShortChunk + r) * inner + h * P + p0 + col) = make_float2(v[0], v[1]);
+      }
+    }
+  }
+  if (holds_state) {
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) probe = fmaf(S[nt][i], 0.f, probe);
+  }
+  if (__syncthreads_or(!(probe == 0.f))) {
+    static_assert(scan_smem(N, kChunkCols, N / 8) <= sizeof(ShortSmem<N>) && N / 8 * kChunkCols <= kShortWarps * 32, "the walk has room");
+    scan_tokens<__nv_bfloat16, 8, true>(reinterpret_cast<float*>(smem_raw), xbc, channels, proj, ld, off_dt, dt_bias, a_log, d_skip, state,
+                                        seq_starts, state_slots, y, H, P, N, G, kChunkCols, h, seq, p0);
+    return;
+  }
+  if (holds_state) {
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        *reinterpret_cast<float2*>(s_glob + (size_t)(s_row + qr + 8 * j) * P + s_col + 8 * nt + 2 * qc) =
+            make_float2(S[nt][2 * j], S[nt][2 * j + 1]);
   }
 }
 #endif  // ERB_ELEM == 1
@@ -1013,20 +1283,24 @@ gated_group_norm_vec_kernel(const void* __restrict__ x_, int x_ld, const T* __re
 }
 
 #if ERB_ELEM == 1
-// Whether the chunk kernel is the faster one: the two costs in microseconds, fitted to both kernels' times over 1 to 64
-// requests of 2 to 2,048 tokens (64 heads of 64 x 128 and 32 of 64 x 64; of 196 pairs measured one is decided wrongly, 33.4 us against 30.3).
-// The walk costs 0.27 us a token of the longest portion or, when the GPU is full, its blocks' tokens and states; a chunk of 128 tokens
-// costs 2.8 us for the longest portion, or as many rounds of blocks as the SMs need, a block an SM.  One request: from 25 tokens on
-// (64 x 128; 24 tokens 9.9 us walked, 10.3 in a chunk; 32 11.7 | 10.2; 64 20.6 | 10.2); 32 requests of equal length: from about 40.
-inline bool chunks_pay(int blocks, int N, int n_tokens, int n_seqs, int longest) {
-  if (longest <= 1) return false;
+// Which form is the fastest: a chunk's tokens of the kernel that takes portions in chunks, 0 for the walk.  The costs in microseconds, fitted to the
+// kernels' times over 1 to 64 requests of 2 to 2,048 tokens (64 heads of 64 x 128 and 32 of 64 x 64; of 196 pairs measured one is decided
+// wrongly, 33.4 us against 30.3).  The walk costs 0.27 us a token of the longest portion or, when the GPU is full, its blocks' tokens and states;
+// a chunk of 128 tokens costs 2.8 us for the longest portion, or as many rounds of blocks as the SMs need, a block an SM.  Portions of at most 64
+// tokens take the kernel for those (its header), at its latency or its blocks.  One request: from 17 tokens on (64 x 128: 16 tokens 6.7 us walked,
+// 7.1 in a chunk; 20 8.5 | 7.3; 8 of 32 x 32: 16 5.9 | 5.0); eight of 24 tokens are walked (41.8 | 45.5), of 32 not (52.0 | 45.8).
+inline int chunk_of(int blocks, int N, int n_tokens, int n_seqs, int longest) {
+  if (longest <= 1) return 0;
   const double size = N / 128.0, extra = (double)n_tokens - n_seqs - (longest - 1);      // tokens beyond one of the other requests
   const double others = fmax(0.0, extra < n_seqs - 1 ? extra : n_seqs - 1);
-  const double longest_chunks = (longest + kChunk - 1) / kChunk, chunks = longest_chunks + (others > 0.0 ? others + extra / kChunk : 0.0);
   const double walk = fmax(3.0 + 0.27 * longest, blocks * size * (0.00165 * n_tokens + 0.008 * n_seqs));
+  if (longest <= kShortChunk) {
+    const double busy = 0.036 * blocks * (1.0 + (others > 0.0 ? others + extra / kShortChunk : 0.0));
+    return fmax(4.6 + 2.75 * size, busy) < fmax(3.0 + 0.27 * longest, blocks * size * (0.0015 * n_tokens + 0.008 * n_seqs)) ? kShortChunk : 0;
+  }
+  const double longest_chunks = (longest + kChunk - 1) / kChunk, chunks = longest_chunks + (others > 0.0 ? others + extra / kChunk : 0.0);
   const double rounds = ceil(blocks * (1.0 + others) / sm_count());
-  const double chunked = fmax(7.0 + 2.7 * longest_chunks, rounds * (2.6 + 2.8 * size + 2.9 * chunks / (1.0 + others)));
-  return chunked < walk;
+  return fmax(7.0 + 2.7 * longest_chunks, rounds * (2.6 + 2.8 * size + 2.9 * chunks / (1.0 + others))) < walk ? kChunk : 0;
 }
 #endif
 
@@ -1069,14 +1343,29 @@ ERB_EXPORT int erb_conv_state_update(const void* proj, int n_seqs, int ld, int o
 
 ERB_EXPORT int erb_ssm_scan(const void* xbc, int channels, const void* proj, int ld, int off_dt, const float* dt_bias,
                             const float* a_log, const float* d_skip, float* state, const int* seq_starts,
-                            const int* state_slots, float* y, int n_seqs, int n_tokens, int longest, int H, int P, int N, int G, int* status,
-                            void* stream) {
+                            const int* state_slots, float* y, int n_seqs, int n_tokens, int longest, int portions, int H, int P, int N, int G,
+                            int* status, void* stream) {
   if (n_seqs <= 0) return ERB_OK;
   if (H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G || P > 512) return fail(ERB_ERR_ARG, "ssm_scan: bad sizes (columns of at most 512)");
+  if (portions <= 0 || portions > n_seqs) portions = n_seqs;
   int most_tokens = INT_MAX;            // what the scan takes: every portion, or single tokens beside the chunk kernel's portions
 #if ERB_ELEM == 1
-  if ((N == 32 || N == 64 || N == 128) && P % kChunkCols == 0 && chunks_pay(H * (P / kChunkCols), N, n_tokens, n_seqs, longest) && channels % 8 == 0 &&
-      !((uintptr_t)xbc & 15) && !((uintptr_t)state & 7) && !((uintptr_t)y & 7)) {
+  const bool fits = (N == 32 || N == 64 || N == 128) && P % kChunkCols == 0 && channels % 8 == 0 && !((uintptr_t)xbc & 15) &&
+                    !((uintptr_t)state & 7) && !((uintptr_t)y & 7);
+  int chunk = fits ? chunk_of(H * (P / kChunkCols), N, n_tokens, n_seqs, longest) : 0;
+  if (chunk == kChunk && ((uintptr_t)y & 15)) chunk = kShortChunk;      // (its stores are of 8 bytes; the other's of 16 cost it a twentieth in two forms)
+  if (chunk == kShortChunk) {
+    const size_t bytes = N == 32 ? sizeof(ShortSmem<32>) : N == 64 ? sizeof(ShortSmem<64>) : sizeof(ShortSmem<128>);
+    auto kern = N == 32 ? ssm_short_kernel<32> : N == 64 ? ssm_short_kernel<64> : ssm_short_kernel<128>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "ssm_scan: %s", cudaGetErrorString(e));
+    launch_chained(kern, dim3(H, portions, P / kChunkCols), dim3((kShortWarps + 1) * 32), bytes, (cudaStream_t)stream, (const elem_t*)xbc, channels,
+                   (const elem_t*)proj, ld, off_dt, dt_bias, a_log, d_skip, state, seq_starts, state_slots, y, H, P, G, n_seqs);
+    const int rc = check_launch("ssm_short");
+    if (rc || n_seqs == 1) return rc;
+    most_tokens = 1;
+    n_tokens = n_seqs;                  // (below: the shape for single tokens)
+  } else if (chunk == kChunk) {
     constexpr size_t bytes = sizeof(ChunkSmem) + 1024;
     auto kern = N == 32 ? ssm_chunk_kernel<32> : N == 64 ? ssm_chunk_kernel<64> : ssm_chunk_kernel<128>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -1086,9 +1375,9 @@ ERB_EXPORT int erb_ssm_scan(const void* xbc, int channels, const void* proj, int
     if ((rc = rows_map(&bc, xbc, n_tokens, channels, channels, kChunk, "ssm_scan")) ||
         (rc = rows_map(&x, xbc, n_tokens, channels, channels, kChunk, "ssm_scan", kChunkCols)))
       return rc;
-    launch_chained(kern, dim3(H, n_seqs, P / kChunkCols), dim3(kChunkThreads), bytes, (cudaStream_t)stream, bc, x,
+    launch_chained(kern, dim3(H, portions, P / kChunkCols), dim3(kChunkThreads), bytes, (cudaStream_t)stream, bc, x,
                    (const elem_t*)xbc, channels, (const elem_t*)proj, ld, off_dt, dt_bias, a_log, d_skip, state, seq_starts,
-                   state_slots, y, H, P, G, status);
+                   state_slots, y, H, P, G, n_seqs, status);
     rc = check_launch("ssm_chunk");
     if (rc || n_seqs == 1) return rc;
     most_tokens = 1;

@@ -113,7 +113,7 @@ _SIGNATURES = {
     "erb_attention_wide_diff": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                 c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_float, c_void_p, c_void_p],
     "erb_ssm_scan": [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "erb_gated_group_norm": [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                              c_float, c_void_p],
     "erb_rms_between": [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_float, c_void_p, c_float, c_void_p,
@@ -130,7 +130,7 @@ _SIGNATURES = {
                            c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                            c_void_p, c_void_p, c_int, c_int, c_void_p],
     "erb_delta_scan": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                       c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+                       c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "erb_head_norm_gate": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
     "erb_moe_route": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p],
@@ -1465,12 +1465,13 @@ def conv_state_update(proj: torch.Tensor, off: int, conv_state: torch.Tensor, n_
 
 def ssm_scan(xbc: torch.Tensor, proj: torch.Tensor, off_dt: int, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, n_seqs: int, seq_starts: torch.Tensor, state_slots: torch.Tensor, y: torch.Tensor,
-             n_groups: int, longest: int | None = None, status: torch.Tensor | None = None) -> None:
+             n_groups: int, longest: int | None = None, status: torch.Tensor | None = None, portions: int = 0) -> None:
     """The recurrence of the state-space mixer over every request's rows, from and to its record in ``state``
     (float ``[slots, heads, N, P]``): ``xbc`` rows ``[x (heads * P) | B (groups * N) | C (groups * N)]``, raw
     step sizes in columns ``off_dt .. off_dt + heads`` of ``proj``; ``y`` float ``[tokens, heads * P]``.  ``longest``: the
     largest number of tokens of a request, by which the kernel is chosen (None: what the totals allow); the results do not
-    depend on it beyond rounding.  ``status``: the word (int32) to which a block that waited for a product in vain reports (code
+    depend on it beyond rounding.  ``portions``: how many of the requests have more than one token (0: not known), so that only these get
+    blocks of the kernels for portions.  ``status``: the word (int32) to which a block that waited for a product in vain reports (code
     7000000, its results are not valid); without one such a block walks its portion token after token."""
     _need(xbc, "xbc"); _need(proj, "proj", xbc.dtype, contiguous=False); _need(state, "state", torch.float32)
     _need(y, "y", torch.float32)
@@ -1485,7 +1486,7 @@ def ssm_scan(xbc: torch.Tensor, proj: torch.Tensor, off_dt: int, dt_bias: torch.
     _call(_fn("ssm", _elem(xbc), "erb_ssm_scan"), xbc, xbc.shape[1], proj,
           proj.stride(0) if n > 1 else proj.shape[1], int(off_dt), dt_bias, a_log, d_skip,
           state, seq_starts, state_slots, y, int(n_seqs), n,
-          n - int(n_seqs) + 1 if longest is None else int(longest), heads, p, n_state,
+          n - int(n_seqs) + 1 if longest is None else int(longest), int(portions), heads, p, n_state,
           int(n_groups), status, _stream())
 
 
@@ -1528,7 +1529,7 @@ def delta_scratch_floats(n_tokens: int, n_heads: int, n_key_heads: int, key_dim:
 def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
                state: torch.Tensor, n_seqs: int, seq_starts: torch.Tensor, state_slots: torch.Tensor, out: torch.Tensor,
                n_key_heads: int, key_dim: int, scratch: torch.Tensor | None = None, longest: int | None = None,
-               status: torch.Tensor | None = None) -> None:
+               status: torch.Tensor | None = None, portions: int = 0) -> None:
     """The gated delta rule over every request's rows, from and to its record in ``state`` (float ``[slots, heads,
     vdim, key_dim]``, the matrix of a head stored with the value index first).  ``qkv``: convolved and activated rows
     ``[q (key heads * key_dim) | k (the same) | v (heads * vdim)]``; the raw write strengths and decay inputs are
@@ -1540,7 +1541,7 @@ def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt
     the sizes allow it, long portions are taken in chunks of 64 tokens; ``longest``: the largest number of tokens of a request,
     by which that is chosen (None: what the totals allow).  The results do not depend on it beyond rounding.  ``status``: the word
     (int32) to which a block that waited for a product in vain reports (code 8000000, its results are not valid); without one
-    such a block walks its portion token after token."""
+    such a block walks its portion token after token.  ``portions``: as in ``ssm_scan``."""
     _need(qkv, "qkv"); _need(proj, "proj", qkv.dtype, contiguous=False); _need(state, "state", torch.float32)
     _need(out, "out", torch.float32); _need(dt_bias, "dt_bias", torch.float32); _need(a_log, "a_log", torch.float32)
     _need(seq_starts, "seq_starts", torch.int32); _need(state_slots, "state_slots", torch.int32); _need(status, "status", torch.int32)
@@ -1560,7 +1561,7 @@ def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, off_b: int, off_a: int, dt
     _call(_fn("delta", _elem(qkv), "erb_delta_scan"), qkv, qkv.shape[1], proj,
           proj.stride(0) if n > 1 else proj.shape[1], int(off_b), int(off_a), dt_bias, a_log,
           state, seq_starts, state_slots, out, scratch, scratch.numel(), int(n_seqs), n,
-          n - int(n_seqs) + 1 if longest is None else int(longest), heads, int(n_key_heads), d, vdim,
+          n - int(n_seqs) + 1 if longest is None else int(longest), int(portions), heads, int(n_key_heads), d, vdim,
           status, _stream())
 
 

@@ -95,7 +95,7 @@ class GatedDeltaRule(Mixer):
         kernels.delta_scan(qkv, proj, self.off_b, self.off_a, self.dt_bias, self.a_log, ctx.state("delta", call.cache_layer),
                            ctx.n_seqs, ctx.seq_starts, ctx.state_slots, o, self.n_key_heads, self.key_dim,
                            ctx.buf("delta.scratch", (scratch,), torch.float32), longest=max(ctx.host_q_len) if chunks else 1,
-                           status=getattr(ctx, "status", None))
+                           status=getattr(ctx, "status", None), portions=sum(n > 1 for n in ctx.host_q_len))
         gated = ctx.buf("delta.gated", (n, self.inner), self.dtype)
         kernels.head_norm_gate(o, proj[:, self.off_gate: self.off_gate + self.inner], self.norm_w, gated, self.n_heads, self.eps)
         n_parts = kernels.linear_parts_count(gated, self.w_o)

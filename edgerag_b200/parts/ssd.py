@@ -78,7 +78,7 @@ class StateSpaceDuality(Mixer):
         kernels.ssm_scan(xbc, proj, inner + self.channels, self.dt_bias, self.a_log, self.d_skip,
                          ctx.state("ssm", call.cache_layer), ctx.n_seqs, ctx.seq_starts, ctx.state_slots, y, self.groups,
                          longest=1 if ctx.batch_invariant else max(ctx.host_q_len),      # (1: walked, whatever shares the step)
-                         status=getattr(ctx, "status", None))
+                         status=getattr(ctx, "status", None), portions=sum(n > 1 for n in ctx.host_q_len))
         normed = ctx.buf("ssd.normed", (n, inner), self.dtype)
         kernels.gated_group_norm(y, self.norm_w, normed, self.eps, self.norm_groups, gate=proj[:, :inner])
         out = ctx.buf("mixer.out", (n, self.hidden), self.dtype)

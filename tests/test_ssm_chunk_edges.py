@@ -40,7 +40,7 @@ def test_chunks_of_128_tokens(N, lens, bad):
 
 @pytest.mark.parametrize("offset", [2, 4])
 def test_outputs_on_8_bytes_come_from_the_chunks_too(offset):
-    """The outputs' alignment does not change who makes them: the bits of the chunks, which the walk's are not."""
+    """Outputs that chunks of 128 tokens cannot store come from chunks of 64, not from the walk, whose bits these have not."""
     H, P, N, G, n = 4, 64, 64, 2, 300
     inner = H * P
     g = torch.Generator().manual_seed(1)
@@ -55,5 +55,6 @@ def test_outputs_on_8_bytes_come_from_the_chunks_too(offset):
 
     y, state = scan(torch.empty(n, inner, device="cuda"), n)
     off_y, off_state = scan(torch.empty(n * inner + offset, device="cuda")[offset:].view(n, inner), n)
-    assert torch.equal(y, off_y) and torch.equal(state, off_state)
-    assert not torch.equal(y, scan(torch.empty_like(y), 1)[0])
+    short_y, short_state = scan(torch.empty_like(y), 64)
+    assert torch.equal(off_y, y if offset == 4 else short_y) and torch.equal(off_state, state if offset == 4 else short_state)
+    assert not torch.equal(off_y, scan(torch.empty_like(y), 1)[0]) and not torch.equal(y, short_y)
