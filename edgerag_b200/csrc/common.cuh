@@ -210,6 +210,17 @@ __device__ __forceinline__ Two silu_two(Two v) {
   return v * Two(0.25f) * fma2(y, r, y);
 }
 
+// The same of one value: the same operations, the same bits.
+__device__ __forceinline__ float silu_one(float v) {
+  const float z = -v, hi = __fmul_rn(z, 1.44269502f), low = __fmaf_rn(z, 1.92596299e-8f, __fmaf_rn(z, 1.44269502f, -hi));
+  float e, y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(hi));
+  const float l = fabsf(hi) < 128.f ? low : 0.f;
+  const float d = fminf(__fmaf_rn(__fmaf_rn(__fmul_rn(e, 0.693147181f), l, e), 0.25f, 0.25f), 3.402823466e38f);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return __fmul_rn(__fmul_rn(v, 0.25f), __fmaf_rn(y, __fmaf_rn(-d, y, 1.f), y));
+}
+
 // The nth request (from 0) with more than one token, or -1; the whole warp asks.
 __device__ __forceinline__ int nth_portion(const int* __restrict__ seq_starts, int n_seqs, int nth) {
   const int lane = threadIdx.x & 31;

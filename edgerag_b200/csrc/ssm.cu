@@ -53,9 +53,7 @@ conv_silu_kernel(const T* __restrict__ proj, int ld, int off, int channels, int 
       acc = fmaf(Elem<T>::load(weight + (size_t)ch * taps + j), v, acc);
     }
 #if ERB_ELEM == 1
-    float s0, s1;
-    silu_two(Two(acc)).get(s0, s1);                            // (as conv_silu_vec_kernel: the same bits)
-    Elem<T>::store(out + (size_t)t * channels + ch, s0);
+    Elem<T>::store(out + (size_t)t * channels + ch, silu_one(acc));      // (as conv_silu_vec_kernel: the same bits)
 #else
     Elem<T>::store(out + (size_t)t * channels + ch, silu_f(acc));
 #endif
@@ -70,7 +68,7 @@ conv_silu_kernel(const T* __restrict__ proj, int ld, int off, int channels, int 
 // instruction, tokens of one request without looking each one's request up, and this silu, four tokens a thread (two 21.8, eight 19.6 us);
 // 64 single tokens 16 us and 3.6 us.
 template <int TT>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, TT == 1 ? 7 : 5)         // (one token a thread: 72 registers, so that 1,000 blocks are one wave)
 conv_silu_vec_kernel(const __nv_bfloat16* __restrict__ proj, int ld, int off, int channels, const __nv_bfloat16* __restrict__ weight,
                      const __nv_bfloat16* __restrict__ bias, const float* __restrict__ conv_state, const int* __restrict__ seq_of_token,
                      const int* __restrict__ seq_starts, const int* __restrict__ state_slots, __nv_bfloat16* __restrict__ out, int n_tokens) {
@@ -78,6 +76,7 @@ conv_silu_vec_kernel(const __nv_bfloat16* __restrict__ proj, int ld, int off, in
   chain_wait();
   const int ch = 8 * (blockIdx.y * blockDim.x + threadIdx.x), t0 = blockIdx.x * TT;
   if (ch >= channels) return;
+  const int first = seq_of_token[t0], place = t0 - seq_starts[first];      // the first token's request, and its index there
   uint4 raw[TT + TAPS - 1];                                   // inputs t0 - (TAPS - 1) .. t0 + TT - 1
 #pragma unroll
   for (int k = 0; k < TT + TAPS - 1; ++k) {
@@ -99,8 +98,7 @@ conv_silu_vec_kernel(const __nv_bfloat16* __restrict__ proj, int ld, int off, in
     }
   }
   // tokens of one request that have their earlier inputs in this portion need no look at the request
-  const int first = seq_of_token[t0];
-  const bool plain = t0 - seq_starts[first] >= TAPS - 1 && seq_of_token[min(t0 + TT, n_tokens) - 1] == first;
+  const bool plain = TT > 1 && place >= TAPS - 1 && seq_of_token[min(t0 + TT, n_tokens) - 1] == first;
 #pragma unroll
   for (int k = 0; k < TT; ++k) {
     const int t = t0 + k;
@@ -108,8 +106,8 @@ conv_silu_vec_kernel(const __nv_bfloat16* __restrict__ proj, int ld, int off, in
     Two acc[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[e] = b[e];
-    int i = TAPS, seq = first;
-    if (!plain) {
+    int i = TT > 1 ? TAPS : place, seq = first;
+    if (TT > 1 && !plain) {
       seq = seq_of_token[t];
       i = t - seq_starts[seq];
     }
