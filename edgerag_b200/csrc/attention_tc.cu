@@ -783,12 +783,14 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
       const uint32_t k_st = sK + (uint32_t)s * kGqaStageBytes, v_st = sV + (uint32_t)s * kGqaStageBytes;
       // Rows past the last key may hold anything (unwritten slots, an earlier tile), rows before the window numbers that are not
       // finite: their scores are masked below, and their values are zeroed here, since 0 * NaN would spoil the product.
-      if (key0 + 16 > n_here || key_abs0 + key0 < k_lo) {
-        for (int k = key0 * 8 + lane; k < (key0 + 16) * 8; k += 32) {
-          const int key = k >> 3, chunk = k & 7;
-          if (key >= n_here || (key_abs0 + key < k_lo && key_abs0 + key >= keep_first))
-            *reinterpret_cast<uint4*>(smem + (v_st - base) + row_of(key) * 128 + chunk * 16) = make_uint4(0, 0, 0, 0);
-        }
+      const int first_seen = tile < kept_tiles ? 0 : k_lo - key_abs0;       // (of a tile that is not of the kept keys; those lie before the window)
+      if (key0 + 16 > n_here || key0 < first_seen) {
+        auto zero = [&](int from, int to) {                 // values of keys of this warp's sixteen
+          for (int k = from * 8 + lane; k < to * 8; k += 32)
+            *reinterpret_cast<uint4*>(smem + (v_st - base) + row_of(k >> 3) * 128 + (k & 7) * 16) = make_uint4(0, 0, 0, 0);
+        };
+        zero(max(n_here, key0), key0 + 16);
+        zero(max(keep_first - key_abs0, key0), min(first_seen, key0 + 16));
         __syncwarp();
       }
       // S for the two blocks of 8 keys
@@ -908,8 +910,7 @@ attention_decode_gqa_kernel(const __grid_constant__ CUtensorMap map_k, const __g
       continue;
     }
     const size_t slot = ((size_t)seq * nq + kvh0 * R + row) * max_splits + split;
-    part_acc[slot * D + 2 * lane] = sum.x;
-    part_acc[slot * D + 2 * lane + 1] = sum.y;
+    *reinterpret_cast<float2*>(part_acc + slot * D + 2 * lane) = sum;
     if (lane == 0) { part_ml[slot * 2] = m; part_ml[slot * 2 + 1] = l; }      // (part_ml may start at any float)
   }
   if (max_splits > 1 && counters)
@@ -990,7 +991,7 @@ ERB_EXPORT int erb_attention_decode_gqa(const void* q, int q_row_stride, const v
   if (q_row_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)k_pages & 127) || ((uintptr_t)v_pages & 127))
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: q rows must be 16-byte aligned, pools 128-byte aligned");
   if (n_seqs > 65535 || nkv > 65535) return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: grid too large");
-  if (counters && max_splits > 1 && !merge_reads(part_acc, head_dim))
+  if (max_splits > 1 && !merge_reads(part_acc, head_dim))
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: part_acc must be aligned to %d bytes", head_dim / 8);
   if (max_splits > kCombineMaxSplits)
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_gqa: %d splits (at most %d)", max_splits, kCombineMaxSplits);
@@ -1051,7 +1052,7 @@ ERB_EXPORT int erb_attention_decode_bulk(const void* q, int q_row_stride, const 
   if (q_row_stride % 8 || ((uintptr_t)q & 15) || ((uintptr_t)k_pages & 15) || ((uintptr_t)v_pages & 15))
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_bulk: rows must be 16-byte aligned");
   if (n_seqs > 65535 || nkv > 65535) return fail(ERB_ERR_UNSUPPORTED, "attention_decode_bulk: grid too large");
-  if (counters && max_splits > 1 && !merge_reads(part_acc, head_dim))
+  if (max_splits > 1 && !merge_reads(part_acc, head_dim))
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_bulk: part_acc must be aligned to %d bytes", head_dim / 8);
   if (max_splits > kCombineMaxSplits)
     return fail(ERB_ERR_UNSUPPORTED, "attention_decode_bulk: %d splits (at most %d)", max_splits, kCombineMaxSplits);
