@@ -1968,6 +1968,8 @@ def _choose_decode_plan(device: int, n_seqs: int, n_kv_heads: int, max_keys: int
 
 
 EVEN_SPLIT_PAGES = 1024      # pages of an equal split at most
+#: several query heads per kv head: (bound on the keys, keys of an equal split at least); beyond, and with one query head per kv head, 128
+EVEN_FEWEST_KEYS = ((256, 48), (512, 64), (768, 96), (2048, 64), (3072, 96))
 
 
 def choose_even_plan(n_seqs: int, n_q_heads: int, n_kv_heads: int, max_keys: int, page_size: int, head_dim: int) -> tuple[int, int, int] | None:
@@ -2001,9 +2003,12 @@ def _choose_even_plan(device: int, n_seqs: int, n_q_heads: int, n_kv_heads: int,
 
     Several query heads per kv head: up to 128 keys one split (9 over 3, 90 keys: a step of 452 us in one split, 519 in two), so the
     other plan; then splits of 48 to 96 keys as far as a wave reaches (15 over 5, steps with splits of 128 | these: 200 keys 8 sequences
-    829 | 720 us, 400 keys 847 | 785; attention of 64 x 7,531 116 | 109, of 8 x 7,531 26.1 | 22.7).  The merge takes eight splits at a time,
-    so the bounds up to 1,024 get 8 or 16 of them: 64 keys for 512 and 1,024, 96 for the one between (attention of 8 x 640 in splits of 48 |
-    64 | 96 | 128: 15 over 5 12.4 | 10.4 | 9.1 | 10.4 us, 9 over 3 8.6 | 7.3 | 6.7 | 7.3; of 8 x 1,000 12.8 | 10.1 | 12.2 | 11.3).
+    829 | 720 us, 400 keys 847 | 785; attention of 64 x 7,531 116 | 109, of 8 x 7,531 26.1 | 22.7).  The merge asks for eight
+    splits at a time, so the bounds up to 1,024 get 8 or 16 of them: 64 keys for 512 and 1,024, 96 for the one between (attention alone in splits of
+    48 | 64 | 96 | 128, 9 over 3: 8 x 500 7.0 | 6.3 | 6.4 | 7.4 us, 8 x 600 7.2 | 6.8 | 6.5 | 7.2, 8 x 1,000 7.8 | 7.3 | 7.8 | 7.4; 15 over 5: 8 x 600 9.4 |
+    9.8 | 9.1 | 10.4).  Behind that: 15 over 5, 4 x 1,400 10.8 | 10.6 | 10.6 | 11.9, 8 x 1,900 11.6 | 11.6 | 12.4 | 13.0, 4 x 2,800 12.7 | 12.4 | 12.0 |
+    12.9; 32 over 8, 1 x 2,800 12.3 | 11.1 | 10.0 | 10.1, and 1 x 3,800 in 64 | 96 | 128 12.0 | 12.0 | 10.5.  Beyond 4,096 keys a batch that these leave
+    half empty keeps the other plan.
 
     One query head per kv head (``single_heads_on_tensor_cores`` says by which kernel): the fewest kv heads per block whose blocks fit into
     one wave, and where they fill a third of it up to 768 keys in one split, which nobody has to merge (32 heads, the other plan | this one, on
@@ -2029,10 +2034,10 @@ def _choose_even_plan(device: int, n_seqs: int, n_q_heads: int, n_kv_heads: int,
             return None
         if not grouped and max_keys <= 768:
             return (-(-max_keys // page_size) * page_size, heads, 1) if blocks >= 0.3 * slots else None
-        fewest_keys = 128 if not grouped else 48 if max_keys <= 256 else 96 if 512 < max_keys <= 768 else 64
+        fewest_keys = next((keys for bound, keys in EVEN_FEWEST_KEYS if max_keys <= bound), 128) if grouped else 128
         by_keys = -(-max_keys // fewest_keys)
         splits = max(1, min(int(0.9 * slots / blocks), by_keys, 64))
-        if splits < by_keys and blocks * splits < 0.6 * slots:
+        if (splits < by_keys or (grouped and max_keys > 4096)) and blocks * splits < 0.6 * slots:
             continue
         split = -(-max_keys // (splits * page_size)) * page_size
         if split > EVEN_SPLIT_PAGES * page_size:
