@@ -192,8 +192,10 @@ def _fn(library: str, elem: str | None, name: str):
 
 
 def _call(fn, *args) -> None:
-    if _host:               # (the call for which the module was loaded)
-        return _host.call(fn, *args)
+    return (_host.call if _host else _call_in_python)(fn, *args)       # (the module's: the call for which it was loaded)
+
+
+def _call_in_python(fn, *args) -> None:
     rc = fn(*(a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args))
     if fn._erb_own:
         launch_counts["own"] += fn._erb_own

@@ -12,7 +12,7 @@ from test_kernels import attention_reference, paged_case, tol
 pytestmark = pytest.mark.gpu
 
 
-def _run(case, nq, nkv, d, splits, split, heads, even=True):
+def _run(case, nq, nkv, d, splits, split, heads, even=True, parts=False):
     dev = {n: case[n].cuda() for n in ("q", "kp", "vp", "tables", "pos")}
     n = case["pos"].numel()
     acc, ml = K.decode_scratch_floats(n, nq, d, splits)
@@ -27,7 +27,36 @@ def _run(case, nq, nkv, d, splits, split, heads, even=True):
         K.attention_decode_gqa(*args, split_keys=split, even=even)
     torch.cuda.synchronize()
     assert int(status) == 0 and int(K.split_counters(out.device, 1).abs().sum()) == 0
-    return out
+    return (part_acc.view(n, nq, splits, d).cpu(), part_ml.view(n, nq, splits, 2).cpu()) if parts else out
+
+
+def _of_the_parts(case, nq, nkv, parts):
+    """The splits' partial results put together in 64 bits, and the same attention in 64 bits."""
+    acc, ml = (p.double() for p in parts)
+    there = ~ml[..., 0].isnan()
+    top = torch.where(there, ml[..., 0], -torch.inf)
+    w = torch.exp2(top - top.amax(-1, keepdim=True))
+    got = (torch.where(there[..., None], acc, 0.0) * w[..., None]).sum(2) / (torch.where(there, ml[..., 1], 0.0) * w).sum(-1, keepdim=True)
+    want = []
+    for t in range(acc.shape[0]):
+        k, v = (x[t].double().repeat_interleave(nq // nkv, 1) for x in (case["ks"], case["vs"]))
+        score = torch.einsum("hd,khd->hk", case["q"][t].double().view(nq, -1), k) * 0.125
+        want.append(torch.einsum("hk,khd->hd", torch.softmax(score, -1), v))
+    return got, torch.stack(want)
+
+
+@pytest.mark.parametrize("nq,nkv,heads", [(8, 8, 2), (5, 5, 4), (9, 9, 8), (4, 4, 1), (15, 5, 0), (6, 3, 0)])
+@pytest.mark.parametrize("splits", [2, 7])
+def test_the_parts_of_equal_splits(nq, nkv, heads, splits):
+    """Every sequence is cut into as many whole pages as its own length gives, not at multiples of the longest's.  One query head per kv head: a
+    weight goes in whole, as three pieces; rounded to 16 bits, weights of several query heads among them, it is off by 2^-9, in two by 2^-18."""
+    ctx_lens = [17, 129, 500, 1300]
+    case = paged_case(torch.bfloat16, 11 + splits, nq, nkv, 64, 16, ctx_lens, [1] * len(ctx_lens))
+    parts = _run(case, nq, nkv, 64, splits, -(-max(ctx_lens) // (splits * 16)) * 16, heads, parts=True)
+    written = [-(-n // (-(-n // (splits * 16)) * 16)) for n in ctx_lens]
+    assert (~parts[1][..., 0].isnan()).sum(-1).tolist() == [[w] * nq for w in written]
+    got, want = _of_the_parts(case, nq, nkv, parts)
+    assert (got - want).norm() < (6e-7 if nq == nkv else 4e-3) * want.norm()
 
 
 @pytest.mark.parametrize("nq,nkv,ps,heads", [(8, 8, 16, 2), (5, 5, 16, 4), (9, 9, 8, 8), (3, 3, 128, 1), (15, 5, 16, 0), (6, 3, 64, 0)])
@@ -67,6 +96,7 @@ def test_the_plan_of_equal_splits(nq, nkv):
                 groups = -(-nkv // (heads or 8))
                 assert split % 16 == 0 and split * splits >= bound and splits <= 64 and n * groups * splits <= slots
     assert K.choose_even_plan(8, nq, nkv, 1024, 16, 128) is None and K.choose_even_plan(8, nq, nkv, 1024, 12, 64) is None
+    assert K.choose_even_plan(8, nq, nkv, 8192, 16, 64) is not None and K.choose_even_plan(64, nq, nkv, 8192, 16, 64) is not None
 
 
 @pytest.mark.parametrize("batch,nq,nkv,context,kernel,equal", [(64, 15, 5, 700, "gqa", True), (8, 32, 32, 1000, "bulk", False), (8, 32, 32, 2500, "bulk", True)])

@@ -47,6 +47,59 @@ def test_every_signature_arrives_in_order(host, name):
     assert host[1] == {"own": 1, "library": 0}
 
 
+@pytest.mark.parametrize("name", sorted(kernels._SIGNATURES))
+def test_every_signature_arrives_without_the_module(monkeypatch, name):
+    """The way through ctypes, where the module cannot be built: tensors become pointers, launches are counted, refusals raised."""
+    types, got, result = kernels._SIGNATURES[name], [], [0]
+    callback = ctypes.CFUNCTYPE(ctypes.c_int, *types)(lambda *a: got.append(a) or result[0])
+    entry = ctypes.CFUNCTYPE(ctypes.c_int)(ctypes.cast(callback, ctypes.c_void_p).value)       # (as a library gives it: no types yet)
+    library = type("Library", (), {name: entry, "erb_last_error": staticmethod(lambda: b"what went wrong")})
+    counts = {"own": 0, "library": 0}
+    for attribute, value in (("_host", False), ("_functions", {}), ("launch_counts", counts), ("_need", kernels._need_in_python)):
+        monkeypatch.setattr(kernels, attribute, value)
+    monkeypatch.setattr(kernels.native, "load", lambda *a: library)
+    fn = kernels._fn("any", None, name)
+    t, numbers = torch.arange(7.0)[3:], itertools.count(3)
+    args = [t if k is ctypes.c_void_p and i % 3 == 0 else None if k is ctypes.c_void_p and i % 3 == 1 else
+            next(numbers) / 4 if k is ctypes.c_float else -next(numbers) if k is ctypes.c_int else (1 << 40) + next(numbers)
+            for i, k in enumerate(types)]
+    call = kernels._call_in_python
+    call(fn, *args)
+    assert got == [tuple(t.data_ptr() if a is t else a for a in args)]
+    own = kernels._LAUNCHES.get(name, 1)
+    assert counts == ({"own": own, "library": 0} if own else {"own": 0, "library": 1})
+    result[0] = 3
+    with pytest.raises(kernels.KernelError, match="what went wrong"):
+        call(fn, *args)
+
+
+@pytest.mark.gpu
+def test_kernels_run_without_the_module():
+    """A norm, a product and decode attention in a program that has no host module: the results of one that has."""
+    import multiprocessing
+
+    context = multiprocessing.get_context("spawn")
+    with context.Pool(1) as pool:
+        alone = pool.apply(_run_a_few, (False,))
+    assert all(a == b for a, b in zip(alone, _run_a_few(True)))
+
+
+def _run_a_few(module):
+    if not module:
+        native.load_host = lambda: None
+    g = torch.Generator().manual_seed(0)
+    rand = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).cuda()       # noqa: E731
+    hidden, normed = torch.randn(4, 512, generator=g).cuda(), torch.empty(4, 512, dtype=torch.bfloat16, device="cuda")
+    kernels.add_rmsnorm(hidden, torch.ones(512, device="cuda"), normed, 1e-5, delta=rand(4, 512))
+    q = torch.empty(4, 512, dtype=torch.bfloat16, device="cuda")
+    kernels.linear(normed, rand(512, 512), q)
+    pages, i32, out = rand(8, 8, 16, 64), lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda"), torch.empty_like(q)      # noqa: E731
+    kernels.attention_decode_bulk(q, pages, pages, i32(0, 1, 2, 3, 4, 5, 6, 7).view(4, 2), i32(0, 1, 2, 3), i32(3, 20, 31, 8), out, 8, 0.125,
+                                  torch.empty(4096, device="cuda"), torch.empty(4096, device="cuda"), 1, i32(0))
+    assert (kernels._host is not False) == module
+    return [t.float().cpu().tolist() for t in (hidden, normed, q, out)]
+
+
 def test_results_counts_and_refusals(host):
     module, counts = host
     fn, got, _a = _entry(module, [ctypes.c_int], result=5, own=0)

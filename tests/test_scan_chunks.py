@@ -48,6 +48,10 @@ def test_state_space_chunks(H, P, N, G, lens, pace):
             want_y, want_s = _ssm_reference(xbc[rows], proj[rows, 1: 1 + H], dt_bias, a_log, skip, before[slots[s]], H, P, N, G)
             assert (y[rows].double() - want_y).abs().max() < 3e-5 * max(1.0, want_y.abs().max()), (s, longest)
             assert (state[slots[s]].double() - want_s).abs().max() < 3e-5 * max(1.0, want_s.abs().max()), (s, longest)
+            # in chunks a few roundings in the mean: operands in two pieces instead of three would be off by some 2^-18 each, 2e-6 in the mean.
+            # (The walk rounds its state once a token, n 2^-25 at worst where nothing decays, which says nothing about pieces.)
+            if longest > 1 and length > 1:
+                assert (y[rows].double() - want_y).norm() < 6e-7 * want_y.norm() and (state[slots[s]].double() - want_s).norm() < 6e-7 * want_s.norm(), s
             at += length
         assert torch.equal(state[0], before[0])     # the slot nobody holds
 
@@ -142,6 +146,8 @@ def test_delta_chunks(H, G, d, dv, lens, pace, alike):
             want, want_s = _delta_reference(qkv[rows], proj[rows, 1: 1 + H], proj[rows, 2 + H: 2 + 2 * H], dt_bias, a_log, before[slots[s]], H, G, d, dv)
             assert (out[rows].double() - want).abs().max() < 3e-5 * max(1.0, want.abs().max()), (s, longest)
             assert (state[slots[s]].double() - want_s).abs().max() < 3e-5 * max(1.0, want_s.abs().max()), (s, longest)
+            if longest > 1 and room and length > 1:      # (as for the state-space chunks; the walk's errors grow along an ill-conditioned portion)
+                assert (out[rows].double() - want).norm() < 8e-7 * want.norm() and (state[slots[s]].double() - want_s).norm() < 8e-7 * want_s.norm(), s
             at += length
         assert torch.equal(state[0], before[0])
 
