@@ -25,7 +25,7 @@
 // the largest weight of a row is no longer exactly 1, and rounding it once would lose 4 % of accuracy against a kernel that
 // moves it with every tile.  The tensor cores have the room for the second piece.
 //
-// What bounds it: the exponentials and what is done to a score besides (about 12 instructions with a cap of the scores); the tensor
+// What bounds it: the exponentials and what is done to a score besides (17 instructions of all warps a score with a cap, 11.5 without); the tensor
 // cores wait for them.  Tiles of 64 keys leave room in TMEM for two accumulators of 128 columns beside the scores, and in shared
 // memory for three to four tiles beside the queries; that, and boxes of 64 columns, is why heads and values are of 64 or 128 (the
 // differential form of 64 and 128: other sizes are diff_attention.cu's).  Differential, 2,048 tokens of 16 heads, capped: 240 us by the mma.sync

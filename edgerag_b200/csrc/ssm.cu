@@ -447,8 +447,8 @@ ssm_scan16_kernel(const T* __restrict__ xbc, int channels, const T* __restrict__
 // exponential where t and s lie in the same 32 tokens; elsewhere it is the product of two factors, from s to the end of its 32 and on to the
 // last token before t's 32, and from there to t, which are made once a token, in double, and rounded once.
 //
-// What bounds it: a chunk's line, about 5,200 clocks: G read 700, the weights 2,500 (shared memory serves the products' operands meanwhile),
-// dS awaited and the state published 1,000, weighted x 700, outputs 400.  2,048 tokens of 64 heads of 64 x 128: 52.3 us; 64.5 us with an
+// What bounds it: a chunk's line, about 5,300 clocks: G read 700, the weights 2,500 (shared memory serves the products' operands meanwhile),
+// dS awaited and the state published 1,000, weighted x 700, outputs 400.  2,048 tokens of 64 heads of 64 x 128: 53.3 us; 64.5 us with an
 // exponential a weight, a lone lane issuing (110 clocks a product; an elected lane of a whole warp has what they take in uniform
 // registers) and steps, stores and weighted x in the line; 132 us in chunks of 64 by mma.sync, 566 us walked.  (The weighted x made by the step warps:
 // 55 us; there they are the longer line.)  Error against float64 1.2e-7 for y, 7.4e-8 for the state, as those.
