@@ -951,7 +951,7 @@ ERB_EXPORT int erb_delta_scan(const void* qkv, int channels, const void* proj, i
     const size_t prep_bytes = d == 64 ? sizeof(DeltaPrepSmem<64>) : sizeof(DeltaPrepSmem<128>);
     cudaError_t e = cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_bytes);
     if (e != cudaSuccess) return fail(ERB_ERR_CUDA, "delta_scan: %s", cudaGetErrorString(e));
-    launch_chained(prep, dim3(H, (n_tokens - (n_seqs - portions)) / kChunk + portions), dim3(kChunkPrepWarps * 32), prep_bytes, (cudaStream_t)stream, (const elem_t*)qkv,
+    launch_chained(prep, dim3(H, n_tokens / kChunk + portions), dim3(kChunkPrepWarps * 32), prep_bytes, (cudaStream_t)stream, (const elem_t*)qkv,
                    channels, (const elem_t*)proj, ld, off_b, off_a, dt_bias, a_log, seq_starts, n_seqs, records, H, G, 1.f / sqrtf((float)d));
     int rc = check_launch("delta_chunk_prepare");
     if (rc) return rc;

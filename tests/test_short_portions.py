@@ -42,7 +42,7 @@ def test_state_space_portions_of_up_to_64_tokens(N, lens, longest):
             assert _error(y[rows], want_y) < 6e-7 and _error(state[s], want_s) < 6e-7, (s, length)
 
 
-@pytest.mark.parametrize("lens", [[1] * 40 + [70], [130, 1, 1, 64, 1], [100] * 3])
+@pytest.mark.parametrize("lens", [[1] * 40 + [70], [130, 1, 1, 64, 1], [100] * 3, [0] * 20 + [63, 65, 0, 65, 0]])
 @pytest.mark.parametrize("scan", ["ssm", "delta"])
 def test_blocks_for_portions_alone(scan, lens):
     """Single tokens get no block of the kernels for portions where the caller counts the portions: the same bits."""
@@ -52,7 +52,7 @@ def test_blocks_for_portions_alone(scan, lens):
     proj = torch.randn(n, 8, generator=g).to(torch.bfloat16).cuda()
     rows = (torch.randn(n, 4 * 64 + 2 * 2 * 64, generator=g) * 0.5).to(torch.bfloat16).cuda()
     before, outs = 0.3 * torch.randn(m, 4, 64, 64, generator=g).cuda(), []
-    for portions in (0, sum(x > 1 for x in lens)):
+    for portions in (0, sum(x > 1 for x in lens)):            # (a request may bring no token at all)
         state, out = before.clone(), torch.full((n, 256), float("nan"), device="cuda")
         if scan == "ssm":
             kernels.ssm_scan(rows, proj[:, :4], 0, *v, state, m, starts, slots, out, 2, longest=1 << 20, portions=portions)
